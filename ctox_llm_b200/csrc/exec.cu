@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "exec.cuh"
+#include "hybrid_prefill.cuh"
 #include "stack.cuh"
 
 using namespace ctox;
@@ -139,6 +140,7 @@ ctox_status ctox_exec_destroy(ctox_exec *e) {
     for (auto &ev : e->phase_ev)
         if (ev) cudaEventDestroy(ev);
     stack_destroy(e);
+    delete e->long_pass;
     delete e;
     return CTOX_OK;
 }
@@ -755,6 +757,7 @@ ctox_status ctox_exec_warmup(ctox_exec *e) {
         }
     }
 #undef WALLOC
+    EX(long_warmup(e));
     CTOX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     e->warmed = true;
     e->position = 0;
@@ -1111,6 +1114,24 @@ ctox_status pass_logits(ctox_exec *e, uint32_t m, const uint32_t *places, uint32
     return CTOX_OK;
 }
 
+// The same for the last long pass (its rows are committed already).
+ctox_status long_pass_logits(ctox_exec *e, const uint32_t *places, uint32_t n, float *out) {
+    ctox_ctx *ctx = e->ctx;
+    const size_t V = e->vocab_l, H = e->cfg.hidden_size;
+    if (n && !e->logits) EX(xalloc(e, (void **)&e->logits, (size_t)kMaxPass * V * 4, true));
+    for (uint32_t i = 0; i < n; i += kMaxPass) {
+        const uint32_t k = n - i < kMaxPass ? n - i : kMaxPass;
+        for (uint32_t j = 0; j < k; ++j)
+            CTOX_CUDA(ctx, cudaMemcpyAsync(e->final_hidden + j * H, e->long_pass->final_hidden + places[i + j] * H, H * 4,
+                                           cudaMemcpyDeviceToDevice, ctx->stream));
+        EX(matvec_stream_pass(e->lm_head, 0, e->final_hidden, CTOX_F32, k, H));
+        matvec_finish_enqueue(e->lm_head, k, e->logits, V);
+        CTOX_CUDA(ctx, cudaMemcpyAsync(out + i * V, e->logits, k * V * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        CTOX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the rows are used again
+    }
+    return CTOX_OK;
+}
+
 ctox_status extend_impl(ctox_exec *e, const uint32_t *tokens, uint64_t n, const uint32_t *want, uint64_t n_want,
                         float *logits_out, const volatile int32_t *cancel, bool *began) {
     ctox_ctx *ctx = e->ctx;
@@ -1118,7 +1139,8 @@ ctox_status extend_impl(ctox_exec *e, const uint32_t *tokens, uint64_t n, const 
     uint64_t w = 0;
     for (uint64_t a = 0; a < n;) {
         if (cancelled(cancel)) return fail(ctx, CTOX_CANCELLED, "prefill cancelled at token %llu", (unsigned long long)a);
-        const uint32_t m = pass_positions(e, n - a);
+        const bool is_long = e->long_pass && n - a >= kLongMin;
+        const uint32_t m = is_long ? (uint32_t)(n - a < e->long_pass->cap ? n - a : e->long_pass->cap) : pass_positions(e, n - a);
         *began = true;
         if (e->cfg.mtp_num_hidden_layers && e->have_hidden && e->position > 0) {
             // keep the MTP cache exact: pairs (token p+1, final hidden p) of the block before
@@ -1128,15 +1150,23 @@ ctox_status extend_impl(ctox_exec *e, const uint32_t *tokens, uint64_t n, const 
             EX(upload_u32(e, e->mtp_tokens_dev, mt, e->hist_n));
             EX(mtp_pass(e, e->hist_n, e->position - e->hist_n + 1, e->mtp_tokens_dev, e->hist_hidden, -1));
         }
-        EX(upload_u32(e, e->tokens_dev, tokens + a, m));
-        EX(target_pass(e, m, e->position));
+        if (is_long) {
+            EX(long_target_pass(e, tokens + a, m));
+        } else {
+            EX(upload_u32(e, e->tokens_dev, tokens + a, m));
+            EX(target_pass(e, m, e->position));
+        }
         places.clear();
         for (; w < n_want && want[w] < a + m; ++w) places.push_back((uint32_t)(want[w] - a));
-        if (!places.empty())
-            EX(pass_logits(e, m, places.data(), (uint32_t)places.size(), logits_out + (w - places.size()) * e->vocab_l));
-        EX(commit_positions(e, m, m));
-        if (e->cfg.mtp_num_hidden_layers)
-            for (uint32_t j = 0; j + 1 < m; ++j) e->hist_tokens[j] = tokens[a + 1 + j];
+        float *to = logits_out + (w - places.size()) * e->vocab_l;
+        if (is_long) {
+            EX(long_pass_logits(e, places.data(), (uint32_t)places.size(), to));
+        } else {
+            if (!places.empty()) EX(pass_logits(e, m, places.data(), (uint32_t)places.size(), to));
+            EX(commit_positions(e, m, m));
+            if (e->cfg.mtp_num_hidden_layers)
+                for (uint32_t j = 0; j + 1 < m; ++j) e->hist_tokens[j] = tokens[a + 1 + j];
+        }
         a += m;
         // `tokens` may be pageable host memory: finish the chunk, and read the device error word
         int32_t dev_err = 0;

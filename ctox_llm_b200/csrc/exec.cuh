@@ -28,6 +28,7 @@ struct LayerS {
 };
 
 struct StackModel;  // a layer stack described layer by layer (stack.cuh)
+struct LongPass;    // buffers of long passes of the hybrid model (hybrid_prefill.cuh)
 }  // namespace ctox
 
 using ctox::kMaxPass;
@@ -90,6 +91,7 @@ struct ctox_exec {
     uint32_t *page_table = nullptr, *mtp_page_table = nullptr;
     uint32_t attn_splits_max = kAttnMaxSplits;
     uint64_t model_bytes = 0, session_bytes = 0;
+    ctox::LongPass *long_pass = nullptr;  // null: passes of up to kMaxPass positions only
     ctox::StackModel *stack = nullptr;  // set: a layer-stack model; the fields of the hybrid model above stay empty
     std::vector<std::pair<void *, size_t>> owned;  // tracked raw allocations (vectors, buffers, states)
 };

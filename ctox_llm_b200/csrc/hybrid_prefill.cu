@@ -1,0 +1,644 @@
+// Long passes of the hybrid model. A prompt portion of up to LongPass::cap positions goes through a layer at once:
+// the packed products on tcgen05 (packed_gemm.cu), between them the kernels below, one CTA per position for what
+// works on rows, a token scan for the recurrence. Arithmetic and order of operations are those of the short passes
+// (decoder.rs:636-938, 1009-1046); sums of many terms are taken in another order.
+//
+// Short passes read every weight once per eight positions and are bound by unpacking it; measured on 8 layers of the
+// flagship's width, 999 tokens: 163 ms in 125 short passes.
+#include "hybrid_prefill.cuh"
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "prep.cuh"
+
+namespace ctox {
+
+__device__ __forceinline__ float lp_out(const LongOut &o, uint32_t row, uint32_t pos) {
+    const float *p = o.y + (size_t)pos * o.rows + row;
+    float v = p[0];
+    for (uint32_t s = 1; s < o.splits; ++s) v += p[s * o.split_stride];  // index order
+    return v;
+}
+template <int OP>  // 0 sum, 1 maximum
+__device__ __forceinline__ float lp_block(float v, float *red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float t = __shfl_xor_sync(0xffffffffu, v, o);
+        v = OP ? fmaxf(v, t) : v + t;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[0];
+    for (uint32_t w = 1; w < blockDim.x / 32; ++w) v = OP ? fmaxf(v, red[w]) : v + red[w];
+    return v;
+}
+
+// ------------------------------------------------------------------ rows: one CTA per position
+// Forms the next product's input row in shared memory and writes it as hi and lo parts. Bound by memory: a
+// projection's fp32 outputs are read once, four bytes per input column are written.
+enum : int { ROWS_NORM, ROWS_SWIGLU, ROWS_ATTENTION, ROWS_DELTA, ROWS_MTP };
+constexpr int kRowsThreads = 512;
+
+struct RowsArgs {
+    LongOut o;              // NORM: addend (o.y null: none); SWIGLU: [gate | up]; ATTENTION, DELTA: where the gates are
+    const float *a, *b;     // NORM: a = input row when `h` starts there (else h); MTP: embedding and hidden rows
+    const float *w, *w2;    // norm weights
+    float *h, *xn_out;      // NORM: residual row (written), normalised row (optional)
+    float eps;
+    uint32_t width;         // columns of h / inter / query width / value width / hidden
+    uint32_t off;           // DELTA: first gate row of o
+    uint32_t q_heads, kv_heads, head_dim, per_group, m;  // ATTENTION
+    LongIn in;
+    const float *s_in;      // of the next product (null: 1)
+    uint32_t blocks_padded;
+    int dt, has_next;
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
+    pdl_launch();
+    pdl_wait();
+    extern __shared__ __align__(16) float vals[];  // [blocks_padded * 64]
+    __shared__ float red[kRowsThreads / 32];
+    const uint32_t pos = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t columns = MODE == ROWS_MTP ? 2 * p.width : p.width;
+    float amax = 0.f;
+    auto put = [&](uint32_t c, float x) {
+        const float v = p.s_in ? x * p.s_in[c] : x;
+        vals[c] = v;
+        amax = fmaxf(amax, fabsf(v));
+    };
+    if constexpr (MODE == ROWS_NORM) {
+        float *h = p.h + (size_t)pos * p.width;
+        float sq = 0.f;
+        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
+            float v = p.a ? p.a[(size_t)pos * p.width + c] : 0.f;
+            if (p.o.y) v += lp_out(p.o, c, pos);
+            h[c] = v;
+            vals[c] = v;
+            sq += v * v;
+        }
+        const float inv = 1.0f / sqrtf(lp_block<0>(sq, red) / (float)p.width + p.eps);
+        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {  // each thread its own columns again
+            const float xn = vals[c] * inv * (1.0f + p.w[c]);
+            if (p.xn_out) p.xn_out[(size_t)pos * p.width + c] = xn;
+            if (p.has_next) put(c, xn);
+        }
+        if (!p.has_next) return;
+    } else if constexpr (MODE == ROWS_MTP) {
+        const float *e = p.a + (size_t)pos * p.width, *h = p.b + (size_t)pos * p.width;
+        float se = 0.f, sh = 0.f;
+        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
+            se += e[c] * e[c];
+            sh += h[c] * h[c];
+        }
+        const float ie = 1.0f / sqrtf(lp_block<0>(se, red) / (float)p.width + p.eps);
+        const float ih = 1.0f / sqrtf(lp_block<0>(sh, red) / (float)p.width + p.eps);
+        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
+            put(c, e[c] * ie * (1.0f + p.w[c]));
+            put(p.width + c, h[c] * ih * (1.0f + p.w2[c]));
+        }
+    } else if constexpr (MODE == ROWS_SWIGLU) {
+        for (uint32_t c = tid; c < p.width; c += kRowsThreads)
+            put(c, silu_f(lp_out(p.o, c, pos)) * lp_out(p.o, p.width + c, pos));
+    } else if constexpr (MODE == ROWS_ATTENTION) {
+        // attention left (unnormalised output, maximum, sum) per group of positions: [kv head][query][head_dim + 2]
+        const uint32_t G = p.q_heads / p.kv_heads, hd = p.head_dim, group = pos / p.per_group, mi = pos % p.per_group;
+        const uint32_t n = min(p.per_group, p.m - group * p.per_group);
+        const float *base = p.a + (size_t)group * p.per_group * p.q_heads * (hd + 2);
+        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
+            const uint32_t hq = c / hd, d = c % hd;
+            const float *r = base + ((size_t)(hq / G) * G * n + mi * G + hq % G) * (hd + 2);
+            const float gate = lp_out(p.o, hq * 2 * hd + hd + d, pos);
+            put(c, r[d] * (1.0f / r[hd + 1]) * (1.0f / (1.0f + expf(-gate))));
+        }
+    } else {
+        // rms_norm_gated per value head (reference.rs:66-93): a warp per head, four columns per lane
+        for (uint32_t head = warp; head < p.width / 128; head += kRowsThreads / 32) {
+            const uint32_t c0 = head * 128 + lane * 4;
+            const float4 v = *reinterpret_cast<const float4 *>(p.a + (size_t)pos * p.width + c0);
+            float sq = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            const float inv = 1.0f / sqrtf(sq / 128.0f + p.eps);
+            const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                put(c0 + j, x[j] * inv * p.w[lane * 4 + j] * silu_f(lp_out(p.o, p.off + c0 + j, pos)));
+        }
+    }
+    for (uint32_t c = columns + tid; c < p.blocks_padded * 64; c += kRowsThreads) vals[c] = 0.f;
+    amax = lp_block<1>(amax, red);  // its barriers also publish vals
+    // One unit per position: the largest value lies in [2^14, 2^15). hi + lo then keep 22 bits of every value above
+    // 2^-18 of the largest, and an absolute 2^-39 of it below.
+    int e = (int)((__float_as_uint(amax) >> 23) & 0xff) - 127;
+    if (!(amax > 0.f) || e > 127) e = 14;  // zero row or non-finite input: factor 1
+    e = max(e, -100);
+    const float f = __uint_as_float((uint32_t)(14 - e + 127) << 23);
+    if (tid == 0) p.in.unit[pos] = __uint_as_float((uint32_t)(e - 14 + 127) << 23);
+    for (uint32_t i = tid; i < p.blocks_padded * 4; i += kRowsThreads) {  // sixteen columns: two chunks of each part
+        const uint32_t block = i >> 2, t = i & 3;
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 x = *reinterpret_cast<const float4 *>(vals + i * 16 + j * 4);
+            v[4 * j] = x.x * f;
+            v[4 * j + 1] = x.y * f;
+            v[4 * j + 2] = x.z * f;
+            v[4 * j + 3] = x.w * f;
+        }
+        __half2 hi[8], lo[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {  // slots 2 s, 2 s + 1 (inv_perm)
+            const float q4a = v[(s >> 2) * 8 + (s & 3)], q4b = v[(s >> 2) * 8 + (s & 3) + 4];
+            const float x = p.dt ? q4a : v[s], y = p.dt ? q4b : v[s + 8];
+            hi[s] = __floats2half2_rn(x, y);
+            lo[s] = __floats2half2_rn(x - __low2float(hi[s]), y - __high2float(hi[s]));
+        }
+        uint8_t *d = p.in.x + ((size_t)block * 2 * p.in.pos_pad + pos) * 128;
+        const uint32_t c0 = ((2 * t) ^ (pos & 7)) * 16, c1 = ((2 * t + 1) ^ (pos & 7)) * 16;
+        const size_t part = (size_t)p.in.pos_pad * 128;
+        *reinterpret_cast<uint4 *>(d + c0) = *reinterpret_cast<uint4 *>(hi);
+        *reinterpret_cast<uint4 *>(d + c1) = *reinterpret_cast<uint4 *>(hi + 4);
+        *reinterpret_cast<uint4 *>(d + part + c0) = *reinterpret_cast<uint4 *>(lo);
+        *reinterpret_cast<uint4 *>(d + part + c1) = *reinterpret_cast<uint4 *>(lo + 4);
+    }
+}
+
+// ------------------------------------------------------------------ linear attention
+// Causal conv + SiLU (reference.rs:159-187) for sixteen positions of 128 channels, which are one head of q, k or v;
+// q and k leave normalised (k^ and q^ / sqrt(128) of delta.cu).
+constexpr int kConvTokens = 16;
+struct LongConv {
+    LongOut o;
+    const float *conv_state, *conv_w;
+    float *qkv;
+    uint32_t key_width, channels, kernel, m;
+};
+__global__ void __launch_bounds__(128) k_long_conv(const LongConv p) {
+    pdl_launch();
+    pdl_wait();
+    __shared__ float red[kConvTokens][4];
+    const uint32_t ch = blockIdx.x * 128 + threadIdx.x, m0 = blockIdx.y * kConvTokens, warp = threadIdx.x >> 5;
+    const uint32_t K = p.kernel;
+    float st[8], cw[8], y[kConvTokens];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        st[j] = cw[j] = 0.f;
+        if ((uint32_t)j < K) {
+            cw[j] = p.conv_w[(size_t)ch * K + j];
+            // st[j]: input of position m0 - K + j
+            const int at = (int)m0 - (int)K + j;
+            st[j] = at >= 0 ? lp_out(p.o, ch, at) : p.conv_state[(size_t)ch * K + (uint32_t)((int)K + at)];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kConvTokens; ++i) y[i] = m0 + i < p.m ? lp_out(p.o, ch, m0 + i) : 0.f;
+#pragma unroll
+    for (int i = 0; i < kConvTokens; ++i) {
+        const float x = y[i];
+#pragma unroll
+        for (int j = 0; j < 7; ++j)
+            if ((uint32_t)j + 1 < K) st[j] = st[j + 1];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if ((uint32_t)j + 1 == K) st[j] = x;
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if ((uint32_t)j < K) sum += st[j] * cw[j];
+        y[i] = silu_f(sum);
+    }
+    if (ch < 2 * p.key_width) {  // all 128 channels of the CTA alike
+#pragma unroll
+        for (int i = 0; i < kConvTokens; ++i) {
+            float s = y[i] * y[i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if ((threadIdx.x & 31) == 0) red[i][warp] = s;
+        }
+        __syncthreads();
+        const float scale = ch < p.key_width ? 1.0f / sqrtf(128.0f) : 1.0f;
+#pragma unroll
+        for (int i = 0; i < kConvTokens; ++i)
+            y[i] = y[i] * (1.0f / sqrtf(red[i][0] + red[i][1] + red[i][2] + red[i][3] + 1e-6f)) * scale;
+    }
+#pragma unroll
+    for (int i = 0; i < kConvTokens; ++i)
+        if (m0 + i < p.m) p.qkv[(size_t)(m0 + i) * p.channels + ch] = y[i];
+}
+
+// Decay and beta of every (position, head) (decoder.rs:29-35,881,897-902), and the conv state after the pass (m is
+// at least the kernel's width). In a kernel of its own: the conv kernel's CTAs read the state before the pass.
+struct LongGates {
+    LongOut o;
+    const float *a_log, *dt_bias;
+    float *decay, *beta, *conv_state;
+    uint32_t heads, off, channels, kernel, m;
+};
+__global__ void __launch_bounds__(256) k_long_gates(const LongGates p) {
+    pdl_launch();
+    pdl_wait();
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x, n = p.m * p.heads;
+    if (i < n) {
+        const uint32_t pos = i / p.heads, h = i % p.heads;
+        const float x = lp_out(p.o, p.off + h, pos) + p.dt_bias[h];
+        const float sp = x > 20.0f ? x : log1pf(expf(x));
+        p.decay[i] = expf(-expf(p.a_log[h]) * sp);
+        p.beta[i] = 1.0f / (1.0f + expf(-lp_out(p.o, p.off + p.heads + h, pos)));
+    } else if (i - n < p.channels * p.kernel) {
+        const uint32_t ch = (i - n) / p.kernel, j = (i - n) % p.kernel;
+        p.conv_state[(i - n)] = lp_out(p.o, ch, p.m - p.kernel + j);
+    }
+}
+
+// The gated-delta recurrence (delta.cu) over all positions. Bound by the chain from token to token: a product with the
+// state, a sum across lanes, the update. A warp owns four value columns with their 128 keys (8 lanes per column, 16
+// state values each in registers), so that chain has three shuffles and no barrier; the tokens' inputs are staged
+// sixteen at a time, a block ahead. A CTA takes 16 columns: 8 CTAs per head.
+constexpr int kScanTokens = 16, kScanCols = 16;
+struct LongScan {
+    const float *qkv, *decay, *beta;
+    float *state, *out;
+    uint32_t key_width, channels, heads, qk_heads, m;
+};
+__global__ void __launch_bounds__(128) k_long_delta(const LongScan p) {
+    pdl_launch();
+    pdl_wait();
+    __shared__ __align__(16) float qs[2][kScanTokens][128], ks[2][kScanTokens][128], vs[2][kScanTokens][kScanCols];
+    __shared__ float ds[2][kScanTokens], bs[2][kScanTokens], os[kScanTokens][kScanCols];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane & 7, c = warp * 4 + (lane >> 3);
+    const uint32_t head = blockIdx.x >> 3, col0 = (blockIdx.x & 7) * kScanCols, kh = head / (p.heads / p.qk_heads);
+    float s[16];
+    float *state = p.state + (size_t)head * 128 * 128 + col0 + c;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s[i] = state[(size_t)((i >> 2) * 32 + sub * 4 + (i & 3)) * 128];
+    auto copy16 = [](void *dst, const void *src) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                     : "memory");
+    };
+    auto copy4 = [](void *dst, const void *src) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                     : "memory");
+    };
+    auto fetch = [&](uint32_t t0, uint32_t b) {
+        const uint32_t n = min((uint32_t)kScanTokens, p.m - t0);
+        for (uint32_t i = tid; i < n * 32; i += 128) {
+            const float *row = p.qkv + (size_t)(t0 + (i >> 5)) * p.channels + kh * 128 + (i & 31) * 4;
+            copy16(&qs[b][i >> 5][(i & 31) * 4], row);
+            copy16(&ks[b][i >> 5][(i & 31) * 4], row + p.key_width);
+        }
+        for (uint32_t i = tid; i < n * 4; i += 128)
+            copy16(&vs[b][i >> 2][(i & 3) * 4],
+                   p.qkv + (size_t)(t0 + (i >> 2)) * p.channels + 2 * p.key_width + head * 128 + col0 + (i & 3) * 4);
+        if (tid < n) {
+            copy4(&ds[b][tid], p.decay + (size_t)(t0 + tid) * p.heads + head);
+            copy4(&bs[b][tid], p.beta + (size_t)(t0 + tid) * p.heads + head);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, 0);
+    for (uint32_t t0 = 0, b = 0; t0 < p.m; t0 += kScanTokens, b ^= 1) {
+        const uint32_t n = min((uint32_t)kScanTokens, p.m - t0);
+        if (t0 + kScanTokens < p.m) {
+            fetch(t0 + kScanTokens, b ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        for (uint32_t t = 0; t < n; ++t) {
+            const float decay = ds[b][t], beta = bs[b][t], v = vs[b][t][c];
+            float k[16], mem[4] = {0.f, 0.f, 0.f, 0.f}, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 x = *reinterpret_cast<const float4 *>(&ks[b][t][i * 32 + sub * 4]);
+                k[4 * i] = x.x;
+                k[4 * i + 1] = x.y;
+                k[4 * i + 2] = x.z;
+                k[4 * i + 3] = x.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                s[i] *= decay;
+                mem[i & 3] = fmaf(s[i], k[i], mem[i & 3]);
+            }
+            float r = (mem[0] + mem[1]) + (mem[2] + mem[3]);
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
+            const float delta = (v - r) * beta;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 x = *reinterpret_cast<const float4 *>(&qs[b][t][i * 32 + sub * 4]);
+                const float q[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    s[4 * i + j] = fmaf(k[4 * i + j], delta, s[4 * i + j]);
+                    o[j] = fmaf(s[4 * i + j], q[j], o[j]);
+                }
+            }
+            r = (o[0] + o[1]) + (o[2] + o[3]);
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
+            if (sub == 0) os[t][c] = r;
+        }
+        __syncthreads();  // outputs complete, and buffer b free for the fetch of the next round
+        for (uint32_t i = tid; i < n * kScanCols; i += 128)
+            p.out[((size_t)(t0 + i / kScanCols) * p.heads + head) * 128 + col0 + i % kScanCols] = os[i / kScanCols][i % kScanCols];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) state[(size_t)((i >> 2) * 32 + sub * 4 + (i & 3)) * 128] = s[i];
+}
+
+// ------------------------------------------------------------------ full attention, before the cache
+// k_attn_pre (layers.cu) for a whole pass: one CTA per position, its angles once, a warp per head.
+struct LongAttnPre {
+    LongOut o;
+    AttnGeom g;
+    const float *q_norm, *k_norm;
+    uint64_t rope_position, cache_slot;
+    float *q;
+    void *k_cache, *v_cache;
+    const uint32_t *page_table;
+    uint32_t page_tokens;
+    int kv_only;
+};
+__device__ __forceinline__ void lp_store(float *p, float v) { *p = v; }
+__device__ __forceinline__ void lp_store(__nv_bfloat16 *p, float v) { *p = __float2bfloat16_rn(v); }
+template <typename T>
+__global__ void __launch_bounds__(256) k_long_attn_pre(const LongAttnPre p) {
+    pdl_launch();
+    pdl_wait();
+    __shared__ float cs[128], sn[128], buf[8][256];
+    const AttnGeom &g = p.g;
+    const uint32_t m = blockIdx.x, hd = g.head_dim, half = g.rotary_dim / 2, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint64_t at = p.cache_slot + m;
+    const size_t slot = (size_t)p.page_table[at / p.page_tokens] * p.page_tokens + at % p.page_tokens;
+    if (threadIdx.x < half) {
+        const float inv_freq = powf(g.theta, -((float)(2 * threadIdx.x)) / (float)g.rotary_dim);
+        const float ang = (float)(p.rope_position + m) * inv_freq;
+        cs[threadIdx.x] = cosf(ang);
+        sn[threadIdx.x] = sinf(ang);
+    }
+    __syncthreads();
+    const uint32_t k_row0 = g.q_heads * 2 * hd, v_row0 = k_row0 + g.kv_heads * hd;
+    for (uint32_t hi = (p.kv_only ? g.q_heads : 0) + warp; hi < g.q_heads + 2 * g.kv_heads; hi += 8) {
+        if (hi >= g.q_heads + g.kv_heads) {
+            const uint32_t kh = hi - g.q_heads - g.kv_heads;
+            T *v = (T *)p.v_cache + (slot * g.kv_heads + kh) * hd;
+            for (uint32_t d = lane; d < hd; d += 32) lp_store(v + d, lp_out(p.o, v_row0 + kh * hd + d, m));
+            continue;
+        }
+        const bool is_q = hi < g.q_heads;
+        const uint32_t head = is_q ? hi : hi - g.q_heads, row0 = is_q ? head * 2 * hd : k_row0 + head * hd;
+        float x[8], sq = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            x[j] = (uint32_t)j * 32 < hd ? lp_out(p.o, row0 + j * 32 + lane, m) : 0.f;  // hd is a multiple of 64
+            sq += x[j] * x[j];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        const float inv = 1.0f / sqrtf(sq / (float)hd + g.eps);
+        const float *w = is_q ? p.q_norm : p.k_norm;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if ((uint32_t)j * 32 < hd) {
+                x[j] = x[j] * inv * (1.0f + w[j * 32 + lane]);
+                buf[warp][j * 32 + lane] = x[j];
+            }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if ((uint32_t)j * 32 < hd) {
+                const uint32_t d = j * 32 + lane;
+                float v = x[j];
+                if (d < half)
+                    v = x[j] * cs[d] - buf[warp][d + half] * sn[d];
+                else if (d < 2 * half)
+                    v = x[j] * cs[d - half] + buf[warp][d - half] * sn[d - half];
+                if (is_q)
+                    p.q[((size_t)m * g.q_heads + head) * hd + d] = v;
+                else
+                    lp_store((T *)p.k_cache + (slot * g.kv_heads + head) * hd + d, v);
+            }
+        __syncwarp();
+    }
+}
+
+// ------------------------------------------------------------------ host side
+namespace {
+
+constexpr uint32_t kLongCap = 1024;  // positions per pass: the buffers take 0.35 GB at the flagship's widths
+
+AttnGeom geom(const ctox_exec *e) {
+    const ctox_model_config &c = e->cfg;
+    return AttnGeom{c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.rotary_dim, c.rope_theta, c.rms_norm_epsilon};
+}
+
+template <int MODE>
+ctox_status rows(ctox_exec *e, RowsArgs &a, uint32_t m, ctox_matvec *next) {
+    ctox_ctx *ctx = e->ctx;
+    a.in = e->long_pass->in;
+    a.has_next = next != nullptr;
+    if (next) {
+        a.s_in = next->s_in;
+        a.blocks_padded = next->blocks_padded;
+        a.dt = next->parts[0].dt;
+    }
+    const size_t smem = (next ? (size_t)next->blocks_padded * 64 : a.width) * 4;
+    CTOX_CUDA(ctx, cudaFuncSetAttribute(k_long_rows<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024));
+    CTOX_CUDA(ctx, launch_pdl(k_long_rows<MODE>, dim3(m), dim3(kRowsThreads), smem, ctx->stream, a));
+    return CTOX_OK;
+}
+
+// h = base (null: 0) + add, then the norm: into xn_out and / or as the input of `next`.
+ctox_status rows_norm(ctox_exec *e, uint32_t m, const float *base, const LongOut *add, const float *w, float *xn_out,
+                      ctox_matvec *next) {
+    RowsArgs a{};
+    if (add) a.o = *add;
+    a.a = base;
+    a.h = e->long_pass->h;
+    a.w = w;
+    a.xn_out = xn_out;
+    a.eps = e->cfg.rms_norm_epsilon;
+    a.width = e->cfg.hidden_size;
+    return rows<ROWS_NORM>(e, a, m, next);
+}
+
+ctox_status product(ctox_exec *e, ctox_matvec *mv, uint32_t m, LongOut *out, uint64_t row0 = 0) {
+    LongPass &L = *e->long_pass;
+    return launch_packed_gemm(mv, L.in, m, row0, mv->rows, L.y, L.y_floats, out);
+}
+
+ctox_status attn_pre(ctox_exec *e, uint32_t l, const LongOut &o, uint32_t m, uint64_t rope_pos0, uint64_t slot0,
+                     const uint32_t *page_table, bool kv_only) {
+    ctox_ctx *ctx = e->ctx;
+    const ctox_model_config &c = e->cfg;
+    const LongAttnPre a{o, geom(e), e->w[l].q_norm, e->w[l].k_norm, rope_pos0, slot0, e->long_pass->aq, e->s[l].k_cache,
+                        e->s[l].v_cache, page_table, c.kv_page_tokens, kv_only};
+    if (c.kv_dtype == CTOX_BF16)
+        CTOX_CUDA(ctx, launch_pdl(k_long_attn_pre<__nv_bfloat16>, dim3(m), dim3(256), 0, ctx->stream, a));
+    else
+        CTOX_CUDA(ctx, launch_pdl(k_long_attn_pre<float>, dim3(m), dim3(256), 0, ctx->stream, a));
+    return CTOX_OK;
+}
+
+// The mixer of layer l; its input projection's output is `o`. Leaves the input of the output projection.
+ctox_status mixer(ctox_exec *e, uint32_t l, const LongOut &o, uint32_t m, uint64_t pos0) {
+    ctox_ctx *ctx = e->ctx;
+    const ctox_model_config &c = e->cfg;
+    LongPass &L = *e->long_pass;
+    LayerW &lw = e->w[l];
+    LayerS &ls = e->s[l];
+    RowsArgs a{};
+    a.o = o;
+    a.eps = c.rms_norm_epsilon;
+    a.m = m;
+    if (lw.full) {
+        const AttnGeom g = geom(e);
+        const int bf16 = c.kv_dtype == CTOX_BF16;
+        EX(attn_pre(e, l, o, m, pos0, pos0, e->page_table, false));
+        timing_begin(ctx);
+        launch_attention_groups(ctx->stream, g, L.aq, ls.k_cache, ls.v_cache, bf16, e->page_table, c.kv_page_tokens, pos0, m,
+                                L.attn);
+        timing_end(ctx, KC_ATTENTION, 2.0 * (double)(pos0 + m) * e->kv_width * (bf16 ? 2 : 4),
+                   4.0 * ((double)pos0 + 0.5 * m) * e->q_width * m);
+        CTOX_CUDA(ctx, cudaGetLastError());
+        a.a = L.attn;
+        a.width = e->q_width;
+        a.q_heads = g.q_heads;
+        a.kv_heads = g.kv_heads;
+        a.head_dim = g.head_dim;
+        a.per_group = attention_group_positions(g, bf16);
+        return rows<ROWS_ATTENTION>(e, a, m, lw.out);
+    }
+    const uint32_t heads = c.linear_num_value_heads, kernel = c.linear_conv_kernel_dim;
+    CTOX_CUDA(ctx, launch_pdl(k_long_conv, dim3(e->channels / 128, (m + kConvTokens - 1) / kConvTokens), dim3(128), 0, ctx->stream,
+                              LongConv{o, ls.conv_state, lw.conv_w, L.qkv, e->key_width, e->channels, kernel, m}));
+    CTOX_CUDA(ctx, launch_pdl(k_long_gates, dim3((m * heads + e->channels * kernel + 255) / 256), dim3(256), 0, ctx->stream,
+                              LongGates{o, lw.a_log, lw.dt_bias, L.g, L.beta, ls.conv_state, heads, e->channels + e->value_width,
+                                        e->channels, kernel, m}));
+    timing_begin(ctx);
+    CTOX_CUDA(ctx, launch_pdl(k_long_delta, dim3(heads * 8), dim3(128), 0, ctx->stream,
+                              LongScan{L.qkv, L.g, L.beta, ls.delta[ls.cur], L.core, e->key_width, e->channels, heads,
+                                       c.linear_num_key_heads, m}));
+    timing_end(ctx, KC_LINEAR_ATTENTION, 2.0 * 4.0 * 128 * 128 * heads, 8.0 * 128 * 128 * heads * m);
+    a.a = L.core;
+    a.w = lw.lin_norm;
+    a.width = e->value_width;
+    a.off = e->channels;
+    return rows<ROWS_DELTA>(e, a, m, lw.out);
+}
+
+}  // namespace
+
+ctox_status long_warmup(ctox_exec *e) {
+    ctox_ctx *ctx = e->ctx;
+    const ctox_model_config &c = e->cfg;
+    if (e->long_pass || e->tp_world > 1 || c.max_context_tokens < 64) return CTOX_OK;
+    std::vector<ctox_matvec *> mats;
+    for (LayerW &lw : e->w)
+        for (ctox_matvec *mv : {lw.in_fan, lw.out, lw.gate_up, lw.down}) mats.push_back(mv);
+    if (e->mtp_fc) mats.push_back(e->mtp_fc);
+    uint32_t blocks = 0;
+    uint64_t rows = 0;
+    for (ctox_matvec *mv : mats) {
+        if (mv->parts.size() != 1 || (size_t)mv->blocks_padded * 256 + 2048 > (size_t)ctx->max_smem_optin) return CTOX_OK;
+        blocks = mv->blocks_padded > blocks ? mv->blocks_padded : blocks;
+        rows = mv->rows > rows ? mv->rows : rows;
+    }
+    const uint32_t cap = c.max_context_tokens < kLongCap ? (c.max_context_tokens + 7) / 8 * 8 : kLongCap;
+    const uint32_t pos_pad = (cap + kLongPosTile - 1) / kLongPosTile * kLongPosTile;
+    LongPass *L = new LongPass();
+    const size_t owned = e->owned.size();
+    const uint64_t session = e->session_bytes;
+    auto get = [&](auto **p, size_t n) { return xalloc(e, (void **)p, n * sizeof(**p), true, false); };
+    L->cap = cap;
+    L->in.pos_pad = pos_pad;
+    L->y_floats = (size_t)cap * rows;
+    const uint64_t H = c.hidden_size;
+    ctox_status rc = get(&L->in.x, long_in_bytes(blocks, pos_pad));
+    if (!rc) rc = get(&L->in.unit, pos_pad);
+    if (!rc) rc = get(&L->y, L->y_floats);
+    if (!rc) rc = get(&L->h, cap * H);
+    if (!rc) rc = get(&L->final_hidden, cap * H);
+    if (!rc) rc = get(&L->qkv, (size_t)cap * e->channels);
+    if (!rc) rc = get(&L->core, (size_t)cap * e->value_width);
+    if (!rc) rc = get(&L->g, (size_t)cap * c.linear_num_value_heads);
+    if (!rc) rc = get(&L->beta, (size_t)cap * c.linear_num_value_heads);
+    if (!rc) rc = get(&L->aq, (size_t)cap * e->q_width);
+    if (!rc) rc = get(&L->attn, (size_t)cap * c.num_attention_heads * (c.head_dim + 2));
+    if (!rc) rc = get(&L->tokens, cap);
+    if (rc) {  // no room: the model runs with short passes alone, as it would without them
+        while (e->owned.size() > owned) {
+            dev_free(ctx, e->owned.back().first, e->owned.back().second);
+            e->owned.pop_back();
+        }
+        e->session_bytes = session;
+        delete L;
+        return CTOX_OK;
+    }
+    e->long_pass = L;
+    return CTOX_OK;
+}
+
+ctox_status long_target_pass(ctox_exec *e, const uint32_t *tokens, uint32_t m) {
+    ctox_ctx *ctx = e->ctx;
+    const ctox_model_config &c = e->cfg;
+    LongPass &L = *e->long_pass;
+    const uint64_t pos0 = e->position;
+    const size_t row = (size_t)c.hidden_size * 4;
+    LongOut o;
+    CTOX_CUDA(ctx, cudaMemcpyAsync(L.tokens, tokens, (size_t)m * 4, cudaMemcpyHostToDevice, ctx->stream));
+    EX(matvec_embed_rows(e->embed, L.tokens, m, L.h));
+    EX(rows_norm(e, m, L.h, nullptr, e->w[0].in_ln, nullptr, e->w[0].in_fan));
+    for (uint32_t l = 0; l < e->n_layers; ++l) {
+        LayerW &lw = e->w[l];
+        const bool last = l + 1 == e->n_layers;
+        EX(product(e, lw.in_fan, m, &o));
+        EX(mixer(e, l, o, m, pos0));
+        EX(product(e, lw.out, m, &o));
+        EX(rows_norm(e, m, L.h, &o, lw.post_ln, nullptr, lw.gate_up));
+        EX(product(e, lw.gate_up, m, &o));
+        RowsArgs a{};
+        a.o = o;
+        a.width = c.intermediate_size;
+        EX(rows<ROWS_SWIGLU>(e, a, m, lw.down));
+        EX(product(e, lw.down, m, &o));
+        EX(rows_norm(e, m, L.h, &o, last ? e->final_norm : e->w[l + 1].in_ln, last ? L.final_hidden : nullptr,
+                     last ? nullptr : e->w[l + 1].in_fan));
+    }
+    // What the pass leaves is committed. The last pairs stay for the next call, as many as a short pass would leave.
+    const uint32_t keep = (m - 1) % kMaxPass + 1, pairs = m - keep;
+    if (c.mtp_num_hidden_layers && pairs) {
+        // The MTP layer over pairs (token p + 1, final hidden p): nothing reads more of it than its cache rows.
+        const uint32_t X = e->n_layers;
+        LayerW &lw = e->w[X];
+        EX(matvec_embed_rows(e->embed, L.tokens + 1, pairs, L.h));
+        RowsArgs a{};
+        a.a = L.h;
+        a.b = L.final_hidden;
+        a.w = e->mtp_norm_e;
+        a.w2 = e->mtp_norm_h;
+        a.eps = c.rms_norm_epsilon;
+        a.width = c.hidden_size;
+        EX(rows<ROWS_MTP>(e, a, pairs, e->mtp_fc));
+        EX(product(e, e->mtp_fc, pairs, &o));
+        EX(rows_norm(e, pairs, nullptr, &o, lw.in_ln, nullptr, lw.in_fan));
+        EX(product(e, lw.in_fan, pairs, &o, 2ull * e->q_width));
+        EX(attn_pre(e, X, o, pairs, pos0 + 1, pos0, e->mtp_page_table, true));
+    }
+    CTOX_CUDA(ctx, cudaMemcpyAsync(e->hist_hidden, L.final_hidden + (size_t)pairs * c.hidden_size, keep * row,
+                                   cudaMemcpyDeviceToDevice, ctx->stream));
+    for (uint32_t j = 0; j + 1 < keep; ++j) e->hist_tokens[j] = tokens[pairs + 1 + j];
+    e->hist_n = keep;
+    e->have_hidden = true;
+    e->position += m;
+    return CTOX_OK;
+}
+
+}  // namespace ctox

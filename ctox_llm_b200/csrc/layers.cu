@@ -8,6 +8,8 @@
 // unless a later step needs it.
 #include "layers.cuh"
 
+#include "hybrid_prefill.cuh"
+
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -399,6 +401,17 @@ void launch_attn_pre(cudaStream_t st, const MvOut &fan, const AttnGeom &g, const
 constexpr int kAttnTile = 32;      // tokens per tile
 constexpr int kAttnThreads = 256;
 
+// Positions of a long pass are dealt to the attention kernels in groups of per_group (blockIdx.y, no split of the
+// context): a CTA sees its group as a pass of its own. A short pass is one group.
+__device__ __forceinline__ void attention_group(const AttnGeom &g, uint32_t per_group, const float *__restrict__ &q, uint64_t &cache_slot,
+                                                int &npos, float *__restrict__ &ws) {
+    const uint32_t first = blockIdx.y * per_group;
+    q += (size_t)first * g.q_heads * g.head_dim;
+    ws += (size_t)first * g.q_heads * (g.head_dim + 2);
+    cache_slot += first;
+    npos = min((int)per_group, npos - (int)first);
+}
+
 // grouped_query_attention (reference.rs:420-499) for the m query positions of one KV head over
 // one split of the context, flash-decoding style: per tile of 32 tokens the K rows are staged in
 // shared memory, every warp scores its queries against the 32 tokens (lane = token), keeps the
@@ -407,11 +420,12 @@ constexpr int kAttnThreads = 256;
 template <typename T, int NQMAX>
 __global__ void __launch_bounds__(kAttnThreads) k_attention(
     AttnGeom g, const float *__restrict__ q, const T *__restrict__ k_cache, const T *__restrict__ v_cache,
-    const uint32_t *__restrict__ page_table, uint32_t page_tokens, uint64_t cache_slot, int npos,
+    const uint32_t *__restrict__ page_table, uint32_t page_tokens, uint64_t cache_slot, int npos, uint32_t per_group,
     uint32_t splits, float *__restrict__ ws) {
     pdl_launch();
     pdl_wait();
     extern __shared__ __align__(128) uint8_t smraw[];
+    attention_group(g, per_group, q, cache_slot, npos, ws);
     const uint32_t hd = g.head_dim, G = g.q_heads / g.kv_heads, NQ = G * npos;
     const uint32_t kh = blockIdx.x / splits, sp = blockIdx.x % splits;
     const uint32_t kstride = hd + 16 / sizeof(T);  // padded row: conflict-free 16-byte reads
@@ -557,9 +571,10 @@ template <int GROUPS>  // 1: up to 16 queries (4 warps), 2: up to 32 queries (8 
 __global__ void __launch_bounds__(GROUPS * 128, 1) k_attention_mma(
     AttnGeom g, const float *__restrict__ q, const __nv_bfloat16 *__restrict__ k_cache,
     const __nv_bfloat16 *__restrict__ v_cache, const uint32_t *__restrict__ page_table, uint32_t page_tokens,
-    uint64_t cache_slot, int npos, uint32_t splits, float *__restrict__ ws) {
+    uint64_t cache_slot, int npos, uint32_t per_group, uint32_t splits, float *__restrict__ ws) {
     pdl_launch();
     extern __shared__ __align__(128) uint8_t smraw[];
+    attention_group(g, per_group, q, cache_slot, npos, ws);
     constexpr int NT = GROUPS * 128, kFaBuffers = fa_buffers(GROUPS);
     const uint32_t G = g.q_heads / g.kv_heads, NQ = G * npos;
     const uint32_t kh = blockIdx.x / splits, sp = blockIdx.x % splits;
@@ -906,7 +921,7 @@ size_t attn_workspace_bytes(const AttnGeom &g, uint32_t m, uint32_t max_splits) 
 template <typename T, int NQMAX>
 static void launch_attention_t(cudaStream_t st, const AttnGeom &g, const float *q, const void *k_cache,
                                const void *v_cache, const uint32_t *page_table, uint32_t page_tokens,
-                               uint64_t cache_slot, uint32_t m, uint32_t splits, float *ws) {
+                               uint64_t cache_slot, uint32_t m, uint32_t per_group, uint32_t splits, float *ws) {
     const size_t smem = (size_t)NQMAX * g.head_dim * 4 + (size_t)NQMAX * kAttnTile * 4 + 3 * NQMAX * 4 +
                         (size_t)kAttnTile * (g.head_dim + 16 / sizeof(T)) * sizeof(T) + 16;
     // the attribute belongs to the device, not to the process: once per device
@@ -917,15 +932,15 @@ static void launch_attention_t(cudaStream_t st, const AttnGeom &g, const float *
         cudaFuncSetAttribute(k_attention<T, NQMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
             cudaSuccess)
         attr_devices |= 1ull << dev;
-    launch_pdl(k_attention<T, NQMAX>, dim3(g.kv_heads * splits), dim3(kAttnThreads), smem, st, 
-        g, q, (const T *)k_cache, (const T *)v_cache, page_table, page_tokens, cache_slot, (int)m, splits, ws);
+    launch_pdl(k_attention<T, NQMAX>, dim3(g.kv_heads * splits, (m + per_group - 1) / per_group), dim3(kAttnThreads), smem, st,
+               g, q, (const T *)k_cache, (const T *)v_cache, page_table, page_tokens, cache_slot, (int)m, per_group, splits, ws);
 }
 
-void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const float *gate,
-                      const void *k_cache, const void *v_cache, int kv_bf16, const uint32_t *page_table,
-                      uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits, float *workspace,
-                      const MvIn &next) {
-    const uint32_t nq = g.q_heads / g.kv_heads * m;
+// Shared by short passes (one group, `splits` parts of the context) and long ones (many groups, one part).
+static void launch_attention_kernel(cudaStream_t st, const AttnGeom &g, const float *q, const void *k_cache,
+                                    const void *v_cache, int kv_bf16, const uint32_t *page_table, uint32_t page_tokens,
+                                    uint64_t cache_slot, uint32_t m, uint32_t per_group, uint32_t splits, float *workspace) {
+    const uint32_t nq = g.q_heads / g.kv_heads * per_group;
     if (kv_bf16 && g.head_dim == kFaHd && nq <= 32) {
         const size_t smem1 = 2 * 32 * kFaStride * 2 + (size_t)fa_buffers(1) * 2 * kFaTile * kFaStride * 2;
         const size_t smem2 = 2 * 32 * kFaStride * 2 + (size_t)fa_buffers(2) * 2 * kFaTile * kFaHd * 2;
@@ -938,36 +953,56 @@ void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const 
             cudaFuncSetAttribute(k_attention_mma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) ==
                 cudaSuccess)
             attr_devices |= 1ull << dev;
+        const dim3 grid(g.kv_heads * splits, (m + per_group - 1) / per_group);
         if (nq <= 16)
-            launch_pdl(k_attention_mma<1>, dim3(g.kv_heads * splits), dim3(128), smem1, st, 
-                g, q, (const __nv_bfloat16 *)k_cache, (const __nv_bfloat16 *)v_cache, page_table, page_tokens,
-                cache_slot, (int)m, splits, workspace);
+            launch_pdl(k_attention_mma<1>, grid, dim3(128), smem1, st, g, q, (const __nv_bfloat16 *)k_cache,
+                       (const __nv_bfloat16 *)v_cache, page_table, page_tokens, cache_slot, (int)m, per_group, splits,
+                       workspace);
         else
-            launch_pdl(k_attention_mma<2>, dim3(g.kv_heads * splits), dim3(256), smem2, st, 
-                g, q, (const __nv_bfloat16 *)k_cache, (const __nv_bfloat16 *)v_cache, page_table, page_tokens,
-                cache_slot, (int)m, splits, workspace);
-        launch_pdl(k_attn_combine_prep, dim3(m * g.q_heads), dim3(g.head_dim), 0, st, g, workspace, gate, (int)m, splits,
-                   next);
+            launch_pdl(k_attention_mma<2>, grid, dim3(256), smem2, st, g, q, (const __nv_bfloat16 *)k_cache,
+                       (const __nv_bfloat16 *)v_cache, page_table, page_tokens, cache_slot, (int)m, per_group, splits,
+                       workspace);
         return;
     }
 #define CTOX_ATTN(T)                                                                                        \
     do {                                                                                                    \
         if (nq <= 8)                                                                                        \
             launch_attention_t<T, 8>(st, g, q, k_cache, v_cache, page_table, page_tokens, cache_slot, m,    \
-                                     splits, workspace);                                                    \
+                                     per_group, splits, workspace);                                         \
         else if (nq <= 24)                                                                                  \
             launch_attention_t<T, 24>(st, g, q, k_cache, v_cache, page_table, page_tokens, cache_slot, m,   \
-                                      splits, workspace);                                                   \
+                                      per_group, splits, workspace);                                        \
         else                                                                                                \
             launch_attention_t<T, 48>(st, g, q, k_cache, v_cache, page_table, page_tokens, cache_slot, m,   \
-                                      splits, workspace);                                                   \
+                                      per_group, splits, workspace);                                        \
     } while (0)
     if (kv_bf16)
         CTOX_ATTN(__nv_bfloat16);
     else
         CTOX_ATTN(float);
 #undef CTOX_ATTN
+}
+
+void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const float *gate,
+                      const void *k_cache, const void *v_cache, int kv_bf16, const uint32_t *page_table,
+                      uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits, float *workspace,
+                      const MvIn &next) {
+    launch_attention_kernel(st, g, q, k_cache, v_cache, kv_bf16, page_table, page_tokens, cache_slot, m, m, splits, workspace);
     launch_pdl(k_attn_combine_prep, dim3(m * g.q_heads), dim3(g.head_dim), 0, st, g, workspace, gate, (int)m, splits, next);
+}
+
+// Positions that share a CTA in a long pass: as many queries as the kernel takes at once (32 on the tensor cores,
+// else what a short pass of eight positions may have).
+uint32_t attention_group_positions(const AttnGeom &g, int kv_bf16) {
+    const uint32_t G = g.q_heads / g.kv_heads;
+    const uint32_t n = kv_bf16 && g.head_dim == kFaHd && G <= 32 ? 32 / G : 8;
+    return n < 8 ? n : 8;
+}
+void launch_attention_groups(cudaStream_t st, const AttnGeom &g, const float *q, const void *k_cache, const void *v_cache,
+                             int kv_bf16, const uint32_t *page_table, uint32_t page_tokens, uint64_t cache_slot, uint32_t m,
+                             float *workspace) {
+    launch_attention_kernel(st, g, q, k_cache, v_cache, kv_bf16, page_table, page_tokens, cache_slot, m,
+                            attention_group_positions(g, kv_bf16), 1, workspace);
 }
 
 }  // namespace ctox

@@ -1,0 +1,85 @@
+"""Long passes of the hybrid model (tensor-core products, row kernels, token scan) against short passes of at most
+16 tokens per call over the same weights: logits, and what speculative blocks do with the state and caches left."""
+import numpy as np
+import pytest
+
+import ctox_llm_b200 as ctox
+from gpu_util import rel_l2
+from oracle_model import OracleModel, tiny_config
+
+pytestmark = pytest.mark.gpu
+
+
+CONFIGS = {
+    # widths that are not whole tiles of 128 rows or 256 columns; CUDA-core attention over both cache types
+    "ragged-f32": dict(kv_dtype=ctox.F32, hidden_size=320, intermediate_size=704),
+    "ragged-bf16": dict(kv_dtype=ctox.BF16, hidden_size=320, intermediate_size=704),
+    # the tensor-core attention kernel, groups of eight positions; every second layer attention
+    "head256": dict(num_attention_heads=4, num_key_value_heads=1, head_dim=256, rotary_dim=64, kv_dtype=ctox.BF16,
+                    full_attention_interval=2),
+}
+
+
+@pytest.mark.parametrize("name", CONFIGS)
+@pytest.mark.parametrize("n", [17, 63, 65, 129, 300, 1025 + 40])
+def test_long_pass_equals_short_passes(orc, name, n):
+    """n crosses the tiles of 64 / 128 / 256 positions, the groups of 8 positions and of 16 tokens, and the 1024
+    positions of one pass. Both sides sum the same products in 32 bits in another order: 1e-4 of the logits for a 32-bit
+    cache; rounding keys and values to 16 bits turns such differences into steps of 2^-9 (1e-3, the bound of the
+    oracle's comparisons)."""
+    be = ctox.B200Backend(0)
+    cfg = tiny_config(max_draft_tokens=3, max_context_tokens=1200, **CONFIGS[name])
+    model = OracleModel(orc, cfg, seed=4)
+    ex = ctox.B200Executor(be, cfg)
+    bound = 1e-4 if cfg.kv_dtype == ctox.F32 else 1e-3
+    try:
+        model.load_into(ex)
+        ex.warmup()
+        ex.keep_logits(True)
+        prompt = [int(t) for t in np.random.default_rng(n).integers(0, cfg.vocab_size, n + 1)]
+        want = sorted({0, 7, 8, n // 2, n - 2, n - 1})
+        runs = []
+        for step in (n, 16):
+            ex.reset_session()
+            rows = []
+            for a in range(0, n, step):
+                b = min(a + step, n)
+                here = [w - a for w in want if a <= w < b]
+                if here:
+                    rows += list(ex.extend(prompt[a:b], here))
+                else:
+                    ex.extend(prompt[a:b])
+            assert ex.position() == n
+            out = [np.stack(rows), ex.last_hidden()[None]]
+            tok = prompt[n]
+            for _ in range(2):  # the MTP cache and the recurrent state
+                ex.decode(tok, mtp_enabled=True, force_accept=0)
+                out += [ex.last_logits(0)[None], np.stack(ex.last_draft_logits()[:1]), np.stack(ex.last_mtp_hidden()[:1])]
+            runs.append(out)
+        for got, ref in zip(*runs):
+            for g, r in zip(got, ref):
+                assert rel_l2(g, r) <= bound
+    finally:
+        ex.unload()
+        be.close()
+
+
+def test_long_pass_on_top_of_a_session_matches_oracle(orc):
+    """A long pass behind a short one and before another: positions, page offsets and carried state against the oracle."""
+    be = ctox.B200Backend(0)
+    cfg = tiny_config(max_draft_tokens=2)
+    model = OracleModel(orc, cfg, seed=6)
+    ex = ctox.B200Executor(be, cfg)
+    try:
+        model.load_into(ex)
+        ex.warmup()
+        prompt = [int(t) for t in np.random.default_rng(5).integers(0, cfg.vocab_size, 48)]
+        _, exp_logits, _ = model.greedy(prompt, 1)
+        ex.reset_session()
+        ex.extend(prompt[:5])
+        ex.extend(prompt[5:42])
+        got = ex.extend(prompt[42:], [5])
+        assert rel_l2(got[0], exp_logits[0]) <= 1e-3
+    finally:
+        ex.unload()
+        be.close()
