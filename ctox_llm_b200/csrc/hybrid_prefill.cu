@@ -191,11 +191,22 @@ __global__ void __launch_bounds__(128) k_long_conv(const LongConv p) {
             cw[j] = p.conv_w[(size_t)ch * K + j];
             // st[j]: input of position m0 - K + j
             const int at = (int)m0 - (int)K + j;
-            st[j] = at >= 0 ? lp_out(p.o, ch, at) : p.conv_state[(size_t)ch * K + (uint32_t)((int)K + at)];
+            st[j] = at >= 0 ? p.o.y[(size_t)at * p.o.rows + ch] : p.conv_state[(size_t)ch * K + (uint32_t)((int)K + at)];
         }
     }
 #pragma unroll
-    for (int i = 0; i < kConvTokens; ++i) y[i] = m0 + i < p.m ? lp_out(p.o, ch, m0 + i) : 0.f;
+    for (int i = 0; i < kConvTokens; ++i) y[i] = m0 + i < p.m ? p.o.y[(size_t)(m0 + i) * p.o.rows + ch] : 0.f;
+    for (uint32_t sp = 1; sp < p.o.splits; ++sp) {  // all loads of a partial sum together
+        const float *o = p.o.y + sp * p.o.split_stride + ch;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int at = (int)m0 - (int)K + j;
+            if ((uint32_t)j < K && at >= 0) st[j] += o[(size_t)at * p.o.rows];
+        }
+#pragma unroll
+        for (int i = 0; i < kConvTokens; ++i)
+            if (m0 + i < p.m) y[i] += o[(size_t)(m0 + i) * p.o.rows];
+    }
 #pragma unroll
     for (int i = 0; i < kConvTokens; ++i) {
         const float x = y[i];
@@ -259,6 +270,31 @@ __global__ void __launch_bounds__(256) k_long_gates(const LongGates p) {
 // state values each in registers), so that chain has three shuffles and no barrier; the tokens' inputs are staged
 // sixteen at a time, a block ahead. A CTA takes 16 columns: 8 CTAs per head.
 constexpr int kScanTokens = 16, kScanCols = 16;
+// Two fp32 values per instruction.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float total4(const unsigned long long (&v)[4]) {
+    float a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) unpack2(v[i], a[i], b[i]);
+    return ((a[0] + b[0]) + (a[1] + b[1])) + ((a[2] + b[2]) + (a[3] + b[3]));
+}
 struct LongScan {
     const float *qkv, *decay, *beta;
     float *state, *out;
@@ -271,10 +307,18 @@ __global__ void __launch_bounds__(128) k_long_delta(const LongScan p) {
     __shared__ float ds[2][kScanTokens], bs[2][kScanTokens], os[kScanTokens][kScanCols];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane & 7, c = warp * 4 + (lane >> 3);
     const uint32_t head = blockIdx.x >> 3, col0 = (blockIdx.x & 7) * kScanCols, kh = head / (p.heads / p.qk_heads);
-    float s[16];
+    // this lane's keys are sub * 4 + 32 i .. + 3, i < 4; two of them per register pair
+    unsigned long long s[8];
     float *state = p.state + (size_t)head * 128 * 128 + col0 + c;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) s[i] = state[(size_t)((i >> 2) * 32 + sub * 4 + (i & 3)) * 128];
+    for (int i = 0; i < 8; ++i) {
+        const float *at = state + (size_t)((i >> 1) * 32 + sub * 4 + (i & 1) * 2) * 128;
+        s[i] = pack2(at[0], at[128]);
+    }
+    auto load = [&](ulonglong2(&d)[4], const float *row) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = *reinterpret_cast<const ulonglong2 *>(row + i * 32 + sub * 4);
+    };
     auto copy16 = [](void *dst, const void *src) {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                      : "memory");
@@ -309,48 +353,61 @@ __global__ void __launch_bounds__(128) k_long_delta(const LongScan p) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
+        ulonglong2 k[4];
+        load(k, ks[b][0]);
+        float decay = ds[b][0], beta = bs[b][0], v = vs[b][0][c], o = 0.f;
         for (uint32_t t = 0; t < n; ++t) {
-            const float decay = ds[b][t], beta = bs[b][t], v = vs[b][t][c];
-            float k[16], mem[4] = {0.f, 0.f, 0.f, 0.f}, o[4] = {0.f, 0.f, 0.f, 0.f};
+            ulonglong2 kn[4], q[4];
+            load(q, qs[b][t]);
+            load(kn, ks[b][t + 1 < n ? t + 1 : t]);
+            const uint32_t tn = t + 1 < n ? t + 1 : t;
+            const float decay_n = ds[b][tn], beta_n = bs[b][tn], v_n = vs[b][tn][c];
+            const unsigned long long d2 = pack2(decay, decay);
+            unsigned long long mem[4] = {0, 0, 0, 0}, out[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float4 x = *reinterpret_cast<const float4 *>(&ks[b][t][i * 32 + sub * 4]);
-                k[4 * i] = x.x;
-                k[4 * i + 1] = x.y;
-                k[4 * i + 2] = x.z;
-                k[4 * i + 3] = x.w;
+                s[2 * i] = mul2(s[2 * i], d2);
+                s[2 * i + 1] = mul2(s[2 * i + 1], d2);
+                mem[i & 1] = fma2(s[2 * i], k[i].x, mem[i & 1]);
+                mem[2 + (i & 1)] = fma2(s[2 * i + 1], k[i].y, mem[2 + (i & 1)]);
             }
+            float r = total4(mem);
+            // the sum over the lanes, side by side with that of the output of the token before
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                s[i] *= decay;
-                mem[i & 3] = fmaf(s[i], k[i], mem[i & 3]);
+            for (int d = 1; d < 8; d <<= 1) {
+                const float r1 = __shfl_xor_sync(0xffffffffu, r, d), o1 = __shfl_xor_sync(0xffffffffu, o, d);
+                r += r1;
+                o += o1;
             }
-            float r = (mem[0] + mem[1]) + (mem[2] + mem[3]);
-#pragma unroll
-            for (int d = 1; d < 8; d <<= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
+            if (sub == 0 && t > 0) os[t - 1][c] = o;
             const float delta = (v - r) * beta;
+            const unsigned long long dl2 = pack2(delta, delta);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float4 x = *reinterpret_cast<const float4 *>(&qs[b][t][i * 32 + sub * 4]);
-                const float q[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    s[4 * i + j] = fmaf(k[4 * i + j], delta, s[4 * i + j]);
-                    o[j] = fmaf(s[4 * i + j], q[j], o[j]);
-                }
+                s[2 * i] = fma2(k[i].x, dl2, s[2 * i]);
+                s[2 * i + 1] = fma2(k[i].y, dl2, s[2 * i + 1]);
+                out[i & 1] = fma2(s[2 * i], q[i].x, out[i & 1]);
+                out[2 + (i & 1)] = fma2(s[2 * i + 1], q[i].y, out[2 + (i & 1)]);
+                k[i] = kn[i];
             }
-            r = (o[0] + o[1]) + (o[2] + o[3]);
-#pragma unroll
-            for (int d = 1; d < 8; d <<= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
-            if (sub == 0) os[t][c] = r;
+            o = total4(out);
+            decay = decay_n;
+            beta = beta_n;
+            v = v_n;
         }
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
+        if (sub == 0) os[n - 1][c] = o;
         __syncthreads();  // outputs complete, and buffer b free for the fetch of the next round
         for (uint32_t i = tid; i < n * kScanCols; i += 128)
             p.out[((size_t)(t0 + i / kScanCols) * p.heads + head) * 128 + col0 + i % kScanCols] = os[i / kScanCols][i % kScanCols];
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) state[(size_t)((i >> 2) * 32 + sub * 4 + (i & 3)) * 128] = s[i];
+    for (int i = 0; i < 8; ++i) {
+        float *at = state + (size_t)((i >> 1) * 32 + sub * 4 + (i & 1) * 2) * 128;
+        unpack2(s[i], at[0], at[128]);
+    }
 }
 
 // ------------------------------------------------------------------ full attention, before the cache
@@ -552,7 +609,7 @@ ctox_status long_warmup(ctox_exec *e) {
         rows = mv->rows > rows ? mv->rows : rows;
     }
     const uint32_t cap = c.max_context_tokens < kLongCap ? (c.max_context_tokens + 7) / 8 * 8 : kLongCap;
-    const uint32_t pos_pad = (cap + kLongPosTile - 1) / kLongPosTile * kLongPosTile;
+    const uint32_t pos_pad = cap + kLongPosTile;  // a last tile may start anywhere below cap
     LongPass *L = new LongPass();
     const size_t owned = e->owned.size();
     const uint64_t session = e->session_bytes;

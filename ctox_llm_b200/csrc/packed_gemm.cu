@@ -3,15 +3,22 @@
 // What bounds it: tensor work. Every weight meets the hi and the lo part of an activation (two fp16 products, as
 // in the streaming matvec), 4 m FLOPs per weight where a plain bf16 product has 2 m. Streaming the same
 // weights once per eight positions, as short passes do, costs 125 passes over the matrix for 1000 positions and is
-// bound by unpacking the codes each time; here a code is unpacked once per 64, 128 or 256 positions.
+// bound by unpacking the codes each time; here a code is unpacked once per up to 256 positions.
 //
-// One CTA of 16 warps per SM works through units (128 rows x N positions x a range of columns):
-//   warp 0     one thread copies the activation tiles (bulk copies into a ring, hi and lo separately)
-//   warp 1     one thread issues tcgen05.mma: per 64-column block lo then hi into one accumulator
+// A CTA of 16 warps per SM works through units (128 rows x n positions x a range of columns):
+//   warp 0     one thread copies the activation tiles (bulk copies, hi and lo parts)
+//   warp 1     issues tcgen05.mma: per 64-column block lo then hi into one accumulator
+//   warp 2     (second CTA of a pair) reports its copies to the first
 //   warps 4-7  unpack codes to fp16 (code - offset, exact) and write them as the swizzled A operand
 //   warps 8-15 take the 64-column sum out of tensor memory and add scale[row][block] * sum to fp32 registers
 // The block scales therefore act in fp32 on sums of 64 products, exactly as in the streaming matvec: folding them
 // into fp16 weights would need a second weight part (scale and code have 15 significant bits).
+//
+// Tiles of more than 128 positions are computed by pairs of CTAs (cta_group::2, 256 rows): each copies half of the
+// positions, which halves what every SM draws from L2 (64 KB per block of 256 positions, 9.7 TB/s over the chip, bound
+// the single-CTA form at 1.01 us a block; a pair takes 0.90). Then the accumulators bound it: with two of 256 columns,
+// products wait for sums to be taken out (two thirds of the tensor time is used). 34816 x 5120 (Q2), 999
+// positions: 573 us, 621 TFLOP/s of a plain product, twice that counting both parts.
 #include "packed_gemm.cuh"
 
 #include <cuda_fp16.h>
@@ -23,21 +30,21 @@ namespace ctox {
 
 constexpr int kPgThreads = 512;
 
-template <uint32_t N>
+// W: widest position tile of the kernel; G: CTAs that share a tile. A launch takes n <= W positions per tile (a
+// multiple of 16 G) and as many stages (weights of 128 rows, activations of n / G positions) as fit.
+template <uint32_t W, uint32_t G>
 struct PgCfg {
-    static constexpr uint32_t kB = N == 256 ? 5 : N == 128 ? 8 : 12;  // activation tiles in the ring
-    static constexpr uint32_t kA = N == 256 ? 3 : 4;                  // weight tiles
-    static constexpr uint32_t kD = N == 256 ? 2 : 4;                  // accumulators in tensor memory
-    static constexpr uint32_t kBBytes = N * 128, kABytes = 128 * 128;
-    static constexpr uint32_t kSmem = kB * kBBytes + kA * kABytes + 1024;
+    static constexpr uint32_t kD = W == 256 ? 2 : 4;  // accumulators in tensor memory
+    static constexpr uint32_t kABytes = 128 * 128;
 };
+constexpr uint32_t kPgStages = 6;
 
 struct PgParams {
     const uint8_t *w, *x;
     const float *unit, *s_out;
     float *y;
     size_t split_stride;
-    uint32_t rows, rt0, units, m, pos_pad, pos_tiles, pairs, kst, kst_s, splits;
+    uint32_t rows, rt0, units, m, pos_pad, pos_tiles, n, stages, pairs, kst, kst_s, splits;
     int32_t *error_word;
 };
 
@@ -68,15 +75,22 @@ __device__ __forceinline__ void pg_q2(uint32_t addr0, uint32_t addr1, uint32_t w
              pg_sub((t & kM6) | kE6, kO6));
 }
 
+// acc[0..1] += s * v[0..1]
+__device__ __forceinline__ void pg_fma2(float *acc, float s, const float *v) {
+    asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %2};\n\tmov.b64 c, {%3, %4};\n\t"
+        "fma.rn.f32x2 a, b, c, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(acc[0]), "+f"(acc[1])
+        : "f"(s), "f"(v[0]), "f"(v[1]));
+}
+
 // A unit of work: rows rt * 128 .., positions n0 .., super-tiles ks0 .. ks1 (256 columns each), partial sum sp.
 struct PgUnit {
     uint32_t rt, n0, sp, ks0, ks1;
 };
-template <uint32_t N>
 __device__ __forceinline__ PgUnit pg_unit(const PgParams &p, uint32_t u) {
     // positions fastest: the CTAs that read the same weights run side by side
     const uint32_t v = u / p.pos_tiles, sp = v % p.splits;
-    return PgUnit{p.rt0 + v / p.splits, (u % p.pos_tiles) * N, sp, (uint32_t)((uint64_t)p.kst * sp / p.splits),
+    return PgUnit{p.rt0 + v / p.splits, (u % p.pos_tiles) * p.n, sp, (uint32_t)((uint64_t)p.kst * sp / p.splits),
                   (uint32_t)((uint64_t)p.kst * (sp + 1) / p.splits)};
 }
 // Super-tile `tile` (0, 1) of row pair `pair` at column super-tile ks.
@@ -86,121 +100,171 @@ __device__ __forceinline__ const uint8_t *pg_tile(const PgParams &p, uint32_t pa
     return p.w + ((((size_t)slice * p.pairs + pair) * p.kst_s + in) * 2 + tile) * Fmt<DT>::kSuperTileBytes;
 }
 
-template <int DT, uint32_t N>
+template <int DT, uint32_t W, uint32_t G>
 __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p) {
     using namespace umma;
-    using C = PgCfg<N>;
+    using C = PgCfg<W, G>;
     extern __shared__ uint8_t raw[];
-    __shared__ __align__(8) uint64_t bars[2 * (C::kB + C::kA + C::kD) + 1];
+    __shared__ __align__(8) uint64_t bars[2 * (kPgStages + C::kD) + 1];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int dead;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t b_base = (smem_addr(raw) + 1023) & ~1023u, a_base = b_base + C::kB * C::kBBytes;
-    const uint32_t b_full = smem_addr(bars), b_empty = b_full + C::kB * 8, a_full = b_empty + C::kB * 8,
-                   a_empty = a_full + C::kA * 8, d_full = a_empty + C::kA * 8, d_empty = d_full + C::kD * 8,
-                   drained = d_empty + C::kD * 8;
-    constexpr uint32_t kCols = C::kD * N;
+    const uint32_t base = (smem_addr(raw) + 1023) & ~1023u, stages = p.stages;
+    const uint32_t half_bytes = p.n / G * 128, stage_bytes = C::kABytes + 2 * half_bytes;  // A | lo | hi
+    const uint32_t full = smem_addr(bars), empty = full + kPgStages * 8, d_full = empty + kPgStages * 8,
+                   d_empty = d_full + C::kD * 8, drained = d_empty + C::kD * 8;
+    constexpr uint32_t kCols = C::kD * W;
+    const uint32_t rank = G == 2 ? cluster_rank() : 0, first_unit = blockIdx.x / G, unit_step = gridDim.x / G;
     if (tid == 0) {
         dead = 0;
-        for (uint32_t i = 0; i < C::kB; ++i) {
-            bar_init(b_full + i * 8, 1);
-            bar_init(b_empty + i * 8, 1);
-        }
-        for (uint32_t i = 0; i < C::kA; ++i) {
-            bar_init(a_full + i * 8, 4);
-            bar_init(a_empty + i * 8, 1);
+        for (uint32_t i = 0; i < stages; ++i) {
+            // the issuing CTA: its copies, its unpacking warps, and the same of the other CTA
+            bar_init(full + i * 8, G == 1 ? 5 : rank == 0 ? 10 : 1);
+            bar_init(empty + i * 8, 1);
         }
         for (uint32_t i = 0; i < C::kD; ++i) {
             bar_init(d_full + i * 8, 1);
-            bar_init(d_empty + i * 8, 8);
+            bar_init(d_empty + i * 8, 8 * G);
         }
         bar_init(drained, 1);
         bar_init_fence();
     }
-    if (warp == 1) tmem_alloc(smem_addr(&tmem_slot), kCols);
+    if (warp == 1) {
+        if constexpr (G == 2)
+            tmem_alloc_pair(smem_addr(&tmem_slot), kCols);
+        else
+            tmem_alloc(smem_addr(&tmem_slot), kCols);
+    }
     fence_before();
     __syncthreads();
+    if constexpr (G == 2) cluster_sync();  // the other CTA's barriers are ready
     fence_after();
     pdl_launch();  // after the allocation (umma.cuh)
     const uint32_t tmem = tmem_slot;
     if (warp < 4) {
-        // N = 256 keeps 128 sums per accumulating thread: those warps take registers from these. The launch has
-        // 512 x 128 registers; 128 x (56 + 96) + 256 x 176 = 64512 of its 65536 are asked for.
-        if constexpr (N == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        // Wide tiles keep up to 128 sums per accumulating thread beside 64 values on their way: those warps take
+        // registers from these. The launch has 512 x 128; 128 x (32 + 64) + 256 x 208 = 65536 are asked for.
+        if constexpr (W > 64) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         if (warp == 0 && lane == 0) {
             pdl_wait();
             asm volatile("fence.proxy.async;" ::: "memory");  // the kernel before wrote x with ordinary stores
-            uint32_t issued = 0;
+            uint32_t st = 0, parity = 1;  // parity of the phase before a ring's first: passes at once
             bool ok = true;
-            for (uint32_t u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-                const PgUnit t = pg_unit<N>(p, u);
-                const uint8_t *src = p.x + ((size_t)t.ks0 * 8 * p.pos_pad + t.n0) * 128;
-                const size_t part = (size_t)p.pos_pad * 128;
-                for (uint32_t i = 0; i < (t.ks1 - t.ks0) * 8; ++i, ++issued) {
-                    const uint32_t s = issued % C::kB, round = issued / C::kB;
-                    if (round > 0 && !(ok = bar_wait(b_empty + s * 8, (round - 1) & 1, &dead))) break;
-                    bar_expect(b_full + s * 8, C::kBBytes);
-                    asm volatile(
-                        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                            b_base + s * C::kBBytes),
-                        "l"(src + (size_t)(i ^ 1) * part), "r"(C::kBBytes), "r"(b_full + s * 8)  // lo, hi, lo, hi ...
-                        : "memory");
-                }
-            }
-            if (!ok) {  // leave no copy in flight behind
-                for (uint32_t s = 0; s < C::kB && s < issued; ++s) {
-                    const uint32_t i = issued - 1 - s;
-                    bar_drain(b_full + (i % C::kB) * 8, (i / C::kB) & 1);
-                }
-            }
-        } else if (warp == 1 && lane == 0) {
-            uint32_t used_b = 0, used_a = 0;
-            bool ok = true;
-            constexpr uint32_t idesc = (1u << 4) | ((N >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 -> fp32
-            for (uint32_t u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-                const PgUnit t = pg_unit<N>(p, u);
-                for (uint32_t k = 0; k < (t.ks1 - t.ks0) * 4; ++k, ++used_a) {
-                    const uint32_t a = used_a % C::kA, d = used_a % C::kD;
-                    if (used_a >= C::kD && !(ok = bar_wait(d_empty + d * 8, (used_a / C::kD - 1) & 1, &dead))) break;
-                    if (!(ok = bar_wait(a_full + a * 8, (used_a / C::kA) & 1, &dead))) break;
-                    for (uint32_t part = 0; part < 2; ++part, ++used_b) {
-                        const uint32_t b = used_b % C::kB;
-                        if (!(ok = bar_wait(b_full + b * 8, (used_b / C::kB) & 1, &dead))) break;
-                        fence_after();
-                        const uint64_t da = smem_desc(a_base + a * C::kABytes, 128), db = smem_desc(b_base + b * C::kBBytes, 128);
+            const size_t part = (size_t)p.pos_pad * 128;
+            for (uint32_t u = first_unit; u < p.units && ok; u += unit_step) {
+                const PgUnit t = pg_unit(p, u);
+                const uint8_t *src = p.x + (size_t)t.ks0 * 8 * part + (size_t)(t.n0 + rank * (p.n / G)) * 128;
+                for (uint32_t i = (t.ks1 - t.ks0) * 4; i > 0; --i) {
+                    const uint32_t bar = full + st * 8, dst = base + st * stage_bytes + C::kABytes;
+                    if (!(ok = bar_wait(empty + st * 8, parity, &dead))) break;
+                    bar_expect(bar, 2 * half_bytes);
 #pragma unroll
-                        for (uint32_t i = 0; i < 4; ++i) mma_f16(tmem + d * N, da + i * 2, db + i * 2, idesc, part > 0 || i > 0);
-                        commit(b_empty + b * 8);
+                    for (uint32_t h = 0; h < 2; ++h)
+                        asm volatile(
+                            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                dst + h * half_bytes),
+                            "l"(src + (h ? 0 : part)), "r"(half_bytes), "r"(bar)
+                            : "memory");
+                    src += 2 * part;
+                    if (++st == stages) {
+                        st = 0;
+                        parity ^= 1;
                     }
-                    if (!ok) break;
-                    commit(a_empty + a * 8);
-                    commit(d_full + d * 8);
                 }
             }
-            if (!ok) {
-                commit(drained);
+            if (!ok) {  // leave no copy in flight behind: a phase lacks other arrivals, so wait for the data as such
+                const long long t0 = clock64();
+                while (clock64() - t0 < 2000000) {
+                }
+            }
+        } else if (warp == 1) {
+            // One thread feeds the tensor cores: 8 products and 4 commits per block. The whole warp runs the loop, so that
+            // its values are uniform and descriptors need no moves between register files; ring positions are kept, not
+            // divided out.
+            const bool issuer = elect_one();
+            uint32_t st = 0, parity = 0, d = 0, d_par = 1;
+            bool ok = true;
+            const uint32_t idesc = (1u << 4) | ((p.n >> 3) << 17) | ((128u * G >> 4) << 24);  // fp16 x fp16 -> fp32
+            const uint64_t desc0 = smem_desc(base, 128);
+            for (uint32_t u = rank == 0 ? first_unit : p.units; u < p.units && ok; u += unit_step) {
+                const PgUnit t = pg_unit(p, u);
+                for (uint32_t k = (t.ks1 - t.ks0) * 4; k > 0; --k) {
+                    if (!(ok = __all_sync(0xffffffffu, bar_wait(d_empty + d * 8, d_par, &dead)))) break;
+                    if (!(ok = __all_sync(0xffffffffu, bar_wait(full + st * 8, parity, &dead)))) break;
+                    fence_after();
+                    const uint64_t da = desc0 + st * (stage_bytes >> 4), db = da + (C::kABytes >> 4);
+                    const uint32_t acc = tmem + d * W;
+                    if (issuer) {
+#pragma unroll
+                        for (uint32_t i = 0; i < 8; ++i) {
+                            const uint64_t a = da + (i & 3) * 2, b = db + (i & 3) * 2 + (i < 4 ? 0 : half_bytes >> 4);
+                            if constexpr (G == 2)
+                                mma_f16_pair(acc, a, b, idesc, i > 0);
+                            else
+                                mma_f16(acc, a, b, idesc, i > 0);
+                        }
+                        if constexpr (G == 2) {
+                            commit_pair(empty + st * 8);
+                            commit_pair(d_full + d * 8);
+                        } else {
+                            commit(empty + st * 8);
+                            commit(d_full + d * 8);
+                        }
+                    }
+                    if (++st == stages) {
+                        st = 0;
+                        parity ^= 1;
+                    }
+                    if (++d == C::kD) {
+                        d = 0;
+                        d_par ^= 1;
+                    }
+                }
+            }
+            if (!ok && issuer) {
+                if constexpr (G == 2)
+                    commit_pair(drained);
+                else
+                    commit(drained);
                 bar_drain(drained, 0);
+            }
+        } else if (G == 2 && warp == 2 && lane == 0 && rank == 1) {
+            // a copy's barrier belongs to the CTA it copies to: tell the issuing CTA
+            uint32_t st = 0, parity = 0;
+            bool ok = true;
+            for (uint32_t u = first_unit; u < p.units && ok; u += unit_step) {
+                const PgUnit t = pg_unit(p, u);
+                for (uint32_t i = (t.ks1 - t.ks0) * 4; i > 0; --i) {
+                    if (!(ok = bar_wait(full + st * 8, parity, &dead))) break;
+                    bar_arrive_cluster(leader_addr(full + st * 8));
+                    if (++st == stages) {
+                        st = 0;
+                        parity ^= 1;
+                    }
+                }
             }
         }
     } else if (warp < 8) {
-        if constexpr (N == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+        if constexpr (W > 64) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
         // Weights do not depend on earlier kernels: no dependency wait. Warp w takes row pair w of the tile; the
         // codes of the super-tile after this one are on their way while this one is unpacked.
         const uint32_t w4 = warp - 4, g = lane >> 2, t4 = lane & 3;
         constexpr uint32_t kVec = DT == 1 ? 4 : 2;
         uint4 q[2][kVec];
-        uint32_t used = 0;
+        uint32_t st = 0, parity = 1;
         bool ok = true;
+        const uint32_t mine = base + (w4 * 32 + g) * 128, report = G == 2 ? leader_addr(full) : full;
+        const uint32_t c0 = ((2 * t4) ^ g) * 16, c1 = ((2 * t4 + 1) ^ g) * 16;
         auto load = [&](const uint8_t *base, bool live, uint32_t tile, uint32_t j) {
             q[tile][j] = live ? __ldg(reinterpret_cast<const uint4 *>(base + tile * Fmt<DT>::kSuperTileBytes + kScaleBytes +
                                                                      j * 512 + lane * 16))
                               : make_uint4(0, 0, 0, 0);
         };
-        for (uint32_t u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-            const PgUnit t = pg_unit<N>(p, u);
-            const uint32_t pair = t.rt * 4 + w4;
+        for (uint32_t u = first_unit; u < p.units && ok; u += unit_step) {
+            const PgUnit t = pg_unit(p, u);
+            const uint32_t pair = (t.rt * G + rank) * 4 + w4;
             const bool live = pair < p.pairs;
-            if (used == 0) {
+            if (u == first_unit) {
                 const uint8_t *first = pg_tile<DT>(p, live ? pair : 0, t.ks0, 0);
 #pragma unroll
                 for (uint32_t j = 0; j < kVec; ++j) {
@@ -214,23 +278,22 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
                 const uint8_t *next;
                 if (ks + 1 < t.ks1) {
                     next = pg_tile<DT>(p, live ? pair : 0, ks + 1, 0);
-                } else if (u + gridDim.x < p.units) {
-                    const PgUnit n = pg_unit<N>(p, u + gridDim.x);
-                    next_live = n.rt * 4 + w4 < p.pairs;
-                    next = pg_tile<DT>(p, next_live ? n.rt * 4 + w4 : 0, n.ks0, 0);
+                } else if (u + unit_step < p.units) {
+                    const PgUnit n = pg_unit(p, u + unit_step);
+                    const uint32_t next_pair = (n.rt * G + rank) * 4 + w4;
+                    next_live = next_pair < p.pairs;
+                    next = pg_tile<DT>(p, next_live ? next_pair : 0, n.ks0, 0);
                 } else {
                     next_live = false;
                     next = p.w;
                 }
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j, ++used) {
-                    const uint32_t a = used % C::kA;
-                    if (used >= C::kA && !__all_sync(0xffffffffu, bar_wait(a_empty + a * 8, (used / C::kA - 1) & 1, &dead))) {
+                for (uint32_t j = 0; j < 4; ++j) {
+                    if (!__all_sync(0xffffffffu, bar_wait(empty + st * 8, parity, &dead))) {
                         ok = false;
                         break;
                     }
-                    const uint32_t row = a_base + a * C::kABytes + (w4 * 32 + g) * 128;
-                    const uint32_t c0 = ((2 * t4) ^ g) * 16, c1 = ((2 * t4 + 1) ^ g) * 16;
+                    const uint32_t row = mine + st * stage_bytes;
 #pragma unroll
                     for (uint32_t tile = 0; tile < 2; ++tile) {
                         const uint32_t r0 = row + tile * 16 * 128, r1 = r0 + 8 * 128;
@@ -250,20 +313,32 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) bar_arrive(a_full + a * 8);
+                    if (lane == 0) {
+                        if constexpr (G == 2)
+                            bar_arrive_cluster(report + st * 8);
+                        else
+                            bar_arrive(report + st * 8);
+                    }
+                    if (++st == stages) {
+                        st = 0;
+                        parity ^= 1;
+                    }
                 }
             }
         }
     } else {
-        if constexpr (N == 256) asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
+        if constexpr (W > 64) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
         pdl_wait();
         const uint32_t quarter = warp & 3, half = (warp - 8) >> 2;  // tensor-memory lanes and columns of this warp
-        const uint32_t src = tmem + half * (N / 2) + ((quarter * 32) << 16);
+        // the two warps of a quarter share its n columns, in chunks of 16
+        const uint32_t first = half ? (p.n + 31) / 32 * 16 : 0, columns = half ? p.n - first : (p.n + 31) / 32 * 16;
+        const uint32_t src = tmem + first + ((quarter * 32) << 16);
         uint32_t used = 0;
+        const uint32_t report = G == 2 ? leader_addr(d_empty) : d_empty;
         bool ok = true;
-        for (uint32_t u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-            const PgUnit t = pg_unit<N>(p, u);
-            const uint32_t pair = t.rt * 4 + quarter, row = t.rt * 128 + quarter * 32 + lane;
+        for (uint32_t u = first_unit; u < p.units && ok; u += unit_step) {
+            const PgUnit t = pg_unit(p, u);
+            const uint32_t pair = (t.rt * G + rank) * 4 + quarter, row = pair * 32 + lane;
             const bool live = pair < p.pairs;
             // scales of this row: four fp16 per super-tile
             const uint32_t sc_off = (lane & 7) * 16 + ((lane >> 3) & 1) * 8;
@@ -272,9 +347,9 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
                            ? __ldg(reinterpret_cast<const uint2 *>(pg_tile<DT>(p, pair, ks, lane >> 4) + sc_off))
                            : make_uint2(0, 0);
             };
-            float acc[N / 2];
+            float acc[W / 2];
 #pragma unroll
-            for (uint32_t i = 0; i < N / 2; ++i) acc[i] = 0.f;
+            for (uint32_t i = 0; i < W / 2; ++i) acc[i] = 0.f;
             uint2 sc = scales(t.ks0);
             for (uint32_t ks = t.ks0; ks < t.ks1 && ok; ++ks) {
                 const uint2 sc_next = scales(ks + 1);
@@ -288,52 +363,81 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
                     fence_after();
                     const uint32_t word = j & 2 ? sc.y : sc.x;
                     const float s = __half2float(__ushort_as_half((uint16_t)(j & 1 ? word >> 16 : word & 0xffff)));
+                    // columns past the tile's belong to the accumulator all the same, and their sums are not stored
+                    constexpr uint32_t kLoad = W > 64 ? 64 : 32;
 #pragma unroll
-                    for (uint32_t c = 0; c < N / 2; c += 32) {
-                        float v[32];
-                        tmem_ld32(src + d * N + c, v);
+                    for (uint32_t c = 0; c < W / 2; c += kLoad) {
+                        if (c >= columns) break;
+                        float v[kLoad];
+                        if constexpr (kLoad == 64)
+                            tmem_ld64(src + d * W + c, v);
+                        else
+                            tmem_ld32(src + d * W + c, v);
                         tmem_ld_wait();
+                        if (c + kLoad >= columns) {  // all of the accumulator is in registers
+                            fence_before();
+                            __syncwarp();
+                            if (lane == 0) {
+                                if constexpr (G == 2)
+                                    bar_arrive_cluster(report + d * 8);
+                                else
+                                    bar_arrive(report + d * 8);
+                            }
+                        }
 #pragma unroll
-                        for (uint32_t i = 0; i < 32; ++i) acc[c + i] = fmaf(s, v[i], acc[c + i]);
+                        for (uint32_t i = 0; i < kLoad; i += 2) pg_fma2(acc + c + i, s, v + i);
                     }
-                    fence_before();
-                    __syncwarp();
-                    if (lane == 0) bar_arrive(d_empty + d * 8);
                 }
                 sc = sc_next;
             }
             if (ok && row < p.rows) {
                 const float so = (p.s_out ? p.s_out[row] : 1.0f) * code_unit(DT);
-                const uint32_t n0 = t.n0 + half * (N / 2);
+                const uint32_t n0 = t.n0 + first;
                 float *y = p.y + t.sp * p.split_stride + (size_t)n0 * p.rows + row;
 #pragma unroll
-                for (uint32_t i = 0; i < N / 2; ++i)
-                    if (n0 + i < p.m) y[(size_t)i * p.rows] = acc[i] * p.unit[n0 + i] * so;
+                for (uint32_t i = 0; i < W / 2; ++i)
+                    if (i < columns && n0 + i < p.m) y[(size_t)i * p.rows] = acc[i] * p.unit[n0 + i] * so;
             }
         }
     }
     __syncwarp();
     __syncthreads();
+    if constexpr (G == 2) cluster_sync();  // no arrival at, and no product from, a CTA that has left
     if (warp == 1) {
         fence_after();
-        tmem_free(tmem, kCols);
+        if constexpr (G == 2)
+            tmem_free_pair(tmem, kCols);
+        else
+            tmem_free(tmem, kCols);
     }
     if (tid == 0 && dead) *p.error_word = DEV_ERR_WAIT_TIMEOUT;
 }
 
 namespace {
 
-template <int DT, uint32_t N>
-ctox_status pg_launch(ctox_ctx *ctx, const PgParams &p) {
-    if constexpr (N == 256) {  // the register split in the kernel counts on 128 per thread at launch
+template <int DT, uint32_t W, uint32_t G>
+ctox_status pg_launch(ctox_ctx *ctx, PgParams &p) {
+    const auto kernel = k_packed_gemm<DT, W, G>;
+    if constexpr (W > 64) {  // the register split in the kernel counts on 128 per thread at launch
         cudaFuncAttributes attr;
-        CTOX_CUDA(ctx, cudaFuncGetAttributes(&attr, k_packed_gemm<DT, N>));
+        CTOX_CUDA(ctx, cudaFuncGetAttributes(&attr, kernel));
         if (attr.numRegs != 128) return fail(ctx, CTOX_INVALID_STATE, "packed product: built with %d registers", attr.numRegs);
     }
-    CTOX_CUDA(ctx, cudaFuncSetAttribute(k_packed_gemm<DT, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PgCfg<N>::kSmem));
-    const uint32_t grid = p.units < (uint32_t)ctx->sm_count ? p.units : (uint32_t)ctx->sm_count;
-    CTOX_CUDA(ctx, launch_pdl(k_packed_gemm<DT, N>, dim3(grid), dim3(kPgThreads), PgCfg<N>::kSmem, ctx->stream, p));
+    const uint32_t stage = PgCfg<W, G>::kABytes + p.n / G * 256;
+    p.stages = ((uint32_t)ctx->max_smem_optin - 2048) / stage;
+    if (p.stages > kPgStages) p.stages = kPgStages;
+    const size_t smem = (size_t)p.stages * stage + 1024;
+    CTOX_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024));
+    const uint32_t slots = (uint32_t)ctx->sm_count / G, grid = (p.units < slots ? p.units : slots) * G;
+    if constexpr (G == 2)
+        CTOX_CUDA(ctx, launch_pdl_cluster(kernel, dim3(grid), dim3(kPgThreads), smem, ctx->stream, 2, p));
+    else
+        CTOX_CUDA(ctx, launch_pdl(kernel, dim3(grid), dim3(kPgThreads), smem, ctx->stream, p));
     return CTOX_OK;
+}
+template <int DT>
+ctox_status pg_launch(ctox_ctx *ctx, PgParams &p) {
+    return p.n > 128 ? pg_launch<DT, 256, 2>(ctx, p) : p.n > 64 ? pg_launch<DT, 128, 1>(ctx, p) : pg_launch<DT, 64, 1>(ctx, p);
 }
 
 }  // namespace
@@ -342,7 +446,7 @@ ctox_status launch_packed_gemm(ctox_matvec *mv, const LongIn &in, uint32_t m, ui
                                size_t capacity, LongOut *out) {
     ctox_ctx *ctx = mv->ctx;
     const MatvecPart &part = mv->parts[0];
-    if (mv->parts.size() != 1 || m == 0 || m > in.pos_pad || in.pos_pad % kLongPosTile || row_end > mv->rows ||
+    if (mv->parts.size() != 1 || m == 0 || row_end > mv->rows ||
         (size_t)m * mv->rows > capacity)
         return fail(ctx, CTOX_SHAPE, "packed product: %u positions of a %llu-row matrix", m, (unsigned long long)mv->rows);
     PgParams p{};
@@ -361,31 +465,32 @@ ctox_status launch_packed_gemm(ctox_matvec *mv, const LongIn &in, uint32_t m, ui
     p.kst = part.kst_s * part.slices;
     p.error_word = ctx->dev_error;
     const uint32_t row_tiles = (uint32_t)((row_end + 127) / 128) - p.rt0;
-    // Tile width and column split by the time of the longest chain of units on an SM: a 64-column block takes
-    // `step` (measured, in units of a block of 256 positions), a unit `start` more for filling its pipeline and
-    // writing its sums. A split is only as good as the extra partial sums its consumer reads.
-    uint32_t best_n = 0;
+    // Tile width and column split by the time of the longest chain of units on an SM, from what a 64-column block of n
+    // positions was measured to take (us, one B200, 999 and 37 positions, four matrix shapes): 0.56 at 48, 0.60 at 96,
+    // 0.64 at 128 (one CTA); 0.76 at 160, 0.90 at 256 (a pair). A unit costs about a microsecond more for filling its
+    // pipeline and writing its sums; a partial sum beyond the first is written and read again at about 5 TB/s.
     double best = 1e30;
-    for (uint32_t n : {64u, 128u, 256u}) {
-        const double step = n == 256 ? 1.0 : n == 128 ? 0.6 : 0.4, start = n == 256 ? 6.0 : n == 128 ? 5.0 : 4.0;
-        const uint32_t tiles = (m + n - 1) / n;
+    for (uint32_t n = 32; n <= 256; n += n < 128 ? 16 : 32) {
+        const uint32_t G = n > 128 ? 2 : 1, slots = (uint32_t)ctx->sm_count / G;
+        const double step = G == 2 ? 0.53 + 0.00146 * n : 0.52 + 0.0009 * n;
+        const uint32_t tiles = (m + n - 1) / n, tiles_r = (row_tiles + G - 1) / G;
+        if (tiles * n > in.pos_pad || p.rt0 % G) continue;
         for (uint32_t s = 1; s <= p.kst && s <= 16 && s * p.split_stride <= capacity; ++s) {
-            const uint32_t units = row_tiles * tiles * s, rounds = (units + ctx->sm_count - 1) / ctx->sm_count;
-            const double cost = rounds * (((p.kst + s - 1) / s) * 4 * step + start) + (s - 1) * 2.0;
+            const uint32_t units = tiles_r * tiles * s, rounds = (units + slots - 1) / slots;
+            const double cost = rounds * (((p.kst + s - 1) / s) * 4 * step + 1.0) + (s - 1) * (0.5 + 1.6e-6 * p.split_stride);
             if (cost < best) {
                 best = cost;
-                best_n = n;
+                p.n = n;
                 p.splits = s;
+                p.units = units;
             }
         }
     }
-    p.pos_tiles = (m + best_n - 1) / best_n;
-    p.units = row_tiles * p.pos_tiles * p.splits;
+    if (p.n == 0) return fail(ctx, CTOX_SHAPE, "packed product: %u positions exceed the buffer's %u", m, in.pos_pad);
+    p.pos_tiles = (m + p.n - 1) / p.n;
+    if (p.n > 128) p.rt0 /= 2;
     timing_begin(ctx);
-    if (part.dt)
-        EX(best_n == 256 ? (pg_launch<1, 256>(ctx, p)) : best_n == 128 ? (pg_launch<1, 128>(ctx, p)) : (pg_launch<1, 64>(ctx, p)));
-    else
-        EX(best_n == 256 ? (pg_launch<0, 256>(ctx, p)) : best_n == 128 ? (pg_launch<0, 128>(ctx, p)) : (pg_launch<0, 64>(ctx, p)));
+    EX(part.dt ? pg_launch<1>(ctx, p) : pg_launch<0>(ctx, p));
     timing_end(ctx, KC_GEMM, (double)part.prep_bytes + 4.0 * m * ((double)mv->columns + mv->rows),
                2.0 * (double)(row_end - row0) * (double)mv->columns * m);
     *out = LongOut{y, p.rows, p.splits, p.split_stride};

@@ -11,14 +11,14 @@ namespace ctox {
 
 // Activations of a long pass: hi and lo fp16 parts of x * s_in / unit[position], one power-of-two unit per
 // position, as [block of 64 columns][part: hi, lo][position][128 bytes]. The columns of a row are in the
-// slot order of inv_perm (layout.cuh), its 16-byte chunks XOR-swizzled by position & 7, so that any 64, 128
-// or 256 positions of a block are a ready shared-memory operand and one contiguous copy.
+// slot order of inv_perm (layout.cuh), its 16-byte chunks XOR-swizzled by position & 7, so that any run of
+// positions that starts at a multiple of eight is a ready shared-memory operand and one contiguous copy.
 struct LongIn {
     uint8_t *x;
     float *unit;
-    uint32_t pos_pad;  // positions of a block's row of the buffer: a multiple of kLongPosTile
+    uint32_t pos_pad;  // positions of a block's row of the buffer (a multiple of eight): those of the pass and a tile
 };
-constexpr uint32_t kLongPosTile = 256;
+constexpr uint32_t kLongPosTile = 256;  // widest tile of positions
 inline size_t long_in_bytes(uint32_t blocks_padded, uint32_t pos_pad) { return (size_t)blocks_padded * 2 * pos_pad * 128; }
 
 // Output of such a product: `splits` partial sums [position][rows], to be added up in index order.
