@@ -1,12 +1,14 @@
 // Persistent tensor-core product for long passes: one CTA per SM, 128 x BN tiles, operands staged by TMA
 // (one thread), multiplied by tcgen05.mma (one thread), accumulators double-buffered in tensor memory so
-// that four epilogue warps drain a tile while the next one is computed.
+// that four epilogue warps drain a tile while the next one is computed. Large products take pairs of CTAs
+// (G = 2, cta_group::2): 256 x 256 tiles, each CTA with half of the rows of either operand, so that an SM draws 32
+// instead of 48 KB from L2 per 512 cycles of tensor work.
 #include "gemm.cuh"
 #include "umma.cuh"
 
 namespace ctox {
 
-constexpr int kGmThreads = 192;  // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue
+constexpr int kGmThreads = 224;  // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue, warp 6: reports copies to the pair's first CTA
 constexpr uint32_t kGmM = 128, kGmK = 64, kGmStageMax = 8;
 
 ctox_status tensor_map_bf16(ctox_ctx *ctx, CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint64_t ld,
@@ -125,101 +127,156 @@ __device__ __forceinline__ void gemm_store(const GemmOut &o, float *v, uint32_t 
     }
 }
 
-template <uint32_t BN>
+template <uint32_t BN, uint32_t G>
 __global__ void __launch_bounds__(kGmThreads, 1)
     k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmPages pa, GemmPages pb,
            uint32_t M, uint32_t N, uint32_t K, uint32_t stages, GemmOut out, int32_t *error_word) {
     using namespace umma;
-    constexpr uint32_t kABytes = kGmM * kGmK * 2, kBBytes = BN * kGmK * 2, kBBox = BN < 128 ? BN : 128;
-    constexpr uint32_t kCols = 2 * BN < 32 ? 32 : 2 * BN;
+    constexpr uint32_t kBRows = BN / G, kABytes = kGmM * kGmK * 2, kBBytes = kBRows * kGmK * 2;  // of this CTA
+    constexpr uint32_t kBBox = kBRows < 128 ? kBRows : 128, kBoxes = kBRows / kBBox;
+    constexpr uint32_t kCols = 2 * BN;
     extern __shared__ uint8_t raw[];
     __shared__ __align__(8) uint64_t bars[2 * kGmStageMax + 5];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int dead;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = G == 2 ? cluster_rank() : 0;
     const uint32_t base = (smem_addr(raw) + 1023) & ~1023u;
     const uint32_t full = smem_addr(bars), empty = full + kGmStageMax * 8, acc_full = empty + kGmStageMax * 8,
                    acc_empty = acc_full + 16, drained = acc_empty + 16;
     if (tid == 0) {
         dead = 0;
         for (uint32_t i = 0; i < stages; ++i) {
-            bar_init(full + i * 8, 1);
+            bar_init(full + i * 8, G == 2 && rank == 0 ? 2 : 1);  // own copies, and the report of the other CTA's
             bar_init(empty + i * 8, 1);
         }
         for (uint32_t i = 0; i < 2; ++i) {
             bar_init(acc_full + i * 8, 1);
-            bar_init(acc_empty + i * 8, 4);
+            bar_init(acc_empty + i * 8, 4 * G);
         }
         bar_init(drained, 1);
         bar_init_fence();
         tma_prefetch_map(&map_a);
         tma_prefetch_map(&map_b);
     }
-    if (warp == 1) tmem_alloc(smem_addr(&tmem_slot), kCols);
+    if (warp == 1) {
+        if constexpr (G == 2)
+            tmem_alloc_pair(smem_addr(&tmem_slot), kCols);
+        else
+            tmem_alloc(smem_addr(&tmem_slot), kCols);
+    }
     fence_before();
     __syncthreads();
+    if constexpr (G == 2) cluster_sync();  // the other CTA's barriers are ready
     fence_after();
     pdl_launch();  // a later kernel's allocation must not come before this one's (see umma.cuh)
     const uint32_t tmem = tmem_slot;
-    const uint32_t tiles_m = (M + kGmM - 1) / kGmM, tiles_n = (N + BN - 1) / BN, tiles = tiles_m * tiles_n;
-    const uint32_t ksteps = (K + kGmK - 1) / kGmK;
+    const uint32_t tiles_m = (M + kGmM * G - 1) / (kGmM * G), tiles_n = (N + BN - 1) / BN, tiles = tiles_m * tiles_n;
+    const uint32_t ksteps = (K + kGmK - 1) / kGmK, first = blockIdx.x / G, step = gridDim.x / G;
     pdl_wait();
     if (warp == 0) {
         if (lane == 0) {
-            uint32_t issued = 0;
+            uint32_t issued = 0, s = 0, parity = 1;  // parity of the phase before a ring's first: passes at once
             bool ok = true;
-            for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-                const uint32_t m0 = t % tiles_m * kGmM, n0 = t / tiles_m * BN;
-                const int ra = operand_row(pa, m0);
-                int rb[(BN + 127) / 128];
+            for (uint32_t t = first; t < tiles && ok; t += step) {
+                const uint32_t m0 = (t % tiles_m * G + rank) * kGmM, n0 = t / tiles_m * BN + rank * kBRows;
+                const int ra = m0 < M ? operand_row(pa, m0) : (int)m0;
+                int rb[kBoxes];
 #pragma unroll
-                for (uint32_t i = 0; i < (BN + 127) / 128; ++i) rb[i] = n0 + i * 128 < N ? operand_row(pb, n0 + i * 128) : (int)(n0 + i * 128);
+                for (uint32_t i = 0; i < kBoxes; ++i) rb[i] = n0 + i * 128 < N ? operand_row(pb, n0 + i * 128) : (int)(n0 + i * 128);
                 for (uint32_t k = 0; k < ksteps; ++k, ++issued) {
-                    const uint32_t s = issued % stages, round = issued / stages;
-                    if (round > 0 && !(ok = bar_wait(empty + s * 8, (round - 1) & 1, &dead))) break;
+                    if (!(ok = bar_wait(empty + s * 8, parity, &dead))) break;
                     const uint32_t bar = full + s * 8, dst = base + s * (kABytes + kBBytes);
                     bar_expect(bar, kABytes + kBBytes);
                     tma_load(dst, &map_a, bar, (int)(k * kGmK), ra);
 #pragma unroll
-                    for (uint32_t i = 0; i < (BN + 127) / 128; ++i)
+                    for (uint32_t i = 0; i < kBoxes; ++i)
                         tma_load(dst + kABytes + i * kBBox * kGmK * 2, &map_b, bar, (int)(k * kGmK), rb[i]);
+                    if (++s == stages) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
             }
-            if (!ok) {  // leave no copy in flight behind
-                for (uint32_t s = 0; s < stages && s < issued; ++s) bar_drain(full + s * 8, ((issued - 1 - s) / stages) & 1);
+            if (!ok) {  // leave no copy in flight behind; the first CTA of a pair may lack the other's report, so by time
+                if constexpr (G == 2) {
+                    const long long t0 = clock64();
+                    while (clock64() - t0 < 2000000) {
+                    }
+                } else {
+                    for (uint32_t i = 0; i < stages && i < issued; ++i)
+                        bar_drain(full + (issued - 1 - i) % stages * 8, ((issued - 1 - i) / stages) & 1);
+                }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t used = 0, n_tile = 0;
-            bool ok = true;
-            const uint32_t idesc = idesc_bf16(kGmM, BN);
-            for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++n_tile) {
-                const uint32_t acc = n_tile & 1, d = tmem + acc * BN;
-                if (n_tile >= 2 && !(ok = bar_wait(acc_empty + acc * 8, ((n_tile >> 1) - 1) & 1, &dead))) break;
+        // The whole warp runs the loop and one lane issues: its values are uniform, so that descriptors need no moves
+        // between register files. The second CTA of a pair issues nothing.
+        const bool issuer = elect_one();
+        uint32_t s = 0, parity = 0, n_tile = 0;
+        bool ok = true;
+        const uint32_t idesc = idesc_bf16(kGmM * G, BN);
+        const uint64_t desc0 = smem_desc(base, 128);
+        for (uint32_t t = rank == 0 ? first : tiles; t < tiles && ok; t += step, ++n_tile) {
+            const uint32_t acc = n_tile & 1, d = tmem + acc * BN;
+            if (!(ok = __all_sync(0xffffffffu, bar_wait(acc_empty + acc * 8, ((n_tile >> 1) & 1) ^ 1, &dead)))) break;
+            fence_after();
+            for (uint32_t k = 0; k < ksteps; ++k) {
+                if (!(ok = __all_sync(0xffffffffu, bar_wait(full + s * 8, parity, &dead)))) break;
                 fence_after();
-                for (uint32_t k = 0; k < ksteps; ++k, ++used) {
-                    const uint32_t s = used % stages;
-                    if (!(ok = bar_wait(full + s * 8, (used / stages) & 1, &dead))) break;
-                    fence_after();
-                    const uint32_t src = base + s * (kABytes + kBBytes);
-                    const uint64_t da = smem_desc(src, 128), db = smem_desc(src + kABytes, 128);
+                const uint64_t da = desc0 + s * ((kABytes + kBBytes) >> 4), db = da + (kABytes >> 4);
+                if (issuer) {
 #pragma unroll
-                    for (uint32_t i = 0; i < kGmK / 16; ++i) mma_f16(d, da + i * 2, db + i * 2, idesc, k > 0 || i > 0);
-                    commit(empty + s * 8);
+                    for (uint32_t i = 0; i < kGmK / 16; ++i) {
+                        if constexpr (G == 2)
+                            mma_f16_pair(d, da + i * 2, db + i * 2, idesc, k > 0 || i > 0);
+                        else
+                            mma_f16(d, da + i * 2, db + i * 2, idesc, k > 0 || i > 0);
+                    }
+                    if constexpr (G == 2)
+                        commit_pair(empty + s * 8);
+                    else
+                        commit(empty + s * 8);
                 }
-                if (ok) commit(acc_full + acc * 8);
+                if (++s == stages) {
+                    s = 0;
+                    parity ^= 1;
+                }
             }
-            if (!ok) {
+            if (ok && issuer) {
+                if constexpr (G == 2)
+                    commit_pair(acc_full + acc * 8);
+                else
+                    commit(acc_full + acc * 8);
+            }
+        }
+        if (!ok && issuer) {
+            if constexpr (G == 2)
+                commit_pair(drained);
+            else
                 commit(drained);
-                bar_drain(drained, 0);
-            }
+            bar_drain(drained, 0);
+        }
+    } else if (warp == 6) {
+        if (G == 2 && rank == 1 && lane == 0) {  // a copy's barrier is in the CTA it copies to: tell the issuing CTA
+            uint32_t s = 0, parity = 0;
+            bool ok = true;
+            for (uint32_t t = first; t < tiles && ok; t += step)
+                for (uint32_t k = 0; k < ksteps; ++k) {
+                    if (!(ok = bar_wait(full + s * 8, parity, &dead))) break;
+                    bar_arrive_cluster(leader_addr(full + s * 8));
+                    if (++s == stages) {
+                        s = 0;
+                        parity ^= 1;
+                    }
+                }
         }
     } else {
         const uint32_t quarter = warp & 3;  // the lanes of tensor memory this warp may read
+        const uint32_t report = G == 2 ? leader_addr(acc_empty) : acc_empty;
         uint32_t n_tile = 0;
-        for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, ++n_tile) {
-            const uint32_t acc = n_tile & 1, m = t % tiles_m * kGmM + quarter * 32 + lane, n0 = t / tiles_m * BN;
+        for (uint32_t t = first; t < tiles; t += step, ++n_tile) {
+            const uint32_t acc = n_tile & 1, m = (t % tiles_m * G + rank) * kGmM + quarter * 32 + lane, n0 = t / tiles_m * BN;
             if (!__all_sync(0xffffffffu, bar_wait(acc_full + acc * 8, (n_tile >> 1) & 1, &dead))) break;
             fence_after();
             const uint32_t src = tmem + acc * BN + ((quarter * 32) << 16);
@@ -232,23 +289,32 @@ __global__ void __launch_bounds__(kGmThreads, 1)
             }
             fence_before();
             __syncwarp();
-            if (lane == 0) bar_arrive(acc_empty + acc * 8);
+            if (lane == 0) {
+                if constexpr (G == 2)
+                    bar_arrive_cluster(report + acc * 8);
+                else
+                    bar_arrive(report + acc * 8);
+            }
         }
     }
     __syncwarp();
     __syncthreads();
+    if constexpr (G == 2) cluster_sync();  // no arrival at, and no product from, a CTA that has left
     if (warp == 1) {
         fence_after();
-        tmem_free(tmem, kCols);
+        if constexpr (G == 2)
+            tmem_free_pair(tmem, kCols);
+        else
+            tmem_free(tmem, kCols);
     }
     if (tid == 0 && dead) *error_word = DEV_ERR_WAIT_TIMEOUT;
 }
 
 namespace {
 
-template <uint32_t BN>
+template <uint32_t BN, uint32_t G>
 ctox_status gemm_launch(ctox_ctx *ctx, const GemmOperand &a, const GemmOperand &b, const GemmOut &out) {
-    const uint32_t stage_bytes = kGmM * kGmK * 2 + BN * kGmK * 2;
+    const uint32_t stage_bytes = kGmM * kGmK * 2 + BN / G * kGmK * 2;
     uint32_t stages = ((uint32_t)ctx->max_smem_optin - 2048) / stage_bytes;
     if (stages > kGmStageMax) stages = kGmStageMax;
     const size_t smem = (size_t)stages * stage_bytes + 1024;
@@ -257,14 +323,18 @@ ctox_status gemm_launch(ctox_ctx *ctx, const GemmOperand &a, const GemmOperand &
         return tensor_map_bf16(ctx, m, o.p, o.page_table ? o.store_rows : o.rows, o.cols, o.ld, box, kGmK);
     };
     ctox_status rc = encode(&ma, a, kGmM);
-    if (!rc) rc = encode(&mb, b, BN < 128 ? BN : 128);
+    if (!rc) rc = encode(&mb, b, BN / G < 128 ? BN / G : 128);
     if (rc) return rc;
-    CTOX_CUDA(ctx, cudaFuncSetAttribute(k_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const uint32_t tiles = ((a.rows + kGmM - 1) / kGmM) * ((b.rows + BN - 1) / BN);
-    const uint32_t grid = tiles < (uint32_t)ctx->sm_count ? tiles : (uint32_t)ctx->sm_count;
-    CTOX_CUDA(ctx, launch_pdl(k_gemm<BN>, dim3(grid), dim3(kGmThreads), smem, ctx->stream, ma, mb,
-                              GemmPages{a.page_table, a.page_tokens, a.row0}, GemmPages{b.page_table, b.page_tokens, b.row0},
-                              a.rows, b.rows, a.cols, stages, out, ctx->dev_error));
+    CTOX_CUDA(ctx, cudaFuncSetAttribute(k_gemm<BN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const uint32_t tiles = ((a.rows + kGmM * G - 1) / (kGmM * G)) * ((b.rows + BN - 1) / BN);
+    const uint32_t slots = (uint32_t)ctx->sm_count / G, grid = (tiles < slots ? tiles : slots) * G;
+    const GemmPages pa{a.page_table, a.page_tokens, a.row0}, pb{b.page_table, b.page_tokens, b.row0};
+    if constexpr (G == 2)
+        CTOX_CUDA(ctx, launch_pdl_cluster(k_gemm<BN, G>, dim3(grid), dim3(kGmThreads), smem, ctx->stream, 2, ma, mb, pa, pb,
+                                          a.rows, b.rows, a.cols, stages, out, ctx->dev_error));
+    else
+        CTOX_CUDA(ctx, launch_pdl(k_gemm<BN, G>, dim3(grid), dim3(kGmThreads), smem, ctx->stream, ma, mb, pa, pb, a.rows, b.rows,
+                                  a.cols, stages, out, ctx->dev_error));
     return CTOX_OK;
 }
 
@@ -276,19 +346,22 @@ ctox_status launch_gemm(ctox_ctx *ctx, const GemmOperand &a, const GemmOperand &
     for (const GemmOperand *o : {&a, &b})
         if (o->page_table && (o->page_tokens % 128 || o->row0 % 128))
             return fail(ctx, CTOX_SHAPE, "gemm: pages of %u tokens are not whole tiles", o->page_tokens);
-    // tile width by rounds over the SMs; a narrower tile has less reuse, hence the constant
+    // tile by rounds over the SMs (an SM's work per round, in columns); a narrower tile has less reuse, hence the constant
     uint32_t best = 0, best_cost = 0xffffffffu;
-    for (uint32_t bn : {256u, 128u, 64u}) {
-        const uint32_t tiles = ((a.rows + kGmM - 1) / kGmM) * ((b.rows + bn - 1) / bn);
-        const uint32_t cost = ((tiles + ctx->sm_count - 1) / ctx->sm_count) * (bn + 64);
+    for (uint32_t bn : {512u, 256u, 128u, 64u}) {  // 512: a pair's 256 x 256
+        const uint32_t G = bn == 512 ? 2 : 1, w = bn == 512 ? 256 : bn, slots = (uint32_t)ctx->sm_count / G;
+        const uint32_t tiles = ((a.rows + kGmM * G - 1) / (kGmM * G)) * ((b.rows + w - 1) / w);
+        const uint32_t cost = ((tiles + slots - 1) / slots) * (G == 2 ? 270 : w + 64);
         if (cost < best_cost) {
             best_cost = cost;
             best = bn;
         }
     }
     timing_begin(ctx);
-    EX(best == 256 ? gemm_launch<256>(ctx, a, b, out) : best == 128 ? gemm_launch<128>(ctx, a, b, out)
-                                                                   : gemm_launch<64>(ctx, a, b, out));
+    EX(best == 512   ? (gemm_launch<256, 2>(ctx, a, b, out))
+       : best == 256 ? (gemm_launch<256, 1>(ctx, a, b, out))
+       : best == 128 ? (gemm_launch<128, 1>(ctx, a, b, out))
+                     : (gemm_launch<64, 1>(ctx, a, b, out)));
     timing_end(ctx, KC_GEMM, 2.0 * ((double)a.rows + b.rows) * a.cols + (out.bf16 ? 2.0 : 4.0) * a.rows * b.rows,
                2.0 * a.rows * b.rows * a.cols);
     return CTOX_OK;
