@@ -57,113 +57,7 @@ __device__ __forceinline__ void merge_stat(NodeStat &a, const NodeStat &b) {
     }
 }
 
-// One sweep over the vocabulary rows for the `npos` positions of the current pass.
-__global__ void __launch_bounds__(kHeadThreads) k_head_stats(
-    const float *__restrict__ partial, const uint8_t *__restrict__ pieces, const float *__restrict__ s_out,
-    const float *__restrict__ bias, uint32_t rows, uint32_t slices, uint32_t max_pieces, uint32_t node0,
-    uint32_t npos,
-    float inv_temperature, unsigned long long seed, unsigned long long step, TreeDesc tree,
-    NodeStat *__restrict__ cta_stats, float *__restrict__ child_z, float *__restrict__ logits_out,
-    unsigned long long logits_stride, uint32_t row_offset, const float *__restrict__ plain) {
-    pdl_launch();
-    pdl_wait();
-    __shared__ NodeStat sh[kHeadThreads / 32][kMaxPosPerPass];
-    NodeStat st[kMaxPosPerPass];
-#pragma unroll
-    for (int m = 0; m < kMaxPosPerPass; ++m) st[m] = NodeStat{0ull, 0ull, 0.f, 0.f, 0u, 0u};
-    for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
-        const uint32_t pr = row / kPairRows, rl = row % kPairRows;
-        float lg[kMaxPosPerPass];
-#pragma unroll
-        for (int m = 0; m < kMaxPosPerPass; ++m)
-            lg[m] = plain && (uint32_t)m < npos ? plain[(size_t)m * logits_stride + row] : 0.f;
-        for (uint32_t sl = 0; sl < slices; ++sl) {  // no slices when the logits are given
-            // a slot is [position][32 rows]: the 32 rows of a pair are one coalesced line per position
-            const float *base = partial + ((size_t)pr * slices + sl) * max_pieces * (kPairRows * kMaxPosPerPass) + rl;
-            const uint32_t n = pieces[pr * slices + sl];
-            for (uint32_t q = 0; q < n; ++q) {
-                const float *sl_q = base + q * (kPairRows * kMaxPosPerPass);
-#pragma unroll
-                for (int m = 0; m < kMaxPosPerPass; ++m)
-                    if ((uint32_t)m < npos) lg[m] += sl_q[m * kPairRows];
-            }
-        }
-        const float so = s_out ? s_out[row] : 1.0f, bi = bias ? bias[row] : 0.0f;
-#pragma unroll
-        for (int m = 0; m < kMaxPosPerPass; ++m) lg[m] = (lg[m] + bi) * so;
-#pragma unroll
-        for (int m = 0; m < kMaxPosPerPass; ++m) {
-            if ((uint32_t)m >= npos) break;
-            const uint32_t node = node0 + m;
-            const float logit = lg[m];
-            if (logits_out) logits_out[(size_t)node * logits_stride + row] = logit;
-            if (!isfinite(logit)) {
-                st[m].nonfinite = 1;
-                continue;
-            }
-            const uint32_t token = row + row_offset;  // rows of a vocabulary shard start at row_offset
-            const unsigned long long pk = pack_key_index(logit, token);
-            st[m].argmax = pk > st[m].argmax ? pk : st[m].argmax;
-            if (inv_temperature > 0.f) {
-                const float z = logit * inv_temperature;
-                if (st[m].sum > 0.f) {
-                    if (z > st[m].max) {
-                        st[m].sum = st[m].sum * expf(st[m].max - z) + 1.0f;
-                        st[m].max = z;
-                    } else {
-                        st[m].sum += expf(z - st[m].max);
-                    }
-                } else {
-                    st[m].max = z;
-                    st[m].sum = 1.0f;
-                }
-                bool is_child = false;
-                for (uint32_t c = node + 1; c < tree.n_nodes; ++c)
-                    if ((uint32_t)tree.parent[c] == node && tree.token[c] == token) {
-                        is_child = true;
-                        child_z[c] = z;  // one writer: the row is unique
-                    }
-                if (!is_child) {
-                    const unsigned long long gk = pack_key_index(z + gumbel_noise(seed, step, node, token), token);
-                    st[m].gumbel = gk > st[m].gumbel ? gk : st[m].gumbel;
-                }
-            }
-        }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int m = 0; m < kMaxPosPerPass; ++m) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            NodeStat other;
-            other.argmax = __shfl_xor_sync(0xffffffffu, st[m].argmax, o);
-            other.gumbel = __shfl_xor_sync(0xffffffffu, st[m].gumbel, o);
-            other.max = __shfl_xor_sync(0xffffffffu, st[m].max, o);
-            other.sum = __shfl_xor_sync(0xffffffffu, st[m].sum, o);
-            other.nonfinite = __shfl_xor_sync(0xffffffffu, st[m].nonfinite, o);
-            merge_stat(st[m], other);
-        }
-        if (lane == 0) sh[warp][m] = st[m];
-    }
-    __syncthreads();
-    if (threadIdx.x < kMaxPosPerPass) {
-        NodeStat a = sh[0][threadIdx.x];
-        for (int w = 1; w < kHeadThreads / 32; ++w) merge_stat(a, sh[w][threadIdx.x]);
-        cta_stats[(size_t)blockIdx.x * kMaxPosPerPass + threadIdx.x] = a;
-    }
-}
-
-// Merges the per-CTA statistics of one pass into node_stats[node0 .. node0+npos): one warp per
-// position, lanes stride over the CTAs, then a butterfly (max/sum merges are order-insensitive up
-// to rounding; the lane order is fixed, so the result is reproducible).
-__global__ void k_head_merge(const NodeStat *__restrict__ cta_stats, uint32_t n_ctas, uint32_t node0,
-                             uint32_t npos, NodeStat *__restrict__ node_stats) {
-    pdl_launch();
-    pdl_wait();
-    const uint32_t m = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (m >= npos) return;
-    NodeStat a{0ull, 0ull, 0.f, 0.f, 0u, 0u};
-    for (uint32_t c = lane; c < n_ctas; c += 32) merge_stat(a, cta_stats[(size_t)c * kMaxPosPerPass + m]);
+__device__ __forceinline__ void warp_merge(NodeStat &a) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         NodeStat other;
@@ -174,6 +68,137 @@ __global__ void k_head_merge(const NodeStat *__restrict__ cta_stats, uint32_t n_
         other.nonfinite = __shfl_xor_sync(0xffffffffu, a.nonfinite, o);
         merge_stat(a, other);
     }
+}
+
+// One sweep over the vocabulary rows: blockIdx.y = position of the current pass, four consecutive rows per thread and
+// trip. Bound by arithmetic (Philox and two logarithms per logit where a temperature is set): one position per CTA
+// keeps one set of statistics in registers, and the four rows' noise comes from one Philox block where their tokens share a
+// counter. (All positions of a row in one thread, a Philox block per logit: 50 us for 8 x 248320 logits.)
+__global__ void __launch_bounds__(kHeadThreads) k_head_stats(
+    const float *__restrict__ partial, const uint8_t *__restrict__ pieces, const float *__restrict__ s_out,
+    const float *__restrict__ bias, uint32_t rows, uint32_t slices, uint32_t max_pieces, uint32_t node0,
+    float inv_temperature, unsigned long long seed, unsigned long long step, const __grid_constant__ TreeDesc tree,
+    NodeStat *__restrict__ cta_stats, float *__restrict__ child_z, float *__restrict__ logits_out,
+    unsigned long long logits_stride, uint32_t row_offset, const float *__restrict__ plain) {
+    pdl_launch();
+    pdl_wait();
+    __shared__ NodeStat sh[kHeadThreads / 32];
+    __shared__ uint32_t child_token[kMaxNodes], child_node[kMaxNodes], children;
+    const uint32_t m = blockIdx.y, node = node0 + m;
+    if (threadIdx.x == 0) {
+        uint32_t n = 0;
+        for (uint32_t c = node + 1; c < tree.n_nodes; ++c)
+            if ((uint32_t)tree.parent[c] == node) {
+                child_node[n] = c;
+                child_token[n++] = tree.token[c];
+            }
+        children = n;
+    }
+    __syncthreads();
+    float *out = logits_out ? logits_out + (size_t)node * logits_stride : nullptr;
+    const bool vec_out = out && ((uintptr_t)out & 15) == 0;
+    NodeStat st{0ull, 0ull, 0.f, 0.f, 0u, 0u};
+    for (uint32_t row0 = (blockIdx.x * kHeadThreads + threadIdx.x) * 4; row0 < rows; row0 += gridDim.x * kHeadThreads * 4) {
+        float lg[4] = {0.f, 0.f, 0.f, 0.f};
+        if (plain) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i)
+                if (row0 + i < rows) lg[i] = plain[(size_t)m * logits_stride + row0 + i];
+        }
+        const uint32_t pr = row0 / kPairRows, rl = row0 % kPairRows;
+        for (uint32_t sl = 0; sl < slices; ++sl) {  // no slices when the logits are given
+            // a slot is [position][32 rows]
+            const float *base = partial + ((size_t)pr * slices + sl) * max_pieces * (kPairRows * kMaxPosPerPass) +
+                                m * kPairRows + rl;
+            const uint32_t n = pieces[pr * slices + sl];
+            for (uint32_t q = 0; q < n; ++q) {
+                const float4 v = *reinterpret_cast<const float4 *>(base + q * (kPairRows * kMaxPosPerPass));
+                lg[0] += v.x;
+                lg[1] += v.y;
+                lg[2] += v.z;
+                lg[3] += v.w;
+            }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i)
+            if (row0 + i < rows) lg[i] = (lg[i] + (bias ? bias[row0 + i] : 0.0f)) * (s_out ? s_out[row0 + i] : 1.0f);
+        if (vec_out && row0 + 4 <= rows)
+            *reinterpret_cast<float4 *>(out + row0) = make_float4(lg[0], lg[1], lg[2], lg[3]);
+        uint4 noise = make_uint4(0u, 0u, 0u, 0u);
+        uint32_t counter = 0xffffffffu;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            const uint32_t row = row0 + i;
+            if (row >= rows) continue;
+            const float logit = lg[i];
+            if (out && !(vec_out && row0 + 4 <= rows)) out[row] = logit;
+            if (!isfinite(logit)) {
+                st.nonfinite = 1;
+                continue;
+            }
+            const uint32_t token = row + row_offset;  // rows of a vocabulary shard start at row_offset
+            const unsigned long long pk = pack_key_index(logit, token);
+            st.argmax = pk > st.argmax ? pk : st.argmax;
+            if (inv_temperature > 0.f) {
+                const float z = logit * inv_temperature;
+                if (st.sum > 0.f) {
+                    if (z > st.max) {
+                        st.sum = st.sum * expf(st.max - z) + 1.0f;
+                        st.max = z;
+                    } else {
+                        st.sum += expf(z - st.max);
+                    }
+                } else {
+                    st.max = z;
+                    st.sum = 1.0f;
+                }
+                bool is_child = false;
+                for (uint32_t c = 0; c < children; ++c)
+                    if (child_token[c] == token) {
+                        is_child = true;
+                        child_z[child_node[c]] = z;  // one writer: the row is unique
+                    }
+                if (!is_child) {
+                    if ((token >> 2) != counter) {
+                        counter = token >> 2;
+                        noise = gumbel_block(seed, step, node, token);
+                    }
+                    const unsigned long long gk = pack_key_index(z + gumbel_of(noise, token), token);
+                    st.gumbel = gk > st.gumbel ? gk : st.gumbel;
+                }
+            }
+        }
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    warp_merge(st);
+    if (lane == 0) sh[warp] = st;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        NodeStat a = sh[0];
+        for (int w = 1; w < kHeadThreads / 32; ++w) merge_stat(a, sh[w]);
+        cta_stats[(size_t)blockIdx.x * kMaxPosPerPass + m] = a;
+    }
+}
+
+// Merges the per-CTA statistics of one pass into node_stats[node0 .. node0+npos): one warp per
+// position, lanes stride over the CTAs (eight loads at a time), then a butterfly (max/sum merges are
+// order-insensitive up to rounding; the lane order is fixed, so the result is reproducible).
+__global__ void k_head_merge(const NodeStat *__restrict__ cta_stats, uint32_t n_ctas, uint32_t node0,
+                             uint32_t npos, NodeStat *__restrict__ node_stats) {
+    pdl_launch();
+    pdl_wait();
+    const uint32_t m = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (m >= npos) return;
+    NodeStat a{0ull, 0ull, 0.f, 0.f, 0u, 0u};
+    for (uint32_t c0 = lane; c0 < n_ctas; c0 += 256) {
+        NodeStat b[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            b[i] = c0 + i * 32 < n_ctas ? cta_stats[(size_t)(c0 + i * 32) * kMaxPosPerPass + m] : NodeStat{0ull, 0ull, 0.f, 0.f, 0u, 0u};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) merge_stat(a, b[i]);
+    }
+    warp_merge(a);
     if (lane == 0) node_stats[node0 + m] = a;
 }
 
@@ -656,11 +681,13 @@ ctox_status head_stats_enqueue(ctox_ctx *ctx, const ctox_matvec *mv, const float
     tree.token = tokens_dev;
     for (uint32_t i = 0; i < n_nodes; ++i) tree.parent[i] = parent[i];
     const MatvecPart *p = mv ? &mv->parts[0] : nullptr;
-    uint32_t grid = (rows + kHeadThreads - 1) / kHeadThreads;
-    if (grid > kHeadGridMax) grid = kHeadGridMax;
-    launch_pdl(k_head_stats, dim3(grid), dim3(kHeadThreads), 0, ctx->stream, p ? p->partial : nullptr,
+    // four CTAs per SM over all positions (their registers allow no more), each with four rows per thread at least
+    uint32_t grid = (rows + kHeadThreads * 4 - 1) / (kHeadThreads * 4), most = 4 * (uint32_t)ctx->sm_count / npos;
+    if (most > kHeadGridMax) most = kHeadGridMax;
+    if (grid > most) grid = most;
+    launch_pdl(k_head_stats, dim3(grid, npos), dim3(kHeadThreads), 0, ctx->stream, p ? p->partial : nullptr,
                p ? p->split[npos > 4 ? 1 : 0].pieces : nullptr, mv ? mv->s_out : nullptr, mv ? mv->bias : nullptr, rows,
-               p ? p->slices : 0u, p ? p->max_pieces : 0u, node0, npos, inv_t, seed, step, tree, hs.cta_stats, hs.child_z,
+               p ? p->slices : 0u, p ? p->max_pieces : 0u, node0, inv_t, seed, step, tree, hs.cta_stats, hs.child_z,
                logits_out_dev, (unsigned long long)logits_stride, row_offset, plain);
     launch_pdl(k_head_merge, dim3(1), dim3(32 * kMaxPosPerPass), 0, ctx->stream, hs.cta_stats, grid, node0, npos, hs.node_stats);
     CTOX_CUDA(ctx, cudaGetLastError());

@@ -58,12 +58,13 @@ __device__ __forceinline__ float gumbel_from_bits(uint32_t bits) {
     const float u = __fmul_rn(__fadd_rn((float)(bits >> 8), 0.5f), 1.0f / 16777216.0f);
     return -det_ln(-det_ln(u));
 }
-// Counter layout: (token / 4 or 0xffffffff, node, step lo, step hi), key = seed.
-__device__ __forceinline__ float gumbel_noise(uint64_t seed, uint64_t step, uint32_t node, uint32_t token) {
-    const uint4 r = philox4x32_10(make_uint4(token >> 2, node, (uint32_t)step, (uint32_t)(step >> 32)),
-                                  make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
-    const uint32_t w = (token & 3u) == 0 ? r.x : (token & 3u) == 1 ? r.y : (token & 3u) == 2 ? r.z : r.w;
-    return gumbel_from_bits(w);
+// Counter layout: (token / 4 or 0xffffffff, node, step lo, step hi), key = seed. A block serves the four tokens of a counter.
+__device__ __forceinline__ uint4 gumbel_block(uint64_t seed, uint64_t step, uint32_t node, uint32_t token) {
+    return philox4x32_10(make_uint4(token >> 2, node, (uint32_t)step, (uint32_t)(step >> 32)),
+                         make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
+}
+__device__ __forceinline__ float gumbel_of(const uint4 &block, uint32_t token) {
+    return gumbel_from_bits((token & 3u) == 0 ? block.x : (token & 3u) == 1 ? block.y : (token & 3u) == 2 ? block.z : block.w);
 }
 __device__ __forceinline__ float accept_draw(uint64_t seed, uint64_t step, uint32_t node) {
     const uint4 r = philox4x32_10(make_uint4(0xffffffffu, node, (uint32_t)step, (uint32_t)(step >> 32)),
