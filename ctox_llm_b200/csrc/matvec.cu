@@ -35,6 +35,7 @@
 
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 namespace ctox {
@@ -245,6 +246,55 @@ struct StreamParams {
     uint32_t warps_per_slice;  // warps that take work (<= units per slice)
     uint32_t npos, max_pieces;
 };
+// Activations for a launch that forms its own fragments.
+struct StreamInput {
+    const void *x;  // null: fragments are prepared (xfrag, meta)
+    const float *s_in;
+    long long stride;
+    uint32_t columns;
+    int bf16, vec;  // vec: rows are aligned for loads of four values
+};
+// The matrices of one launch; matrix i takes the CTAs from first_cta[i] on.
+constexpr int kStreamItems = 4;
+struct StreamArgs {
+    StreamParams item[kStreamItems];
+    uint32_t first_cta[kStreamItems];
+    uint32_t items;
+    StreamInput in;
+};
+
+__device__ __forceinline__ const StreamParams &stream_item(const StreamParams &p, uint32_t) { return p; }
+__device__ __forceinline__ const StreamParams &stream_item(const StreamArgs &a, uint32_t i) { return a.item[i]; }
+
+// Columns k .. k + 3 of an activation row times s_in.
+__device__ __forceinline__ void load_activations(const StreamInput &in, uint32_t k, uint32_t m, float (&v)[4]) {
+    const long long at = (long long)m * in.stride + k;
+    if (in.vec && k + 4 <= in.columns) {
+        if (in.bf16) {
+            const uint2 w = *reinterpret_cast<const uint2 *>((const __nv_bfloat16 *)in.x + at);
+            v[0] = __uint_as_float(w.x << 16);
+            v[1] = __uint_as_float(w.x & 0xffff0000u);
+            v[2] = __uint_as_float(w.y << 16);
+            v[3] = __uint_as_float(w.y & 0xffff0000u);
+        } else {
+            const float4 w = *reinterpret_cast<const float4 *>((const float *)in.x + at);
+            v[0] = w.x;
+            v[1] = w.y;
+            v[2] = w.z;
+            v[3] = w.w;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            v[j] = k + j >= in.columns ? 0.f
+                   : in.bf16           ? __bfloat162float(((const __nv_bfloat16 *)in.x)[at + j])
+                                       : ((const float *)in.x)[at + j];
+    }
+    if (in.s_in)
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            if (k + j < in.columns) v[j] *= in.s_in[k + j];
+}
 
 // Four MMAs of one 16-row x 64-column block; cw = this lane's code vector(s).
 template <int DT>
@@ -268,9 +318,18 @@ __device__ __forceinline__ void block_mma(float (&c)[4], uint32_t w0, uint32_t w
     }
 }
 
-template <int DT, int WARPS, int STAGES, int NT>
-__global__ void __launch_bounds__(WARPS * 32, 1) k_matvec_stream(const StreamParams p) {
+// DISPATCH: a stand-alone dispatch. The matrices of a fan-out share the launch, and where that is little work every CTA forms
+// the fragments of its slice itself instead of waiting for a kernel that does (kOwnGroups).
+template <int DT, int WARPS, int STAGES, int NT, bool DISPATCH>
+__global__ void __launch_bounds__(WARPS * 32, 1)
+    k_matvec_stream(const __grid_constant__ std::conditional_t<DISPATCH, StreamArgs, StreamParams> args) {
     pdl_launch();
+    uint32_t cta = blockIdx.x, which = 0;
+    if constexpr (DISPATCH) {
+        while (which + 1 < args.items && cta >= args.first_cta[which + 1]) ++which;
+        cta -= args.first_cta[which];
+    }
+    const StreamParams &p = stream_item(args, which);
     using F = Fmt<DT>;
     constexpr uint32_t kST = F::kSuperTileBytes;
     constexpr uint32_t kUnitBytes = 2 * kST;                      // one tile pair
@@ -292,8 +351,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_matvec_stream(const StreamPar
 
     // This CTA works inside one column slice; its warps split the slice's units
     // (tile pair x super-tile of the slice, pair-major) evenly: [beg, end).
-    const uint32_t slice = blockIdx.x / p.ctas_per_slice;
-    const uint32_t lw = (blockIdx.x % p.ctas_per_slice) * WARPS + warp;
+    const uint32_t slice = cta / p.ctas_per_slice;
+    const uint32_t lw = (cta % p.ctas_per_slice) * WARPS + warp;
     const uint64_t total = (uint64_t)p.pairs * p.kst_s;
     const bool active = lw < p.warps_per_slice;
     uint64_t beg = 0, end = 0;
@@ -325,7 +384,20 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_matvec_stream(const StreamPar
     // The activations come from the kernels before this one: wait for them here, with the first
     // STAGES chunks of every warp already on their way.
     pdl_wait();
-    if (threadIdx.x == 0) {
+    bool own = false;
+    if constexpr (DISPATCH) own = args.in.x != nullptr;
+    if (own) {
+        if constexpr (DISPATCH) {  // a group of 16 lanes takes a block of one position
+            const uint32_t i = threadIdx.x & 15, gid = threadIdx.x >> 4;
+            if (gid < slice_blocks * p.npos) {
+                float v[4];
+                load_activations(args.in, (slice * slice_blocks + gid / p.npos) * 64 + i * 4, gid % p.npos, v);
+                prep_block(v, (int)i, (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu, (int)(gid / p.npos), (int)(gid % p.npos),
+                           (int)p.npos, DT, xs, reinterpret_cast<float2 *>(ms));
+            }
+        }
+        __syncthreads();
+    } else if (threadIdx.x == 0) {
         fence_proxy_async();
         mbar_expect_tx(xbar, xfrag_bytes + meta_bytes);
         const uint8_t *xsrc = p.xfrag + (size_t)slice * xfrag_bytes;
@@ -339,7 +411,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_matvec_stream(const StreamPar
                  meta_bytes, xbar);
     }
     if (!active || nchunks == 0) return;  // warp 0 of every CTA is active and waits for xbar below
-    bool ok = mbar_wait(xbar, 0);
+    bool ok = own || mbar_wait(xbar, 0);
 
     // lanes whose B column / position does not exist read zeros with stride 0
     uint32_t b_base[NT], b_stride[NT], b_half[NT], m_base[NT], m_stride[NT];
@@ -777,11 +849,11 @@ StreamCfg pick_stream_cfg(ctox_ctx *ctx, int dt, uint32_t slice_blocks, uint32_t
 template <int DT, int NT>
 void launch_stream_nt(StreamCfg cfg, unsigned grid, size_t smem, cudaStream_t st, const StreamParams &sp) {
     if (cfg.warps == 16)
-        launch_pdl(k_matvec_stream<DT, 16, 2, NT>, dim3(grid), dim3(512), smem, st, sp);
+        launch_pdl(k_matvec_stream<DT, 16, 2, NT, false>, dim3(grid), dim3(512), smem, st, sp);
     else if (cfg.stages == 4)
-        launch_pdl(k_matvec_stream<DT, 8, 4, NT>, dim3(grid), dim3(256), smem, st, sp);
+        launch_pdl(k_matvec_stream<DT, 8, 4, NT, false>, dim3(grid), dim3(256), smem, st, sp);
     else
-        launch_pdl(k_matvec_stream<DT, 8, 2, NT>, dim3(grid), dim3(256), smem, st, sp);
+        launch_pdl(k_matvec_stream<DT, 8, 2, NT, false>, dim3(grid), dim3(256), smem, st, sp);
 }
 
 template <int DT>
@@ -790,6 +862,77 @@ void launch_stream(StreamCfg cfg, unsigned grid, size_t smem, cudaStream_t st, c
         launch_stream_nt<DT, 2>(cfg, grid, smem, st, sp);
     else
         launch_stream_nt<DT, 1>(cfg, grid, smem, st, sp);
+}
+
+// One matrix of a stand-alone dispatch and where its outputs go.
+struct DispatchItem {
+    ctox_matvec *mv;
+    MatvecPart *part;
+    float *y;
+    uint64_t y_stride;
+};
+
+StreamParams stream_params(ctox_ctx *ctx, const MatvecPart &p, uint32_t npos) {
+    const MatvecPart::Split &split = p.split[npos > 4 ? 1 : 0];
+    StreamParams sp{};
+    sp.wprep = p.prep;
+    sp.partial = p.partial;
+    sp.error_flag = ctx->dev_error;
+    sp.pairs = p.pairs;
+    sp.kst_s = p.kst_s;
+    sp.slices = p.slices;
+    sp.ctas_per_slice = split.ctas_per_slice;
+    sp.warps_per_slice = split.warps_per_slice;
+    sp.npos = npos;
+    sp.max_pieces = p.max_pieces;
+    return sp;
+}
+
+// Blocks x positions of a slice that a 16-warp CTA takes in one trip, a group of 16 lanes each. In place of the preparation
+// kernel that is worth 1.4 us of 7.2 (1024 x 1024, one position); each further trip costs 0.9 us, more than the kernel it
+// replaces, which overlaps the weights' arrival (17408 x 5120, two trips: 12.4 against 11.1 us; nine trips: 18.8
+// against 10.9).
+constexpr uint32_t kOwnGroups = 32;
+
+// How the SMs are dealt to the `n` matrices of a launch over the same activations; false where they cannot share one. All
+// take the 16-warp shape with the same slices (one shared-memory size). With several matrices each gets SMs by its
+// bytes, so its warps are fewer than prepared and its row pairs are cut differently: into no more pieces than the prepared
+// slots hold when the shortest warp has `least` units.
+bool plan_merged(ctox_ctx *ctx, const DispatchItem *it, uint32_t n, uint32_t npos, StreamArgs *a) {
+    if (n > (uint32_t)kStreamItems) return false;
+    uint64_t total = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const MatvecPart &p = *it[i].part;
+        const MatvecPart::Split &split = p.split[npos > 4 ? 1 : 0];
+        if (split.warps != 16 || split.stages != 2 || p.kst_s != it[0].part->kst_s || p.dt != it[0].part->dt) return false;
+        total += (uint64_t)p.pairs * p.slices * p.kst_s;
+    }
+    uint32_t cta = 0;
+    a->items = n;
+    for (uint32_t i = 0; i < n; ++i) {
+        const MatvecPart &p = *it[i].part;
+        StreamParams sp = stream_params(ctx, p, npos);
+        if (n > 1) {
+            const uint64_t units = (uint64_t)p.pairs * p.kst_s;
+            uint32_t ctas = (uint32_t)((uint64_t)ctx->sm_count * units / total);  // per slice
+            if (ctas == 0) ctas = 1;
+            uint64_t warps = (uint64_t)ctas * 16;
+            if (warps > units) warps = units;
+            if (warps < sp.warps_per_slice) {
+                uint64_t least = units / warps;
+                while (least < units && (p.kst_s - 1) / least + 2 > p.max_pieces) ++least;
+                if ((p.kst_s - 1) / least + 2 > p.max_pieces) return false;
+                warps = units / least;
+                if ((units + 1) * warps + units >= (1ull << 32)) return false;
+                sp.warps_per_slice = (uint32_t)warps;
+                sp.ctas_per_slice = (uint32_t)((warps + 15) / 16);
+            }
+        }
+        a->item[i] = sp;
+        a->first_cta[i] = cta;
+        cta += sp.ctas_per_slice * p.slices;
+    }
+    return true;
 }
 
 void free_matvec(ctox_matvec *mv) {
@@ -907,18 +1050,22 @@ ctox_status set_smem_attr(ctox_ctx *ctx) {
 #define CTOX_SMEM_ATTR(...)                                                                        \
     CTOX_CUDA(ctx, cudaFuncSetAttribute(k_matvec_stream<__VA_ARGS__>,                              \
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin))
-    CTOX_SMEM_ATTR(0, 16, 2, 1);
-    CTOX_SMEM_ATTR(1, 16, 2, 1);
-    CTOX_SMEM_ATTR(0, 8, 4, 1);
-    CTOX_SMEM_ATTR(1, 8, 4, 1);
-    CTOX_SMEM_ATTR(0, 8, 2, 1);
-    CTOX_SMEM_ATTR(1, 8, 2, 1);
-    CTOX_SMEM_ATTR(0, 16, 2, 2);
-    CTOX_SMEM_ATTR(1, 16, 2, 2);
-    CTOX_SMEM_ATTR(0, 8, 4, 2);
-    CTOX_SMEM_ATTR(1, 8, 4, 2);
-    CTOX_SMEM_ATTR(0, 8, 2, 2);
-    CTOX_SMEM_ATTR(1, 8, 2, 2);
+    CTOX_SMEM_ATTR(0, 16, 2, 1, true);
+    CTOX_SMEM_ATTR(1, 16, 2, 1, true);
+    CTOX_SMEM_ATTR(0, 16, 2, 2, true);
+    CTOX_SMEM_ATTR(1, 16, 2, 2, true);
+    CTOX_SMEM_ATTR(0, 16, 2, 1, false);
+    CTOX_SMEM_ATTR(1, 16, 2, 1, false);
+    CTOX_SMEM_ATTR(0, 8, 4, 1, false);
+    CTOX_SMEM_ATTR(1, 8, 4, 1, false);
+    CTOX_SMEM_ATTR(0, 8, 2, 1, false);
+    CTOX_SMEM_ATTR(1, 8, 2, 1, false);
+    CTOX_SMEM_ATTR(0, 16, 2, 2, false);
+    CTOX_SMEM_ATTR(1, 16, 2, 2, false);
+    CTOX_SMEM_ATTR(0, 8, 4, 2, false);
+    CTOX_SMEM_ATTR(1, 8, 4, 2, false);
+    CTOX_SMEM_ATTR(0, 8, 2, 2, false);
+    CTOX_SMEM_ATTR(1, 8, 2, 2, false);
 #undef CTOX_SMEM_ATTR
     done_device = ctx->device;
     return CTOX_OK;
@@ -933,6 +1080,66 @@ ctox_status check_device_error(ctox_ctx *ctx, const char *what) {
     if (code == DEV_ERR_WAIT_TIMEOUT)
         return fail(ctx, CTOX_INVALID_STATE, "%s: a bounded device wait ran out", what);
     if (code) return fail(ctx, CTOX_INVALID_STATE, "%s: device error %d", what, code);
+    return CTOX_OK;
+}
+
+// Positions m0 .. m0 + npos of a dispatch over one or several matrices of one input.
+ctox_status dispatch_pass(ctox_ctx *ctx, const DispatchItem *it, uint64_t n, const void *x, uint32_t x_dtype, uint64_t x_stride,
+                          uint32_t npos) {
+    ctox_matvec *first = it[0].mv;
+    const size_t esz = x_dtype == CTOX_BF16 ? 2 : 4;
+    const StreamInput in{x, first->s_in, (long long)x_stride, (uint32_t)first->columns, x_dtype == CTOX_BF16,
+                         (uintptr_t)x % (4 * esz) == 0 && x_stride % 4 == 0};
+    bool prepared = false;
+    auto prepare = [&](int dt) {
+        if (prepared) return;
+        const int groups = (int)(first->blocks_padded * npos);
+        launch_pdl(k_prep_x, dim3((groups * 16 + 255) / 256), dim3(256), 0, ctx->stream, x, (int)(x_dtype == CTOX_BF16),
+                   (long long)x_stride, (const float *)first->s_in, (int)first->columns, (int)first->blocks_padded, (int)npos, dt,
+                   first->xfrag, first->meta);
+        prepared = true;
+    };
+    for (uint64_t i0 = 0; i0 < n; i0 += kFinishItems) {
+        const uint32_t k = n - i0 < (uint64_t)kFinishItems ? (uint32_t)(n - i0) : (uint32_t)kFinishItems;
+        FinishArgs f{};
+        for (uint32_t i = 0; i < k; ++i) f.item[i] = finish_item(it[i0 + i].mv, *it[i0 + i].part, npos, it[i0 + i].y, it[i0 + i].y_stride);
+        StreamArgs a{};
+        const MatvecPart &p0 = *it[i0].part;
+        const bool own = p0.kst_s * 4 * npos <= kOwnGroups;
+        if ((own || k > 1) && plan_merged(ctx, it + i0, k, npos, &a)) {
+            if (own)
+                a.in = in;
+            else
+                prepare(p0.dt);
+            double bytes = 0, rows = 0;
+            for (uint32_t i = 0; i < k; ++i) {
+                a.item[i].xfrag = first->xfrag;
+                a.item[i].meta = first->meta;
+                if (k > 1) f.item[i].warps_per_slice = a.item[i].warps_per_slice;  // cut anew
+                bytes += (double)it[i0 + i].part->prep_bytes;
+                rows += (double)it[i0 + i].part->rows;
+            }
+            const uint32_t grid = a.first_cta[k - 1] + a.item[k - 1].ctas_per_slice * a.item[k - 1].slices;
+            const size_t smem = stream_smem_bytes(p0.dt, StreamCfg{16, 2}, p0.kst_s * 4, npos);
+            timing_begin(ctx);
+            if (p0.dt && npos > 4)
+                launch_pdl(k_matvec_stream<1, 16, 2, 2, true>, dim3(grid), dim3(512), smem, ctx->stream, a);
+            else if (p0.dt)
+                launch_pdl(k_matvec_stream<1, 16, 2, 1, true>, dim3(grid), dim3(512), smem, ctx->stream, a);
+            else if (npos > 4)
+                launch_pdl(k_matvec_stream<0, 16, 2, 2, true>, dim3(grid), dim3(512), smem, ctx->stream, a);
+            else
+                launch_pdl(k_matvec_stream<0, 16, 2, 1, true>, dim3(grid), dim3(512), smem, ctx->stream, a);
+            timing_end(ctx, KC_STREAM_MATVEC, bytes, 2.0 * rows * (double)first->columns * npos);
+        } else {
+            prepare(p0.dt);
+            for (uint32_t i = 0; i < k; ++i) {
+                ctox_matvec *mv = it[i0 + i].mv;
+                EX(matvec_stream_prepared(mv, (size_t)(it[i0 + i].part - mv->parts.data()), npos, first));
+            }
+        }
+        launch_finish(ctx->stream, f, k, npos);
+    }
     return CTOX_OK;
 }
 
@@ -971,19 +1178,9 @@ ctox_status matvec_stream_prepared(ctox_matvec *mv, size_t part_index, uint32_t 
         return fail(ctx, CTOX_MEMORY_BUDGET, "streaming kernel: %u positions of %llu columns exceed shared memory",
                     npos, (unsigned long long)mv->columns);
     }
-    StreamParams sp;
-    sp.wprep = p.prep;
+    StreamParams sp = stream_params(ctx, p, npos);
     sp.xfrag = fragments_of ? fragments_of->xfrag : mv->xfrag;
     sp.meta = fragments_of ? fragments_of->meta : mv->meta;
-    sp.partial = p.partial;
-    sp.error_flag = ctx->dev_error;
-    sp.pairs = p.pairs;
-    sp.kst_s = p.kst_s;
-    sp.slices = p.slices;
-    sp.ctas_per_slice = split.ctas_per_slice;
-    sp.warps_per_slice = split.warps_per_slice;
-    sp.npos = npos;
-    sp.max_pieces = p.max_pieces;
     const size_t smem = stream_smem_bytes(p.dt, cfg, p.kst_s * 4, npos);
     const unsigned grid = split.ctas_per_slice * p.slices;
     timing_begin(ctx);
@@ -1233,12 +1430,9 @@ ctox_status ctox_matvec_dispatch(ctox_matvec *mv, const void *x_dev, uint32_t x_
     for (uint32_t m0 = 0; m0 < positions; m0 += per_pass) {
         const uint32_t npos = positions - m0 < per_pass ? positions - m0 : per_pass;
         const uint8_t *xp = (const uint8_t *)x_dev + (size_t)m0 * x_stride * esz;
-        for (size_t pi = 0; pi < mv->parts.size(); ++pi) {
-            ctox_status rc = matvec_stream_pass(mv, pi, xp, x_dtype, npos, x_stride);
-            if (rc) return rc;
-            FinishArgs a{};
-            a.item[0] = finish_item(mv, mv->parts[pi], npos, y_dev + (size_t)m0 * y_stride + mv->parts[pi].row_start, y_stride);
-            launch_finish(st, a, 1, npos);
+        for (MatvecPart &part : mv->parts) {  // the fragments depend on a part's code format
+            const DispatchItem item{mv, &part, y_dev + (size_t)m0 * y_stride + part.row_start, y_stride};
+            EX(dispatch_pass(ctx, &item, 1, xp, x_dtype, x_stride, npos));
         }
     }
     CTOX_CUDA(ctx, cudaGetLastError());
@@ -1271,24 +1465,13 @@ ctox_status ctox_matvec_fanout_dispatch(ctox_matvec *const *mvs, uint64_t n, con
         per_pass = pp < per_pass ? pp : per_pass;
     }
     const size_t esz = x_dtype == CTOX_BF16 ? 2 : 4;
+    std::vector<DispatchItem> items(n);
     for (uint32_t m0 = 0; m0 < positions; m0 += per_pass) {
         const uint32_t npos = positions - m0 < per_pass ? positions - m0 : per_pass;
         const uint8_t *xp = (const uint8_t *)x_dev + (size_t)m0 * x_stride * esz;
-        const int groups = (int)(first->blocks_padded * npos);
-        launch_pdl(k_prep_x, dim3((groups * 16 + 255) / 256), dim3(256), 0, ctx->stream, (const void *)xp,
-                   (int)(x_dtype == CTOX_BF16), (long long)x_stride, (const float *)first->s_in, (int)first->columns,
-                   (int)first->blocks_padded, (int)npos, first->parts[0].dt, first->xfrag, first->meta);
-        for (uint64_t i0 = 0; i0 < n; i0 += kFinishItems) {
-            FinishArgs a{};
-            uint32_t items = 0;
-            for (uint64_t i = i0; i < n && items < (uint32_t)kFinishItems; ++i, ++items) {
-                ctox_matvec *mv = mvs[i];
-                ctox_status rc = matvec_stream_prepared(mv, 0, npos, first);
-                if (rc) return rc;
-                a.item[items] = finish_item(mv, mv->parts[0], npos, y_devs[i] + (size_t)m0 * y_strides[i], y_strides[i]);
-            }
-            launch_finish(ctx->stream, a, items, npos);
-        }
+        for (uint64_t i = 0; i < n; ++i)
+            items[i] = DispatchItem{mvs[i], &mvs[i]->parts[0], y_devs[i] + (size_t)m0 * y_strides[i], y_strides[i]};
+        EX(dispatch_pass(ctx, items.data(), n, xp, x_dtype, x_stride, npos));
     }
     CTOX_CUDA(ctx, cudaGetLastError());
     return CTOX_OK;
@@ -1560,19 +1743,10 @@ extern "C" ctox_status ctox_matvec_dispatch_static(ctox_matvec *mv, const void *
             launch_pdl(k_prep_x, dim3((groups * 16 + 255) / 256), dim3(256), 0, st, xp, x_dtype == CTOX_BF16, (long long)x_stride,
                                                                mv->s_in, (int)mv->columns,
                                                                (int)mv->blocks_padded, (int)npos, p.dt, xfrag, meta);
-            StreamParams sp;
-            sp.wprep = p.prep;
+            StreamParams sp = stream_params(ctx, p, npos);
             sp.xfrag = xfrag;
             sp.meta = meta;
             sp.partial = partial;
-            sp.error_flag = ctx->dev_error;
-            sp.pairs = p.pairs;
-            sp.kst_s = p.kst_s;
-            sp.slices = p.slices;
-            sp.ctas_per_slice = split.ctas_per_slice;
-            sp.warps_per_slice = split.warps_per_slice;
-            sp.npos = npos;
-            sp.max_pieces = p.max_pieces;
             const StreamCfg cfg{split.warps, split.stages};
             const size_t smem = stream_smem_bytes(p.dt, cfg, p.kst_s * 4, npos);
             const unsigned grid = split.ctas_per_slice * p.slices;
