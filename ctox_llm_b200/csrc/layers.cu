@@ -412,11 +412,30 @@ __device__ __forceinline__ void attention_group(const AttnGeom &g, uint32_t per_
     npos = min((int)per_group, npos - (int)first);
 }
 
+// Eight bf16 or four fp32 cache values of a 16-byte word.
+__device__ __forceinline__ void kv_unpack(const uint4 &w, float (&v)[8], const __nv_bfloat16 *) {
+    const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        v[2 * i] = __uint_as_float(u[i] << 16);
+        v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+    }
+}
+__device__ __forceinline__ void kv_unpack(const uint4 &w, float (&v)[4], const float *) {
+    v[0] = __uint_as_float(w.x);
+    v[1] = __uint_as_float(w.y);
+    v[2] = __uint_as_float(w.z);
+    v[3] = __uint_as_float(w.w);
+}
+
 // grouped_query_attention (reference.rs:420-499) for the m query positions of one KV head over
-// one split of the context, flash-decoding style: per tile of 32 tokens the K rows are staged in
+// one split of the context, flash-decoding style: per tile of 32 tokens the K and V rows are staged in
 // shared memory, every warp scores its queries against the 32 tokens (lane = token), keeps the
-// running max / sum per query, and each thread then owns one output dimension of all queries.
+// running max / sum per query, and each thread then owns one output dimension of its queries.
 // Partial (max, sum, unnormalised output) go to the workspace; k_attn_combine_prep merges them.
+// Bound by latency at short contexts and by shared-memory reads at long ones: both tiles come with all loads of a thread in
+// flight, keys are read 16 bytes at a time for all queries of a warp, weights four tokens at a time. (V rows read
+// from the cache token by token, keys and weights value by value: 23 us at 45 tokens, 8 queries of 128.)
 template <typename T, int NQMAX>
 __global__ void __launch_bounds__(kAttnThreads) k_attention(
     AttnGeom g, const float *__restrict__ q, const T *__restrict__ k_cache, const T *__restrict__ v_cache,
@@ -426,25 +445,30 @@ __global__ void __launch_bounds__(kAttnThreads) k_attention(
     pdl_wait();
     extern __shared__ __align__(128) uint8_t smraw[];
     attention_group(g, per_group, q, cache_slot, npos, ws);
+    constexpr uint32_t kWarps = kAttnThreads / 32, kQ = (NQMAX + kWarps - 1) / kWarps, kVec = 16 / sizeof(T);
     const uint32_t hd = g.head_dim, G = g.q_heads / g.kv_heads, NQ = G * npos;
     const uint32_t kh = blockIdx.x / splits, sp = blockIdx.x % splits;
-    const uint32_t kstride = hd + 16 / sizeof(T);  // padded row: conflict-free 16-byte reads
+    const uint32_t kstride = hd + kVec;  // padded row: conflict-free 16-byte reads
     float *q_s = reinterpret_cast<float *>(smraw);                       // [NQ][hd]
     float *p_s = q_s + NQMAX * hd;                                        // [NQ][tile]
     float *m_run = p_s + NQMAX * kAttnTile, *l_run = m_run + NQMAX, *alpha = l_run + NQMAX;
     T *k_s = reinterpret_cast<T *>(alpha + NQMAX);                        // [tile][kstride]
+    T *v_s = k_s + kAttnTile * kstride;                                   // [tile][kstride]
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint64_t total = cache_slot + (uint64_t)npos;  // tokens visible to the last query
     const uint64_t tiles = (total + kAttnTile - 1) / kAttnTile;
     const uint64_t tile_beg = tiles * sp / splits, tile_end = tiles * (sp + 1) / splits;
-    for (uint32_t i = tid; i < NQ * hd; i += kAttnThreads) {
-        const uint32_t qi = i / hd, d = i % hd, mi = qi / G, gq = qi % G;
-        q_s[i] = q[((size_t)mi * g.q_heads + kh * G + gq) * hd + d];
+    for (uint32_t i = tid; i < NQ * hd / 4; i += kAttnThreads) {
+        const uint32_t qi = i / (hd / 4), d = i % (hd / 4), mi = qi / G, gq = qi % G;
+        *reinterpret_cast<float4 *>(q_s + i * 4) =
+            *reinterpret_cast<const float4 *>(q + ((size_t)mi * g.q_heads + kh * G + gq) * hd + d * 4);
     }
     if (tid < NQMAX) {
         m_run[tid] = -INFINITY;
         l_run[tid] = 0.f;
     }
+    // outputs: thread group `part` of hd threads takes the queries qi % parts == part
+    const uint32_t parts = kAttnThreads / hd == 4 ? 4 : kAttnThreads / hd == 2 ? 2 : 1, part = tid / hd, dim = tid % hd;
     float o[NQMAX];
 #pragma unroll
     for (int i = 0; i < NQMAX; ++i) o[i] = 0.f;
@@ -452,39 +476,76 @@ __global__ void __launch_bounds__(kAttnThreads) k_attention(
     __syncthreads();
     for (uint64_t tile = tile_beg; tile < tile_end; ++tile) {
         const uint64_t t0 = tile * kAttnTile;
-        // stage K rows (16-byte chunks, coalesced)
-        const uint32_t chunks_per_row = hd * sizeof(T) / 16;
-        for (uint32_t c = tid; c < kAttnTile * chunks_per_row; c += kAttnThreads) {
-            const uint32_t r = c / chunks_per_row, cc = c % chunks_per_row;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (t0 + r < total) {
-                const size_t slot = kv_slot(page_table, page_tokens, t0 + r);
-                v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(
-                        k_cache + (slot * g.kv_heads + kh) * hd) + cc * 16);
+        // stage K and V rows (16-byte chunks, coalesced), four chunks of each at a time
+        const uint32_t chunks_per_row = hd / kVec, chunks = kAttnTile * chunks_per_row;
+        for (uint32_t c0 = tid; c0 < chunks; c0 += kAttnThreads * 4) {
+            size_t at[4];
+            uint4 kv[4], vv[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint32_t c = c0 + j * kAttnThreads, r = c / chunks_per_row;
+                at[j] = c < chunks && t0 + r < total
+                            ? (kv_slot(page_table, page_tokens, t0 + r) * g.kv_heads + kh) * hd + c % chunks_per_row * kVec
+                            : ~(size_t)0;
             }
-            *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(k_s + r * kstride) + cc * 16) = v;
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                kv[j] = vv[j] = make_uint4(0, 0, 0, 0);
+                if (at[j] != ~(size_t)0) {
+                    kv[j] = *reinterpret_cast<const uint4 *>(k_cache + at[j]);
+                    vv[j] = *reinterpret_cast<const uint4 *>(v_cache + at[j]);
+                }
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint32_t c = c0 + j * kAttnThreads;
+                if (c < chunks) {
+                    const uint32_t to = c / chunks_per_row * kstride + c % chunks_per_row * kVec;
+                    *reinterpret_cast<uint4 *>(k_s + to) = kv[j];
+                    *reinterpret_cast<uint4 *>(v_s + to) = vv[j];
+                }
+            }
         }
         __syncthreads();
         // scores + running softmax: warp w takes queries w, w+8, ...; lane = token of the tile
         const uint64_t t = t0 + lane;
-        for (uint32_t qi = warp; qi < NQ; qi += kAttnThreads / 32) {
-            const uint32_t mi = qi / G;
-            float s = 0.f;
-            const T *kr = k_s + lane * kstride;
-            const float *qr = q_s + qi * hd;
-            for (uint32_t d = 0; d < hd; ++d) s += qr[d] * kv_load(kr + d);
-            s *= scale;
+        float s[kQ];
+#pragma unroll
+        for (uint32_t j = 0; j < kQ; ++j) s[j] = 0.f;
+        for (uint32_t d = 0; d < hd; d += kVec) {
+            float kf[kVec];
+            kv_unpack(*reinterpret_cast<const uint4 *>(k_s + lane * kstride + d), kf, (const T *)nullptr);
+#pragma unroll
+            for (uint32_t j = 0; j < kQ; ++j) {
+                if (warp + j * kWarps >= NQ) break;
+                const float *qr = q_s + (warp + j * kWarps) * hd + d;
+#pragma unroll
+                for (uint32_t i = 0; i < kVec; i += 4) {
+                    const float4 qv = *reinterpret_cast<const float4 *>(qr + i);
+                    s[j] = fmaf(qv.x, kf[i], s[j]);
+                    s[j] = fmaf(qv.y, kf[i + 1], s[j]);
+                    s[j] = fmaf(qv.z, kf[i + 2], s[j]);
+                    s[j] = fmaf(qv.w, kf[i + 3], s[j]);
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kQ; ++j) {
+            const uint32_t qi = warp + j * kWarps, mi = qi / G;
+            if (qi >= NQ) break;
+            float sv = s[j] * scale;
             const bool valid = t < total && t <= cache_slot + mi;  // causal inside the pass
-            if (!valid) s = -INFINITY;
-            float tmax = s;
+            if (!valid) sv = -INFINITY;
+            float tmax = sv;
 #pragma unroll
             for (int of = 16; of > 0; of >>= 1) tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, of));
             const float m_old = m_run[qi], m_new = fmaxf(m_old, tmax);
-            const float p = (valid && m_new > -INFINITY) ? expf(s - m_new) : 0.f;
+            const float p = (valid && m_new > -INFINITY) ? expf(sv - m_new) : 0.f;
             float psum = p;
 #pragma unroll
             for (int of = 16; of > 0; of >>= 1) psum += __shfl_xor_sync(0xffffffffu, psum, of);
             p_s[qi * kAttnTile + lane] = p;
+            __syncwarp();
             if (lane == 0) {
                 const float a = m_old > -INFINITY ? expf(m_old - m_new) : 0.f;
                 alpha[qi] = a;
@@ -493,27 +554,34 @@ __global__ void __launch_bounds__(kAttnThreads) k_attention(
             }
         }
         __syncthreads();
-        // output: thread d owns dimension d of every query
-        if (tid < hd) {
+        // output: each thread one dimension (tokens past the last have weight and value zero)
+        if (part < parts) {
 #pragma unroll
             for (int qi = 0; qi < NQMAX; ++qi)
-                if ((uint32_t)qi < NQ) o[qi] *= alpha[qi];
-            for (uint32_t r = 0; r < (uint32_t)kAttnTile && t0 + r < total; ++r) {
-                const size_t slot = kv_slot(page_table, page_tokens, t0 + r);
-                const float vv = kv_load(v_cache + (slot * g.kv_heads + kh) * hd + tid);
+                if ((uint32_t)qi < NQ && (qi & (parts - 1)) == part) o[qi] *= alpha[qi];
+            for (uint32_t r = 0; r < (uint32_t)kAttnTile; r += 4) {
+                float vv[4];
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) vv[j] = kv_load(v_s + (r + j) * kstride + dim);
 #pragma unroll
                 for (int qi = 0; qi < NQMAX; ++qi)
-                    if ((uint32_t)qi < NQ) o[qi] += p_s[qi * kAttnTile + r] * vv;
+                    if ((uint32_t)qi < NQ && (qi & (parts - 1)) == part) {
+                        const float4 p = *reinterpret_cast<const float4 *>(p_s + qi * kAttnTile + r);
+                        o[qi] = fmaf(p.x, vv[0], o[qi]);
+                        o[qi] = fmaf(p.y, vv[1], o[qi]);
+                        o[qi] = fmaf(p.z, vv[2], o[qi]);
+                        o[qi] = fmaf(p.w, vv[3], o[qi]);
+                    }
             }
         }
         __syncthreads();
     }
     // workspace: [kv head][split][query][hd + 2]
     float *out = ws + ((size_t)(kh * splits + sp) * NQ) * (hd + 2);
-    if (tid < hd) {
+    if (part < parts) {
 #pragma unroll
         for (int qi = 0; qi < NQMAX; ++qi)
-            if ((uint32_t)qi < NQ) out[(size_t)qi * (hd + 2) + tid] = o[qi];
+            if ((uint32_t)qi < NQ && (qi & (parts - 1)) == part) out[(size_t)qi * (hd + 2) + dim] = o[qi];
     }
     if (tid < NQ) {
         out[(size_t)tid * (hd + 2) + hd] = m_run[tid];
@@ -923,7 +991,7 @@ static void launch_attention_t(cudaStream_t st, const AttnGeom &g, const float *
                                const void *v_cache, const uint32_t *page_table, uint32_t page_tokens,
                                uint64_t cache_slot, uint32_t m, uint32_t per_group, uint32_t splits, float *ws) {
     const size_t smem = (size_t)NQMAX * g.head_dim * 4 + (size_t)NQMAX * kAttnTile * 4 + 3 * NQMAX * 4 +
-                        (size_t)kAttnTile * (g.head_dim + 16 / sizeof(T)) * sizeof(T) + 16;
+                        2 * (size_t)kAttnTile * (g.head_dim + 16 / sizeof(T)) * sizeof(T) + 16;
     // the attribute belongs to the device, not to the process: once per device
     static thread_local unsigned long long attr_devices = 0;
     int dev = 0;

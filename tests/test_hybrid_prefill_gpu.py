@@ -83,3 +83,31 @@ def test_long_pass_on_top_of_a_session_matches_oracle(orc):
     finally:
         ex.unload()
         be.close()
+
+
+@pytest.mark.parametrize("kv", [ctox.F32, ctox.BF16])
+@pytest.mark.parametrize("head_dim,heads,kv_heads", [(64, 4, 2), (64, 12, 2), (128, 4, 4), (128, 6, 1), (192, 4, 2)])
+def test_attention_on_cuda_cores_matches_oracle(orc, head_dim, heads, kv_heads, kv):
+    """Four, two and one groups of threads per head dimension; 8, 24 and 48 queries per CTA; a context that ends inside a tile
+    of 32 tokens; long and short passes and single positions."""
+    be = ctox.B200Backend(0)
+    cfg = tiny_config(max_draft_tokens=2, num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=head_dim, rotary_dim=32,
+                      kv_dtype=kv, full_attention_interval=2)
+    model = OracleModel(orc, cfg, seed=8)
+    ex = ctox.B200Executor(be, cfg)
+    try:
+        model.load_into(ex)
+        ex.warmup()
+        ex.keep_logits(True)
+        prompt = [int(t) for t in np.random.default_rng(head_dim).integers(0, cfg.vocab_size, 75)]
+        tokens, logits, _ = model.greedy(prompt, 2)
+        for cuts in ((0, 75), (0, 8, 16, 60, 68, 75)):
+            ex.reset_session()
+            for a, b in zip(cuts, cuts[1:]):
+                got = ex.extend(prompt[a:b], [b - a - 1])
+            assert rel_l2(got[0], logits[0]) <= 1e-3
+            ex.decode(tokens[0], mtp_enabled=True, force_accept=0)
+            assert rel_l2(ex.last_logits(0), logits[1]) <= 1e-3
+    finally:
+        ex.unload()
+        be.close()
