@@ -10,6 +10,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "f32x2.cuh"
 #include "prep.cuh"
 
 namespace ctox {
@@ -270,26 +271,7 @@ __global__ void __launch_bounds__(256) k_long_gates(const LongGates p) {
 // state values each in registers), so that chain has three shuffles and no barrier; the tokens' inputs are staged
 // sixteen at a time, a block ahead. A CTA takes 16 columns: 8 CTAs per head.
 constexpr int kScanTokens = 16, kScanCols = 16;
-// Two fp32 values per instruction.
-__device__ __forceinline__ unsigned long long pack2(float a, float b) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float &a, float &b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ float total4(const unsigned long long (&v)[4]) {
+__device__ __forceinline__ float total4(const f32x2 (&v)[4]) {
     float a[4], b[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) unpack2(v[i], a[i], b[i]);
@@ -308,7 +290,7 @@ __global__ void __launch_bounds__(128) k_long_delta(const LongScan p) {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane & 7, c = warp * 4 + (lane >> 3);
     const uint32_t head = blockIdx.x >> 3, col0 = (blockIdx.x & 7) * kScanCols, kh = head / (p.heads / p.qk_heads);
     // this lane's keys are sub * 4 + 32 i .. + 3, i < 4; two of them per register pair
-    unsigned long long s[8];
+    f32x2 s[8];
     float *state = p.state + (size_t)head * 128 * 128 + col0 + c;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -362,8 +344,8 @@ __global__ void __launch_bounds__(128) k_long_delta(const LongScan p) {
             load(kn, ks[b][t + 1 < n ? t + 1 : t]);
             const uint32_t tn = t + 1 < n ? t + 1 : t;
             const float decay_n = ds[b][tn], beta_n = bs[b][tn], v_n = vs[b][tn][c];
-            const unsigned long long d2 = pack2(decay, decay);
-            unsigned long long mem[4] = {0, 0, 0, 0}, out[4] = {0, 0, 0, 0};
+            const f32x2 d2 = pack2(decay, decay);
+            f32x2 mem[4] = {0, 0, 0, 0}, out[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 s[2 * i] = mul2(s[2 * i], d2);
@@ -381,7 +363,7 @@ __global__ void __launch_bounds__(128) k_long_delta(const LongScan p) {
             }
             if (sub == 0 && t > 0) os[t - 1][c] = o;
             const float delta = (v - r) * beta;
-            const unsigned long long dl2 = pack2(delta, delta);
+            const f32x2 dl2 = pack2(delta, delta);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 s[2 * i] = fma2(k[i].x, dl2, s[2 * i]);
