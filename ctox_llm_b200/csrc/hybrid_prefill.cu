@@ -21,6 +21,19 @@ __device__ __forceinline__ float lp_out(const LongOut &o, uint32_t row, uint32_t
     for (uint32_t s = 1; s < o.splits; ++s) v += p[s * o.split_stride];  // index order
     return v;
 }
+// Four rows row .. row + 3 (a multiple of four, o.rows too).
+__device__ __forceinline__ float4 lp_out4(const LongOut &o, uint32_t row, uint32_t pos) {
+    const float *p = o.y + (size_t)pos * o.rows + row;
+    float4 v = *reinterpret_cast<const float4 *>(p);
+    for (uint32_t s = 1; s < o.splits; ++s) {
+        const float4 w = *reinterpret_cast<const float4 *>(p + s * o.split_stride);
+        v.x += w.x;
+        v.y += w.y;
+        v.z += w.z;
+        v.w += w.w;
+    }
+    return v;
+}
 template <int OP>  // 0 sum, 1 maximum
 __device__ __forceinline__ float lp_block(float v, float *red) {
 #pragma unroll
@@ -71,21 +84,35 @@ __global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
         vals[c] = v;
         amax = fmaxf(amax, fabsf(v));
     };
+    // widths are multiples of 64: NORM and SWIGLU take four columns per thread and trip
+    auto put4 = [&](uint32_t c, float4 x) {
+        if (p.s_in) {
+            const float4 w = *reinterpret_cast<const float4 *>(p.s_in + c);
+            x = make_float4(x.x * w.x, x.y * w.y, x.z * w.z, x.w * w.w);
+        }
+        *reinterpret_cast<float4 *>(vals + c) = x;
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+    };
     if constexpr (MODE == ROWS_NORM) {
         float *h = p.h + (size_t)pos * p.width;
         float sq = 0.f;
-        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
-            float v = p.a ? p.a[(size_t)pos * p.width + c] : 0.f;
-            if (p.o.y) v += lp_out(p.o, c, pos);
-            h[c] = v;
-            vals[c] = v;
-            sq += v * v;
+        for (uint32_t c = tid * 4; c < p.width; c += kRowsThreads * 4) {
+            float4 v = p.a ? *reinterpret_cast<const float4 *>(p.a + (size_t)pos * p.width + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (p.o.y) {
+                const float4 y = lp_out4(p.o, c, pos);
+                v = make_float4(v.x + y.x, v.y + y.y, v.z + y.z, v.w + y.w);
+            }
+            *reinterpret_cast<float4 *>(h + c) = v;
+            *reinterpret_cast<float4 *>(vals + c) = v;
+            sq += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
         }
         const float inv = 1.0f / sqrtf(lp_block<0>(sq, red) / (float)p.width + p.eps);
-        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {  // each thread its own columns again
-            const float xn = vals[c] * inv * (1.0f + p.w[c]);
-            if (p.xn_out) p.xn_out[(size_t)pos * p.width + c] = xn;
-            if (p.has_next) put(c, xn);
+        for (uint32_t c = tid * 4; c < p.width; c += kRowsThreads * 4) {  // each thread its own columns again
+            const float4 v = *reinterpret_cast<const float4 *>(vals + c), w = *reinterpret_cast<const float4 *>(p.w + c);
+            const float4 xn = make_float4(v.x * inv * (1.0f + w.x), v.y * inv * (1.0f + w.y), v.z * inv * (1.0f + w.z),
+                                          v.w * inv * (1.0f + w.w));
+            if (p.xn_out) *reinterpret_cast<float4 *>(p.xn_out + (size_t)pos * p.width + c) = xn;
+            if (p.has_next) put4(c, xn);
         }
         if (!p.has_next) return;
     } else if constexpr (MODE == ROWS_MTP) {
@@ -102,8 +129,11 @@ __global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
             put(p.width + c, h[c] * ih * (1.0f + p.w2[c]));
         }
     } else if constexpr (MODE == ROWS_SWIGLU) {
-        for (uint32_t c = tid; c < p.width; c += kRowsThreads)
-            put(c, silu_f(lp_out(p.o, c, pos)) * lp_out(p.o, p.width + c, pos));
+#pragma unroll 2
+        for (uint32_t c = tid * 4; c < p.width; c += kRowsThreads * 4) {
+            const float4 g = lp_out4(p.o, c, pos), u = lp_out4(p.o, p.width + c, pos);
+            put4(c, make_float4(silu_f(g.x) * u.x, silu_f(g.y) * u.y, silu_f(g.z) * u.z, silu_f(g.w) * u.w));
+        }
     } else if constexpr (MODE == ROWS_ATTENTION) {
         // attention left (unnormalised output, maximum, sum) per group of positions: [kv head][query][head_dim + 2]
         const uint32_t G = p.q_heads / p.kv_heads, hd = p.head_dim, group = pos / p.per_group, mi = pos % p.per_group;
