@@ -49,8 +49,31 @@ __device__ __forceinline__ int operand_row(const GemmPages &p, uint32_t row) {
     return (int)(p.table[pos / p.page_tokens] * p.page_tokens + pos % p.page_tokens);
 }
 
-// 32 columns n0 .. n0 + 32 of one output row.
-__device__ __forceinline__ void gemm_store(const GemmOut &o, float *v, uint32_t m, uint32_t n0, uint32_t N) {
+// A warp's 32 rows m0 .. of BYTES bytes each, chunk c of this lane's row in w[c], to d + row * pitch: through shared memory, so
+// that neighbouring lanes store neighbouring chunks. (A row per lane, each store touched 32 lines: a product over 512
+// columns spent most of its 40 us on them.)
+constexpr uint32_t kStoreStage = 32 * (128 + 16);  // bytes of shared memory per warp
+template <uint32_t BYTES>
+__device__ __forceinline__ void store_rows(uint8_t *d, size_t pitch, const uint4 *w, uint32_t rows, uint8_t *stage) {
+    constexpr uint32_t C = BYTES / 16, kPitch = BYTES + 16;
+    const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();  // the rows before have been read
+#pragma unroll
+    for (uint32_t c = 0; c < C; ++c) *reinterpret_cast<uint4 *>(stage + lane * kPitch + c * 16) = w[c];
+    __syncwarp();
+#pragma unroll
+    for (uint32_t i = 0; i < C; ++i) {
+        const uint32_t r = (i * 32 + lane) / C, c = (i * 32 + lane) % C;
+        const uint4 x = *reinterpret_cast<const uint4 *>(stage + r * kPitch + c * 16);
+        if (r < rows) *reinterpret_cast<uint4 *>(d + r * pitch + c * 16) = x;
+    }
+}
+
+// 32 columns n0 .. n0 + 32 of the output rows of a warp; m: this lane's row (the warp's 32 rows follow one another). Lanes
+// past the last row take part.
+__device__ __forceinline__ void gemm_store(const GemmOut &o, float *v, uint32_t m, uint32_t n0, uint32_t M, uint32_t N,
+                                           uint8_t *stage) {
+    const uint32_t m0 = m - (threadIdx.x & 31), rows = M - m0 < 32 ? M - m0 : 32;  // m0 < M
     if (o.bias) {
 #pragma unroll
         for (int j = 0; j < 32; ++j)
@@ -58,15 +81,15 @@ __device__ __forceinline__ void gemm_store(const GemmOut &o, float *v, uint32_t 
     }
     if (o.kind == OUT_CLAMPED_GLU) {
         __nv_bfloat16 *d = (__nv_bfloat16 *)o.d + (size_t)m * o.ld + n0 / 2;
-        __nv_bfloat162 h[8];
+        alignas(16) __nv_bfloat162 h[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             h[j] = __floats2bfloat162_rn(clamped_glu(v[4 * j], v[4 * j + 1], o.cap, o.slope),
                                          clamped_glu(v[4 * j + 2], v[4 * j + 3], o.cap, o.slope));
         if (n0 + 32 <= N && o.ld % 8 == 0) {
-            *reinterpret_cast<uint4 *>(d) = *reinterpret_cast<uint4 *>(h);
-            *reinterpret_cast<uint4 *>(d + 8) = *reinterpret_cast<uint4 *>(h + 4);
-        } else {
+            store_rows<32>((uint8_t *)((__nv_bfloat16 *)o.d + (size_t)m0 * o.ld + n0 / 2), (size_t)o.ld * 2,
+                           reinterpret_cast<const uint4 *>(h), rows, stage);
+        } else if (m < M) {
 #pragma unroll
             for (int j = 0; j < 16; ++j)
                 if (n0 + 2 * j < N) d[j] = j & 1 ? h[j / 2].y : h[j / 2].x;
@@ -83,7 +106,7 @@ __device__ __forceinline__ void gemm_store(const GemmOut &o, float *v, uint32_t 
         uint32_t w = n0 % o.head_width;  // heads are a multiple of 16 wide: w is even, a pair never straddles two
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
-            if (w >= o.rope0 && w < o.rope0 + o.rope_dims) {
+            if (m < M && w >= o.rope0 && w < o.rope0 + o.rope_dims) {
                 const float2 cs = o.table[(size_t)m * (o.rope_dims / 2) + ((w - o.rope0) >> 1)];
                 const float a = v[j] * cs.x - v[j + 1] * cs.y, b = v[j + 1] * cs.x + v[j] * cs.y;
                 v[j] = a;
@@ -95,6 +118,7 @@ __device__ __forceinline__ void gemm_store(const GemmOut &o, float *v, uint32_t 
     }
     const bool full = n0 + 32 <= N;
     if (o.split && n0 >= o.split) {
+        if (m >= M) return;
         float *d = o.d2 + (size_t)m * o.ld2 + (n0 - o.split);
 #pragma unroll
         for (int j = 0; j < 32; ++j)
@@ -102,14 +126,12 @@ __device__ __forceinline__ void gemm_store(const GemmOut &o, float *v, uint32_t 
     } else if (o.bf16) {
         __nv_bfloat16 *d = (__nv_bfloat16 *)o.d + (size_t)m * o.ld + n0;
         if (full && o.ld % 8 == 0) {
+            alignas(16) __nv_bfloat162 h[16];
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-                __nv_bfloat162 h[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[j + 2 * i], v[j + 2 * i + 1]);
-                *reinterpret_cast<uint4 *>(d + j) = *reinterpret_cast<uint4 *>(h);
-            }
-        } else {
+            for (int j = 0; j < 16; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            store_rows<64>((uint8_t *)((__nv_bfloat16 *)o.d + (size_t)m0 * o.ld + n0), (size_t)o.ld * 2,
+                           reinterpret_cast<const uint4 *>(h), rows, stage);
+        } else if (m < M) {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
                 if (n0 + j < N) d[j] = __float2bfloat16_rn(v[j]);
@@ -117,9 +139,9 @@ __device__ __forceinline__ void gemm_store(const GemmOut &o, float *v, uint32_t 
     } else {
         float *d = (float *)o.d + (size_t)m * o.ld + n0;
         if (full && o.ld % 4 == 0) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(d + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        } else {
+            store_rows<128>((uint8_t *)((float *)o.d + (size_t)m0 * o.ld + n0), (size_t)o.ld * 4, reinterpret_cast<const uint4 *>(v),
+                            rows, stage);
+        } else if (m < M) {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
                 if (n0 + j < N) d[j] = v[j];
@@ -274,6 +296,7 @@ __global__ void __launch_bounds__(kGmThreads, 1)
     } else {
         const uint32_t quarter = warp & 3;  // the lanes of tensor memory this warp may read
         const uint32_t report = G == 2 ? leader_addr(acc_empty) : acc_empty;
+        uint8_t *raw_stage = raw + (base - smem_addr(raw)) + stages * (kABytes + kBBytes) + quarter * kStoreStage;
         uint32_t n_tile = 0;
         for (uint32_t t = first; t < tiles; t += step, ++n_tile) {
             const uint32_t acc = n_tile & 1, m = (t % tiles_m * G + rank) * kGmM + quarter * 32 + lane, n0 = t / tiles_m * BN;
@@ -282,10 +305,10 @@ __global__ void __launch_bounds__(kGmThreads, 1)
             const uint32_t src = tmem + acc * BN + ((quarter * 32) << 16);
 #pragma unroll 1
             for (uint32_t c = 0; c < BN; c += 32) {
-                float v[32];
+                alignas(16) float v[32];
                 tmem_ld32(src + c, v);
                 tmem_ld_wait();
-                if (m < M && n0 + c < N) gemm_store(out, v, m, n0 + c, N);
+                if (m - lane < M && n0 + c < N) gemm_store(out, v, m, n0 + c, M, N, raw_stage);
             }
             fence_before();
             __syncwarp();
@@ -315,9 +338,9 @@ namespace {
 template <uint32_t BN, uint32_t G>
 ctox_status gemm_launch(ctox_ctx *ctx, const GemmOperand &a, const GemmOperand &b, const GemmOut &out) {
     const uint32_t stage_bytes = kGmM * kGmK * 2 + BN / G * kGmK * 2;
-    uint32_t stages = ((uint32_t)ctx->max_smem_optin - 2048) / stage_bytes;
+    uint32_t stages = ((uint32_t)ctx->max_smem_optin - 2048 - 4 * kStoreStage) / stage_bytes;
     if (stages > kGmStageMax) stages = kGmStageMax;
-    const size_t smem = (size_t)stages * stage_bytes + 1024;
+    const size_t smem = (size_t)stages * stage_bytes + 1024 + 4 * kStoreStage;
     CUtensorMap ma, mb;
     auto encode = [&](CUtensorMap *m, const GemmOperand &o, uint32_t box) {
         return tensor_map_bf16(ctx, m, o.p, o.page_table ? o.store_rows : o.rows, o.cols, o.ld, box, kGmK);
