@@ -18,7 +18,9 @@ struct LongPass {
     uint32_t *tokens = nullptr;
 };
 
-// Fewest remaining tokens worth a long pass: two short passes of eight positions take as long (hybrid_prefill.cu).
+// Fewest remaining tokens worth a long pass. Its products unpack every weight for a tile of positions whatever it holds: 17
+// tokens take 2.41 ms against 2.90 in three short passes (8 layers of width 5120), 0.49 against 0.98 (4 layers of
+// width 1024); 16 take 2.40 against 2.15 in two short passes of the wide model.
 constexpr uint32_t kLongMin = 17;
 
 // Allocates the buffers; leaves e->long_pass null (short passes only) where they do not fit or do not apply.
