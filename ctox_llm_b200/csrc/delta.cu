@@ -306,6 +306,13 @@ void launch_commit_batch(cudaStream_t st, const CommitLayer *layers_dev, const C
                rescan ? 1 : 0, (int)heads, (int)qk_heads, channels, conv_kernel);
 }
 
+void launch_delta_rescan(cudaStream_t st, const float *q, const float *k, const float *v, const float *log_decay,
+                         const float *beta, const float *state_in, float *state_out, float *out, uint32_t tokens,
+                         uint32_t heads, uint32_t qk_heads) {
+    launch_pdl(k_gated_delta_scan128<float>, dim3(heads * 4), dim3(128), 0, st, q, k, v, log_decay, beta, state_in, state_out,
+               out, (int)tokens, (int)heads, (int)qk_heads);
+}
+
 // Any head geometry: one thread per (head, value column), the reference's loop order.
 __global__ void k_gated_delta_scan_generic(const float *__restrict__ q, const float *__restrict__ k,
                                            const float *__restrict__ v, const float *__restrict__ log_decay,

@@ -1011,8 +1011,8 @@ ctox_status commit_positions(ctox_exec *e, uint32_t m, uint32_t n) {
             if (e->w[l].full) continue;
             LayerS &ls = e->s[l];
             if (n < m)
-                EX(ctox_gated_delta_scan(ctx, ls.q, ls.k, ls.v, ls.g, ls.beta, ls.delta[ls.cur], ls.delta[ls.cur ^ 1],
-                                         e->lcore, n, c.linear_num_value_heads, c.linear_num_key_heads, 128, 128));
+                launch_delta_rescan(ctx->stream, ls.q, ls.k, ls.v, ls.g, ls.beta, ls.delta[ls.cur], ls.delta[ls.cur ^ 1],
+                                    e->lcore, n, c.linear_num_value_heads, c.linear_num_key_heads);
             ls.cur ^= 1;
             launch_conv_commit(ctx->stream, ls.conv_state, ls.conv_in, e->channels, c.linear_conv_kernel_dim, n);
         }

@@ -110,6 +110,10 @@ struct CommitLayer {
 struct CommitCur {
     uint64_t lo, hi;  // bit j: index (0 / 1) of the committed state buffer of linear layer j < 128
 };
+// The re-scan of one layer, when there are more layers than a batch takes: like the batch, bit for bit what the pass computed.
+void launch_delta_rescan(cudaStream_t st, const float *q, const float *k, const float *v, const float *log_decay,
+                         const float *beta, const float *state_in, float *state_out, float *out, uint32_t tokens,
+                         uint32_t heads, uint32_t qk_heads);
 void launch_commit_batch(cudaStream_t st, const CommitLayer *layers_dev, const CommitCur &cur, uint32_t n_layers,
                          uint32_t n, bool rescan, uint32_t heads, uint32_t qk_heads, uint32_t channels,
                          uint32_t conv_kernel);
