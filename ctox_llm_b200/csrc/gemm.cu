@@ -8,7 +8,7 @@
 
 namespace ctox {
 
-constexpr int kGmThreads = 224;  // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue, warp 6: reports copies to the pair's first CTA
+constexpr int kGmThreads = 192;  // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue
 constexpr uint32_t kGmM = 128, kGmK = 64, kGmStageMax = 8;
 
 ctox_status tensor_map_bf16(ctox_ctx *ctx, CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint64_t ld,
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kGmThreads, 1)
     if (tid == 0) {
         dead = 0;
         for (uint32_t i = 0; i < stages; ++i) {
-            bar_init(full + i * 8, G == 2 && rank == 0 ? 2 : 1);  // own copies, and the report of the other CTA's
+            bar_init(full + i * 8, 1);  // at the first CTA of a pair: the copies of both
             bar_init(empty + i * 8, 1);
         }
         for (uint32_t i = 0; i < 2; ++i) {
@@ -209,18 +209,23 @@ __global__ void __launch_bounds__(kGmThreads, 1)
                 for (uint32_t k = 0; k < ksteps; ++k, ++issued) {
                     if (!(ok = bar_wait(empty + s * 8, parity, &dead))) break;
                     const uint32_t bar = full + s * 8, dst = base + s * (kABytes + kBBytes);
-                    bar_expect(bar, kABytes + kBBytes);
-                    tma_load(dst, &map_a, bar, (int)(k * kGmK), ra);
+                    auto load = [&](uint32_t to, const CUtensorMap *map, int row) {
+                        if constexpr (G == 2)
+                            tma_load_pair(to, map, leader_addr(bar), (int)(k * kGmK), row);
+                        else
+                            tma_load(to, map, bar, (int)(k * kGmK), row);
+                    };
+                    if (rank == 0) bar_expect(bar, G * (kABytes + kBBytes));
+                    load(dst, &map_a, ra);
 #pragma unroll
-                    for (uint32_t i = 0; i < kBoxes; ++i)
-                        tma_load(dst + kABytes + i * kBBox * kGmK * 2, &map_b, bar, (int)(k * kGmK), rb[i]);
+                    for (uint32_t i = 0; i < kBoxes; ++i) load(dst + kABytes + i * kBBox * kGmK * 2, &map_b, rb[i]);
                     if (++s == stages) {
                         s = 0;
                         parity ^= 1;
                     }
                 }
             }
-            if (!ok) {  // leave no copy in flight behind; the first CTA of a pair may lack the other's report, so by time
+            if (!ok) {  // leave no copy in flight behind; a pair's barrier may lack the other CTA's part, so by time
                 if constexpr (G == 2) {
                     const long long t0 = clock64();
                     while (clock64() - t0 < 2000000) {
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(kGmThreads, 1)
         const uint64_t desc0 = smem_desc(base, 128);
         for (uint32_t t = rank == 0 ? first : tiles; t < tiles && ok; t += step, ++n_tile) {
             const uint32_t acc = n_tile & 1, d = tmem + acc * BN;
-            if (!(ok = __all_sync(0xffffffffu, bar_wait(acc_empty + acc * 8, ((n_tile >> 1) & 1) ^ 1, &dead)))) break;
+            if (!(ok = __all_sync(0xffffffffu, bar_wait<G == 2 ? BAR_PAIR_TURN : BAR_CTA>(acc_empty + acc * 8, ((n_tile >> 1) & 1) ^ 1, &dead)))) break;
             fence_after();
             for (uint32_t k = 0; k < ksteps; ++k) {
                 if (!(ok = __all_sync(0xffffffffu, bar_wait(full + s * 8, parity, &dead)))) break;
@@ -279,20 +284,6 @@ __global__ void __launch_bounds__(kGmThreads, 1)
                 commit(drained);
             bar_drain(drained, 0);
         }
-    } else if (warp == 6) {
-        if (G == 2 && rank == 1 && lane == 0) {  // a copy's barrier is in the CTA it copies to: tell the issuing CTA
-            uint32_t s = 0, parity = 0;
-            bool ok = true;
-            for (uint32_t t = first; t < tiles && ok; t += step)
-                for (uint32_t k = 0; k < ksteps; ++k) {
-                    if (!(ok = bar_wait(full + s * 8, parity, &dead))) break;
-                    bar_arrive_cluster(leader_addr(full + s * 8));
-                    if (++s == stages) {
-                        s = 0;
-                        parity ^= 1;
-                    }
-                }
-        }
     } else {
         const uint32_t quarter = warp & 3;  // the lanes of tensor memory this warp may read
         const uint32_t report = G == 2 ? leader_addr(acc_empty) : acc_empty;
@@ -314,7 +305,7 @@ __global__ void __launch_bounds__(kGmThreads, 1)
             __syncwarp();
             if (lane == 0) {
                 if constexpr (G == 2)
-                    bar_arrive_cluster(report + acc * 8);
+                    bar_turn_leader(report + acc * 8);
                 else
                     bar_arrive(report + acc * 8);
             }

@@ -8,7 +8,7 @@
 // A CTA of 16 warps per SM works through units (128 rows x n positions x a range of columns):
 //   warp 0     one thread copies the activation tiles (bulk copies, hi and lo parts)
 //   warp 1     issues tcgen05.mma: per 64-column block lo then hi into one accumulator
-//   warp 2     (second CTA of a pair) reports its copies to the first
+//   warp 2     (second CTA of a pair) reports its stages to the first
 //   warps 4-7  unpack codes to fp16 (code - offset, exact) and write them as the swizzled A operand
 //   warps 8-15 take the 64-column sum out of tensor memory and add scale[row][block] * sum to fp32 registers
 // The block scales therefore act in fp32 on sums of 64 products, exactly as in the streaming matvec: folding them
@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
     if (tid == 0) {
         dead = 0;
         for (uint32_t i = 0; i < stages; ++i) {
-            // the issuing CTA: its copies, its unpacking warps, and the same of the other CTA
-            bar_init(full + i * 8, G == 1 ? 5 : rank == 0 ? 10 : 1);
+            // this CTA's copies and unpacking warps; at the issuing CTA of a pair also the other's report of the same
+            bar_init(full + i * 8, G == 2 && rank == 0 ? 6 : 5);
             bar_init(empty + i * 8, 1);
         }
         for (uint32_t i = 0; i < C::kD; ++i) {
@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
             for (uint32_t u = rank == 0 ? first_unit : p.units; u < p.units && ok; u += unit_step) {
                 const PgUnit t = pg_unit(p, u);
                 for (uint32_t k = (t.ks1 - t.ks0) * 4; k > 0; --k) {
-                    if (!(ok = __all_sync(0xffffffffu, bar_wait(d_empty + d * 8, d_par, &dead)))) break;
-                    if (!(ok = __all_sync(0xffffffffu, bar_wait(full + st * 8, parity, &dead)))) break;
+                    if (!(ok = __all_sync(0xffffffffu, bar_wait<G == 2 ? BAR_PAIR_TURN : BAR_CTA>(d_empty + d * 8, d_par, &dead)))) break;
+                    if (!(ok = __all_sync(0xffffffffu, bar_wait<G == 2 ? BAR_PAIR : BAR_CTA>(full + st * 8, parity, &dead)))) break;
                     fence_after();
                     const uint64_t da = desc0 + st * (stage_bytes >> 4), db = da + (C::kABytes >> 4);
                     const uint32_t acc = tmem + d * W;
@@ -229,14 +229,14 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
                 bar_drain(drained, 0);
             }
         } else if (G == 2 && warp == 2 && lane == 0 && rank == 1) {
-            // a copy's barrier belongs to the CTA it copies to: tell the issuing CTA
+            // this CTA's copies and unpacked weights of a stage are complete: tell the issuing CTA
             uint32_t st = 0, parity = 0;
             bool ok = true;
             for (uint32_t u = first_unit; u < p.units && ok; u += unit_step) {
                 const PgUnit t = pg_unit(p, u);
                 for (uint32_t i = (t.ks1 - t.ks0) * 4; i > 0; --i) {
                     if (!(ok = bar_wait(full + st * 8, parity, &dead))) break;
-                    bar_arrive_cluster(leader_addr(full + st * 8));
+                    bar_release_leader(leader_addr(full + st * 8));
                     if (++st == stages) {
                         st = 0;
                         parity ^= 1;
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
         uint4 q[2][kVec];
         uint32_t st = 0, parity = 1;
         bool ok = true;
-        const uint32_t mine = base + (w4 * 32 + g) * 128, report = G == 2 ? leader_addr(full) : full;
+        const uint32_t mine = base + (w4 * 32 + g) * 128;
         const uint32_t c0 = ((2 * t4) ^ g) * 16, c1 = ((2 * t4 + 1) ^ g) * 16;
         auto load = [&](const uint8_t *base, bool live, uint32_t tile, uint32_t j) {
             q[tile][j] = live ? __ldg(reinterpret_cast<const uint4 *>(base + tile * Fmt<DT>::kSuperTileBytes + kScaleBytes +
@@ -313,12 +313,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) {
-                        if constexpr (G == 2)
-                            bar_arrive_cluster(report + st * 8);
-                        else
-                            bar_arrive(report + st * 8);
-                    }
+                    if (lane == 0) bar_arrive(full + st * 8);
                     if (++st == stages) {
                         st = 0;
                         parity ^= 1;
@@ -379,7 +374,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
                             __syncwarp();
                             if (lane == 0) {
                                 if constexpr (G == 2)
-                                    bar_arrive_cluster(report + d * 8);
+                                    bar_turn_leader(report + d * 8);
                                 else
                                     bar_arrive(report + d * 8);
                             }

@@ -44,24 +44,38 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// What a wait orders: the arrivals of this CTA (the default), or also those that threads of the other CTA of a pair made:
+// with what they released (BAR_PAIR, against bar_release_leader), or only the turn of tensor memory, which the
+// tcgen05 fences on both sides order (BAR_PAIR_TURN, against bar_turn_leader).
+enum BarScope { BAR_CTA, BAR_PAIR, BAR_PAIR_TURN };
+template <BarScope S = BAR_CTA>
 __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+#define CTOX_BAR_TRY(SEM)                                                   \
+    asm volatile(                                                           \
+        "{\n\t.reg .pred p;\n\t"                                            \
+        "mbarrier.try_wait.parity" SEM ".shared::cta.b64 p, [%1], %2;\n\t" \
+        "selp.u32 %0, 1, 0, p;\n\t}"                                       \
+        : "=r"(ok)                                                          \
+        : "r"(bar), "r"(parity)                                             \
+        : "memory")
+    if constexpr (S == BAR_PAIR)
+        CTOX_BAR_TRY(".acquire.cluster");
+    else if constexpr (S == BAR_PAIR_TURN)
+        CTOX_BAR_TRY(".relaxed.cluster");
+    else
+        CTOX_BAR_TRY("");
+#undef CTOX_BAR_TRY
     return ok != 0;
 }
 // Waits for a phase of a barrier, for about a second at most. On a time-out, or when another role of the
 // CTA has given up (*dead), returns false: the caller leaves its loop.
 constexpr long long kWaitCycles = 2000000000ll;
+template <BarScope S = BAR_CTA>
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int *dead) {
-    if (bar_try(bar, parity)) return true;
+    if (bar_try<S>(bar, parity)) return true;
     const long long t0 = clock64();
-    while (!bar_try(bar, parity)) {
+    while (!bar_try<S>(bar, parity)) {
         if (*dead) return false;
         if (clock64() - t0 > kWaitCycles) {
             *dead = 1;
@@ -80,6 +94,15 @@ __device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap *map, u
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
         "l"(map), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+}
+// A copy by either CTA of a pair into its own shared memory that completes at a barrier of the first (leader_addr): the
+// CTA that issues the pair's products waits for both halves there, with no thread between them.
+__device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap *map, uint32_t leader_bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];" ::"r"(
+            dst),
+        "l"(map), "r"(leader_bar), "r"(x), "r"(y)
         : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map) {
@@ -153,16 +176,20 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Address of this CTA's `bar` in the CTA of rank 0, and an arrival there. (Release at cluster scope would be a memory
-// barrier of about a thousand cycles. What these arrivals order goes through the async proxy, which the caller's
-// proxy fence covers, or through tensor memory.)
+// Address of this CTA's `bar` in the CTA of rank 0, and arrivals there. A release at cluster scope is a memory barrier of
+// about a thousand cycles for the arriving thread: one thread of the second CTA makes it for all (it has waited for them
+// at a barrier of its own CTA), beside the work. An accumulator's turn needs no release: its readers have waited for
+// their loads and passed fence_before().
 __device__ __forceinline__ uint32_t leader_addr(uint32_t bar) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(bar));
     return r;
 }
-__device__ __forceinline__ void bar_arrive_cluster(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+__device__ __forceinline__ void bar_release_leader(uint32_t leader_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_bar) : "memory");
+}
+__device__ __forceinline__ void bar_turn_leader(uint32_t leader_bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_bar) : "memory");
 }
 // Instruction descriptor: bf16 x bf16 -> fp32, both operands k-major.
 __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t m, uint32_t n) {
