@@ -1139,7 +1139,7 @@ ctox_status extend_impl(ctox_exec *e, const uint32_t *tokens, uint64_t n, const 
     uint64_t w = 0;
     for (uint64_t a = 0; a < n;) {
         if (cancelled(cancel)) return fail(ctx, CTOX_CANCELLED, "prefill cancelled at token %llu", (unsigned long long)a);
-        const bool is_long = e->long_pass && n - a >= kLongMin;
+        const bool is_long = e->long_pass && n - a >= long_min(e);
         const uint32_t m = is_long ? (uint32_t)(n - a < e->long_pass->cap ? n - a : e->long_pass->cap) : pass_positions(e, n - a);
         *began = true;
         if (e->cfg.mtp_num_hidden_layers && e->have_hidden && e->position > 0) {

@@ -10,6 +10,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "f32x2.cuh"
 #include "prep.cuh"
 
@@ -49,6 +51,15 @@ __device__ __forceinline__ float lp_block(float v, float *red) {
     return v;
 }
 
+// Row of the attention kernels' workspace that holds a query's part of one split: per group of positions
+// [kv head][split][position][head of the kv head].
+__device__ __forceinline__ size_t attn_row(uint32_t pos, uint32_t head, uint32_t split, uint32_t m, uint32_t per_group,
+                                           uint32_t splits, uint32_t q_heads, uint32_t kv_heads) {
+    const uint32_t G = q_heads / kv_heads, group = pos / per_group, n = min(per_group, m - group * per_group);
+    return (size_t)group * per_group * splits * q_heads +
+           ((size_t)(head / G) * splits + split) * G * n + pos % per_group * G + head % G;
+}
+
 // ------------------------------------------------------------------ rows: one CTA per position
 // Forms the next product's input row in shared memory and writes it as hi and lo parts. Bound by memory: a
 // projection's fp32 outputs are read once, four bytes per input column are written.
@@ -63,7 +74,7 @@ struct RowsArgs {
     float eps;
     uint32_t width;         // columns of h / inter / query width / value width / hidden
     uint32_t off;           // DELTA: first gate row of o
-    uint32_t q_heads, kv_heads, head_dim, per_group, m;  // ATTENTION
+    uint32_t q_heads, kv_heads, head_dim, per_group, splits, m;  // ATTENTION
     LongIn in;
     const float *s_in;      // of the next product (null: 1)
     uint32_t blocks_padded;
@@ -135,13 +146,11 @@ __global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
             put4(c, make_float4(silu_f(g.x) * u.x, silu_f(g.y) * u.y, silu_f(g.z) * u.z, silu_f(g.w) * u.w));
         }
     } else if constexpr (MODE == ROWS_ATTENTION) {
-        // attention left (unnormalised output, maximum, sum) per group of positions: [kv head][query][head_dim + 2]
-        const uint32_t G = p.q_heads / p.kv_heads, hd = p.head_dim, group = pos / p.per_group, mi = pos % p.per_group;
-        const uint32_t n = min(p.per_group, p.m - group * p.per_group);
-        const float *base = p.a + (size_t)group * p.per_group * p.q_heads * (hd + 2);
+        // attention left (unnormalised output, maximum, sum) of each query; of several splits the first holds the merged one
+        const uint32_t hd = p.head_dim;
         for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
             const uint32_t hq = c / hd, d = c % hd;
-            const float *r = base + ((size_t)(hq / G) * G * n + mi * G + hq % G) * (hd + 2);
+            const float *r = p.a + attn_row(pos, hq, 0, p.m, p.per_group, p.splits, p.q_heads, p.kv_heads) * (hd + 2);
             const float gate = lp_out(p.o, hq * 2 * hd + hd + d, pos);
             put(c, r[d] * (1.0f / r[hd + 1]) * (1.0f / (1.0f + expf(-gate))));
         }
@@ -498,8 +507,62 @@ __global__ void __launch_bounds__(256) k_long_attn_pre(const LongAttnPre p) {
     }
 }
 
+// The splits of a query's context merged into the first one's row (sum 1: normalised). One CTA per (position, head), a
+// thread per dimension; a warp forms the splits' weights.
+struct LongMerge {
+    float *ws;
+    uint32_t q_heads, kv_heads, per_group, splits, m;
+};
+__global__ void __launch_bounds__(256) k_long_attn_merge(const LongMerge p) {
+    pdl_launch();
+    pdl_wait();
+    __shared__ float wgt[kAttnMaxSplits];
+    const uint32_t hd = blockDim.x, pos = blockIdx.x / p.q_heads, head = blockIdx.x % p.q_heads, d = threadIdx.x;
+    float *r = p.ws + attn_row(pos, head, 0, p.m, p.per_group, p.splits, p.q_heads, p.kv_heads) * (hd + 2);
+    const size_t stride = (attn_row(pos, head, 1, p.m, p.per_group, p.splits, p.q_heads, p.kv_heads) -
+                           attn_row(pos, head, 0, p.m, p.per_group, p.splits, p.q_heads, p.kv_heads)) * (hd + 2);
+    if (d < 32) {
+        float mx = -INFINITY, den = 0.f;
+        for (uint32_t s = d; s < p.splits; s += 32) mx = fmaxf(mx, r[s * stride + hd]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (uint32_t s = d; s < p.splits; s += 32) {
+            const float ms = r[s * stride + hd], w = ms > -INFINITY ? expf(ms - mx) : 0.f;
+            wgt[s] = w;
+            den += r[s * stride + hd + 1] * w;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+        for (uint32_t s = d; s < p.splits; s += 32) wgt[s] /= den;
+    }
+    __syncthreads();
+    float acc = 0.f;
+#pragma unroll 8
+    for (uint32_t s = 0; s < p.splits; ++s) acc += r[s * stride + d] * wgt[s];
+    r[d] = acc;
+    if (d == 0) r[hd + 1] = 1.0f;
+}
+
 // ------------------------------------------------------------------ host side
 namespace {
+
+// Splits of the context in a long pass of m positions. A group's CTAs are one per KV head, too few of them where the pass is
+// short: 17 positions at four KV heads are 16 CTAs. The parts are as many as finish soonest, counted in rounds over the SMs
+// of tiles of 64 tokens with two tiles' time for a CTA's start and end, and no more than the workspace holds.
+uint32_t attention_splits(const ctox_exec *e, uint32_t per_group, uint64_t pos0, uint32_t m) {
+    const uint64_t tiles = (pos0 + m + 63) / 64, sms = (uint64_t)e->ctx->sm_count;
+    const uint64_t ctas = (uint64_t)e->cfg.num_key_value_heads * ((m + per_group - 1) / per_group);
+    uint64_t most = std::min<uint64_t>(e->attn_splits_max, e->long_pass->cap / m), best = 1, best_cost = ~0ull;
+    most = std::min(most, tiles);
+    for (uint64_t s = 1; s <= most; ++s) {
+        const uint64_t cost = (ctas * s + sms - 1) / sms * ((tiles + s - 1) / s + 2);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = s;
+        }
+    }
+    return (uint32_t)best;
+}
 
 constexpr uint32_t kLongCap = 1024;  // positions per pass: the buffers take 0.35 GB at the flagship's widths
 
@@ -571,9 +634,14 @@ ctox_status mixer(ctox_exec *e, uint32_t l, const LongOut &o, uint32_t m, uint64
         const AttnGeom g = geom(e);
         const int bf16 = c.kv_dtype == CTOX_BF16;
         EX(attn_pre(e, l, o, m, pos0, pos0, e->page_table, false));
+        a.per_group = attention_group_positions(g, bf16, m);
+        a.splits = attention_splits(e, a.per_group, pos0, m);
         timing_begin(ctx);
         launch_attention_groups(ctx->stream, g, L.aq, ls.k_cache, ls.v_cache, bf16, e->page_table, c.kv_page_tokens, pos0, m,
-                                L.attn);
+                                a.splits, L.attn);
+        if (a.splits > 1)
+            launch_pdl(k_long_attn_merge, dim3(m * g.q_heads), dim3(g.head_dim), 0, ctx->stream,
+                       LongMerge{L.attn, g.q_heads, g.kv_heads, a.per_group, a.splits, m});
         timing_end(ctx, KC_ATTENTION, 2.0 * (double)(pos0 + m) * e->kv_width * (bf16 ? 2 : 4),
                    4.0 * ((double)pos0 + 0.5 * m) * e->q_width * m);
         CTOX_CUDA(ctx, cudaGetLastError());
@@ -582,7 +650,6 @@ ctox_status mixer(ctox_exec *e, uint32_t l, const LongOut &o, uint32_t m, uint64
         a.q_heads = g.q_heads;
         a.kv_heads = g.kv_heads;
         a.head_dim = g.head_dim;
-        a.per_group = attention_group_positions(g, bf16);
         return rows<ROWS_ATTENTION>(e, a, m, lw.out);
     }
     const uint32_t heads = c.linear_num_value_heads, kernel = c.linear_conv_kernel_dim;
@@ -604,6 +671,11 @@ ctox_status mixer(ctox_exec *e, uint32_t l, const LongOut &o, uint32_t m, uint64
 }
 
 }  // namespace
+
+uint32_t long_min(const ctox_exec *e) {
+    const bool cores = !attention_on_tensor_cores(geom(e), e->cfg.kv_dtype == CTOX_BF16);
+    return cores && e->position > kDeepCores ? kLongMinDeepCores : kLongMin;
+}
 
 ctox_status long_warmup(ctox_exec *e) {
     ctox_ctx *ctx = e->ctx;

@@ -10,6 +10,8 @@
 
 #include "hybrid_prefill.cuh"
 
+#include <algorithm>
+
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -401,13 +403,13 @@ void launch_attn_pre(cudaStream_t st, const MvOut &fan, const AttnGeom &g, const
 constexpr int kAttnTile = 32;      // tokens per tile
 constexpr int kAttnThreads = 256;
 
-// Positions of a long pass are dealt to the attention kernels in groups of per_group (blockIdx.y, no split of the
-// context): a CTA sees its group as a pass of its own. A short pass is one group.
+// Positions of a long pass are dealt to the attention kernels in groups of per_group (blockIdx.y): a CTA sees its group as
+// a pass of its own. A short pass is one group.
 __device__ __forceinline__ void attention_group(const AttnGeom &g, uint32_t per_group, const float *__restrict__ &q, uint64_t &cache_slot,
-                                                int &npos, float *__restrict__ &ws) {
+                                                int &npos, uint32_t splits, float *__restrict__ &ws) {
     const uint32_t first = blockIdx.y * per_group;
     q += (size_t)first * g.q_heads * g.head_dim;
-    ws += (size_t)first * g.q_heads * (g.head_dim + 2);
+    ws += (size_t)first * splits * g.q_heads * (g.head_dim + 2);
     cache_slot += first;
     npos = min((int)per_group, npos - (int)first);
 }
@@ -444,7 +446,7 @@ __global__ void __launch_bounds__(kAttnThreads) k_attention(
     pdl_launch();
     pdl_wait();
     extern __shared__ __align__(128) uint8_t smraw[];
-    attention_group(g, per_group, q, cache_slot, npos, ws);
+    attention_group(g, per_group, q, cache_slot, npos, splits, ws);
     constexpr uint32_t kWarps = kAttnThreads / 32, kQ = (NQMAX + kWarps - 1) / kWarps, kVec = 16 / sizeof(T);
     const uint32_t hd = g.head_dim, G = g.q_heads / g.kv_heads, NQ = G * npos;
     const uint32_t kh = blockIdx.x / splits, sp = blockIdx.x % splits;
@@ -642,7 +644,7 @@ __global__ void __launch_bounds__(GROUPS * 128, 1) k_attention_mma(
     uint64_t cache_slot, int npos, uint32_t per_group, uint32_t splits, float *__restrict__ ws) {
     pdl_launch();
     extern __shared__ __align__(128) uint8_t smraw[];
-    attention_group(g, per_group, q, cache_slot, npos, ws);
+    attention_group(g, per_group, q, cache_slot, npos, splits, ws);
     constexpr int NT = GROUPS * 128, kFaBuffers = fa_buffers(GROUPS);
     const uint32_t G = g.q_heads / g.kv_heads, NQ = G * npos;
     const uint32_t kh = blockIdx.x / splits, sp = blockIdx.x % splits;
@@ -1004,7 +1006,7 @@ static void launch_attention_t(cudaStream_t st, const AttnGeom &g, const float *
                g, q, (const T *)k_cache, (const T *)v_cache, page_table, page_tokens, cache_slot, (int)m, per_group, splits, ws);
 }
 
-// Shared by short passes (one group, `splits` parts of the context) and long ones (many groups, one part).
+// Shared by short passes (one group) and long ones (many groups).
 static void launch_attention_kernel(cudaStream_t st, const AttnGeom &g, const float *q, const void *k_cache,
                                     const void *v_cache, int kv_bf16, const uint32_t *page_table, uint32_t page_tokens,
                                     uint64_t cache_slot, uint32_t m, uint32_t per_group, uint32_t splits, float *workspace) {
@@ -1059,18 +1061,24 @@ void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const 
     launch_pdl(k_attn_combine_prep, dim3(m * g.q_heads), dim3(g.head_dim), 0, st, g, workspace, gate, (int)m, splits, next);
 }
 
-// Positions that share a CTA in a long pass: as many queries as the kernel takes at once (32 on the tensor cores,
-// else what a short pass of eight positions may have).
-uint32_t attention_group_positions(const AttnGeom &g, int kv_bf16) {
+// Which kernel a long pass takes (its groups have 32 queries at most on the tensor cores).
+bool attention_on_tensor_cores(const AttnGeom &g, int kv_bf16) {
+    return kv_bf16 && g.head_dim == kFaHd && g.q_heads / g.kv_heads <= 32;
+}
+// Positions that share a CTA in a long pass of m: as many queries as the kernel takes at once (32 on the tensor cores, else
+// what a short pass of eight positions may have), dealt evenly to as many groups as that makes: a CTA's time follows its
+// queries (17 positions on 32000 tokens, 24 heads of 256, 32-bit cache: groups of 8, 8, 1 took 3.76 ms for four layers).
+uint32_t attention_group_positions(const AttnGeom &g, int kv_bf16, uint32_t m) {
     const uint32_t G = g.q_heads / g.kv_heads;
-    const uint32_t n = kv_bf16 && g.head_dim == kFaHd && G <= 32 ? 32 / G : 8;
-    return n < 8 ? n : 8;
+    const uint32_t most = attention_on_tensor_cores(g, kv_bf16) ? std::min(32 / G, 8u) : 8u;
+    const uint32_t groups = (m + most - 1) / most;
+    return (m + groups - 1) / groups;
 }
 void launch_attention_groups(cudaStream_t st, const AttnGeom &g, const float *q, const void *k_cache, const void *v_cache,
                              int kv_bf16, const uint32_t *page_table, uint32_t page_tokens, uint64_t cache_slot, uint32_t m,
-                             float *workspace) {
+                             uint32_t splits, float *workspace) {
     launch_attention_kernel(st, g, q, k_cache, v_cache, kv_bf16, page_table, page_tokens, cache_slot, m,
-                            attention_group_positions(g, kv_bf16), 1, workspace);
+                            attention_group_positions(g, kv_bf16, m), splits, workspace);
 }
 
 }  // namespace ctox
