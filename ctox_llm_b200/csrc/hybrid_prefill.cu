@@ -85,7 +85,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
     pdl_launch();
     pdl_wait();
-    extern __shared__ __align__(16) float vals[];  // [blocks_padded * 64]
+    extern __shared__ __align__(16) float vals[];  // [blocks_padded * 64], then the largest value of each block
     __shared__ float red[kRowsThreads / 32];
     const uint32_t pos = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t columns = MODE == ROWS_MTP ? 2 * p.width : p.width;
@@ -172,14 +172,39 @@ __global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
     for (uint32_t c = columns + tid; c < p.blocks_padded * 64; c += kRowsThreads) vals[c] = 0.f;
     amax = lp_block<1>(amax, red);  // its barriers also publish vals
     // One unit per position: the largest value lies in [2^14, 2^15). hi + lo then keep 22 bits of every value above
-    // 2^-18 of the largest, and an absolute 2^-39 of it below.
-    int e = (int)((__float_as_uint(amax) >> 23) & 0xff) - 127;
-    if (!(amax > 0.f) || e > 127) e = 14;  // zero row or non-finite input: factor 1
-    e = max(e, -100);
-    const float f = __uint_as_float((uint32_t)(14 - e + 127) << 23);
-    if (tid == 0) p.in.unit[pos] = __uint_as_float((uint32_t)(e - 14 + 127) << 23);
+    // 2^-28 of the largest, and an absolute 2^-50 of it below. A streaming product has a unit for each block and keeps 22
+    // bits above 2^-13 (4-bit codes) or 2^-9 of the block's largest value, 2^-35 or 2^-31 of it below: the row's unit leaves
+    // no block fewer unless its largest value is below 2^-15 of the row's. Then every block gets its own unit.
+    float *block_max = vals + p.blocks_padded * 64;
+    auto exponent = [](float x) { return (int)((__float_as_uint(x) >> 23) & 0xff) - 127; };
+    int spread = 0;
+    for (uint32_t i = tid; i < p.blocks_padded * 4; i += kRowsThreads) {  // four neighbouring lanes: a block
+        float mx = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 x = *reinterpret_cast<const float4 *>(vals + i * 16 + j * 4);
+            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+        }
+        const uint32_t lanes = 0xfu << (lane & 28);
+        mx = fmaxf(mx, __shfl_xor_sync(lanes, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(lanes, mx, 2));
+        if ((i & 3) == 0) block_max[i >> 2] = mx;
+        if (mx > 0.f && exponent(mx) < exponent(amax) - 15) spread = 1;
+    }
+    spread = __syncthreads_or(spread);
+    auto unit_exponent = [&](float largest) {
+        const int e = exponent(largest);
+        return max(!(largest > 0.f) || e > 127 ? 14 : e, -100);  // zero or non-finite: factor 1
+    };
+    if (tid == 0) {
+        p.in.unit[pos] = __uint_as_float((uint32_t)(unit_exponent(amax) - 14 + 127) << 23);
+        p.in.spread[pos] = spread ? 0xff : 0;
+    }
     for (uint32_t i = tid; i < p.blocks_padded * 4; i += kRowsThreads) {  // sixteen columns: two chunks of each part
         const uint32_t block = i >> 2, t = i & 3;
+        const int e = unit_exponent(spread ? block_max[block] : amax);
+        const float f = __uint_as_float((uint32_t)(14 - e + 127) << 23);
+        if (t == 0) p.in.block_unit[(size_t)block * p.in.pos_pad + pos] = __uint_as_float((uint32_t)(e - 14 + 127) << 23);
         float v[16];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -195,7 +220,8 @@ __global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
             const float q4a = v[(s >> 2) * 8 + (s & 3)], q4b = v[(s >> 2) * 8 + (s & 3) + 4];
             const float x = p.dt ? q4a : v[s], y = p.dt ? q4b : v[s + 8];
             hi[s] = __floats2half2_rn(x, y);
-            lo[s] = __floats2half2_rn(x - __low2float(hi[s]), y - __high2float(hi[s]));
+            lo[s] = __floats2half2_rn((x - __low2float(hi[s])) * (float)(1 << kLoShift),
+                                      (y - __high2float(hi[s])) * (float)(1 << kLoShift));
         }
         uint8_t *d = p.in.x + ((size_t)block * 2 * p.in.pos_pad + pos) * 128;
         const uint32_t c0 = ((2 * t) ^ (pos & 7)) * 16, c1 = ((2 * t + 1) ^ (pos & 7)) * 16;
@@ -581,7 +607,7 @@ ctox_status rows(ctox_exec *e, RowsArgs &a, uint32_t m, ctox_matvec *next) {
         a.blocks_padded = next->blocks_padded;
         a.dt = next->parts[0].dt;
     }
-    const size_t smem = (next ? (size_t)next->blocks_padded * 64 : a.width) * 4;
+    const size_t smem = (next ? (size_t)next->blocks_padded * 65 : a.width) * 4;
     CTOX_CUDA(ctx, cudaFuncSetAttribute(k_long_rows<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024));
     CTOX_CUDA(ctx, launch_pdl(k_long_rows<MODE>, dim3(m), dim3(kRowsThreads), smem, ctx->stream, a));
     return CTOX_OK;
@@ -688,7 +714,7 @@ ctox_status long_warmup(ctox_exec *e) {
     uint32_t blocks = 0;
     uint64_t rows = 0;
     for (ctox_matvec *mv : mats) {
-        if (mv->parts.size() != 1 || (size_t)mv->blocks_padded * 256 + 2048 > (size_t)ctx->max_smem_optin) return CTOX_OK;
+        if (mv->parts.size() != 1 || (size_t)mv->blocks_padded * 260 + 2048 > (size_t)ctx->max_smem_optin) return CTOX_OK;
         blocks = mv->blocks_padded > blocks ? mv->blocks_padded : blocks;
         rows = mv->rows > rows ? mv->rows : rows;
     }
@@ -704,6 +730,8 @@ ctox_status long_warmup(ctox_exec *e) {
     const uint64_t H = c.hidden_size;
     ctox_status rc = get(&L->in.x, long_in_bytes(blocks, pos_pad));
     if (!rc) rc = get(&L->in.unit, pos_pad);
+    if (!rc) rc = get(&L->in.block_unit, (size_t)blocks * pos_pad + kUnitTail);
+    if (!rc) rc = get(&L->in.spread, pos_pad + kUnitTail);
     if (!rc) rc = get(&L->y, L->y_floats);
     if (!rc) rc = get(&L->h, cap * H);
     if (!rc) rc = get(&L->final_hidden, cap * H);

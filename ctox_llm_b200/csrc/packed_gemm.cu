@@ -10,7 +10,9 @@
 //   warp 1     issues tcgen05.mma: per 64-column block lo then hi into one accumulator
 //   warp 2     (second CTA of a pair) reports its stages to the first
 //   warps 4-7  unpack codes to fp16 (code - offset, exact) and write them as the swizzled A operand
-//   warps 8-15 take the 64-column sum out of tensor memory and add scale[row][block] * sum to fp32 registers
+//   warps 8-15 take the 64-column sum out of tensor memory and add scale[row][block] * sum to fp32 registers; where a
+//              position of the tile is marked (packed_gemm.cuh), scale[row][block] * unit[block][position] * sum, which
+//              takes a third longer (999 positions of a 9088 x 5056 and a 5056 x 4544 product, all marked: 497 against 376 us)
 // The block scales therefore act in fp32 on sums of 64 products, exactly as in the streaming matvec: folding them
 // into fp16 weights would need a second weight part (scale and code have 15 significant bits).
 //
@@ -22,6 +24,8 @@
 #include "packed_gemm.cuh"
 
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "layout.cuh"
 #include "umma.cuh"
@@ -41,7 +45,8 @@ constexpr uint32_t kPgStages = 6;
 
 struct PgParams {
     const uint8_t *w, *x;
-    const float *unit, *s_out;
+    const float *unit, *block_unit, *s_out;
+    const uint8_t *spread;
     float *y;
     size_t split_stride;
     uint32_t rows, rt0, units, m, pos_pad, pos_tiles, n, stages, pairs, kst, kst_s, splits;
@@ -108,6 +113,8 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
     __shared__ __align__(8) uint64_t bars[2 * (kPgStages + C::kD) + 1];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int dead;
+    __shared__ volatile uint32_t marked_tiles[8];
+    __shared__ __align__(16) float unit_stage[8][W / 2];  // of an accumulating warp's columns
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t base = (smem_addr(raw) + 1023) & ~1023u, stages = p.stages;
     const uint32_t half_bytes = p.n / G * 128, stage_bytes = C::kABytes + 2 * half_bytes;  // A | lo | hi
@@ -198,7 +205,9 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
 #pragma unroll
                         for (uint32_t i = 0; i < 8; ++i) {
                             const uint64_t a = da + (i & 3) * 2, b = db + (i & 3) * 2 + (i < 4 ? 0 : half_bytes >> 4);
-                            if constexpr (G == 2)
+                            if (i == 4)  // the lo parts are summed: back to the unit of the hi parts
+                                mma_f16_shifted<G, kLoShift>(acc, a, b, idesc);
+                            else if constexpr (G == 2)
                                 mma_f16_pair(acc, a, b, idesc, i > 0);
                             else
                                 mma_f16(acc, a, b, idesc, i > 0);
@@ -331,6 +340,17 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
         uint32_t used = 0;
         const uint32_t report = G == 2 ? leader_addr(d_empty) : d_empty;
         bool ok = true;
+        // Bit i: this warp's columns of tile i hold a position that is marked. In shared memory, because the loop below has no
+        // register to spare.
+        uint32_t tiles = 0;
+        for (uint32_t i = 0; i < p.pos_tiles; ++i) {
+            const uint32_t n0 = i * p.n + first, end = n0 >= p.m ? 0 : min(columns, p.m - n0);
+            const uint32_t marks = lane * 4 < end ? *reinterpret_cast<const uint32_t *>(p.spread + n0 + lane * 4) : 0;
+            const uint32_t live = end >= lane * 4 + 4 ? 0xffffffffu : (1u << (8 * (end & 3))) - 1;
+            if (__any_sync(0xffffffffu, (marks & live) != 0)) tiles |= 1u << i;
+        }
+        if (lane == 0) marked_tiles[warp - 8] = tiles;
+        __syncwarp();
         for (uint32_t u = first_unit; u < p.units && ok; u += unit_step) {
             const PgUnit t = pg_unit(p, u);
             const uint32_t pair = (t.rt * G + rank) * 4 + quarter, row = pair * 32 + lane;
@@ -345,45 +365,90 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
             float acc[W / 2];
 #pragma unroll
             for (uint32_t i = 0; i < W / 2; ++i) acc[i] = 0.f;
-            uint2 sc = scales(t.ks0);
-            for (uint32_t ks = t.ks0; ks < t.ks1 && ok; ++ks) {
-                const uint2 sc_next = scales(ks + 1);
+            auto sweep = [&](auto marked_units) {
+                // The marked form takes the units of 32 columns at a time from shared memory, where the warp puts those of
+                // the next block once this block's have been read.
+                constexpr bool kMarked = decltype(marked_units)::value;
+                constexpr uint32_t kLoad = kMarked || W <= 64 ? 32 : 64;
+                float *units = unit_stage[warp - 8];
+                float next_units[W / 64];
+                auto fetch = [&](uint32_t block) {
+#pragma unroll
+                    for (uint32_t i = 0; i < W / 64; ++i)
+                        next_units[i] = block < p.kst * 4 ? p.block_unit[(size_t)block * p.pos_pad + t.n0 + first + i * 32 + lane] : 0.f;
+                };
+                if constexpr (kMarked) fetch(t.ks0 * 4);
+                uint2 sc = scales(t.ks0);
+                for (uint32_t ks = t.ks0; ks < t.ks1 && ok; ++ks) {
+                    const uint2 sc_next = scales(ks + 1);
 #pragma unroll 1
-                for (uint32_t j = 0; j < 4; ++j, ++used) {
-                    const uint32_t d = used % C::kD;
-                    if (!__all_sync(0xffffffffu, bar_wait(d_full + d * 8, (used / C::kD) & 1, &dead))) {
-                        ok = false;
-                        break;
-                    }
-                    fence_after();
-                    const uint32_t word = j & 2 ? sc.y : sc.x;
-                    const float s = __half2float(__ushort_as_half((uint16_t)(j & 1 ? word >> 16 : word & 0xffff)));
-                    // columns past the tile's belong to the accumulator all the same, and their sums are not stored
-                    constexpr uint32_t kLoad = W > 64 ? 64 : 32;
+                    for (uint32_t j = 0; j < 4; ++j, ++used) {
+                        const uint32_t d = used % C::kD;
+                        if constexpr (kMarked) {
+                            __syncwarp();  // the block before has been read
 #pragma unroll
-                    for (uint32_t c = 0; c < W / 2; c += kLoad) {
-                        if (c >= columns) break;
-                        float v[kLoad];
-                        if constexpr (kLoad == 64)
-                            tmem_ld64(src + d * W + c, v);
-                        else
-                            tmem_ld32(src + d * W + c, v);
-                        tmem_ld_wait();
-                        if (c + kLoad >= columns) {  // all of the accumulator is in registers
-                            fence_before();
+                            for (uint32_t i = 0; i < W / 64; ++i) units[i * 32 + lane] = next_units[i];
+                            fetch(ks * 4 + j + 1);
                             __syncwarp();
-                            if (lane == 0) {
-                                if constexpr (G == 2)
-                                    bar_turn_leader(report + d * 8);
-                                else
-                                    bar_arrive(report + d * 8);
-                            }
                         }
+                        if (!__all_sync(0xffffffffu, bar_wait(d_full + d * 8, (used / C::kD) & 1, &dead))) {
+                            ok = false;
+                            break;
+                        }
+                        fence_after();
+                        const uint32_t word = j & 2 ? sc.y : sc.x;
+                        const float s = __half2float(__ushort_as_half((uint16_t)(j & 1 ? word >> 16 : word & 0xffff)));
+                        // columns past the tile's belong to the accumulator all the same, and their sums are not stored
 #pragma unroll
-                        for (uint32_t i = 0; i < kLoad; i += 2) pg_fma2(acc + c + i, s, v + i);
+                        for (uint32_t c = 0; c < W / 2; c += kLoad) {
+                            if (c >= columns) break;
+                            float v[kLoad];
+                            if constexpr (kLoad == 64)
+                                tmem_ld64(src + d * W + c, v);
+                            else
+                                tmem_ld32(src + d * W + c, v);
+                            tmem_ld_wait();
+                            if (c + kLoad >= columns) {  // all of the accumulator is in registers
+                                fence_before();
+                                __syncwarp();
+                                if (lane == 0) {
+                                    if constexpr (G == 2)
+                                        bar_turn_leader(report + d * 8);
+                                    else
+                                        bar_arrive(report + d * 8);
+                                }
+                            }
+                            if constexpr (kMarked) {
+#pragma unroll
+                                for (uint32_t i = 0; i < kLoad; i += 4) {
+                                    const float4 x = *reinterpret_cast<const float4 *>(units + c + i);
+                                    v[i] *= x.x;
+                                    v[i + 1] *= x.y;
+                                    v[i + 2] *= x.z;
+                                    v[i + 3] *= x.w;
+                                }
+                            }
+#pragma unroll
+                            for (uint32_t i = 0; i < kLoad; i += 2) pg_fma2(acc + c + i, s, v + i);
+                        }
                     }
+                    sc = sc_next;
                 }
-                sc = sc_next;
+            };
+            // the units of blocks for all positions of this warp, if one is marked
+            if ((marked_tiles[warp - 8] >> (u % p.pos_tiles)) & 1)
+                sweep(std::true_type());
+            else
+                sweep(std::false_type());
+            {  // what is left of the units: a factor per column, one for marked tiles
+                const bool in_blocks = (marked_tiles[warp - 8] >> (u % p.pos_tiles)) & 1;
+                __syncwarp();
+#pragma unroll
+                for (uint32_t i = 0; i < W / 64; ++i) {
+                    const uint32_t at = t.n0 + first + i * 32 + lane;
+                    unit_stage[warp - 8][i * 32 + lane] = in_blocks || at >= p.m ? 1.0f : p.unit[at];
+                }
+                __syncwarp();
             }
             if (ok && row < p.rows) {
                 const float so = (p.s_out ? p.s_out[row] : 1.0f) * code_unit(DT);
@@ -391,7 +456,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
                 float *y = p.y + t.sp * p.split_stride + (size_t)n0 * p.rows + row;
 #pragma unroll
                 for (uint32_t i = 0; i < W / 2; ++i)
-                    if (i < columns && n0 + i < p.m) y[(size_t)i * p.rows] = acc[i] * p.unit[n0 + i] * so;
+                    if (i < columns && n0 + i < p.m) y[(size_t)i * p.rows] = acc[i] * unit_stage[warp - 8][i] * so;
             }
         }
     }
@@ -419,10 +484,10 @@ ctox_status pg_launch(ctox_ctx *ctx, PgParams &p) {
         if (attr.numRegs != 128) return fail(ctx, CTOX_INVALID_STATE, "packed product: built with %d registers", attr.numRegs);
     }
     const uint32_t stage = PgCfg<W, G>::kABytes + p.n / G * 256;
-    p.stages = ((uint32_t)ctx->max_smem_optin - 2048) / stage;
+    p.stages = ((uint32_t)ctx->max_smem_optin - 2048 - 16 * W) / stage;  // beside the barriers and 16 W bytes of units
     if (p.stages > kPgStages) p.stages = kPgStages;
     const size_t smem = (size_t)p.stages * stage + 1024;
-    CTOX_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024));
+    CTOX_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024 - 16 * (int)W));
     const uint32_t slots = (uint32_t)ctx->sm_count / G, grid = (p.units < slots ? p.units : slots) * G;
     if constexpr (G == 2)
         CTOX_CUDA(ctx, launch_pdl_cluster(kernel, dim3(grid), dim3(kPgThreads), smem, ctx->stream, 2, p));
@@ -448,6 +513,8 @@ ctox_status launch_packed_gemm(ctox_matvec *mv, const LongIn &in, uint32_t m, ui
     p.w = part.prep;
     p.x = in.x;
     p.unit = in.unit;
+    p.block_unit = in.block_unit;
+    p.spread = in.spread;
     p.s_out = mv->s_out;
     p.y = y;
     p.rows = (uint32_t)mv->rows;
@@ -469,7 +536,7 @@ ctox_status launch_packed_gemm(ctox_matvec *mv, const LongIn &in, uint32_t m, ui
         const uint32_t G = n > 128 ? 2 : 1, slots = (uint32_t)ctx->sm_count / G;
         const double step = G == 2 ? 0.53 + 0.00146 * n : 0.52 + 0.0009 * n;
         const uint32_t tiles = (m + n - 1) / n, tiles_r = (row_tiles + G - 1) / G;
-        if (tiles * n > in.pos_pad || p.rt0 % G) continue;
+        if (tiles * n > in.pos_pad || p.rt0 % G || tiles > 32) continue;
         for (uint32_t s = 1; s <= p.kst && s <= 16 && s * p.split_stride <= capacity; ++s) {
             const uint32_t units = tiles_r * tiles * s, rounds = (units + slots - 1) / slots;
             const double cost = rounds * (((p.kst + s - 1) / s) * 4 * step + 1.0) + (s - 1) * (0.5 + 1.6e-6 * p.split_stride);

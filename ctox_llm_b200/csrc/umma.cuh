@@ -162,6 +162,15 @@ __device__ __forceinline__ void mma_f16_pair(uint32_t d, uint64_t a, uint64_t b,
         "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
         : "memory");
 }
+// D = A B + D / 2^SHIFT, by one CTA or a pair.
+template <uint32_t G, uint32_t SHIFT>
+__device__ __forceinline__ void mma_f16_shifted(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::%4.kind::f16 [%0], %1, %2, %3, p, %5;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "n"(G), "n"(SHIFT)
+        : "memory");
+}
 __device__ __forceinline__ void commit_pair(uint32_t bar) {
     asm volatile(
         "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),

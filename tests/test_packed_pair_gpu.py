@@ -79,7 +79,7 @@ def exact(m, tokens):
 
 
 @pytest.mark.parametrize("dtype", [ctox.Q4B64, ctox.Q2B64])
-@pytest.mark.parametrize("outlier", [0, 14])
+@pytest.mark.parametrize("outlier", [0, 14, 24, 40])
 def test_pair_products_against_64_bits(dtype, outlier):
     """160, 200 and 256 positions: tiles of 160 to 256, the last one full or cut, over 71 row tiles and 39.5 of them. The sums
     of 79 and of 71 blocks are 32-bit: roundings of 2^-24 that add up at worst like their number, 9e-6 over both products
