@@ -35,6 +35,11 @@ struct TimedLaunch {
     int kind;
     double bytes, flops;
 };
+// Memory that its owner can do without: release(owner) frees it and returns true, or false if it is in use now.
+struct Spare {
+    void *owner;
+    bool (*release)(void *owner);
+};
 }
 struct ctox_ctx {
     int device = 0;
@@ -49,6 +54,7 @@ struct ctox_ctx {
     size_t pinned_bytes = 0;
     void *scratch = nullptr;        // context-owned device scratch of the selection kernels
     size_t scratch_bytes = 0;
+    std::vector<ctox::Spare> spares;  // given back, latest first, when an allocation of the context fails
     std::string last_error;
     // tensor parallelism: NCCL communicator over the GPUs of one box (tp.cu); world 1 = none
     int tp_rank = 0, tp_world = 1;
@@ -96,7 +102,8 @@ inline ctox_status fail(ctox_ctx *ctx, ctox_status code, const char *fmt, ...) {
 
 // Tracked allocation: every byte is accounted on the context so that a caller
 // can assert "nothing left" after destroying its handles.
-ctox_status dev_alloc(ctox_ctx *ctx, void **ptr, size_t bytes);
+// `optional`: memory the caller can do without, for which no spare is given back.
+ctox_status dev_alloc(ctox_ctx *ctx, void **ptr, size_t bytes, bool optional = false);
 void dev_free(ctox_ctx *ctx, void *ptr, size_t bytes);
 ctox_status ensure_pinned(ctox_ctx *ctx, size_t bytes);
 // Context-owned device scratch (not counted as a caller-visible allocation); grows on demand.

@@ -7,12 +7,26 @@
 namespace ctox {
 thread_local std::string g_create_error;
 
-ctox_status dev_alloc(ctox_ctx *ctx, void **ptr, size_t bytes) {
+static cudaError_t malloc_from_spares(ctox_ctx *ctx, void **ptr, size_t bytes) {
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    for (size_t i = ctx->spares.size(); e == cudaErrorMemoryAllocation && i > 0; --i) {
+        cudaGetLastError();
+        const Spare s = ctx->spares[i - 1];
+        if (!s.release(s.owner)) continue;
+        ctx->spares.erase(ctx->spares.begin() + (i - 1));
+        e = cudaMalloc(ptr, bytes);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
+ctox_status dev_alloc(ctox_ctx *ctx, void **ptr, size_t bytes, bool optional) {
     *ptr = nullptr;
     if (bytes == 0) return CTOX_OK;
-    cudaError_t e = cudaMalloc(ptr, bytes);
+    cudaError_t e = optional ? cudaMalloc(ptr, bytes) : malloc_from_spares(ctx, ptr, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
+        *ptr = nullptr;
         return fail(ctx, CTOX_MEMORY_BUDGET, "cudaMalloc(%zu) failed: %s", bytes,
                     cudaGetErrorString(e));
     }
@@ -45,9 +59,9 @@ ctox_status ensure_scratch(ctox_ctx *ctx, size_t bytes) {
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
     const size_t want = bytes < (1u << 20) ? (1u << 20) : bytes;
-    cudaError_t e = cudaMalloc(&ctx->scratch, want);
+    cudaError_t e = malloc_from_spares(ctx, &ctx->scratch, want);
     if (e != cudaSuccess) {
-        cudaGetLastError();
+        ctx->scratch = nullptr;
         return fail(ctx, CTOX_MEMORY_BUDGET, "cudaMalloc(%zu) failed: %s", want, cudaGetErrorString(e));
     }
     ctx->scratch_bytes = want;

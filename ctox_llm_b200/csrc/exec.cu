@@ -140,7 +140,9 @@ ctox_status ctox_exec_destroy(ctox_exec *e) {
     for (auto &ev : e->phase_ev)
         if (ev) cudaEventDestroy(ev);
     stack_destroy(e);
-    delete e->long_pass;
+    auto &spares = e->ctx->spares;
+    spares.erase(std::remove_if(spares.begin(), spares.end(), [e](const Spare &s) { return s.owner == e; }), spares.end());
+    long_release(e);
     delete e;
     return CTOX_OK;
 }
@@ -684,7 +686,8 @@ ctox_status ctox_exec_warmup(ctox_exec *e) {
         return fail(ctx, CTOX_INVALID_STATE, "warmup: MTP tensors missing");
     ctox_status rc = build_draft_head(e);
     if (rc) return rc;
-    if (e->h) {  // buffers exist from an earlier warmup
+    if (e->h) {  // buffers exist from an earlier warmup (those of long passes may have been given back)
+        EX(long_warmup(e));
         e->warmed = true;
         return ctox_exec_reset_session(e);
     }
@@ -1106,7 +1109,6 @@ ctox_status pass_logits(ctox_exec *e, uint32_t m, const uint32_t *places, uint32
         }
         return CTOX_OK;
     }
-    if (!e->logits) EX(xalloc(e, (void **)&e->logits, (size_t)kMaxPass * V * 4, true));
     EX(matvec_stream_prepared(e->lm_head, 0, m));
     matvec_finish_enqueue(e->lm_head, m, e->logits, V);
     for (uint32_t i = 0; i < n; ++i)
@@ -1118,7 +1120,6 @@ ctox_status pass_logits(ctox_exec *e, uint32_t m, const uint32_t *places, uint32
 ctox_status long_pass_logits(ctox_exec *e, const uint32_t *places, uint32_t n, float *out) {
     ctox_ctx *ctx = e->ctx;
     const size_t V = e->vocab_l, H = e->cfg.hidden_size;
-    if (n && !e->logits) EX(xalloc(e, (void **)&e->logits, (size_t)kMaxPass * V * 4, true));
     for (uint32_t i = 0; i < n; i += kMaxPass) {
         const uint32_t k = n - i < kMaxPass ? n - i : kMaxPass;
         for (uint32_t j = 0; j < k; ++j)
@@ -1137,11 +1138,20 @@ ctox_status extend_impl(ctox_exec *e, const uint32_t *tokens, uint64_t n, const 
     ctox_ctx *ctx = e->ctx;
     std::vector<uint32_t> places;
     uint64_t w = 0;
+    struct Busy {
+        ctox_exec *e;
+        ~Busy() {
+            if (e->long_pass) e->long_pass->busy = false;
+        }
+    } busy{e};
+    // ahead of the first pass: the allocation may give the long passes' buffers back
+    if (n_want && !e->stack && !e->logits) EX(xalloc(e, (void **)&e->logits, (size_t)kMaxPass * e->vocab_l * 4, true));
     for (uint64_t a = 0; a < n;) {
         if (cancelled(cancel)) return fail(ctx, CTOX_CANCELLED, "prefill cancelled at token %llu", (unsigned long long)a);
         const bool is_long = e->long_pass && n - a >= long_min(e);
         const uint32_t m = is_long ? (uint32_t)(n - a < e->long_pass->cap ? n - a : e->long_pass->cap) : pass_positions(e, n - a);
         *began = true;
+        if (is_long) e->long_pass->busy = true;
         if (e->cfg.mtp_num_hidden_layers && e->have_hidden && e->position > 0) {
             // keep the MTP cache exact: pairs (token p+1, final hidden p) of the block before
             uint32_t mt[kMaxPass];

@@ -590,7 +590,7 @@ uint32_t attention_splits(const ctox_exec *e, uint32_t per_group, uint64_t pos0,
     return (uint32_t)best;
 }
 
-constexpr uint32_t kLongCap = 1024;  // positions per pass: the buffers take 0.35 GB at the flagship's widths
+constexpr uint32_t kLongCap = 1024;  // positions per pass: the buffers take 0.39 GB at the flagship's widths
 
 AttnGeom geom(const ctox_exec *e) {
     const ctox_model_config &c = e->cfg;
@@ -721,9 +721,15 @@ ctox_status long_warmup(ctox_exec *e) {
     const uint32_t cap = c.max_context_tokens < kLongCap ? (c.max_context_tokens + 7) / 8 * 8 : kLongCap;
     const uint32_t pos_pad = cap + kLongPosTile;  // a last tile may start anywhere below cap
     LongPass *L = new LongPass();
-    const size_t owned = e->owned.size();
-    const uint64_t session = e->session_bytes;
-    auto get = [&](auto **p, size_t n) { return xalloc(e, (void **)p, n * sizeof(**p), true, false); };
+    e->long_pass = L;
+    auto get = [&](auto **p, size_t n) {
+        const ctox_status rc = dev_alloc(ctx, (void **)p, n * sizeof(**p), true);
+        if (!rc) {
+            L->owned.emplace_back((void *)*p, n * sizeof(**p));
+            e->session_bytes += n * sizeof(**p);
+        }
+        return rc;
+    };
     L->cap = cap;
     L->in.pos_pad = pos_pad;
     L->y_floats = (size_t)cap * rows;
@@ -742,17 +748,26 @@ ctox_status long_warmup(ctox_exec *e) {
     if (!rc) rc = get(&L->aq, (size_t)cap * e->q_width);
     if (!rc) rc = get(&L->attn, (size_t)cap * c.num_attention_heads * (c.head_dim + 2));
     if (!rc) rc = get(&L->tokens, cap);
-    if (rc) {  // no room: the model runs with short passes alone, as it would without them
-        while (e->owned.size() > owned) {
-            dev_free(ctx, e->owned.back().first, e->owned.back().second);
-            e->owned.pop_back();
-        }
-        e->session_bytes = session;
-        delete L;
-        return CTOX_OK;
-    }
-    e->long_pass = L;
+    if (rc)  // no room: the model runs with short passes alone, as it would without them
+        long_release(e);
+    else
+        ctx->spares.push_back(Spare{e, [](void *owner) {
+            ctox_exec *e = (ctox_exec *)owner;
+            if (e->long_pass->busy || cudaStreamSynchronize(e->ctx->stream) != cudaSuccess) return false;
+            long_release(e);
+            return true;
+        }});
     return CTOX_OK;
+}
+
+void long_release(ctox_exec *e) {
+    if (!e->long_pass) return;
+    for (auto &o : e->long_pass->owned) {
+        dev_free(e->ctx, o.first, o.second);
+        e->session_bytes -= o.second;
+    }
+    delete e->long_pass;
+    e->long_pass = nullptr;
 }
 
 ctox_status long_target_pass(ctox_exec *e, const uint32_t *tokens, uint32_t m) {

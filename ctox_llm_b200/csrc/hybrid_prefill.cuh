@@ -5,9 +5,11 @@
 
 namespace ctox {
 
-// Buffers of long passes, allocated at warm-up.
+// Buffers of long passes, allocated at warm-up and given back when another allocation of the context fails.
 struct LongPass {
     uint32_t cap = 0;  // positions
+    bool busy = false;  // a call that takes long passes is on its way
+    std::vector<std::pair<void *, size_t>> owned;
     LongIn in{};
     float *y = nullptr;  // outputs of a projection (partial sums)
     size_t y_floats = 0;
@@ -31,6 +33,7 @@ uint32_t long_min(const ctox_exec *e);
 
 // Allocates the buffers; leaves e->long_pass null (short passes only) where they do not fit or do not apply.
 ctox_status long_warmup(ctox_exec *e);
+void long_release(ctox_exec *e);
 // Consumes m tokens (long_min .. cap) at the session's position: target layers, committed state, the MTP cache of
 // all but the last (m - 1) % 8 + 1 pairs, which like those of a short pass are left to the next call.
 ctox_status long_target_pass(ctox_exec *e, const uint32_t *tokens, uint32_t m);
