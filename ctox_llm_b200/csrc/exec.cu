@@ -1161,7 +1161,7 @@ ctox_status extend_impl(ctox_exec *e, const uint32_t *tokens, uint64_t n, const 
             EX(mtp_pass(e, e->hist_n, e->position - e->hist_n + 1, e->mtp_tokens_dev, e->hist_hidden, -1));
         }
         if (is_long) {
-            EX(long_target_pass(e, tokens + a, m));
+            EX(long_target_pass(e, tokens + a, m, cancel));
         } else {
             EX(upload_u32(e, e->tokens_dev, tokens + a, m));
             EX(target_pass(e, m, e->position));

@@ -748,6 +748,8 @@ ctox_status long_warmup(ctox_exec *e) {
     if (!rc) rc = get(&L->aq, (size_t)cap * e->q_width);
     if (!rc) rc = get(&L->attn, (size_t)cap * c.num_attention_heads * (c.head_dim + 2));
     if (!rc) rc = get(&L->tokens, cap);
+    for (cudaEvent_t &ev : L->layer_done)
+        if (!rc && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) rc = CTOX_INVALID_STATE;
     if (rc)  // no room: the model runs with short passes alone, as it would without them
         long_release(e);
     else
@@ -766,11 +768,13 @@ void long_release(ctox_exec *e) {
         dev_free(e->ctx, o.first, o.second);
         e->session_bytes -= o.second;
     }
+    for (cudaEvent_t ev : e->long_pass->layer_done)
+        if (ev) cudaEventDestroy(ev);
     delete e->long_pass;
     e->long_pass = nullptr;
 }
 
-ctox_status long_target_pass(ctox_exec *e, const uint32_t *tokens, uint32_t m) {
+ctox_status long_target_pass(ctox_exec *e, const uint32_t *tokens, uint32_t m, const volatile int32_t *cancel) {
     ctox_ctx *ctx = e->ctx;
     const ctox_model_config &c = e->cfg;
     LongPass &L = *e->long_pass;
@@ -783,6 +787,10 @@ ctox_status long_target_pass(ctox_exec *e, const uint32_t *tokens, uint32_t m) {
     for (uint32_t l = 0; l < e->n_layers; ++l) {
         LayerW &lw = e->w[l];
         const bool last = l + 1 == e->n_layers;
+        if (cancel) {
+            if (l >= 2) CTOX_CUDA(ctx, cudaEventSynchronize(L.layer_done[l & 1]));
+            if (*cancel) return fail(ctx, CTOX_CANCELLED, "prefill cancelled in layer %u of a pass of %u tokens", l, m);
+        }
         EX(product(e, lw.in_fan, m, &o));
         EX(mixer(e, l, o, m, pos0));
         EX(product(e, lw.out, m, &o));
@@ -795,6 +803,7 @@ ctox_status long_target_pass(ctox_exec *e, const uint32_t *tokens, uint32_t m) {
         EX(product(e, lw.down, m, &o));
         EX(rows_norm(e, m, L.h, &o, last ? e->final_norm : e->w[l + 1].in_ln, last ? L.final_hidden : nullptr,
                      last ? nullptr : e->w[l + 1].in_fan));
+        if (cancel) CTOX_CUDA(ctx, cudaEventRecord(L.layer_done[l & 1], ctx->stream));
     }
     // What the pass leaves is committed. The last pairs stay for the next call, as many as a short pass would leave.
     const uint32_t keep = (m - 1) % kMaxPass + 1, pairs = m - keep;

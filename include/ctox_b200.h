@@ -531,8 +531,9 @@ ctox_status ctox_exec_warmup(ctox_exec *exec);
 ctox_status ctox_exec_reset_session(ctox_exec *exec);
 /* Cancellation (engine.rs:364-377 CancellationToken = Arc<AtomicBool>): `cancel` points to a
  * word another thread may set to non-zero at any time, or is NULL. It is read on the host at
- * entry and between passes; a call that sees it returns CTOX_CANCELLED (error.rs:5-29). A
- * cancelled decode leaves the session as it was before the call; a cancelled prefill leaves no
+ * entry and between passes (prompts of the hybrid model in passes of up to 1024 tokens: also before
+ * every layer, two layers ahead of the device); a call that sees it returns CTOX_CANCELLED
+ * (error.rs:5-29). A cancelled decode leaves the session as it was before the call; a cancelled prefill leaves no
  * usable session (reset_session or a new prefill). */
 
 /* prefill(): runs the tokens through the target (and the MTP cache) in chunks;
