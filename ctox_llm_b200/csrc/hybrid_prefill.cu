@@ -608,7 +608,6 @@ ctox_status rows(ctox_exec *e, RowsArgs &a, uint32_t m, ctox_matvec *next) {
         a.dt = next->parts[0].dt;
     }
     const size_t smem = (next ? (size_t)next->blocks_padded * 65 : a.width) * 4;
-    CTOX_CUDA(ctx, cudaFuncSetAttribute(k_long_rows<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024));
     CTOX_CUDA(ctx, launch_pdl(k_long_rows<MODE>, dim3(m), dim3(kRowsThreads), smem, ctx->stream, a));
     return CTOX_OK;
 }
@@ -718,6 +717,12 @@ ctox_status long_warmup(ctox_exec *e) {
         blocks = mv->blocks_padded > blocks ? mv->blocks_padded : blocks;
         rows = mv->rows > rows ? mv->rows : rows;
     }
+    bool usable = false;
+    EX(packed_gemm_init(ctx, &usable));
+    if (!usable) return CTOX_OK;
+    for (auto kernel : {k_long_rows<ROWS_NORM>, k_long_rows<ROWS_SWIGLU>, k_long_rows<ROWS_ATTENTION>, k_long_rows<ROWS_DELTA>,
+                        k_long_rows<ROWS_MTP>})
+        CTOX_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024));
     const uint32_t cap = c.max_context_tokens < kLongCap ? (c.max_context_tokens + 7) / 8 * 8 : kLongCap;
     const uint32_t pos_pad = cap + kLongPosTile;  // a last tile may start anywhere below cap
     LongPass *L = new LongPass();

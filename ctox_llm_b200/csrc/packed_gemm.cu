@@ -476,18 +476,21 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_packed_gemm(const PgParams p)
 namespace {
 
 template <int DT, uint32_t W, uint32_t G>
+ctox_status pg_init(ctox_ctx *ctx, bool *usable) {
+    const auto kernel = k_packed_gemm<DT, W, G>;
+    cudaFuncAttributes attr;
+    CTOX_CUDA(ctx, cudaFuncGetAttributes(&attr, kernel));
+    if (W > 64 && attr.numRegs != 128) *usable = false;  // the split in the kernel counts on 128 per thread at launch
+    CTOX_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024 - 16 * (int)W));
+    return CTOX_OK;
+}
+template <int DT, uint32_t W, uint32_t G>
 ctox_status pg_launch(ctox_ctx *ctx, PgParams &p) {
     const auto kernel = k_packed_gemm<DT, W, G>;
-    if constexpr (W > 64) {  // the register split in the kernel counts on 128 per thread at launch
-        cudaFuncAttributes attr;
-        CTOX_CUDA(ctx, cudaFuncGetAttributes(&attr, kernel));
-        if (attr.numRegs != 128) return fail(ctx, CTOX_INVALID_STATE, "packed product: built with %d registers", attr.numRegs);
-    }
     const uint32_t stage = PgCfg<W, G>::kABytes + p.n / G * 256;
     p.stages = ((uint32_t)ctx->max_smem_optin - 2048 - 16 * W) / stage;  // beside the barriers and 16 W bytes of units
     if (p.stages > kPgStages) p.stages = kPgStages;
     const size_t smem = (size_t)p.stages * stage + 1024;
-    CTOX_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin - 1024 - 16 * (int)W));
     const uint32_t slots = (uint32_t)ctx->sm_count / G, grid = (p.units < slots ? p.units : slots) * G;
     if constexpr (G == 2)
         CTOX_CUDA(ctx, launch_pdl_cluster(kernel, dim3(grid), dim3(kPgThreads), smem, ctx->stream, 2, p));
@@ -501,6 +504,16 @@ ctox_status pg_launch(ctox_ctx *ctx, PgParams &p) {
 }
 
 }  // namespace
+
+ctox_status packed_gemm_init(ctox_ctx *ctx, bool *usable) {
+    *usable = true;
+    EX((pg_init<0, 64, 1>(ctx, usable)));
+    EX((pg_init<1, 64, 1>(ctx, usable)));
+    EX((pg_init<0, 128, 1>(ctx, usable)));
+    EX((pg_init<1, 128, 1>(ctx, usable)));
+    EX((pg_init<0, 256, 2>(ctx, usable)));
+    return pg_init<1, 256, 2>(ctx, usable);
+}
 
 ctox_status launch_packed_gemm(ctox_matvec *mv, const LongIn &in, uint32_t m, uint64_t row0, uint64_t row_end, float *y,
                                size_t capacity, LongOut *out) {

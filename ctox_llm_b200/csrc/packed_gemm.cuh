@@ -32,6 +32,9 @@ struct LongOut {
     size_t split_stride;  // floats between two partial sums
 };
 
+// Makes the kernels ready on the context's device; *usable: false where this build's kernels do not have the registers that
+// their warps share out.
+ctox_status packed_gemm_init(ctox_ctx *ctx, bool *usable);
 // y = W x for m positions; rows row0 .. row_end only (row0 rounded down to a tile of 128). `capacity`: floats
 // behind y. Recovery scales are applied; the result is in *out.
 ctox_status launch_packed_gemm(ctox_matvec *mv, const LongIn &in, uint32_t m, uint64_t row0, uint64_t row_end, float *y,
