@@ -14,17 +14,19 @@ CONFIGS = {
     # widths that are not whole tiles of 128 rows or 256 columns; CUDA-core attention over both cache types
     "ragged-f32": dict(kv_dtype=ctox.F32, hidden_size=320, intermediate_size=704),
     "ragged-bf16": dict(kv_dtype=ctox.BF16, hidden_size=320, intermediate_size=704),
-    # the tensor-core attention kernel, groups of eight positions; every second layer attention
+    # the tensor-core attention kernel; every second layer attention; groups of eight positions, and of five
     "head256": dict(num_attention_heads=4, num_key_value_heads=1, head_dim=256, rotary_dim=64, kv_dtype=ctox.BF16,
                     full_attention_interval=2),
+    "head256-6": dict(num_attention_heads=6, num_key_value_heads=1, head_dim=256, rotary_dim=64, kv_dtype=ctox.BF16,
+                      full_attention_interval=2),
 }
 
 
 @pytest.mark.parametrize("name", CONFIGS)
-@pytest.mark.parametrize("n", [9, 16, 17, 63, 65, 129, 300, 1025 + 40])
+@pytest.mark.parametrize("n", [17, 18, 31, 63, 65, 129, 300, 1025 + 40])
 def test_long_pass_equals_short_passes(orc, name, n):
-    """n crosses the tiles of 64 / 128 / 256 positions, the groups of 8 positions and of 16 tokens, and the 1024
-    positions of one pass. Both sides sum the same products in 32 bits in another order: 1e-4 of the logits for a 32-bit
+    """n crosses the groups of 5 and 8 positions and of 16 tokens, and the 1024 positions of one pass; at these widths the
+    products take tiles of 32 to 112 positions, one to ten of them (test_packed_pair_gpu.py has the wide ones). Both sides sum the same products in 32 bits in another order: 1e-4 of the logits for a 32-bit
     cache; rounding keys and values to 16 bits turns such differences into steps of 2^-9 (1e-3, the bound of the
     oracle's comparisons)."""
     be = ctox.B200Backend(0)
@@ -39,7 +41,13 @@ def test_long_pass_equals_short_passes(orc, name, n):
         prompt = [int(t) for t in np.random.default_rng(n).integers(0, cfg.vocab_size, n + 1)]
         want = sorted({0, 7, 8, n // 2, n - 2, n - 1})
         runs = []
+        launches = {}
         for step in (n, 8):
+            ex.reset_session()
+            before = be.kernel_launches()
+            for a in range(0, n, step):
+                ex.extend(prompt[a:min(a + step, n)])
+            launches[step] = be.kernel_launches() - before
             ex.reset_session()
             rows = []
             for a in range(0, n, step):
@@ -56,6 +64,7 @@ def test_long_pass_equals_short_passes(orc, name, n):
                 ex.decode(tok, mtp_enabled=True, force_accept=0)
                 out += [ex.last_logits(0)[None], np.stack(ex.last_draft_logits()[:1]), np.stack(ex.last_mtp_hidden()[:1])]
             runs.append(out)
+        assert launches[n] < 0.8 * launches[8], "a long pass where the other side has three short ones or more"
         for got, ref in zip(*runs):
             for g, r in zip(got, ref):
                 assert rel_l2(g, r) <= bound
