@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(512, 1) k_linear_attention(LinearAttnArgs a, i
         }
     }
     __syncthreads();
-    // L2 norms of q and k for all positions at once, with the reduction tree of the stand-alone scan
+    // L2 norms of q and k for all positions at once, with the reduction tree of delta_scan128_body
     // (value d in lane d % 32 of warp d / 32, butterfly, then the four warp sums in order); then the
     // normalised key and the scaled query replace q and k in shared memory, as in the scan
     if (warp < 8) {
