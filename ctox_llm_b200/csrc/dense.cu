@@ -1,6 +1,7 @@
 // Matrix-vector products with dense bf16 weights for short passes, the norms of longer passes, and
 // the small kernels that go with them (embedding rows, weight layout).
 #include "dense.cuh"
+#include "dense_device.cuh"
 
 #include <map>
 #include <mutex>
@@ -11,28 +12,9 @@ namespace ctox {
 constexpr int kDvThreads = 256, kDvWarps = kDvThreads / 32;
 constexpr uint64_t kUnitCost = 20000;                        // of a unit of rows, in columns
 constexpr uint32_t kBatch = 4;                               // vectors a thread requests at once
+constexpr uint32_t kMergeBatch = 16;                        // the same where attention splits are merged
 constexpr int kSplitLanes = (kAttnSplitsDense + 31) / 32;  // splits per lane of a merging warp
 
-// Columns c .. c + 3 of p, zero from `end` on.
-__device__ __forceinline__ float4 load4(const float *p, uint32_t c, uint32_t end, bool vec) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (c + 4 <= end && vec) return *reinterpret_cast<const float4 *>(p + c);
-    if (c < end) v.x = p[c];
-    if (c + 1 < end) v.y = p[c + 1];
-    if (c + 2 < end) v.z = p[c + 2];
-    if (c + 3 < end) v.w = p[c + 3];
-    return v;
-}
-__device__ __forceinline__ void store4(float *p, uint32_t c, uint32_t end, const float4 &v) {
-    if (c + 4 <= end && ((uintptr_t)p & 15) == 0) {
-        *reinterpret_cast<float4 *>(p + c) = v;
-        return;
-    }
-    if (c < end) p[c] = v.x;
-    if (c + 1 < end) p[c + 1] = v.y;
-    if (c + 2 < end) p[c + 2] = v.z;
-    if (c + 3 < end) p[c + 3] = v.w;
-}
 __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // Sum over the kDvThreads / M threads of a position (whole warps); every thread of the CTA calls it.
@@ -50,39 +32,6 @@ __device__ __forceinline__ float position_sum(float v, float *red) {
 #pragma unroll
     for (int i = 0; i < W; ++i) s += red[warp / W * W + i];
     return s;
-}
-
-__device__ void latent_append_row(const LatentAppend &a, uint32_t m, uint32_t tid, uint32_t nthreads, float *red) {
-    const float *row = a.fan + (size_t)m * a.fan_stride + a.fan_off;
-    float sq = 0.f;
-    for (uint32_t c = tid; c < a.kv_rank; c += nthreads) sq += row[c] * row[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    __syncthreads();
-    if ((tid & 31) == 0) red[tid >> 5] = sq;
-    __syncthreads();
-    float total = 0.f;
-    for (uint32_t w = 0; w < nthreads / 32; ++w) total += red[w];
-    const float inv = 1.0f / sqrtf(total / (float)a.kv_rank + a.eps);
-    const uint32_t pos = a.pos0 + m;
-    const size_t base = paged_slot(a.page_table, a.page_tokens, pos) * (a.kv_pad + a.rot_pad);
-    auto store = [&](uint32_t c, float v) {
-        if (a.bf16)
-            ((__nv_bfloat16 *)a.cache)[base + c] = __float2bfloat16_rn(v);
-        else
-            ((float *)a.cache)[base + c] = v;
-    };
-    for (uint32_t c = tid; c < a.kv_pad; c += nthreads) store(c, c < a.kv_rank ? row[c] * inv * a.norm_w[c] : 0.f);
-    for (uint32_t i = tid; i < a.rot_pad / 2; i += nthreads) {
-        float u = 0.f, v = 0.f;
-        if (2 * i < a.rot_dim) {
-            u = row[a.kv_rank + 2 * i];
-            v = row[a.kv_rank + 2 * i + 1];
-            rope_pair(u, v, (float)pos * a.freq[i]);
-        }
-        store(a.kv_pad + 2 * i, u);
-        store(a.kv_pad + 2 * i + 1, v);
-    }
 }
 
 // One warp group of 2^lpr_log2 lanes per R rows, `ks` warps side by side on the columns of the same
@@ -105,7 +54,7 @@ __global__ void __launch_bounds__(kDvThreads, 2)
     k_dense_matvec(const __nv_bfloat16 *__restrict__ W, uint32_t ld, uint32_t rows_per_group, uint32_t units_per_group,
                    uint32_t units, uint32_t ks, uint32_t lpr_log2, uint32_t npos, VecIn in, VecOut out,
                    LatentAppend ap, uint32_t append_positions) {
-    pdl_launch();
+    if (!append_positions) pdl_launch();  // else after the wait (dense.cuh)
     extern __shared__ __align__(16) float xs[];  // [M][ldx]
     __shared__ float red[kDvWarps];
     __shared__ float part[kDvWarps][32 * 4];  // partial sums of the column parts: [warp][subgroup rows x positions]
@@ -114,6 +63,7 @@ __global__ void __launch_bounds__(kDvThreads, 2)
     const uint32_t grid = gridDim.x - append_positions;
     if (blockIdx.x >= grid) {
         pdl_wait();
+        pdl_launch();
         latent_append_row(ap, blockIdx.x - grid, tid, kDvThreads, red);
         return;
     }
@@ -179,14 +129,14 @@ __global__ void __launch_bounds__(kDvThreads, 2)
             each(ldx, [&](uint32_t c) {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (c < end)
-                    for (uint32_t s0 = 0; s0 < in.splits; s0 += kBatch * 2) {
-                        float4 o[kBatch * 2];
+                    for (uint32_t s0 = 0; s0 < in.splits; s0 += kMergeBatch) {
+                        float4 o[kMergeBatch];
 #pragma unroll
-                        for (uint32_t i = 0; i < kBatch * 2; ++i)
+                        for (uint32_t i = 0; i < kMergeBatch; ++i)
                             o[i] = s0 + i < in.splits ? *reinterpret_cast<const float4 *>(in.ws_o + ((size_t)(s0 + i) * in.ws_rows + row) * cols + c)
                                                       : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                        for (uint32_t i = 0; i < kBatch * 2; ++i) {
+                        for (uint32_t i = 0; i < kMergeBatch; ++i) {
                             const float w = s0 + i < in.splits ? mw[pm][s0 + i] : 0.f;
                             v.x = fmaf(w, o[i].x, v.x);
                             v.y = fmaf(w, o[i].y, v.y);
@@ -301,9 +251,10 @@ __global__ void __launch_bounds__(kDvThreads, 2)
 #pragma unroll
         for (int d = 0; d < D; ++d) fetch(base, row0, d, buf[d]);
         if (group != staged) {
-            if (staged == 0xffffffffu)
+            if (staged == 0xffffffffu) {
                 pdl_wait();
-            else
+                if (append_positions) pdl_launch();
+            } else
                 __syncthreads();
             stage(group);
             __syncthreads();
@@ -377,28 +328,7 @@ __global__ void __launch_bounds__(kDvThreads, 2)
                     }
                 const uint32_t m = k / R, row = row0 + k % R;
                 if (m >= npos || row >= rows_per_group) continue;
-                if (out.bias) {
-                    v += out.bias[(size_t)group * rows_per_group + row];
-                    if ((row ^ 1u) < rows_per_group) pair += out.bias[(size_t)group * rows_per_group + (row ^ 1u)];
-                }
-                if (out.kind == OUT_CLAMPED_GLU) {
-                    if (!(row & 1)) out.y[(size_t)m * out.y_stride + (row >> 1)] = clamped_glu(v, pair, out.cap, out.slope);
-                    continue;
-                }
-                if (out.kind == OUT_RELU2) {
-                    v = v > 0.f ? v * v : 0.f;
-                } else if (out.kind == OUT_SOFTCAP) {
-                    v = out.cap * tanhf(v / out.cap);
-                } else if (out.kind == OUT_ROPE) {
-                    const uint32_t w = row % out.head_width;
-                    if (w >= out.rope0 && w < out.rope0 + out.rope_dims) {
-                        const float angle = (float)(out.pos0 + m) * out.freq[(w - out.rope0) >> 1];
-                        float a = (w & 1) ? pair : v, b = (w & 1) ? v : pair;
-                        rope_pair(a, b, angle);
-                        v = (w & 1) ? b : a;
-                    }
-                }
-                out.y[(size_t)m * out.y_stride + (size_t)group * rows_per_group + row] = v;
+                emit_row(out, m, group * rows_per_group, row, v, pair, row_constants(out, m, row, rows_per_group, group * rows_per_group));
             }
         }
     }
@@ -454,6 +384,11 @@ ctox_status matvec_launch(ctox_ctx *ctx, const DenseMat &w, uint32_t groups, uin
 
 ctox_status launch_dense_matvec(ctox_ctx *ctx, const DenseMat &w, uint32_t groups, uint32_t m, const VecIn &in,
                                 const VecOut &out, const LatentAppend *append) {
+    if (m == 1 && groups == 1) {
+        bool taken = false;
+        EX(launch_dense_stream(ctx, w, in, out, append, &taken));
+        if (taken) return CTOX_OK;
+    }
     uint32_t lpr_log2 = 5;  // lanes per row: fewer for narrow matrices
     while (lpr_log2 > 3 && w.ld <= (8u << (lpr_log2 - 1))) --lpr_log2;
     const uint32_t span = 8u << lpr_log2, nsteps = (w.ld + span - 1) / span;

@@ -74,9 +74,19 @@ struct LatentAppend {
 };
 
 // y = W x for m <= kDensePass positions; groups > 1: rows and inputs come in `groups` equal parts. With
-// `append`, extra CTAs of the same launch append the m positions to the latent cache.
+// `append`, extra CTAs of the same launch append the m positions to the latent cache, and the launch lets the next kernel start
+// only after its own dependency wait: a kernel that starts later may then read what earlier passes left in the
+// cache ahead of its own wait (stack_attention.cu).
 ctox_status launch_dense_matvec(ctox_ctx *ctx, const DenseMat &w, uint32_t groups, uint32_t m, const VecIn &in,
                                 const VecOut &out, const LatentAppend *append);
+
+// One position and one group through k_dense_stream (dense_stream.cu), where the matrix has at least kDenseStreamBytes and its
+// rows fit that kernel's shape; *taken says whether.
+// (Taken from 1, 4 and 12 MB on, 16 tokens of the latent model take 16.8, 16.8 and 17.1 ms, a Vasanex request 17.5, 17.2 and 17.2;
+// that was before the ring was cut to kDsRoom.)
+constexpr size_t kDenseStreamBytes = 4 << 20;
+ctox_status launch_dense_stream(ctox_ctx *ctx, const DenseMat &w, const VecIn &in, const VecOut &out, const LatentAppend *append,
+                                bool *taken);
 
 // x <- x + layer_norm(y; wb), or x + y without wb (y may be null; x_out may equal x), then the norm (w) of
 // the result as fp32 and / or bf16. One CTA per row; `rows` (device, may be null) picks input rows.
@@ -120,12 +130,15 @@ ctox_status launch_fill_normal_f32(ctox_ctx *ctx, float *out, uint64_t n, float 
 
 #ifdef __CUDACC__
 namespace ctox {
-__device__ __forceinline__ void rope_pair(float &u, float &v, float angle) {
-    float s, c;
-    sincosf(angle, &s, &c);
+__device__ __forceinline__ void turn_pair(float &u, float &v, float s, float c) {
     const float a = u * c - v * s, b = v * c + u * s;
     u = a;
     v = b;
+}
+__device__ __forceinline__ void rope_pair(float &u, float &v, float angle) {
+    float s, c;
+    sincosf(angle, &s, &c);
+    turn_pair(u, v, s, c);
 }
 // Gated feed-forward with clamped inputs: g = min(gate, limit), u = clamp(up, +-limit); g sigmoid(slope g) (u + 1).
 __device__ __forceinline__ float clamped_glu(float gate, float up, float limit, float slope) {
