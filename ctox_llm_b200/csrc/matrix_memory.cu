@@ -6,14 +6,18 @@
 namespace ctox {
 
 namespace cg = cooperative_groups;
-constexpr int kMmThreads = 256, kMmWarps = kMmThreads / 32, kMmRows = 4;  // state rows a warp works on at once
+constexpr int kMmThreads = 256, kMmWarps = kMmThreads / 32;
+// State rows a warp works on at once. A decode step is a chain of round trips: with nine rows a CTA of 65 (512 value dimensions over
+// eight CTAs, and the normaliser) takes one trip to its state instead of three.
+__host__ __device__ constexpr int mm_rows(int m) { return m == 1 ? 9 : 4; }
 
 // A cluster per head, its CTAs share the state's rows (value dimensions, the normaliser behind them). A row stays
 // in registers for all M positions: the gates' scales of every position are known before the state is touched.
 // The head's norm needs the outputs of all CTAs: they meet through distributed shared memory.
 template <int M>
-__global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, const float *__restrict__ fan, uint32_t fan_stride,
+__global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, const float *fan, uint32_t fan_stride,
                                                               uint32_t gate_off, uint32_t npos, uint32_t rows_per, float *__restrict__ out) {
+    constexpr int kMmRows = mm_rows(M);
     pdl_launch();
     extern __shared__ __align__(16) float sm[];
     __shared__ float keep[M], take[M], floor_s[M], part[kMmWarps][M];
@@ -29,8 +33,17 @@ __global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, co
     const uint32_t rows = row_beg < all ? min(rows_per, all - row_beg) : 0;
     float *state = a.state + (size_t)head * (a.vdim_pad + kMemRows) * a.dim_pad;
     auto state_row = [&](uint32_t r) { return state + (size_t)(r < a.vdim ? r : a.vdim_pad) * a.dim_pad; };
+    // The state may still be in HBM: ask L2 for it ahead of the wait (its values are read after it).
+    for (uint32_t i = tid; i < rows * (a.dim_pad / 32); i += kMmThreads)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(state_row(row_beg + i / (a.dim_pad / 32)) + i % (a.dim_pad / 32) * 32));
+    // What a thread's first output needs at the end: the norm's weight is a constant, the gate comes with the other inputs. (fan is
+    // not __restrict__: loads from const __restrict__ memory may be moved ahead of the wait.)
+    const uint32_t out_t = rows ? tid / rows : 0, out_v = rows ? row_beg + tid % rows : 0;
+    const bool has_out = rows && out_t < npos && out_v < a.vdim;
+    const float norm_w = has_out ? a.norm_w[head * a.vdim + out_v] : 0.f;
     pdl_wait();
     const uint32_t k_off = a.heads * a.dim_pad, v_off = 2 * k_off, g_off = v_off + a.heads * a.vdim_pad;
+    const float gate = has_out ? fan[(size_t)out_t * fan_stride + g_off + head * a.vdim_pad + out_v] : 0.f;
     if (warp == 0) {  // lane = position; the running maximum goes from lane to lane
         float i = 0.f, f = 0.f, top = a.top[head], before = 0.f, after = 0.f;
         if (lane < npos) {
@@ -77,6 +90,7 @@ __global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, co
 #pragma unroll
             for (int t = 0; t < M; ++t) acc[r][t] = 0.f;
         }
+#pragma unroll(M == 1 ? 2 : 1)
         for (uint32_t d = lane * 4; d < a.dim_pad; d += 128) {
             float4 s[kMmRows];
 #pragma unroll
@@ -147,9 +161,10 @@ __global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, co
     for (uint32_t i = tid; i < npos * rows; i += kMmThreads) {
         const uint32_t t = i / rows, r = i % rows, v = row_beg + r;
         if (v >= a.vdim) continue;
-        const float g = fan[(size_t)t * fan_stride + g_off + head * a.vdim_pad + v];
+        const bool first = i == tid;
+        const float g = first ? gate : fan[(size_t)t * fan_stride + g_off + head * a.vdim_pad + v];
         out[(size_t)t * a.heads * a.vdim_pad + head * a.vdim_pad + v] =
-            num[t * rows_per + r] * part[0][t] * part[1][t] * a.norm_w[head * a.vdim + v] * sigmoid(g);
+            num[t * rows_per + r] * part[0][t] * part[1][t] * (first ? norm_w : a.norm_w[head * a.vdim + v]) * sigmoid(g);
     }
     if (rank == 0)
         for (uint32_t i = tid; i < npos * (a.vdim_pad - a.vdim); i += kMmThreads)

@@ -8,7 +8,6 @@ constexpr int kQkvThreads = 512;
 // One CTA per (position, share of the outputs). Every CTA of a position brings the projections into shared memory and
 // forms the norms over the whole query and key projection itself; a thread then makes groups of four outputs.
 __global__ void __launch_bounds__(kQkvThreads) k_qkv_prep(QkvPrep a) {
-    pdl_launch();
     extern __shared__ __align__(16) float sm[];
     __shared__ float red[2][kQkvThreads / 32];
     const uint32_t m = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pos = a.pos0 + m;
@@ -20,12 +19,16 @@ __global__ void __launch_bounds__(kQkvThreads) k_qkv_prep(QkvPrep a) {
         sincosf((float)pos * a.freq[i], &s, &c);
         cs_s[i] = make_float2(c, s);
     }
+    // the slot and the mixing weight are constants
+    const size_t base = paged_slot(a.page_table, a.page_tokens, pos) * (a.kv_heads * (a.dim_pad + a.vdim_pad));
+    const float mix = a.v_mix ? *a.v_mix : 0.f;
     // the norms' weights are constants: bring their lines in before the wait
     for (uint32_t c = tid * 32; c < nq + nk; c += kQkvThreads * 32) {
         const float *w = c < nq ? a.q_norm : a.k_norm;
         if (w) asm volatile("prefetch.global.L1 [%0];" ::"l"(w + (c < nq ? c : c - nq)));
     }
     pdl_wait();
+    pdl_launch();  // not before: the attention after it reads earlier passes' cache rows ahead of its own wait
     const float *row = a.fan + (size_t)m * a.fan_stride;
     float sq = 0.f, sk = 0.f;
     auto add = [&](uint32_t c, float v) {
@@ -112,8 +115,6 @@ __global__ void __launch_bounds__(kQkvThreads) k_qkv_prep(QkvPrep a) {
         }
     };
     const uint32_t q_groups = a.heads * a.dim_pad / 4, part = a.dim_pad + a.vdim_pad, slot_cols = a.kv_heads * part;
-    const size_t base = paged_slot(a.page_table, a.page_tokens, pos) * slot_cols;
-    const float mix = a.v_mix ? *a.v_mix : 0.f;
     for (uint32_t g = blockIdx.x * kQkvThreads + tid; g < q_groups + slot_cols / 4; g += gridDim.x * kQkvThreads) {
         __align__(16) float r[4];
         if (g < q_groups) {

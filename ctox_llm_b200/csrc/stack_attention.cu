@@ -54,39 +54,45 @@ __device__ void merge_splits(const CacheAttn &a, const PartRows<true> &pr, uint3
     for (uint32_t r = row0 + warp; r < row0 + tile_rows && r < pr.n; r += blockDim.x >> 5) {
         const uint32_t row = pr.row(r);
         const float sink = a.sink ? a.sink[row % a.heads] : -INFINITY;
-        float mv[kSplitLanes], mx = sink, den = 0.f;
+        // the first splits' values are on their way while the weights are formed
+        constexpr uint32_t kBatch = 16;
+        float4 o[kBatch];
+        auto fetch = [&](uint32_t c, uint32_t s0) {
+#pragma unroll
+            for (uint32_t i = 0; i < kBatch; ++i)
+                o[i] = s0 + i < splits && c < a.val_cols
+                           ? __ldcg(reinterpret_cast<const float4 *>(a.ws_o + ((size_t)(s0 + i) * rows + row) * a.val_cols + c))
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        fetch(lane * 4, 0);
+        float mv[kSplitLanes], sv[kSplitLanes], mx = sink, den = 0.f;
 #pragma unroll
         for (int i = 0; i < kSplitLanes; ++i) {
             const uint32_t sp = lane + i * 32;
             const float2 ml = sp < splits ? __ldcg(reinterpret_cast<const float2 *>(a.ws_ml + ((size_t)sp * rows + row) * 2))
                                           : make_float2(-INFINITY, 0.f);
             mv[i] = ml.x;
+            sv[i] = ml.y;
             mx = fmaxf(mx, ml.x);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
 #pragma unroll
         for (int i = 0; i < kSplitLanes; ++i) {
-            const uint32_t sp = lane + i * 32;
             mv[i] = mv[i] == -INFINITY ? 0.f : expf(mv[i] - mx);
-            if (sp < splits) den += __ldcg(a.ws_ml + ((size_t)sp * rows + row) * 2 + 1) * mv[i];
+            if (lane + i * 32 < splits) den += sv[i] * mv[i];
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+        for (int d = 16; d > 0; d >>= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
         if (a.sink) den += expf(sink - mx);
         const float inv = 1.0f / den;
         for (uint32_t c0 = 0; c0 < a.val_cols; c0 += 128) {
             const uint32_t c = c0 + lane * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (uint32_t s0 = 0; s0 < splits; s0 += 8) {
-                float4 o[8];
+            for (uint32_t s0 = 0; s0 < splits; s0 += kBatch) {
+                if (c0 || s0) fetch(c, s0);
 #pragma unroll
-                for (uint32_t i = 0; i < 8; ++i)
-                    o[i] = s0 + i < splits && c < a.val_cols
-                               ? __ldcg(reinterpret_cast<const float4 *>(a.ws_o + ((size_t)(s0 + i) * rows + row) * a.val_cols + c))
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (uint32_t i = 0; i < 8; ++i) {
+                for (uint32_t i = 0; i < kBatch; ++i) {
                     const uint32_t sp = s0 + i;
                     float w = 0.f;
 #pragma unroll
@@ -265,7 +271,6 @@ __global__ void __launch_bounds__(kCaThreads, NT <= 2 ? 2 : 1) k_cache_attention
     const uint32_t tiles = (kr.hi - kr.lo + kCaTileMma - 1) / kCaTileMma;
     const uint32_t t_beg = (uint32_t)((uint64_t)tiles * sp / splits), t_end = (uint32_t)((uint64_t)tiles * (sp + 1) / splits);
     const uint32_t chunks = a.head_cols / 8;
-    pdl_wait();
     auto load_tile = [&](uint32_t tile, uint32_t stage) {
         // lane i < 8 looks the slot of this warp's row i up, for all lanes
         const uint32_t mine = kr.lo + tile * kCaTileMma + warp + (lane & 7) * kCaWarps;
@@ -283,8 +288,17 @@ __global__ void __launch_bounds__(kCaThreads, NT <= 2 ? 2 : 1) k_cache_attention
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (t_beg < t_end) load_tile(t_beg, 0);
-    if (stages == 2 && t_beg + 1 < t_end) load_tile(t_beg + 1, 1);
+    // Tiles of earlier passes' tokens are requested ahead of the dependency wait: the kernel of this pass that appends to the
+    // cache lets no later one start before all of the pass before has finished (dense.cuh, qkv.cu). A tile with tokens of this
+    // pass comes after the wait.
+    const uint32_t first = t_beg < t_end ? 1 + (stages == 2 && t_beg + 1 < t_end) : 0;
+    uint32_t asked = 0;
+    while (asked < first && kr.lo + (t_beg + asked + 1) * kCaTileMma <= a.pos0) {
+        load_tile(t_beg + asked, asked);
+        ++asked;
+    }
+    pdl_wait();
+    for (; asked < first; ++asked) load_tile(t_beg + asked, asked);
     // ---- this warp's part of the queries: steps warp, warp + 8, ... as operand fragments
     const float qscale = a.scale * 1.4426950408889634f;  // scores in units of log 2
     uint32_t qh[NK][4], ql[NK][4];
