@@ -49,6 +49,7 @@ struct ctox_ctx {
     int max_smem_optin = 0;
     uint64_t allocated = 0;
     int32_t *dev_error = nullptr;   // device error word (kernels set, host reads)
+    uint32_t *arrived = nullptr;    // behind it: arrival counters of the selection kernels, zero between launches
     int32_t *host_error = nullptr;  // pinned mirror
     void *pinned = nullptr;         // pinned staging for the host-form calls
     size_t pinned_bytes = 0;

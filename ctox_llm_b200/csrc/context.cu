@@ -147,12 +147,13 @@ ctox_status ctox_ctx_create(int32_t device, void *stream, ctox_ctx **out) {
         }
         ctx->owns_stream = true;
     }
-    if (cudaMalloc(&ctx->dev_error, sizeof(int32_t)) != cudaSuccess ||
+    if (cudaMalloc(&ctx->dev_error, 4 * sizeof(int32_t)) != cudaSuccess ||
         cudaMallocHost(&ctx->host_error, sizeof(int32_t)) != cudaSuccess ||
-        cudaMemset(ctx->dev_error, 0, sizeof(int32_t)) != cudaSuccess) {
+        cudaMemset(ctx->dev_error, 0, 4 * sizeof(int32_t)) != cudaSuccess) {
         ctox_ctx_destroy(ctx);
         return fail(nullptr, CTOX_MEMORY_BUDGET, "context allocation failed");
     }
+    ctx->arrived = reinterpret_cast<uint32_t *>(ctx->dev_error) + 2;
     *out = ctx;
     return CTOX_OK;
 }

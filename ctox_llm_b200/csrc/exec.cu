@@ -1041,41 +1041,61 @@ ctox_status mtp_pass(ctox_exec *e, uint32_t m, uint64_t abs_pos0, const uint32_t
     launch_mtp_pre(ctx->stream, e->embed_rows, hidden_rows, e->mtp_norm_e, e->mtp_norm_h, c.rms_norm_epsilon,
                    c.hidden_size, m, &fc_in);
     EX(matvec_stream_prepared(e->mtp_fc, 0, m));
-    CTOX_CUDA(ctx, cudaMemsetAsync(e->mtp_h, 0, (size_t)m * c.hidden_size * 4, ctx->stream));
     const MvOut fc = mv_out(e->mtp_fc, m);
     const MvIn lin = mv_in(e->w[L].in_fan);
     launch_residual_norm_prep(ctx->stream, e->mtp_h, &fc, e->w[L].in_ln, c.rms_norm_epsilon, c.hidden_size, m, nullptr,
-                              &lin, e->norm_scratch);
+                              &lin, e->norm_scratch, true);
+    const bool restricted = c.draft_vocab != 0;
+    // null: no draft, or no draft row on this rank. A pass of one pair ends with the head's fragments.
+    ctox_matvec *head = draft_slot < 0 ? nullptr : restricted ? e->draft_head : e->lm_head;
     EX(layer_body(e, L, e->mtp_h, m, abs_pos0, abs_pos0 - 1, e->mtp_page_table, e->mtp_norm, e->mtp_hidden,
-                  nullptr));
+                  m == 1 ? head : nullptr));
     if (e->keep_logits && e->mtp_trace && e->mtp_trace_n + m <= 2 * kMaxPass) {
         CTOX_CUDA(ctx, cudaMemcpyAsync(e->mtp_trace + (size_t)e->mtp_trace_n * c.hidden_size, e->mtp_hidden,
                                        (size_t)m * c.hidden_size * 4, cudaMemcpyDeviceToDevice, ctx->stream));
         e->mtp_trace_n += m;
     }
     if (draft_slot >= 0) {
-        const bool restricted = c.draft_vocab != 0;
-        ctox_matvec *head = restricted ? e->draft_head : e->lm_head;  // null: no draft row on this rank
+        const uint32_t *ids = restricted ? e->draft_ids + e->draft_lo : nullptr;
+        uint32_t *token = e->tokens_dev + draft_slot;
         if (head) {
-            EX(matvec_stream_pass(head, 0, e->mtp_hidden + (size_t)(m - 1) * c.hidden_size, CTOX_F32, 1,
-                                  c.hidden_size));
-            matvec_finish_enqueue(head, 1, e->draft_logits, head->rows);
-            if (e->keep_logits && e->draft_trace && e->draft_trace_n < kMaxPass && head->rows <= e->draft_rows) {
-                CTOX_CUDA(ctx, cudaMemcpyAsync(e->draft_trace + (size_t)e->draft_trace_n * e->draft_rows,
-                                               e->draft_logits, (size_t)head->rows * 4, cudaMemcpyDeviceToDevice,
-                                               ctx->stream));
-                e->draft_trace_n += 1;
+            if (m == 1)
+                EX(matvec_stream_prepared(head, 0, 1));
+            else
+                EX(matvec_stream_pass(head, 0, e->mtp_hidden + (size_t)(m - 1) * c.hidden_size, CTOX_F32, 1, c.hidden_size));
+            float *logits = e->draft_logits;
+            if (e->keep_logits && e->draft_trace && e->draft_trace_n < kMaxPass && head->rows <= e->draft_rows)
+                logits = e->draft_trace + (size_t)e->draft_trace_n++ * e->draft_rows;
+            if (head->activation == CTOX_ACT_IDENTITY) {
+                EX(argmax_matvec_enqueue(head, logits, ids, e->vocab_off, token, nullptr));
+                return CTOX_OK;
             }
+            matvec_finish_enqueue(head, 1, logits, head->rows);
+            EX(argmax_enqueue(ctx, logits, (uint32_t)head->rows, ids, e->vocab_off, token, nullptr));
+            return CTOX_OK;
         }
-        EX(argmax_enqueue(ctx, e->draft_logits, head ? (uint32_t)head->rows : 0,
-                          restricted ? e->draft_ids + e->draft_lo : nullptr, e->vocab_off,
-                          e->tokens_dev + draft_slot, nullptr));
+        EX(argmax_enqueue(ctx, e->draft_logits, 0, ids, e->vocab_off, token, nullptr));
     }
     return CTOX_OK;
 }
 
+struct FewTokens {
+    uint32_t v[kMaxPass + 1];
+};
+__global__ void k_store_tokens(const __grid_constant__ FewTokens t, uint32_t n, uint32_t *dst) {
+    pdl_launch();
+    pdl_wait();
+    if (threadIdx.x < n) dst[threadIdx.x] = t.v[threadIdx.x];
+}
+
 ctox_status upload_u32(ctox_exec *e, uint32_t *dst, const uint32_t *src, uint32_t n) {
     ctox_ctx *ctx = e->ctx;
+    if (n <= kMaxPass + 1) {  // travel with the launch: a copy would keep the kernels around it from overlapping
+        FewTokens t{};
+        for (uint32_t i = 0; i < n; ++i) t.v[i] = src[i];
+        CTOX_CUDA(ctx, launch_pdl(k_store_tokens, dim3(1), dim3(32), 0, ctx->stream, t, n, dst));
+        return CTOX_OK;
+    }
     // pageable source: the copy is staged by the runtime before the call returns
     CTOX_CUDA(ctx, cudaMemcpyAsync(dst, src, n * 4, cudaMemcpyHostToDevice, ctx->stream));
     return CTOX_OK;
@@ -1240,25 +1260,28 @@ ctox_status decode_impl(ctox_exec *e, uint32_t token, int32_t mtp_enabled, float
     for (uint32_t i = 0; i < m; ++i) parent[i] = (int32_t)i - 1;
     const float inv_t = temperature > 0.f ? 1.0f / temperature : 0.f;
     const uint64_t step_id = e->step_counter++;
+    // one GPU: the kernel of the statistics walks the tree as well; a tensor-parallel group merges the ranks' first
+    const int force = force_accept < 0 ? -1 : (force_accept > (int32_t)k ? (int32_t)k : force_accept);
+    const int *walk = ctx->tp_world > 1 ? nullptr : &force;
     if (e->stack) {
         EX(stack_head_last(e));
-        EX(head_verify_logits_enqueue(ctx, e->logits, m, parent, e->tokens_dev, inv_t, seed, step_id, e->vocab_l));
+        EX(head_verify_logits_enqueue(ctx, e->logits, m, parent, e->tokens_dev, inv_t, seed, step_id, e->vocab_l, walk));
     } else {
         EX(matvec_stream_prepared(e->lm_head, 0, m));
         EX(head_verify_enqueue(e->lm_head, 0, m, m, parent, e->tokens_dev, inv_t, seed, step_id, e->vocab_l,
-                               e->keep_logits ? e->logits : nullptr, e->vocab_off));
+                               e->keep_logits ? e->logits : nullptr, e->vocab_off, walk));
     }
-    EX(head_tp_merge_enqueue(ctx, m, parent, e->tokens_dev, e->vocab_l));
     ctox_spec_record *rec_dev = nullptr;
-    EX(head_accept_enqueue(ctx, m, parent, e->tokens_dev, inv_t, seed, step_id,
-                           force_accept < 0 ? -1 : (force_accept > (int32_t)k ? (int32_t)k : force_accept),
-                           &rec_dev));
+    if (walk) {
+        EX(head_record(ctx, &rec_dev));
+    } else {
+        EX(head_tp_merge_enqueue(ctx, m, parent, e->tokens_dev, e->vocab_l));
+        EX(head_accept_enqueue(ctx, m, parent, e->tokens_dev, inv_t, seed, step_id, force, &rec_dev));
+    }
     if (e->phase_timing) cudaEventRecord(e->phase_ev[3], ctx->stream);
     EX(ensure_pinned(ctx, sizeof(ctox_spec_record) + 16));
-    CTOX_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, rec_dev, sizeof(ctox_spec_record), cudaMemcpyDeviceToHost,
+    CTOX_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, rec_dev, sizeof(ctox_spec_record) + sizeof(int32_t), cudaMemcpyDeviceToHost,
                                    ctx->stream));
-    CTOX_CUDA(ctx, cudaMemcpyAsync((uint8_t *)ctx->pinned + sizeof(ctox_spec_record), ctx->dev_error, 4,
-                                   cudaMemcpyDeviceToHost, ctx->stream));
     e->last_enqueue_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t_begin).count();
     CTOX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the one host read of the block
     if (e->phase_timing)

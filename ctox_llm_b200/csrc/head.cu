@@ -7,7 +7,7 @@
 // with ONE CTA); greedy MTP verification engine.rs:915-963 and the one-thread
 // accept kernel vendor/cuda/tensorrt_llm_mtp/mtp_accept_draft_token_sm86.cu:64-80.
 // The reference has no stochastic acceptance (engine.rs:583-590 fails closed);
-// the rule implemented here is stated in k_spec_accept.
+// the rule implemented here is stated at accept_walk.
 //
 // The lm_head logits are never written out: the streaming matvec leaves raw
 // per-piece sums, and k_head_stats turns them into per-position (argmax, max,
@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "head.cuh"
 #include "matvec.cuh"
+#include "prep.cuh"
 
 #include <cmath>
 #include <cstddef>
@@ -70,16 +71,126 @@ __device__ __forceinline__ void warp_merge(NodeStat &a) {
     }
 }
 
+// Walks the draft tree with the statistics of every node. One thread: the walk is
+// a dependent chain of at most kMaxNodes steps; the rest of the record is written side by side.
+//
+// Node 0 is the root (the current position). At node n with children c1..cm in
+// index order: with temperature 0, child c is accepted iff its token equals
+// argmax of n's logits (engine.rs:939-962); otherwise c is accepted with
+// probability p_n(c) / (1 - mass of its rejected elder siblings) on the draw
+// accept_draw(seed, step, c). The drafter is deterministic, so this is speculative
+// sampling with a point-mass proposal and the emitted token is distributed as
+// softmax(logits / T). When no child is accepted the token is the Gumbel-max
+// sample of p_n restricted to non-children (greedy: the argmax).
+//
+// Called by a whole CTA of at least kMaxNodes + 1 threads; node: shared memory, the statistics of all nodes.
+struct AcceptArgs {
+    float inv_temperature;
+    unsigned long long seed, step;
+    int force_accept;
+    ctox_spec_record *rec;  // null: no walk
+    const int32_t *error;   // the context's error word: its value is left behind the record, one copy brings both to the host
+};
+__device__ __forceinline__ void accept_walk(const NodeStat *node_stats, const float *child_z, const TreeDesc &tree, const AcceptArgs &a) {
+    __shared__ uint32_t token[kMaxNodes];
+    __shared__ float z[kMaxNodes];
+    const uint32_t t = threadIdx.x;
+    ctox_spec_record *rec = a.rec;
+    if (t < tree.n_nodes) {
+        rec->node_token[t] = token[t] = tree.token[t];
+        z[t] = __ldcg(child_z + t);
+    }
+    if (t < kMaxNodes) {
+        rec->node_argmax[t] = t < tree.n_nodes ? (uint32_t)(node_stats[t].argmax & 0xffffffffull) : 0u;
+        rec->path[t] = -1;
+    }
+    if (t <= kMaxNodes) rec->emitted[t] = 0;
+    __syncthreads();
+    if (t != 0) return;
+    uint32_t count = 0, node = 0, status = 0;
+    for (uint32_t n = 0; n < tree.n_nodes; ++n)
+        if (node_stats[n].nonfinite) status = 1;
+    if (status == 0 && a.force_accept >= 0) {
+        // throughput buckets: accept exactly force_accept drafts of the chain, then the target's token
+        while (count < (uint32_t)a.force_accept && node + 1 < tree.n_nodes) {
+            rec->path[count] = (int32_t)(node + 1);
+            rec->emitted[count++] = token[node + 1];
+            ++node;
+        }
+        rec->emitted[count++] = (uint32_t)(node_stats[node].argmax & 0xffffffffull);
+    } else if (status == 0) {
+        for (;;) {
+            const NodeStat st = node_stats[node];
+            bool moved = false;
+            if (!(a.inv_temperature > 0.f)) {
+                const uint32_t target = (uint32_t)(st.argmax & 0xffffffffull);
+                for (uint32_t c = node + 1; c < tree.n_nodes; ++c)
+                    if ((uint32_t)tree.parent[c] == node && token[c] == target) {
+                        rec->path[count] = (int32_t)c;
+                        rec->emitted[count++] = target;
+                        node = c;
+                        moved = true;
+                        break;
+                    }
+                if (!moved) {
+                    rec->emitted[count++] = target;
+                    break;
+                }
+                continue;
+            }
+            float residual = 1.0f;
+            for (uint32_t c = node + 1; c < tree.n_nodes; ++c) {
+                if ((uint32_t)tree.parent[c] != node) continue;
+                const float p = expf(z[c] - st.max) / st.sum;
+                const float u = accept_draw(a.seed, a.step, c);
+                if (u * residual < p) {
+                    rec->path[count] = (int32_t)c;
+                    rec->emitted[count++] = token[c];
+                    node = c;
+                    moved = true;
+                    break;
+                }
+                residual -= p;
+                if (residual < 0.f) residual = 0.f;
+            }
+            if (moved) continue;
+            rec->emitted[count++] = (uint32_t)(st.gumbel & 0xffffffffull);
+            break;
+        }
+    }
+    rec->n_emitted = count;
+    rec->status = status;
+    *reinterpret_cast<int32_t *>(rec + 1) = __ldcg(a.error);
+}
+
+// True in the CTA of a launch that arrives last (every CTA calls it once, with all threads). What the others wrote before is
+// visible there, through loads that pass L1 by (__ldcg). The word is zero again afterwards.
+__device__ __forceinline__ bool last_to_arrive(uint32_t *arrived) {
+    __shared__ uint32_t last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(arrived, 1u) == gridDim.x * gridDim.y - 1;
+        if (last) *arrived = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+}
+
 // One sweep over the vocabulary rows: blockIdx.y = position of the current pass, four consecutive rows per thread and
 // trip. Bound by arithmetic (Philox and two logarithms per logit where a temperature is set): one position per CTA
 // keeps one set of statistics in registers, and the four rows' noise comes from one Philox block where their tokens share a
 // counter. (All positions of a row in one thread, a Philox block per logit: 50 us for 8 x 248320 logits.)
+// The CTA that arrives last merges the positions' statistics over the CTAs (a warp per position; the lane order is fixed, so the
+// result is reproducible) and, where accept.rec is set, walks the tree: two launches less between the logits and the record.
 __global__ void __launch_bounds__(kHeadThreads) k_head_stats(
     const float *__restrict__ partial, const uint8_t *__restrict__ pieces, const float *__restrict__ s_out,
     const float *__restrict__ bias, uint32_t rows, uint32_t slices, uint32_t max_pieces, uint32_t node0,
     float inv_temperature, unsigned long long seed, unsigned long long step, const __grid_constant__ TreeDesc tree,
-    NodeStat *__restrict__ cta_stats, float *__restrict__ child_z, float *__restrict__ logits_out,
-    unsigned long long logits_stride, uint32_t row_offset, const float *__restrict__ plain) {
+    NodeStat *cta_stats, float *child_z, float *__restrict__ logits_out,
+    unsigned long long logits_stride, uint32_t row_offset, const float *__restrict__ plain, NodeStat *node_stats,
+    const __grid_constant__ AcceptArgs accept, uint32_t *arrived) {
     pdl_launch();
     pdl_wait();
     __shared__ NodeStat sh[kHeadThreads / 32];
@@ -178,28 +289,33 @@ __global__ void __launch_bounds__(kHeadThreads) k_head_stats(
         for (int w = 1; w < kHeadThreads / 32; ++w) merge_stat(a, sh[w]);
         cta_stats[(size_t)blockIdx.x * kMaxPosPerPass + m] = a;
     }
-}
-
-// Merges the per-CTA statistics of one pass into node_stats[node0 .. node0+npos): one warp per
-// position, lanes stride over the CTAs (eight loads at a time), then a butterfly (max/sum merges are
-// order-insensitive up to rounding; the lane order is fixed, so the result is reproducible).
-__global__ void k_head_merge(const NodeStat *__restrict__ cta_stats, uint32_t n_ctas, uint32_t node0,
-                             uint32_t npos, NodeStat *__restrict__ node_stats) {
-    pdl_launch();
-    pdl_wait();
-    const uint32_t m = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (m >= npos) return;
-    NodeStat a{0ull, 0ull, 0.f, 0.f, 0u, 0u};
-    for (uint32_t c0 = lane; c0 < n_ctas; c0 += 256) {
-        NodeStat b[8];
+    if (!last_to_arrive(arrived)) return;
+    __shared__ NodeStat all[kMaxNodes];
+    const uint32_t n_ctas = gridDim.x, npos = gridDim.y;
+    static_assert(kHeadThreads / 32 >= kMaxPosPerPass);
+    if ((uint32_t)warp < npos) {
+        NodeStat a{0ull, 0ull, 0.f, 0.f, 0u, 0u};
+        for (uint32_t c0 = lane; c0 < n_ctas; c0 += 128) {
+            uint4 b[4][2];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            b[i] = c0 + i * 32 < n_ctas ? cta_stats[(size_t)(c0 + i * 32) * kMaxPosPerPass + m] : NodeStat{0ull, 0ull, 0.f, 0.f, 0u, 0u};
+            for (int i = 0; i < 4; ++i) {
+                const uint4 *p = reinterpret_cast<const uint4 *>(cta_stats + (size_t)(c0 + i * 32) * kMaxPosPerPass + warp);
+                const bool in = c0 + i * 32 < n_ctas;
+                b[i][0] = in ? __ldcg(p) : make_uint4(0, 0, 0, 0);
+                b[i][1] = in ? __ldcg(p + 1) : make_uint4(0, 0, 0, 0);
+            }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) merge_stat(a, b[i]);
+            for (int i = 0; i < 4; ++i)
+                merge_stat(a, NodeStat{(unsigned long long)b[i][0].y << 32 | b[i][0].x, (unsigned long long)b[i][0].w << 32 | b[i][0].z,
+                                       __uint_as_float(b[i][1].x), __uint_as_float(b[i][1].y), b[i][1].z, 0u});
+        }
+        warp_merge(a);
+        if (lane == 0) node_stats[node0 + warp] = all[node0 + warp] = a;
     }
-    warp_merge(a);
-    if (lane == 0) node_stats[node0 + m] = a;
+    if (!accept.rec) return;
+    if (threadIdx.x < node0) all[threadIdx.x] = node_stats[threadIdx.x];  // of earlier passes
+    __syncthreads();
+    accept_walk(all, child_z, tree, accept);
 }
 
 // Tensor-parallel vocabulary: every rank holds the statistics of its shard and the logit of the
@@ -223,82 +339,15 @@ __global__ void k_head_merge_ranks(const RankStats *__restrict__ gathered, uint3
     out->child_z[n] = gathered[owner].child_z[n];
 }
 
-// Walks the draft tree with the statistics of every node. One thread: the walk is
-// a dependent chain of at most kMaxNodes steps.
-//
-// Node 0 is the root (the current position). At node n with children c1..cm in
-// index order: with temperature 0, child c is accepted iff its token equals
-// argmax of n's logits (engine.rs:939-962); otherwise c is accepted with
-// probability p_n(c) / (1 - mass of its rejected elder siblings) on the draw
-// accept_draw(seed, step, c). The drafter is deterministic, so this is speculative
-// sampling with a point-mass proposal and the emitted token is distributed as
-// softmax(logits / T). When no child is accepted the token is the Gumbel-max
-// sample of p_n restricted to non-children (greedy: the argmax).
-__global__ void k_spec_accept(const NodeStat *__restrict__ node_stats, const float *__restrict__ child_z,
-                              TreeDesc tree, float inv_temperature, unsigned long long seed,
-                              unsigned long long step, int force_accept, ctox_spec_record *__restrict__ rec) {
+// The walk by itself, after the statistics of a tensor-parallel group have been merged.
+__global__ void k_spec_accept(const NodeStat *node_stats, const float *child_z, const __grid_constant__ TreeDesc tree,
+                              const __grid_constant__ AcceptArgs accept) {
     pdl_launch();
     pdl_wait();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    uint32_t count = 0, node = 0, status = 0;
-    for (uint32_t n = 0; n < tree.n_nodes; ++n) rec->node_token[n] = tree.token[n];
-    for (uint32_t n = 0; n < tree.n_nodes; ++n) {
-        rec->node_argmax[n] = (uint32_t)(node_stats[n].argmax & 0xffffffffull);
-        if (node_stats[n].nonfinite) status = 1;
-    }
-    for (uint32_t n = tree.n_nodes; n < kMaxNodes; ++n) rec->node_argmax[n] = 0;
-    for (uint32_t i = 0; i < kMaxNodes; ++i) rec->path[i] = -1;
-    if (status == 0 && force_accept >= 0) {
-        // throughput buckets: accept exactly force_accept drafts of the chain, then the target's token
-        while (count < (uint32_t)force_accept && node + 1 < tree.n_nodes) {
-            rec->path[count] = (int32_t)(node + 1);
-            rec->emitted[count++] = tree.token[node + 1];
-            ++node;
-        }
-        rec->emitted[count++] = (uint32_t)(node_stats[node].argmax & 0xffffffffull);
-    } else if (status == 0) {
-        for (;;) {
-            const NodeStat st = node_stats[node];
-            bool moved = false;
-            if (!(inv_temperature > 0.f)) {
-                const uint32_t target = (uint32_t)(st.argmax & 0xffffffffull);
-                for (uint32_t c = node + 1; c < tree.n_nodes; ++c)
-                    if ((uint32_t)tree.parent[c] == node && tree.token[c] == target) {
-                        rec->path[count] = (int32_t)c;
-                        rec->emitted[count++] = target;
-                        node = c;
-                        moved = true;
-                        break;
-                    }
-                if (!moved) {
-                    rec->emitted[count++] = target;
-                    break;
-                }
-                continue;
-            }
-            float residual = 1.0f;
-            for (uint32_t c = node + 1; c < tree.n_nodes; ++c) {
-                if ((uint32_t)tree.parent[c] != node) continue;
-                const float p = expf(child_z[c] - st.max) / st.sum;
-                const float u = accept_draw(seed, step, c);
-                if (u * residual < p) {
-                    rec->path[count] = (int32_t)c;
-                    rec->emitted[count++] = tree.token[c];
-                    node = c;
-                    moved = true;
-                    break;
-                }
-                residual -= p;
-                if (residual < 0.f) residual = 0.f;
-            }
-            if (moved) continue;
-            rec->emitted[count++] = (uint32_t)(st.gumbel & 0xffffffffull);
-            break;
-        }
-    }
-    for (uint32_t i = count; i < kMaxNodes + 1; ++i) rec->emitted[i] = 0;
-    rec->n_emitted = count;
-    rec->status = status;
+    __shared__ NodeStat all[kMaxNodes];
+    if (threadIdx.x < tree.n_nodes) all[threadIdx.x] = node_stats[threadIdx.x];
+    __syncthreads();
+    accept_walk(all, child_z, tree, accept);
 }
 
 // ------------------------------------------------------------------ plain argmax
@@ -308,52 +357,74 @@ struct ArgmaxPartial {
     uint32_t pad;
 };
 
-__global__ void __launch_bounds__(kHeadThreads) k_argmax_partial(const float *__restrict__ logits, uint32_t n,
-                                                               ArgmaxPartial *__restrict__ out) {
+// Where the values of an argmax come from: finished logits, or the partial sums of a streamed matvec (partial set), whose
+// outputs are then stored as well.
+struct ArgmaxSource {
+    const float *logits;
+    const float *partial;
+    const uint8_t *pieces;
+    const float *s_out, *bias;
+    uint32_t slices, max_pieces, kst_s, warps_per_slice, pairs;
+    float *out;
+};
+
+// The CTA that arrives last merges the others' results: result[0] = token (mapped through row_ids when given,
+// engine.rs:203-217), result[1] = status (1 = a logit is not finite, kernels/cuda/q2q4_fused_matvec_sm86.cu:2583-2585).
+// With packed_out the (key, token) pair is stored as well, for the merge over a tensor-parallel group.
+__global__ void __launch_bounds__(kHeadThreads) k_argmax(const __grid_constant__ ArgmaxSource src, uint32_t n, ArgmaxPartial *parts,
+                                                         const uint32_t *__restrict__ row_ids, uint32_t row_offset,
+                                                         uint32_t *token_out, uint32_t *status_out, ArgmaxPartial *packed_out,
+                                                         uint32_t *arrived) {
     pdl_launch();
     pdl_wait();
     __shared__ ArgmaxPartial sh[kHeadThreads / 32];
-    unsigned long long best = 0ull;
-    uint32_t bad = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float v = logits[i];
-        if (!isfinite(v)) bad = 1;
-        const unsigned long long pk = pack_key_index(v, i);
-        best = pk > best ? pk : best;
-    }
+    auto reduce = [&](unsigned long long best, uint32_t bad) {  // thread 0 receives the CTA's result
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
-        best = ob > best ? ob : best;
-        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-    }
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = ArgmaxPartial{best, bad, 0};
-    __syncthreads();
-    if (threadIdx.x == 0) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+            best = ob > best ? ob : best;
+            bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+        }
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = ArgmaxPartial{best, bad, 0};
+        __syncthreads();
         ArgmaxPartial a = sh[0];
         for (int w = 1; w < kHeadThreads / 32; ++w) {
             a.best = sh[w].best > a.best ? sh[w].best : a.best;
             a.nonfinite |= sh[w].nonfinite;
         }
-        out[blockIdx.x] = a;
+        return a;
+    };
+    unsigned long long best = 0ull;
+    uint32_t bad = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        float v;
+        if (src.partial) {  // as in k_matvec_finish
+            v = src.warps_per_slice ? matvec_output_n(src.partial, piece_count(i / kPairRows, src.kst_s, src.warps_per_slice, src.pairs),
+                                                      src.slices, src.max_pieces, nullptr, i, 0)
+                                    : matvec_output(src.partial, src.pieces, src.slices, src.max_pieces, nullptr, i, 0);
+            if (src.bias) v += src.bias[i];
+            if (src.s_out) v *= src.s_out[i];
+            src.out[i] = v;
+        } else {
+            v = src.logits[i];
+        }
+        if (!isfinite(v)) bad = 1;
+        const unsigned long long pk = pack_key_index(v, i);
+        best = pk > best ? pk : best;
     }
-}
-
-// result[0] = token (mapped through row_ids when given, engine.rs:203-217), result[1] = status
-// (1 = a logit is not finite, kernels/cuda/q2q4_fused_matvec_sm86.cu:2583-2585).
-// With packed_out the (key, token) pair is stored as well, for the merge over a tensor-parallel group.
-__global__ void k_argmax_final(const ArgmaxPartial *__restrict__ parts, uint32_t n_parts,
-                               const uint32_t *__restrict__ row_ids, uint32_t row_offset,
-                               uint32_t *__restrict__ token_out, uint32_t *__restrict__ status_out,
-                               ArgmaxPartial *__restrict__ packed_out) {
-    pdl_launch();
-    pdl_wait();
+    ArgmaxPartial a = reduce(best, bad);
+    if (threadIdx.x == 0) parts[blockIdx.x] = a;
+    if (!last_to_arrive(arrived)) return;
+    best = 0ull;
+    bad = 0;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += kHeadThreads) {
+        const uint4 p = __ldcg(reinterpret_cast<const uint4 *>(parts + i));
+        const unsigned long long b = (unsigned long long)p.y << 32 | p.x;
+        best = b > best ? b : best;
+        bad |= p.z;
+    }
+    a = reduce(best, bad);
     if (threadIdx.x != 0) return;
-    ArgmaxPartial a = parts[0];
-    for (uint32_t i = 1; i < n_parts; ++i) {
-        a.best = parts[i].best > a.best ? parts[i].best : a.best;
-        a.nonfinite |= parts[i].nonfinite;
-    }
     const uint32_t row = (uint32_t)(a.best & 0xffffffffull);
     const uint32_t token = row_ids ? row_ids[row] : row + row_offset;
     if (token_out) *token_out = token;
@@ -549,7 +620,7 @@ struct HeadScratch {
     float *child_z;        // [kMaxNodes]   } tensor-parallel merge
     RankStats *gathered;   // [kMaxTpWorld]
     ArgmaxPartial *argmax_send, *argmax_gathered;  // [1], [kMaxTpWorld]
-    ctox_spec_record *record;
+    ctox_spec_record *record;  // and the error word (AcceptArgs)
     ArgmaxPartial *argmax_parts;  // [grid]
     uint32_t *argmax_result;      // [2]
     uint32_t *tokens;             // [kMaxNodes] node tokens of the host-form verify call
@@ -568,7 +639,7 @@ ctox_status head_scratch(ctox_ctx *ctx, HeadScratch &hs) {
     const size_t o_gath = take(sizeof(RankStats) * kMaxTpWorld);
     const size_t o_as = take(sizeof(ArgmaxPartial));
     const size_t o_ag = take(sizeof(ArgmaxPartial) * kMaxTpWorld);
-    const size_t o_rec = take(sizeof(ctox_spec_record));
+    const size_t o_rec = take(sizeof(ctox_spec_record) + sizeof(int32_t));
     const size_t o_ap = take(sizeof(ArgmaxPartial) * kHeadGridMax);
     const size_t o_ar = take(sizeof(uint32_t) * 2);
     const size_t o_tok = take(sizeof(uint32_t) * kMaxNodes);
@@ -602,9 +673,10 @@ ctox_status ctox_argmax_f32(ctox_ctx *ctx, const float *logits_dev, uint32_t n, 
     uint32_t grid = (n + kHeadThreads * 4 - 1) / (kHeadThreads * 4);
     if (grid > kHeadGridMax) grid = kHeadGridMax;
     if (grid == 0) grid = 1;
-    launch_pdl(k_argmax_partial, dim3(grid), dim3(kHeadThreads), 0, ctx->stream, logits_dev, n, hs.argmax_parts);
-    launch_pdl(k_argmax_final, dim3(1), dim3(32), 0, ctx->stream, hs.argmax_parts, grid, row_ids_dev, 0, result_dev, result_dev + 1,
-                                              nullptr);
+    ArgmaxSource src{};
+    src.logits = logits_dev;
+    launch_pdl(k_argmax, dim3(grid), dim3(kHeadThreads), 0, ctx->stream, src, n, hs.argmax_parts, row_ids_dev, 0u, result_dev,
+               result_dev + 1, nullptr, ctx->arrived + 1);
     CTOX_CUDA(ctx, cudaGetLastError());
     return CTOX_OK;
 }
@@ -671,7 +743,7 @@ namespace {
 ctox_status head_stats_enqueue(ctox_ctx *ctx, const ctox_matvec *mv, const float *plain, uint64_t logits_stride,
                                uint32_t node0, uint32_t npos, uint32_t n_nodes, const int32_t *parent,
                                const uint32_t *tokens_dev, float inv_t, uint64_t seed, uint64_t step, uint32_t rows,
-                               float *logits_out_dev, uint32_t row_offset) {
+                               float *logits_out_dev, uint32_t row_offset, const int *accept) {
     HeadScratch hs;
     ctox_status rc = head_scratch(ctx, hs);
     if (rc) return rc;
@@ -688,8 +760,8 @@ ctox_status head_stats_enqueue(ctox_ctx *ctx, const ctox_matvec *mv, const float
     launch_pdl(k_head_stats, dim3(grid, npos), dim3(kHeadThreads), 0, ctx->stream, p ? p->partial : nullptr,
                p ? p->split[npos > 4 ? 1 : 0].pieces : nullptr, mv ? mv->s_out : nullptr, mv ? mv->bias : nullptr, rows,
                p ? p->slices : 0u, p ? p->max_pieces : 0u, node0, inv_t, seed, step, tree, hs.cta_stats, hs.child_z,
-               logits_out_dev, (unsigned long long)logits_stride, row_offset, plain);
-    launch_pdl(k_head_merge, dim3(1), dim3(32 * kMaxPosPerPass), 0, ctx->stream, hs.cta_stats, grid, node0, npos, hs.node_stats);
+               logits_out_dev, (unsigned long long)logits_stride, row_offset, plain, hs.node_stats,
+               AcceptArgs{inv_t, seed, step, accept ? *accept : -1, accept ? hs.record : nullptr, ctx->dev_error}, ctx->arrived);
     CTOX_CUDA(ctx, cudaGetLastError());
     return CTOX_OK;
 }
@@ -698,16 +770,23 @@ ctox_status head_stats_enqueue(ctox_ctx *ctx, const ctox_matvec *mv, const float
 
 ctox_status head_verify_enqueue(ctox_matvec *mv, uint32_t node0, uint32_t npos, uint32_t n_nodes,
                                 const int32_t *parent, const uint32_t *tokens_dev, float inv_t, uint64_t seed,
-                                uint64_t step, uint32_t rows, float *logits_out_dev, uint32_t row_offset) {
+                                uint64_t step, uint32_t rows, float *logits_out_dev, uint32_t row_offset, const int *accept) {
     return head_stats_enqueue(mv->ctx, mv, nullptr, mv->rows, node0, npos, n_nodes, parent, tokens_dev, inv_t, seed, step,
-                              rows, logits_out_dev, row_offset);
+                              rows, logits_out_dev, row_offset, accept);
 }
 
 ctox_status head_verify_logits_enqueue(ctox_ctx *ctx, const float *logits, uint32_t npos, const int32_t *parent,
                                        const uint32_t *tokens_dev, float inv_t, uint64_t seed, uint64_t step,
-                                       uint32_t rows) {
+                                       uint32_t rows, const int *accept) {
     return head_stats_enqueue(ctx, nullptr, logits, rows, 0, npos, npos, parent, tokens_dev, inv_t, seed, step, rows,
-                              nullptr, 0);
+                              nullptr, 0, accept);
+}
+
+ctox_status head_record(ctox_ctx *ctx, ctox_spec_record **record_dev) {
+    HeadScratch hs;
+    EX(head_scratch(ctx, hs));
+    *record_dev = hs.record;
+    return CTOX_OK;
 }
 
 ctox_status head_accept_enqueue(ctox_ctx *ctx, uint32_t n_nodes, const int32_t *parent,
@@ -721,15 +800,16 @@ ctox_status head_accept_enqueue(ctox_ctx *ctx, uint32_t n_nodes, const int32_t *
     tree.n_nodes = n_nodes;
     tree.token = tokens_dev;
     for (uint32_t i = 0; i < n_nodes; ++i) tree.parent[i] = parent[i];
-    launch_pdl(k_spec_accept, dim3(1), dim3(32), 0, ctx->stream, hs.node_stats, hs.child_z, tree, inv_t, seed, step, force_accept,
-                                            hs.record);
+    launch_pdl(k_spec_accept, dim3(1), dim3(32), 0, ctx->stream, hs.node_stats, hs.child_z, tree,
+               AcceptArgs{inv_t, seed, step, force_accept, hs.record, ctx->dev_error});
     CTOX_CUDA(ctx, cudaGetLastError());
     *record_dev = hs.record;
     return CTOX_OK;
 }
 
-ctox_status argmax_enqueue(ctox_ctx *ctx, const float *logits_dev, uint32_t n, const uint32_t *row_ids_dev,
-                           uint32_t row_offset, uint32_t *token_dev, uint32_t *status_dev) {
+namespace {
+ctox_status argmax_any(ctox_ctx *ctx, const ArgmaxSource &src, uint32_t n, const uint32_t *row_ids_dev, uint32_t row_offset,
+                       uint32_t *token_dev, uint32_t *status_dev) {
     HeadScratch hs;
     ctox_status rc = head_scratch(ctx, hs);
     if (rc) return rc;
@@ -738,13 +818,12 @@ ctox_status argmax_enqueue(ctox_ctx *ctx, const float *logits_dev, uint32_t n, c
         if (!tp) return fail(ctx, CTOX_INVALID_ARTIFACT, "greedy logits are empty");
         CTOX_CUDA(ctx, cudaMemsetAsync(hs.argmax_send, 0, sizeof(ArgmaxPartial), ctx->stream));
     } else {
-        uint32_t grid = (n + kHeadThreads * 4 - 1) / (kHeadThreads * 4);
+        // a row per thread where the sums of a matvec are read (several round trips each), else four
+        const uint32_t per = src.partial ? kHeadThreads : kHeadThreads * 4;
+        uint32_t grid = (n + per - 1) / per;
         if (grid > kHeadGridMax) grid = kHeadGridMax;
-        if (grid == 0) grid = 1;
-        launch_pdl(k_argmax_partial, dim3(grid), dim3(kHeadThreads), 0, ctx->stream, logits_dev, n, hs.argmax_parts);
-        launch_pdl(k_argmax_final, dim3(1), dim3(32), 0, ctx->stream, hs.argmax_parts, grid, row_ids_dev, row_offset,
-                                                  tp ? nullptr : token_dev, tp ? nullptr : status_dev,
-                                                  tp ? hs.argmax_send : nullptr);
+        launch_pdl(k_argmax, dim3(grid), dim3(kHeadThreads), 0, ctx->stream, src, n, hs.argmax_parts, row_ids_dev, row_offset,
+                   tp ? nullptr : token_dev, tp ? nullptr : status_dev, tp ? hs.argmax_send : nullptr, ctx->arrived + 1);
     }
     if (tp) {
         rc = tp_all_gather(ctx, hs.argmax_send, hs.argmax_gathered, sizeof(ArgmaxPartial));
@@ -753,6 +832,25 @@ ctox_status argmax_enqueue(ctox_ctx *ctx, const float *logits_dev, uint32_t n, c
     }
     CTOX_CUDA(ctx, cudaGetLastError());
     return CTOX_OK;
+}
+
+}  // namespace
+
+ctox_status argmax_enqueue(ctox_ctx *ctx, const float *logits_dev, uint32_t n, const uint32_t *row_ids_dev,
+                           uint32_t row_offset, uint32_t *token_dev, uint32_t *status_dev) {
+    ArgmaxSource src{};
+    src.logits = logits_dev;
+    return argmax_any(ctx, src, n, row_ids_dev, row_offset, token_dev, status_dev);
+}
+ctox_status argmax_matvec_enqueue(ctox_matvec *mv, float *logits_out, const uint32_t *row_ids_dev, uint32_t row_offset,
+                                  uint32_t *token_dev, uint32_t *status_dev) {
+    const MatvecPart &p = mv->parts[0];
+    const MatvecPart::Split &sp = p.split[0];
+    const uint64_t units = (uint64_t)p.pairs * p.kst_s;
+    const bool fits = (units + 1) * sp.warps_per_slice + units < (1ull << 32);  // piece_count() in 32 bits
+    const ArgmaxSource src{nullptr, p.partial, sp.pieces, mv->s_out, mv->bias, p.slices, p.max_pieces, p.kst_s,
+                           fits ? sp.warps_per_slice : 0, p.pairs, logits_out};
+    return argmax_any(mv->ctx, src, (uint32_t)mv->rows, row_ids_dev, row_offset, token_dev, status_dev);
 }
 
 // Tensor-parallel vocabulary: exchanges the per-rank statistics and leaves the merged ones where
@@ -827,14 +925,12 @@ ctox_status ctox_lmhead_verify(ctox_matvec *mv, const void *hidden_dev, uint32_t
         rc = matvec_stream_pass(mv, 0, (const uint8_t *)hidden_dev + (size_t)n0 * hidden_stride * esz,
                                 hidden_dtype, npos, hidden_stride);
         if (rc) return rc;
+        const int accept = -1;  // the last pass walks the tree
         rc = head_verify_enqueue(mv, n0, npos, n_nodes, parent, hs.tokens, inv_t, seed, step, rows,
-                                 logits_out_dev, 0);
+                                 logits_out_dev, 0, n0 + npos == n_nodes ? &accept : nullptr);
         if (rc) return rc;
     }
-    ctox_spec_record *rec_dev = nullptr;
-    rc = head_accept_enqueue(ctx, n_nodes, parent, hs.tokens, inv_t, seed, step, -1, &rec_dev);
-    if (rc) return rc;
-    CTOX_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, rec_dev, sizeof(ctox_spec_record), cudaMemcpyDeviceToHost,
+    CTOX_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, hs.record, sizeof(ctox_spec_record), cudaMemcpyDeviceToHost,
                                    ctx->stream));
     CTOX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     memcpy(record, ctx->pinned, sizeof(ctox_spec_record));

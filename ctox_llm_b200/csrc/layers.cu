@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kRnColumns / CL, 1) k_residual_norm_prep(float
     pdl_wait();
     float v = 0.f;
     if (c < hidden) {
-        v = h[(size_t)m * hidden + c];
+        if (has_add != 2) v = h[(size_t)m * hidden + c];  // 2: the stream begins here
         if (has_add) {
             v += out_at(add, ar, c, m);
             h[(size_t)m * hidden + c] = v;
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kRnColumns / CL, 1) k_residual_norm_prep(float
 }
 
 void launch_residual_norm_prep(cudaStream_t st, float *h, const MvOut *add, const float *w, float eps,
-                               uint32_t hidden, uint32_t m, float *xn_out, const MvIn *next, float *scratch) {
+                               uint32_t hidden, uint32_t m, float *xn_out, const MvIn *next, float *scratch, bool fresh) {
     static const bool merged = [] {
         const char *v = getenv("CTOX_MERGED_NORM");
         return !(v && v[0] == '0');
@@ -162,14 +162,15 @@ void launch_residual_norm_prep(cudaStream_t st, float *h, const MvOut *add, cons
         }
         if (m <= 2 && dev < 64 && (wide_ok >> dev & 1ull))
             launch_pdl_cluster(k_residual_norm_prep<kRnClusterWide>, dim3(kRnClusterWide, m),
-                               dim3(kRnColumns / kRnClusterWide), 0, st, kRnClusterWide, h, a, add != nullptr, hidden, w,
+                               dim3(kRnColumns / kRnClusterWide), 0, st, kRnClusterWide, h, a, add ? 1 + fresh : 0, hidden, w,
                                eps, (int)m, xn_out, n, next != nullptr, nblocks);
         else
             launch_pdl_cluster(k_residual_norm_prep<kRnCluster>, dim3(kRnCluster, m), dim3(kRnColumns / kRnCluster), 0, st,
-                               kRnCluster, h, a, add != nullptr, hidden, w, eps, (int)m, xn_out, n, next != nullptr,
+                               kRnCluster, h, a, add ? 1 + fresh : 0, hidden, w, eps, (int)m, xn_out, n, next != nullptr,
                                nblocks);
         return;
     }
+    if (fresh) cudaMemsetAsync(h, 0, (size_t)m * hidden * sizeof(float), st);
     launch_residual_add(st, h, add, hidden, m, scratch);
     launch_norm_prep(st, h, w, eps, hidden, m, xn_out, next, scratch);
 }

@@ -44,10 +44,11 @@ struct AttnGeom {
     float theta, eps;
 };
 
-// h[m] (+= matvec output) ; xn = rmsnorm_1p(h[m], w) ; optional copy of xn ; fragments of xn * s_in.
+// h[m] (+= matvec output; = it where `fresh`) ; xn = rmsnorm_1p(h[m], w) ; optional copy of xn ; fragments of xn * s_in.
 // scratch: m * ceil(hidden / 256) floats.
 void launch_residual_norm_prep(cudaStream_t st, float *h, const MvOut *add, const float *w, float eps,
-                               uint32_t hidden, uint32_t m, float *xn_out, const MvIn *next, float *scratch);
+                               uint32_t hidden, uint32_t m, float *xn_out, const MvIn *next, float *scratch,
+                               bool fresh = false);
 // h[m] (+= matvec output) and the partial sums of squares of the result: scratch[m][ceil(hidden/256)],
 // the form launch_norm_prep reads.
 void launch_residual_add(cudaStream_t st, float *h, const MvOut *add, uint32_t hidden, uint32_t m, float *scratch);

@@ -74,14 +74,17 @@ ctox_status matvec_embed_rows(ctox_matvec *mv, const uint32_t *row_ids_dev, uint
 // y[pos][row] from the partial sums of the last streamed pass.
 void matvec_finish_enqueue(ctox_matvec *mv, uint32_t npos, float *y, uint64_t y_stride);
 // Selection over the partial sums of an lm_head pass (head.cu). Statistics of verify nodes
-// node0 .. node0+npos; then the acceptance walk over all nodes, whose record stays on the device.
+// node0 .. node0+npos; with `accept` (the force_accept of head_accept_enqueue; one GPU, the pass of the last nodes) also the
+// acceptance walk over all nodes, whose record stays on the device.
 ctox_status head_verify_enqueue(ctox_matvec *mv, uint32_t node0, uint32_t npos, uint32_t n_nodes,
                                 const int32_t *parent, const uint32_t *tokens_dev, float inv_t, uint64_t seed,
-                                uint64_t step, uint32_t rows, float *logits_out_dev, uint32_t row_offset);
+                                uint64_t step, uint32_t rows, float *logits_out_dev, uint32_t row_offset, const int *accept);
 // The same from finished logits [npos][rows] (a head that writes them).
 ctox_status head_verify_logits_enqueue(ctox_ctx *ctx, const float *logits, uint32_t npos, const int32_t *parent,
                                        const uint32_t *tokens_dev, float inv_t, uint64_t seed, uint64_t step,
-                                       uint32_t rows);
+                                       uint32_t rows, const int *accept);
+// Where the record of an acceptance walk is left, the value of the context's error word behind it.
+ctox_status head_record(ctox_ctx *ctx, ctox_spec_record **record_dev);
 // Tensor-parallel vocabulary: merges the ranks' statistics (all-gather) before the acceptance walk.
 ctox_status head_tp_merge_enqueue(ctox_ctx *ctx, uint32_t n_nodes, const int32_t *parent,
                                   const uint32_t *tokens_dev, uint32_t shard_rows);
@@ -90,6 +93,9 @@ ctox_status head_accept_enqueue(ctox_ctx *ctx, uint32_t n_nodes, const int32_t *
                                 int force_accept, ctox_spec_record **record_dev);
 // Greedy token of a logit vector; token = row_ids[row] or row + row_offset. In a tensor-parallel
 // group every rank passes its shard and all ranks receive the group's token.
+// The same over the outputs of a streamed pass of one position (identity activation), which go to logits_out.
+ctox_status argmax_matvec_enqueue(ctox_matvec *mv, float *logits_out, const uint32_t *row_ids_dev, uint32_t row_offset,
+                                  uint32_t *token_dev, uint32_t *status_dev);
 ctox_status argmax_enqueue(ctox_ctx *ctx, const float *logits_dev, uint32_t n, const uint32_t *row_ids_dev,
                            uint32_t row_offset, uint32_t *token_dev, uint32_t *status_dev);
 }  // namespace ctox
