@@ -178,17 +178,25 @@ void launch_residual_norm_prep(cudaStream_t st, float *h, const MvOut *add, cons
 // [rmsnorm(embed) | rmsnorm(prev_hidden)] -> fragments (2 * hidden columns). One CTA per
 // (16 blocks of 64 columns, position); every CTA adds up both sums of squares itself (40 KB from L2),
 // then each 16-lane group writes one block.
-__global__ void __launch_bounds__(256) k_mtp_pre(const float *__restrict__ embed_rows,
-                                               const float *__restrict__ prev_hidden,
+__global__ void __launch_bounds__(256) k_mtp_pre(const float *embed_rows, const float *prev_hidden,
                                                const float *__restrict__ w_embed,
                                                const float *__restrict__ w_hidden, float eps, uint32_t hidden,
                                                int npos, MvIn next) {
     pdl_launch();
-    pdl_wait();
     __shared__ float red[8];
     const int m = blockIdx.y;
     const float *e = embed_rows + (size_t)m * hidden, *h = prev_hidden + (size_t)m * hidden;
+    // this thread's weights are constants: ahead of the wait
+    float w[4], sc[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t c = (blockIdx.x * 16 + (threadIdx.x >> 4)) * 64 + (threadIdx.x & 15) * 4 + j;
+        w[j] = c < hidden ? w_embed[c] : c < 2 * hidden ? w_hidden[c - hidden] : 0.f;
+        sc[j] = next.s_in && c < 2 * hidden ? next.s_in[c] : 1.0f;
+    }
+    pdl_wait();
     float sq_e = 0.f, sq_h = 0.f;
+#pragma unroll 4
     for (uint32_t c = threadIdx.x; c < hidden; c += blockDim.x) {
         const float a = e[c], b = h[c];
         sq_e += a * a;
@@ -207,8 +215,8 @@ __global__ void __launch_bounds__(256) k_mtp_pre(const float *__restrict__ embed
         if (c < 2 * hidden) {
             const bool second = c >= hidden;
             const uint32_t cc = second ? c - hidden : c;
-            const float xn = second ? h[cc] * inv_h * (1.0f + w_hidden[cc]) : e[cc] * inv_e * (1.0f + w_embed[cc]);
-            v[j] = xn * (next.s_in ? next.s_in[c] : 1.0f);
+            const float xn = second ? h[cc] * inv_h * (1.0f + w[j]) : e[cc] * inv_e * (1.0f + w[j]);
+            v[j] = xn * sc[j];
         }
     }
     const unsigned gmask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
@@ -348,7 +356,6 @@ __global__ void __launch_bounds__(256) k_attn_pre(MvOut fan, AttnGeom g, const f
                                                   T *__restrict__ v_cache, const uint32_t *__restrict__ page_table,
                                                   uint32_t page_tokens) {
     pdl_launch();
-    pdl_wait();
     __shared__ float buf[256];
     __shared__ float red[8];
     const uint32_t heads_total = g.q_heads + 2 * g.kv_heads;
@@ -356,29 +363,38 @@ __global__ void __launch_bounds__(256) k_attn_pre(MvOut fan, AttnGeom g, const f
     const int m = blockIdx.x / heads_total;
     const uint32_t hd = g.head_dim, d = threadIdx.x;  // blockDim.x == head_dim
     const uint32_t k_row0 = g.q_heads * 2 * hd, v_row0 = k_row0 + g.kv_heads * hd;
+    // What does not depend on earlier kernels, ahead of the wait: the cache slot, the norm's weight, the turn of this dimension
+    // and where the projection's sums lie.
     const size_t slot = kv_slot(page_table, page_tokens, cache_slot + m);
-    if (hi >= g.q_heads + g.kv_heads) {  // value head: plain copy into the cache
-        const uint32_t kh = hi - g.q_heads - g.kv_heads;
-        kv_store(v_cache + (slot * g.kv_heads + kh) * hd + d, out_of(fan, v_row0 + kh * hd + d, m));
+    const bool is_q = hi < g.q_heads, is_v = hi >= g.q_heads + g.kv_heads;
+    const uint32_t head = is_q ? hi : is_v ? hi - g.q_heads - g.kv_heads : hi - g.q_heads;
+    const uint32_t row = (is_q ? head * 2 * hd : (is_v ? v_row0 : k_row0) + head * hd) + d;
+    const OutRef ref = out_ref(fan, row), gate_ref = is_q ? out_ref(fan, row + hd) : OutRef{nullptr, 0, 0, 1.0f, false};
+    const float w = is_v ? 0.f : (is_q ? q_norm : k_norm)[d];
+    float cs = 1.f, sn = 0.f;
+    if (!is_v && d < g.rotary_dim) {
+        const uint32_t half = g.rotary_dim / 2, i = d < half ? d : d - half;
+        const float pos = (float)(rope_position + (uint64_t)m);
+        const float inv_freq = powf(g.theta, -((float)(2 * i)) / (float)g.rotary_dim);
+        const float ang = pos * inv_freq;
+        cs = cosf(ang);
+        sn = sinf(ang);
+    }
+    pdl_wait();
+    const float v = out_at(fan, ref, row, m);
+    if (is_v) {  // value head: plain copy into the cache
+        kv_store(v_cache + (slot * g.kv_heads + head) * hd + d, v);
         return;
     }
-    const bool is_q = hi < g.q_heads;
-    const uint32_t head = is_q ? hi : hi - g.q_heads;
-    const uint32_t row0 = is_q ? head * 2 * hd : k_row0 + head * hd;
-    const float v = out_of(fan, row0 + d, m);
-    if (is_q) gate[((size_t)m * g.q_heads + head) * hd + d] = out_of(fan, row0 + hd + d, m);
+    if (is_q) gate[((size_t)m * g.q_heads + head) * hd + d] = out_at(fan, gate_ref, row + hd, m);
     const float sq = block_sum(v * v, red);
     const float inv = 1.0f / sqrtf(sq / (float)hd + g.eps);
-    const float xn = v * inv * (1.0f + (is_q ? q_norm : k_norm)[d]);
+    const float xn = v * inv * (1.0f + w);
     buf[d] = xn;
     __syncthreads();
     float out = xn;
     if (d < g.rotary_dim) {
         const uint32_t half = g.rotary_dim / 2;
-        const uint32_t i = d < half ? d : d - half;
-        const float pos = (float)(rope_position + (uint64_t)m);
-        const float inv_freq = powf(g.theta, -((float)(2 * i)) / (float)g.rotary_dim);
-        const float ang = pos * inv_freq, cs = cosf(ang), sn = sinf(ang);
         out = d < half ? xn * cs - buf[d + half] * sn : xn * cs + buf[d - half] * sn;
     }
     if (is_q)
