@@ -254,13 +254,25 @@ struct StreamInput {
     uint32_t columns;
     int bf16, vec;  // vec: rows are aligned for loads of four values
 };
-// The matrices of one launch; matrix i takes the CTAs from first_cta[i] on.
+// Where the outputs of a matrix go, and the sums they are made from.
+struct FinishItem {
+    const float *partial;
+    const uint8_t *pieces;
+    const float *s_out, *bias;
+    float *y;
+    long long y_stride;
+    uint32_t rows, slices, max_pieces, activation;
+    uint32_t kst_s, warps_per_slice, pairs;  // warps_per_slice == 0: piece counts from the table
+};
+// The matrices of one launch; matrix i takes the CTAs from first_cta[i] on. closed: a CTA takes whole row pairs, a warp per unit, and
+// writes the outputs itself.
 constexpr int kStreamItems = 4;
 struct StreamArgs {
     StreamParams item[kStreamItems];
     uint32_t first_cta[kStreamItems];
-    uint32_t items;
+    uint32_t items, closed;
     StreamInput in;
+    FinishItem out[kStreamItems];
 };
 
 __device__ __forceinline__ const StreamParams &stream_item(const StreamParams &p, uint32_t) { return p; }
@@ -294,6 +306,13 @@ __device__ __forceinline__ void load_activations(const StreamInput &in, uint32_t
 #pragma unroll
         for (uint32_t j = 0; j < 4; ++j)
             if (k + j < in.columns) v[j] *= in.s_in[k + j];
+}
+
+__device__ __forceinline__ float finish_value(const FinishItem &f, float v, float s_out, float bias) {
+    if (f.bias) v += bias;
+    if (f.s_out) v *= s_out;
+    if (f.activation == CTOX_ACT_SILU) v = v / (1.0f + expf(-v));
+    return v;
 }
 
 // Four MMAs of one 16-row x 64-column block; cw = this lane's code vector(s).
@@ -351,12 +370,19 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
 
     // This CTA works inside one column slice; its warps split the slice's units
     // (tile pair x super-tile of the slice, pair-major) evenly: [beg, end).
-    const uint32_t slice = cta / p.ctas_per_slice;
+    const uint32_t slice = cta / p.ctas_per_slice;  // closed: there is one
     const uint32_t lw = (cta % p.ctas_per_slice) * WARPS + warp;
     const uint64_t total = (uint64_t)p.pairs * p.kst_s;
-    const bool active = lw < p.warps_per_slice;
+    bool closed = false;
+    if constexpr (DISPATCH) closed = args.closed;
+    bool active = lw < p.warps_per_slice;
     uint64_t beg = 0, end = 0;
-    if (active) {
+    if (closed) {
+        const uint32_t pair = cta * (WARPS / p.kst_s) + warp / p.kst_s;
+        active = warp < WARPS / p.kst_s * p.kst_s && pair < p.pairs;
+        beg = (uint64_t)pair * p.kst_s + warp % p.kst_s;
+        end = beg + active;
+    } else if (active) {
         beg = ((uint64_t)lw * total) / p.warps_per_slice;
         end = ((uint64_t)(lw + 1) * total) / p.warps_per_slice;
     }
@@ -410,7 +436,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
         bulk_g2s(smem_u32(ms), reinterpret_cast<const uint8_t *>(p.meta) + (size_t)slice * meta_bytes,
                  meta_bytes, xbar);
     }
-    if (!active || nchunks == 0) return;  // warp 0 of every CTA is active and waits for xbar below
+    if (!closed && (!active || nchunks == 0)) return;  // warp 0 of every CTA is active and waits for xbar below
     bool ok = own || mbar_wait(xbar, 0);
 
     // lanes whose B column / position does not exist read zeros with stride 0
@@ -546,7 +572,36 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
         const uint32_t issued = min(nchunks, waited + (uint32_t)STAGES);
         for (uint32_t c = waited; c < issued; ++c)
             mbar_wait(my_bars + 8 * (c % STAGES), (c / STAGES) & 1);
-        return;
+        if (!closed) return;
+    }
+    if constexpr (DISPATCH) {
+        if (closed) {  // the warps of a pair leave their sums in their own stages: [position][32 rows]
+            auto sums_of = [&](uint32_t w) { return reinterpret_cast<float *>(stages + w * STAGES * kChunkBytes); };
+            if (active) {
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+                    if (has_m[nt]) {
+                        float *col = sums_of(warp) + (4 * nt + t) * kPairRows;
+                        col[rloc[0]] = acc[nt][0] + acc[nt][1];
+                        col[rloc[1]] = acc[nt][2] + acc[nt][3];
+                        col[rloc[2]] = acc[nt][4] + acc[nt][5];
+                        col[rloc[3]] = acc[nt][6] + acc[nt][7];
+                    }
+            }
+            __syncthreads();
+            const FinishItem &f = args.out[which];
+            const uint32_t per = WARPS / p.kst_s;
+            for (uint32_t i = threadIdx.x; i < per * p.npos * kPairRows; i += WARPS * 32) {
+                const uint32_t r = i % kPairRows, pos = i / kPairRows % p.npos, q = i / (kPairRows * p.npos);
+                const uint32_t row = (cta * per + q) * kPairRows + r;
+                if (row >= f.rows) continue;
+                float v = 0.f;
+                for (uint32_t k = 0; k < p.kst_s; ++k) v += sums_of(q * p.kst_s + k)[pos * kPairRows + r];
+                f.y[(long long)pos * f.y_stride + row] =
+                    finish_value(f, v, f.s_out ? f.s_out[row] : 1.0f, f.bias ? f.bias[row] : 0.0f);
+            }
+            return;
+        }
     }
     close_pair(cur_pair, cur_ks == p.kst_s);
 }
@@ -556,15 +611,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
 // each, up to eight pieces of a value are requested together (matvec_output_n), and what does not depend on the stream is
 // read ahead of the wait. (A thread per (row, position), positions side by side, took 5.0 us for 5120 x 4 outputs of
 // four slices, one line per lane and one round trip per piece.)
-struct FinishItem {
-    const float *partial;
-    const uint8_t *pieces;
-    const float *s_out, *bias;
-    float *y;
-    long long y_stride;
-    uint32_t rows, slices, max_pieces, activation;
-    uint32_t kst_s, warps_per_slice, pairs;  // warps_per_slice == 0: piece counts from the table
-};
 constexpr int kFinishItems = 4;
 struct FinishArgs {
     FinishItem item[kFinishItems];
@@ -585,10 +631,7 @@ __global__ void __launch_bounds__(256) k_matvec_finish(const __grid_constant__ F
     if (!live) return;
     float v = n ? matvec_output_n(f.partial, n, f.slices, f.max_pieces, nullptr, row, pos)
                 : matvec_output(f.partial, f.pieces, f.slices, f.max_pieces, nullptr, row, pos);
-    if (f.bias) v += bi;
-    if (f.s_out) v *= so;
-    if (f.activation == CTOX_ACT_SILU) v = v / (1.0f + expf(-v));
-    f.y[(long long)pos * f.y_stride + row] = v;
+    f.y[(long long)pos * f.y_stride + row] = finish_value(f, v, so, bi);
 }
 
 // ------------------------------------------------------------------ row-per-warp kernel
@@ -935,6 +978,28 @@ bool plan_merged(ctox_ctx *ctx, const DispatchItem *it, uint32_t n, uint32_t npo
     return true;
 }
 
+// A launch whose CTAs take whole row pairs, a warp per unit, and write the outputs themselves: no second kernel (1024 x 1024, one
+// position: 5.9 -> 3.9 us). For matrices of one slice whose units are no more than the warps of one CTA per SM; with more, a warp's
+// second stage is of use, and the even split over all warps is the better one.
+bool plan_closed(ctox_ctx *ctx, const DispatchItem *it, uint32_t n, uint32_t npos, StreamArgs *a) {
+    if (n > (uint32_t)kStreamItems) return false;
+    uint32_t cta = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const MatvecPart &p = *it[i].part;
+        const MatvecPart::Split &split = p.split[npos > 4 ? 1 : 0];
+        if (split.warps != 16 || split.stages != 2 || p.slices != 1 || p.kst_s > 16 || p.kst_s != it[0].part->kst_s || p.dt != it[0].part->dt)
+            return false;
+        StreamParams sp = stream_params(ctx, p, npos);
+        sp.ctas_per_slice = (p.pairs + 16 / p.kst_s - 1) / (16 / p.kst_s);
+        a->item[i] = sp;
+        a->first_cta[i] = cta;
+        cta += sp.ctas_per_slice;
+    }
+    a->items = n;
+    a->closed = cta <= (uint32_t)ctx->sm_count;
+    return a->closed;
+}
+
 void free_matvec(ctox_matvec *mv) {
     ctox_ctx *ctx = mv->ctx;
     for (auto &p : mv->parts) {
@@ -1106,7 +1171,8 @@ ctox_status dispatch_pass(ctox_ctx *ctx, const DispatchItem *it, uint64_t n, con
         StreamArgs a{};
         const MatvecPart &p0 = *it[i0].part;
         const bool own = p0.kst_s * 4 * npos <= kOwnGroups;
-        if ((own || k > 1) && plan_merged(ctx, it + i0, k, npos, &a)) {
+        const bool closed = own && plan_closed(ctx, it + i0, k, npos, &a);
+        if (closed || ((own || k > 1) && plan_merged(ctx, it + i0, k, npos, &a))) {
             if (own)
                 a.in = in;
             else
@@ -1116,6 +1182,7 @@ ctox_status dispatch_pass(ctox_ctx *ctx, const DispatchItem *it, uint64_t n, con
                 a.item[i].xfrag = first->xfrag;
                 a.item[i].meta = first->meta;
                 if (k > 1) f.item[i].warps_per_slice = a.item[i].warps_per_slice;  // cut anew
+                if (closed) a.out[i] = f.item[i];
                 bytes += (double)it[i0 + i].part->prep_bytes;
                 rows += (double)it[i0 + i].part->rows;
             }
@@ -1138,7 +1205,7 @@ ctox_status dispatch_pass(ctox_ctx *ctx, const DispatchItem *it, uint64_t n, con
                 EX(matvec_stream_prepared(mv, (size_t)(it[i0 + i].part - mv->parts.data()), npos, first));
             }
         }
-        launch_finish(ctx->stream, f, k, npos);
+        if (!closed) launch_finish(ctx->stream, f, k, npos);
     }
     return CTOX_OK;
 }
