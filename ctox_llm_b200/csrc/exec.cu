@@ -871,7 +871,7 @@ namespace {
 AttnGeom attn_geom(const ctox_exec *e) {
     const ctox_model_config &c = e->cfg;
     return AttnGeom{c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.rotary_dim, c.rope_theta,
-                    c.rms_norm_epsilon};
+                    c.rms_norm_epsilon, e->ctx->dev_error};
 }
 
 // Column-split projection in a tensor-parallel group: finish this rank's partial result, sum it

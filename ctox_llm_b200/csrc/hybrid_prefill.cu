@@ -594,7 +594,8 @@ constexpr uint32_t kLongCap = 1024;  // positions per pass: the buffers take 0.3
 
 AttnGeom geom(const ctox_exec *e) {
     const ctox_model_config &c = e->cfg;
-    return AttnGeom{c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.rotary_dim, c.rope_theta, c.rms_norm_epsilon};
+    return AttnGeom{c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.rotary_dim, c.rope_theta, c.rms_norm_epsilon,
+                    e->ctx->dev_error};
 }
 
 template <int MODE>

@@ -355,7 +355,6 @@ __global__ void __launch_bounds__(256) k_attn_pre(MvOut fan, AttnGeom g, const f
                                                   float *__restrict__ gate, T *__restrict__ k_cache,
                                                   T *__restrict__ v_cache, const uint32_t *__restrict__ page_table,
                                                   uint32_t page_tokens) {
-    pdl_launch();
     __shared__ float buf[256];
     __shared__ float red[8];
     const uint32_t heads_total = g.q_heads + 2 * g.kv_heads;
@@ -381,6 +380,7 @@ __global__ void __launch_bounds__(256) k_attn_pre(MvOut fan, AttnGeom g, const f
         sn = sinf(ang);
     }
     pdl_wait();
+    pdl_launch();  // not before: attention reads earlier passes' cache rows ahead of its own wait
     const float v = out_at(fan, ref, row, m);
     if (is_v) {  // value head: plain copy into the cache
         kv_store(v_cache + (slot * g.kv_heads + head) * hd + d, v);
@@ -1074,7 +1074,15 @@ void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const 
                       const void *k_cache, const void *v_cache, int kv_bf16, const uint32_t *page_table,
                       uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits, float *workspace,
                       const MvIn &next) {
-    launch_attention_kernel(st, g, q, k_cache, v_cache, kv_bf16, page_table, page_tokens, cache_slot, m, m, splits, workspace);
+    // tcgen05 from a few tiles per part of the context on: it has more to set up and to merge. Blocks of a four-layer model, all
+    // attention, 24 heads over 4: with three drafts 912 (mma.sync) and 914 us at 4000 tokens, 934 / 922 at 6000, 1174 / 1075 at
+    // 32000; without drafts 493 / 495 at 8000, 517 / 510 at 12000, 615 / 568 at 32000.
+    const uint32_t nq = g.q_heads / g.kv_heads * m;
+    const uint64_t tiles = (cache_slot + m + kFaTile - 1) / kFaTile;
+    if (kv_bf16 && g.head_dim == kFaHd && nq <= 32 && tiles >= (nq <= 16 ? 4u : 3u) * (uint64_t)splits)
+        launch_attention_tensor(st, g, q, k_cache, v_cache, page_table, page_tokens, cache_slot, m, splits, workspace);
+    else
+        launch_attention_kernel(st, g, q, k_cache, v_cache, kv_bf16, page_table, page_tokens, cache_slot, m, m, splits, workspace);
     launch_pdl(k_attn_combine_prep, dim3(m * g.q_heads), dim3(g.head_dim), 0, st, g, workspace, gate, (int)m, splits, next);
 }
 

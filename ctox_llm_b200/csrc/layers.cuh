@@ -42,6 +42,7 @@ constexpr int kAttnMaxSplits = 160;
 struct AttnGeom {
     uint32_t q_heads, kv_heads, head_dim, rotary_dim;
     float theta, eps;
+    int32_t *error_word;
 };
 
 // h[m] (+= matvec output; = it where `fresh`) ; xn = rmsnorm_1p(h[m], w) ; optional copy of xn ; fragments of xn * s_in.
@@ -85,6 +86,11 @@ void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const 
                       const void *k_cache, const void *v_cache, int kv_bf16, const uint32_t *page_table,
                       uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits, float *workspace,
                       const MvIn &next);
+
+// The part of it that runs on tcgen05 (attention_tensor.cu): head_dim 256, bf16 cache, at most 32 query rows.
+void launch_attention_tensor(cudaStream_t st, const AttnGeom &g, const float *q, const void *k_cache, const void *v_cache,
+                             const uint32_t *page_table, uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits,
+                             float *workspace);
 
 // Linear attention of one layer in one kernel: causal conv + SiLU over this head's channels of the
 // fused projection, decay/beta, the gated-delta recurrence over the m positions, rms_norm_gated and
