@@ -452,6 +452,13 @@ __global__ void __launch_bounds__(512, 1) k_linear_attention(LinearAttnArgs a, i
     }
     const bool pieces = total >= 1 && total <= 8;  // otherwise the general fetch per position
     const float so = pieces && o.s_out ? o.s_out[row] : 1.0f;
+    // weights of the gated norm and scales of out_proj for the outputs of this lane (phase 3)
+    float nw[4], si[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        nw[j] = warp < (uint32_t)npos ? a.norm_w[lane * 4 + j] : 0.f;
+        si[j] = warp < (uint32_t)npos && a.next.s_in ? a.next.s_in[head * kDeltaDim + lane * 4 + j] : 1.0f;
+    }
     pdl_wait();
 
     // ---- 1. conv + SiLU, z, decay, beta
@@ -594,12 +601,11 @@ __global__ void __launch_bounds__(512, 1) k_linear_attention(LinearAttnArgs a, i
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
         const float inv = 1.0f / sqrtf(sq / 128.0f + a.eps);
-        const uint32_t ocol = head * kDeltaDim + lane * 4;
         const float cs[4] = {c.x, c.y, c.z, c.w}, gz[4] = {g.x, g.y, g.z, g.w};
         float v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            v[j] = cs[j] * inv * a.norm_w[lane * 4 + j] * silu_f(gz[j]) * (a.next.s_in ? a.next.s_in[ocol + j] : 1.0f);
+            v[j] = cs[j] * inv * nw[j] * silu_f(gz[j]) * si[j];
         const unsigned gmask = (lane & 16) ? 0xffff0000u : 0x0000ffffu;
         prep_block(v, lane & 15, gmask, (int)(head * 2 + (lane >> 4)), m, npos, a.next.dt, a.next.xfrag, a.next.meta);
     }

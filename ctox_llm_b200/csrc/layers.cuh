@@ -225,12 +225,13 @@ __device__ __forceinline__ OutRef out_ref(const MvOut &o, uint32_t row) {
 __device__ __forceinline__ float out_at(const MvOut &o, const OutRef &r, uint32_t row, uint32_t pos) {
     if (!r.pieces) return out_of(o, row, pos);
     const float *first = r.first + pos * 32;
+    constexpr int kTrip = 24;  // pieces requested together: a 5120 x 17408 product leaves 20 (four slices of five)
     float v = 0.f;
     uint32_t sl = 0, q = 0;
-    for (uint32_t k0 = 0; k0 < r.total; k0 += 8) {
-        float buf[8];
+    for (uint32_t k0 = 0; k0 < r.total; k0 += kTrip) {
+        float buf[kTrip];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < kTrip; ++j) {
             buf[j] = 0.f;
             if (k0 + j < r.total) {
                 buf[j] = first[((size_t)sl * o.max_pieces + q) * 256];
@@ -241,7 +242,7 @@ __device__ __forceinline__ float out_at(const MvOut &o, const OutRef &r, uint32_
             }
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < kTrip; ++j)
             if (k0 + j < r.total) v += buf[j];
     }
     return o.s_out ? v * r.so : v;
