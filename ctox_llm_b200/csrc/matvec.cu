@@ -264,16 +264,23 @@ struct FinishItem {
     uint32_t rows, slices, max_pieces, activation;
     uint32_t kst_s, warps_per_slice, pairs;  // warps_per_slice == 0: piece counts from the table
 };
-// The matrices of one launch; matrix i takes the CTAs from first_cta[i] on. closed: a CTA takes whole row pairs, a warp per unit, and
-// writes the outputs itself.
+// The matrices of one launch; matrix i takes the CTAs from first_cta[i] on.
 constexpr int kStreamItems = 4;
 struct StreamArgs {
     StreamParams item[kStreamItems];
     uint32_t first_cta[kStreamItems];
-    uint32_t items, closed;
+    uint32_t items;
     StreamInput in;
+};
+// The same where a CTA takes whole row pairs, a warp per unit, and writes the outputs itself.
+struct ClosedArgs : StreamArgs {
     FinishItem out[kStreamItems];
 };
+// A pass of the executor, a stand-alone dispatch, or a closed one.
+enum StreamForm { STREAM_PASS, STREAM_DISPATCH, STREAM_CLOSED };
+template <StreamForm FORM>
+using StreamFormArgs = std::conditional_t<FORM == STREAM_PASS, StreamParams, std::conditional_t<FORM == STREAM_DISPATCH, StreamArgs, ClosedArgs>>;
+
 
 __device__ __forceinline__ const StreamParams &stream_item(const StreamParams &p, uint32_t) { return p; }
 __device__ __forceinline__ const StreamParams &stream_item(const StreamArgs &a, uint32_t i) { return a.item[i]; }
@@ -337,11 +344,12 @@ __device__ __forceinline__ void block_mma(float (&c)[4], uint32_t w0, uint32_t w
     }
 }
 
-// DISPATCH: a stand-alone dispatch. The matrices of a fan-out share the launch, and where that is little work every CTA forms
+// FORM: in a stand-alone dispatch the matrices of a fan-out share the launch, and where that is little work every CTA forms
 // the fragments of its slice itself instead of waiting for a kernel that does (kOwnGroups).
-template <int DT, int WARPS, int STAGES, int NT, bool DISPATCH>
+template <int DT, int WARPS, int STAGES, int NT, StreamForm FORM>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-    k_matvec_stream(const __grid_constant__ std::conditional_t<DISPATCH, StreamArgs, StreamParams> args) {
+    k_matvec_stream(const __grid_constant__ StreamFormArgs<FORM> args) {
+    constexpr bool DISPATCH = FORM != STREAM_PASS, closed = FORM == STREAM_CLOSED;
     pdl_launch();
     uint32_t cta = blockIdx.x, which = 0;
     if constexpr (DISPATCH) {
@@ -373,11 +381,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
     const uint32_t slice = cta / p.ctas_per_slice;  // closed: there is one
     const uint32_t lw = (cta % p.ctas_per_slice) * WARPS + warp;
     const uint64_t total = (uint64_t)p.pairs * p.kst_s;
-    bool closed = false;
-    if constexpr (DISPATCH) closed = args.closed;
     bool active = lw < p.warps_per_slice;
     uint64_t beg = 0, end = 0;
-    if (closed) {
+    if constexpr (closed) {
         const uint32_t pair = cta * (WARPS / p.kst_s) + warp / p.kst_s;
         active = warp < WARPS / p.kst_s * p.kst_s && pair < p.pairs;
         beg = (uint64_t)pair * p.kst_s + warp % p.kst_s;
@@ -574,34 +580,32 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
             mbar_wait(my_bars + 8 * (c % STAGES), (c / STAGES) & 1);
         if (!closed) return;
     }
-    if constexpr (DISPATCH) {
-        if (closed) {  // the warps of a pair leave their sums in their own stages: [position][32 rows]
-            auto sums_of = [&](uint32_t w) { return reinterpret_cast<float *>(stages + w * STAGES * kChunkBytes); };
-            if (active) {
+    if constexpr (closed) {  // the warps of a pair leave their sums in their own stages: [position][32 rows]
+        auto sums_of = [&](uint32_t w) { return reinterpret_cast<float *>(stages + w * STAGES * kChunkBytes); };
+        if (active) {
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
-                    if (has_m[nt]) {
-                        float *col = sums_of(warp) + (4 * nt + t) * kPairRows;
-                        col[rloc[0]] = acc[nt][0] + acc[nt][1];
-                        col[rloc[1]] = acc[nt][2] + acc[nt][3];
-                        col[rloc[2]] = acc[nt][4] + acc[nt][5];
-                        col[rloc[3]] = acc[nt][6] + acc[nt][7];
-                    }
-            }
-            __syncthreads();
-            const FinishItem &f = args.out[which];
-            const uint32_t per = WARPS / p.kst_s;
-            for (uint32_t i = threadIdx.x; i < per * p.npos * kPairRows; i += WARPS * 32) {
-                const uint32_t r = i % kPairRows, pos = i / kPairRows % p.npos, q = i / (kPairRows * p.npos);
-                const uint32_t row = (cta * per + q) * kPairRows + r;
-                if (row >= f.rows) continue;
-                float v = 0.f;
-                for (uint32_t k = 0; k < p.kst_s; ++k) v += sums_of(q * p.kst_s + k)[pos * kPairRows + r];
-                f.y[(long long)pos * f.y_stride + row] =
-                    finish_value(f, v, f.s_out ? f.s_out[row] : 1.0f, f.bias ? f.bias[row] : 0.0f);
-            }
-            return;
+            for (int nt = 0; nt < NT; ++nt)
+                if (has_m[nt]) {
+                    float *col = sums_of(warp) + (4 * nt + t) * kPairRows;
+                    col[rloc[0]] = acc[nt][0] + acc[nt][1];
+                    col[rloc[1]] = acc[nt][2] + acc[nt][3];
+                    col[rloc[2]] = acc[nt][4] + acc[nt][5];
+                    col[rloc[3]] = acc[nt][6] + acc[nt][7];
+                }
         }
+        __syncthreads();
+        const FinishItem &f = args.out[which];
+        const uint32_t per = WARPS / p.kst_s;
+        for (uint32_t i = threadIdx.x; i < per * p.npos * kPairRows; i += WARPS * 32) {
+            const uint32_t r = i % kPairRows, pos = i / kPairRows % p.npos, q = i / (kPairRows * p.npos);
+            const uint32_t row = (cta * per + q) * kPairRows + r;
+            if (row >= f.rows) continue;
+            float v = 0.f;
+            for (uint32_t k = 0; k < p.kst_s; ++k) v += sums_of(q * p.kst_s + k)[pos * kPairRows + r];
+            f.y[(long long)pos * f.y_stride + row] =
+                finish_value(f, v, f.s_out ? f.s_out[row] : 1.0f, f.bias ? f.bias[row] : 0.0f);
+        }
+        return;
     }
     close_pair(cur_pair, cur_ks == p.kst_s);
 }
@@ -851,9 +855,13 @@ ctox_status upload_f32(ctox_ctx *ctx, const float *src, uint64_t n, float **dst,
 struct StreamCfg {
     int warps, stages;
 };
+// Eight warps with four stages leave room on an SM for the kernels before and after, which then start ahead of their wait: the
+// shape of dispatches that stand alone (5120 x 17408 Q2, four positions 10.9 -> 9.7 us; 17408 x 5120 Q4, one 11.0 -> 10.7 to 11.1;
+// two stages take 9.3 and 9.8, but 35 instead of 28 us for a single Q4 dispatch from an idle GPU). In the executor's chain the body
+// gains from sixteen: two blocks of 64 layers take 12.5 ms with sixteen and 12.9 with eight, and eight for the smallest matrices alone
+// make some models of width 1024 to 2560 4 % faster and others 6 % slower.
 
-FinishItem finish_item(const ctox_matvec *mv, const MatvecPart &p, uint32_t npos, float *y, uint64_t y_stride) {
-    const MatvecPart::Split &sp = p.split[npos > 4 ? 1 : 0];
+FinishItem finish_item(const ctox_matvec *mv, const MatvecPart &p, const MatvecPart::Split &sp, float *y, uint64_t y_stride) {
     const uint64_t units = (uint64_t)p.pairs * p.kst_s;
     const bool fits = (units + 1) * sp.warps_per_slice + units < (1ull << 32);  // piece_count() in 32 bits
     return FinishItem{p.partial, sp.pieces, mv->s_out ? mv->s_out + p.row_start : nullptr,
@@ -892,11 +900,11 @@ StreamCfg pick_stream_cfg(ctox_ctx *ctx, int dt, uint32_t slice_blocks, uint32_t
 template <int DT, int NT>
 void launch_stream_nt(StreamCfg cfg, unsigned grid, size_t smem, cudaStream_t st, const StreamParams &sp) {
     if (cfg.warps == 16)
-        launch_pdl(k_matvec_stream<DT, 16, 2, NT, false>, dim3(grid), dim3(512), smem, st, sp);
+        launch_pdl(k_matvec_stream<DT, 16, 2, NT, STREAM_PASS>, dim3(grid), dim3(512), smem, st, sp);
     else if (cfg.stages == 4)
-        launch_pdl(k_matvec_stream<DT, 8, 4, NT, false>, dim3(grid), dim3(256), smem, st, sp);
+        launch_pdl(k_matvec_stream<DT, 8, 4, NT, STREAM_PASS>, dim3(grid), dim3(256), smem, st, sp);
     else
-        launch_pdl(k_matvec_stream<DT, 8, 2, NT, false>, dim3(grid), dim3(256), smem, st, sp);
+        launch_pdl(k_matvec_stream<DT, 8, 2, NT, STREAM_PASS>, dim3(grid), dim3(256), smem, st, sp);
 }
 
 template <int DT>
@@ -907,6 +915,18 @@ void launch_stream(StreamCfg cfg, unsigned grid, size_t smem, cudaStream_t st, c
         launch_stream_nt<DT, 1>(cfg, grid, smem, st, sp);
 }
 
+template <StreamForm FORM>
+void launch_merged(int dt, uint32_t npos, unsigned grid, size_t smem, cudaStream_t st, const StreamFormArgs<FORM> &a) {
+    if (dt && npos > 4)
+        launch_pdl(k_matvec_stream<1, 16, 2, 2, FORM>, dim3(grid), dim3(512), smem, st, a);
+    else if (dt)
+        launch_pdl(k_matvec_stream<1, 16, 2, 1, FORM>, dim3(grid), dim3(512), smem, st, a);
+    else if (npos > 4)
+        launch_pdl(k_matvec_stream<0, 16, 2, 2, FORM>, dim3(grid), dim3(512), smem, st, a);
+    else
+        launch_pdl(k_matvec_stream<0, 16, 2, 1, FORM>, dim3(grid), dim3(512), smem, st, a);
+}
+
 // One matrix of a stand-alone dispatch and where its outputs go.
 struct DispatchItem {
     ctox_matvec *mv;
@@ -915,8 +935,7 @@ struct DispatchItem {
     uint64_t y_stride;
 };
 
-StreamParams stream_params(ctox_ctx *ctx, const MatvecPart &p, uint32_t npos) {
-    const MatvecPart::Split &split = p.split[npos > 4 ? 1 : 0];
+StreamParams stream_params(ctox_ctx *ctx, const MatvecPart &p, const MatvecPart::Split &split, uint32_t npos) {
     StreamParams sp{};
     sp.wprep = p.prep;
     sp.partial = p.partial;
@@ -954,7 +973,7 @@ bool plan_merged(ctox_ctx *ctx, const DispatchItem *it, uint32_t n, uint32_t npo
     a->items = n;
     for (uint32_t i = 0; i < n; ++i) {
         const MatvecPart &p = *it[i].part;
-        StreamParams sp = stream_params(ctx, p, npos);
+        StreamParams sp = stream_params(ctx, p, p.split[npos > 4 ? 1 : 0], npos);
         if (n > 1) {
             const uint64_t units = (uint64_t)p.pairs * p.kst_s;
             uint32_t ctas = (uint32_t)((uint64_t)ctx->sm_count * units / total);  // per slice
@@ -981,7 +1000,7 @@ bool plan_merged(ctox_ctx *ctx, const DispatchItem *it, uint32_t n, uint32_t npo
 // A launch whose CTAs take whole row pairs, a warp per unit, and write the outputs themselves: no second kernel (1024 x 1024, one
 // position: 5.9 -> 3.9 us). For matrices of one slice whose units are no more than the warps of one CTA per SM; with more, a warp's
 // second stage is of use, and the even split over all warps is the better one.
-bool plan_closed(ctox_ctx *ctx, const DispatchItem *it, uint32_t n, uint32_t npos, StreamArgs *a) {
+bool plan_closed(ctox_ctx *ctx, const DispatchItem *it, uint32_t n, uint32_t npos, ClosedArgs *a) {
     if (n > (uint32_t)kStreamItems) return false;
     uint32_t cta = 0;
     for (uint32_t i = 0; i < n; ++i) {
@@ -989,15 +1008,14 @@ bool plan_closed(ctox_ctx *ctx, const DispatchItem *it, uint32_t n, uint32_t npo
         const MatvecPart::Split &split = p.split[npos > 4 ? 1 : 0];
         if (split.warps != 16 || split.stages != 2 || p.slices != 1 || p.kst_s > 16 || p.kst_s != it[0].part->kst_s || p.dt != it[0].part->dt)
             return false;
-        StreamParams sp = stream_params(ctx, p, npos);
+        StreamParams sp = stream_params(ctx, p, split, npos);
         sp.ctas_per_slice = (p.pairs + 16 / p.kst_s - 1) / (16 / p.kst_s);
         a->item[i] = sp;
         a->first_cta[i] = cta;
         cta += sp.ctas_per_slice;
     }
     a->items = n;
-    a->closed = cta <= (uint32_t)ctx->sm_count;
-    return a->closed;
+    return cta <= (uint32_t)ctx->sm_count;
 }
 
 void free_matvec(ctox_matvec *mv) {
@@ -1062,9 +1080,14 @@ ctox_status prepare_part(ctox_ctx *ctx, ctox_matvec *mv, MatvecPart &part, const
     // (pair, slice) is cut into
     const uint64_t units = (uint64_t)part.pairs * part.kst_s;  // per slice
     part.max_pieces = 1;
-    for (int cls = 0; cls < 2; ++cls) {
+    for (int cls = 0; cls < kSplits; ++cls) {
         MatvecPart::Split &sp = part.split[cls];
-        const StreamCfg cfg = pick_stream_cfg(ctx, part.dt, part.kst_s * 4, cls ? kMaxPosPerPass : 4);
+        StreamCfg cfg = pick_stream_cfg(ctx, part.dt, part.kst_s * 4, cls == 1 ? kMaxPosPerPass : 4);
+        if (cls == kAloneSplit) {
+            const StreamCfg alone{8, 4};
+            if (cfg.warps != 16 || stream_smem_bytes(part.dt, alone, part.kst_s * 4, 4) > (size_t)ctx->max_smem_optin) continue;
+            cfg = alone;
+        }
         sp.warps = cfg.warps;
         sp.stages = cfg.stages;
         if (cfg.warps == 0) continue;
@@ -1115,22 +1138,26 @@ ctox_status set_smem_attr(ctox_ctx *ctx) {
 #define CTOX_SMEM_ATTR(...)                                                                        \
     CTOX_CUDA(ctx, cudaFuncSetAttribute(k_matvec_stream<__VA_ARGS__>,                              \
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin))
-    CTOX_SMEM_ATTR(0, 16, 2, 1, true);
-    CTOX_SMEM_ATTR(1, 16, 2, 1, true);
-    CTOX_SMEM_ATTR(0, 16, 2, 2, true);
-    CTOX_SMEM_ATTR(1, 16, 2, 2, true);
-    CTOX_SMEM_ATTR(0, 16, 2, 1, false);
-    CTOX_SMEM_ATTR(1, 16, 2, 1, false);
-    CTOX_SMEM_ATTR(0, 8, 4, 1, false);
-    CTOX_SMEM_ATTR(1, 8, 4, 1, false);
-    CTOX_SMEM_ATTR(0, 8, 2, 1, false);
-    CTOX_SMEM_ATTR(1, 8, 2, 1, false);
-    CTOX_SMEM_ATTR(0, 16, 2, 2, false);
-    CTOX_SMEM_ATTR(1, 16, 2, 2, false);
-    CTOX_SMEM_ATTR(0, 8, 4, 2, false);
-    CTOX_SMEM_ATTR(1, 8, 4, 2, false);
-    CTOX_SMEM_ATTR(0, 8, 2, 2, false);
-    CTOX_SMEM_ATTR(1, 8, 2, 2, false);
+    CTOX_SMEM_ATTR(0, 16, 2, 1, STREAM_PASS);
+    CTOX_SMEM_ATTR(0, 16, 2, 1, STREAM_DISPATCH);
+    CTOX_SMEM_ATTR(0, 16, 2, 1, STREAM_CLOSED);
+    CTOX_SMEM_ATTR(0, 8, 4, 1, STREAM_PASS);
+    CTOX_SMEM_ATTR(0, 8, 2, 1, STREAM_PASS);
+    CTOX_SMEM_ATTR(0, 16, 2, 2, STREAM_PASS);
+    CTOX_SMEM_ATTR(0, 16, 2, 2, STREAM_DISPATCH);
+    CTOX_SMEM_ATTR(0, 16, 2, 2, STREAM_CLOSED);
+    CTOX_SMEM_ATTR(0, 8, 4, 2, STREAM_PASS);
+    CTOX_SMEM_ATTR(0, 8, 2, 2, STREAM_PASS);
+    CTOX_SMEM_ATTR(1, 16, 2, 1, STREAM_PASS);
+    CTOX_SMEM_ATTR(1, 16, 2, 1, STREAM_DISPATCH);
+    CTOX_SMEM_ATTR(1, 16, 2, 1, STREAM_CLOSED);
+    CTOX_SMEM_ATTR(1, 8, 4, 1, STREAM_PASS);
+    CTOX_SMEM_ATTR(1, 8, 2, 1, STREAM_PASS);
+    CTOX_SMEM_ATTR(1, 16, 2, 2, STREAM_PASS);
+    CTOX_SMEM_ATTR(1, 16, 2, 2, STREAM_DISPATCH);
+    CTOX_SMEM_ATTR(1, 16, 2, 2, STREAM_CLOSED);
+    CTOX_SMEM_ATTR(1, 8, 4, 2, STREAM_PASS);
+    CTOX_SMEM_ATTR(1, 8, 2, 2, STREAM_PASS);
 #undef CTOX_SMEM_ATTR
     done_device = ctx->device;
     return CTOX_OK;
@@ -1145,6 +1172,31 @@ ctox_status check_device_error(ctox_ctx *ctx, const char *what) {
     if (code == DEV_ERR_WAIT_TIMEOUT)
         return fail(ctx, CTOX_INVALID_STATE, "%s: a bounded device wait ran out", what);
     if (code) return fail(ctx, CTOX_INVALID_STATE, "%s: device error %d", what, code);
+    return CTOX_OK;
+}
+
+// One launch over a part, cut as `split` says; the activations' fragments are those of fragments_of.
+ctox_status stream_part(ctox_matvec *mv, const MatvecPart &p, const MatvecPart::Split &split, uint32_t npos, const ctox_matvec *fragments_of) {
+    ctox_ctx *ctx = mv->ctx;
+    const StreamCfg cfg{split.warps, split.stages};
+    if (cfg.warps == 0) {
+        // the class shape does not fit; a smaller position count may (same work split as class 0
+        // only if the shape is the same, so recompute nothing: refuse instead)
+        return fail(ctx, CTOX_MEMORY_BUDGET, "streaming kernel: %u positions of %llu columns exceed shared memory",
+                    npos, (unsigned long long)mv->columns);
+    }
+    StreamParams sp = stream_params(ctx, p, split, npos);
+    sp.xfrag = fragments_of->xfrag;
+    sp.meta = fragments_of->meta;
+    const size_t smem = stream_smem_bytes(p.dt, cfg, p.kst_s * 4, npos);
+    const unsigned grid = split.ctas_per_slice * p.slices;
+    timing_begin(ctx);
+    if (p.dt)
+        launch_stream<1>(cfg, grid, smem, ctx->stream, sp);
+    else
+        launch_stream<0>(cfg, grid, smem, ctx->stream, sp);
+    timing_end(ctx, KC_STREAM_MATVEC, (double)p.prep_bytes, 2.0 * (double)p.rows * (double)mv->columns * npos);
+    CTOX_CUDA(ctx, cudaGetLastError());
     return CTOX_OK;
 }
 
@@ -1166,46 +1218,45 @@ ctox_status dispatch_pass(ctox_ctx *ctx, const DispatchItem *it, uint64_t n, con
     };
     for (uint64_t i0 = 0; i0 < n; i0 += kFinishItems) {
         const uint32_t k = n - i0 < (uint64_t)kFinishItems ? (uint32_t)(n - i0) : (uint32_t)kFinishItems;
+        ClosedArgs a{};
         FinishArgs f{};
-        for (uint32_t i = 0; i < k; ++i) f.item[i] = finish_item(it[i0 + i].mv, *it[i0 + i].part, npos, it[i0 + i].y, it[i0 + i].y_stride);
-        StreamArgs a{};
         const MatvecPart &p0 = *it[i0].part;
         const bool own = p0.kst_s * 4 * npos <= kOwnGroups;
-        const bool closed = own && plan_closed(ctx, it + i0, k, npos, &a);
-        if (closed || ((own || k > 1) && plan_merged(ctx, it + i0, k, npos, &a))) {
-            if (own)
-                a.in = in;
-            else
-                prepare(p0.dt);
+        const bool closed = own && plan_closed(ctx, it + i0, k, npos, &a), merged = closed || ((own || k > 1) && plan_merged(ctx, it + i0, k, npos, &a));
+        auto split_of = [&](const MatvecPart &p) -> const MatvecPart::Split & {
+            return p.split[npos > 4 ? 1 : !merged && p.split[kAloneSplit].warps ? kAloneSplit : 0];
+        };
+        for (uint32_t i = 0; i < k; ++i) {
+            const DispatchItem &d = it[i0 + i];
+            f.item[i] = finish_item(d.mv, *d.part, split_of(*d.part), d.y, d.y_stride);
+        }
+        if (own && merged)
+            a.in = in;
+        else
+            prepare(p0.dt);
+        if (merged) {
             double bytes = 0, rows = 0;
             for (uint32_t i = 0; i < k; ++i) {
                 a.item[i].xfrag = first->xfrag;
                 a.item[i].meta = first->meta;
                 if (k > 1) f.item[i].warps_per_slice = a.item[i].warps_per_slice;  // cut anew
-                if (closed) a.out[i] = f.item[i];
+                a.out[i] = f.item[i];
                 bytes += (double)it[i0 + i].part->prep_bytes;
                 rows += (double)it[i0 + i].part->rows;
             }
             const uint32_t grid = a.first_cta[k - 1] + a.item[k - 1].ctas_per_slice * a.item[k - 1].slices;
             const size_t smem = stream_smem_bytes(p0.dt, StreamCfg{16, 2}, p0.kst_s * 4, npos);
             timing_begin(ctx);
-            if (p0.dt && npos > 4)
-                launch_pdl(k_matvec_stream<1, 16, 2, 2, true>, dim3(grid), dim3(512), smem, ctx->stream, a);
-            else if (p0.dt)
-                launch_pdl(k_matvec_stream<1, 16, 2, 1, true>, dim3(grid), dim3(512), smem, ctx->stream, a);
-            else if (npos > 4)
-                launch_pdl(k_matvec_stream<0, 16, 2, 2, true>, dim3(grid), dim3(512), smem, ctx->stream, a);
+            if (closed)
+                launch_merged<STREAM_CLOSED>(p0.dt, npos, grid, smem, ctx->stream, a);
             else
-                launch_pdl(k_matvec_stream<0, 16, 2, 1, true>, dim3(grid), dim3(512), smem, ctx->stream, a);
+                launch_merged<STREAM_DISPATCH>(p0.dt, npos, grid, smem, ctx->stream, a);
             timing_end(ctx, KC_STREAM_MATVEC, bytes, 2.0 * rows * (double)first->columns * npos);
+            if (closed) continue;
         } else {
-            prepare(p0.dt);
-            for (uint32_t i = 0; i < k; ++i) {
-                ctox_matvec *mv = it[i0 + i].mv;
-                EX(matvec_stream_prepared(mv, (size_t)(it[i0 + i].part - mv->parts.data()), npos, first));
-            }
+            for (uint32_t i = 0; i < k; ++i) EX(stream_part(it[i0 + i].mv, *it[i0 + i].part, split_of(*it[i0 + i].part), npos, first));
         }
-        if (!closed) launch_finish(ctx->stream, f, k, npos);
+        launch_finish(ctx->stream, f, k, npos);
     }
     return CTOX_OK;
 }
@@ -1235,29 +1286,8 @@ uint32_t matvec_positions_per_pass(ctox_matvec *mv) {
 
 // fragments_of: another matrix of the same fan-out group whose fragment buffers hold the activations.
 ctox_status matvec_stream_prepared(ctox_matvec *mv, size_t part_index, uint32_t npos, const ctox_matvec *fragments_of) {
-    ctox_ctx *ctx = mv->ctx;
     MatvecPart &p = mv->parts[part_index];
-    const MatvecPart::Split &split = p.split[npos > 4 ? 1 : 0];
-    StreamCfg cfg{split.warps, split.stages};
-    if (cfg.warps == 0) {
-        // the class shape does not fit; a smaller position count may (same work split as class 0
-        // only if the shape is the same, so recompute nothing: refuse instead)
-        return fail(ctx, CTOX_MEMORY_BUDGET, "streaming kernel: %u positions of %llu columns exceed shared memory",
-                    npos, (unsigned long long)mv->columns);
-    }
-    StreamParams sp = stream_params(ctx, p, npos);
-    sp.xfrag = fragments_of ? fragments_of->xfrag : mv->xfrag;
-    sp.meta = fragments_of ? fragments_of->meta : mv->meta;
-    const size_t smem = stream_smem_bytes(p.dt, cfg, p.kst_s * 4, npos);
-    const unsigned grid = split.ctas_per_slice * p.slices;
-    timing_begin(ctx);
-    if (p.dt)
-        launch_stream<1>(cfg, grid, smem, ctx->stream, sp);
-    else
-        launch_stream<0>(cfg, grid, smem, ctx->stream, sp);
-    timing_end(ctx, KC_STREAM_MATVEC, (double)p.prep_bytes, 2.0 * (double)p.rows * (double)mv->columns * npos);
-    CTOX_CUDA(ctx, cudaGetLastError());
-    return CTOX_OK;
+    return stream_part(mv, p, p.split[npos > 4 ? 1 : 0], npos, fragments_of ? fragments_of : mv);
 }
 
 ctox_status matvec_stream_pass(ctox_matvec *mv, size_t part_index, const void *x, uint32_t x_dtype,
@@ -1334,7 +1364,7 @@ ctox_status matvec_embed_rows(ctox_matvec *mv, const uint32_t *row_ids_dev, uint
 
 void matvec_finish_enqueue(ctox_matvec *mv, uint32_t npos, float *y, uint64_t y_stride) {
     FinishArgs a{};
-    a.item[0] = finish_item(mv, mv->parts[0], npos, y, y_stride);
+    a.item[0] = finish_item(mv, mv->parts[0], mv->parts[0].split[npos > 4 ? 1 : 0], y, y_stride);
     launch_finish(mv->ctx->stream, a, 1, npos);
 }
 
@@ -1810,7 +1840,7 @@ extern "C" ctox_status ctox_matvec_dispatch_static(ctox_matvec *mv, const void *
             launch_pdl(k_prep_x, dim3((groups * 16 + 255) / 256), dim3(256), 0, st, xp, x_dtype == CTOX_BF16, (long long)x_stride,
                                                                mv->s_in, (int)mv->columns,
                                                                (int)mv->blocks_padded, (int)npos, p.dt, xfrag, meta);
-            StreamParams sp = stream_params(ctx, p, npos);
+            StreamParams sp = stream_params(ctx, p, split, npos);
             sp.xfrag = xfrag;
             sp.meta = meta;
             sp.partial = partial;
@@ -1824,7 +1854,7 @@ extern "C" ctox_status ctox_matvec_dispatch_static(ctox_matvec *mv, const void *
                 launch_stream<0>(cfg, grid, smem, st, sp);
             timing_end(ctx);
             FinishArgs a{};
-            a.item[0] = finish_item(mv, p, npos, y_dev + (size_t)m0 * y_stride + p.row_start, y_stride);
+            a.item[0] = finish_item(mv, p, split, y_dev + (size_t)m0 * y_stride + p.row_start, y_stride);
             a.item[0].partial = partial;
             launch_finish(st, a, 1, npos);
         }

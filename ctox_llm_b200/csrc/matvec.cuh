@@ -13,6 +13,8 @@ constexpr int kMaxPosPerPass = 8;  // positions per pass of the streaming kernel
 constexpr int kPairRows = 32;      // rows of a tile pair (the unit of work and of the partial sums)
 }  // namespace ctox
 
+constexpr int kSplits = 3, kAloneSplit = 2;
+
 struct MatvecPart {
     int dt = 0;  // 0 Q2, 1 Q4
     uint64_t row_start = 0, rows = 0;
@@ -26,13 +28,14 @@ struct MatvecPart {
     float *partial = nullptr;
     size_t partial_bytes = 0;
     // The work split depends on the launch shape, which depends on the number of positions
-    // (shared memory); one table per shape class: [0] 1..4 positions, [1] 5..8 positions.
+    // (shared memory); one table per shape class: [0] 1..4 positions, [1] 5..8 positions, [kAloneSplit] 1..4 positions of
+    // one matrix dispatched by itself (warps == 0: as [0]).
     struct Split {
         int warps = 0, stages = 0;       // launch shape; warps == 0: does not fit
         uint32_t ctas_per_slice = 0, warps_per_slice = 0, max_pieces = 1;
         uint8_t *pieces = nullptr;       // [pairs][slices] partial-sum pieces
         size_t pieces_bytes = 0;
-    } split[2];
+    } split[kSplits];
     uint32_t max_pieces = 1;  // slot stride of `partial`: max over both splits
 };
 
