@@ -23,7 +23,10 @@ def fill(leave):
     for chunk in (1 << 30, 64 << 20, 2 << 20):
         while torch.cuda.mem_get_info()[0] >= leave + chunk:
             n = (torch.cuda.mem_get_info()[0] - leave) // chunk * chunk
-            held.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
+            if n < 10 << 20:  # torch takes 20 MB from the device for a request of 1 to 10 MB, and 2 MB for two of 1 MB
+                held += [torch.empty(1 << 20, dtype=torch.uint8, device="cuda") for _ in range(n >> 20)]
+            else:
+                held.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
     return held
 
 
