@@ -331,63 +331,174 @@ __global__ void __launch_bounds__(256) k_long_gates(const LongGates p) {
     }
 }
 
-// The gated-delta recurrence (delta.cu) over all positions. Bound by the chain from token to token: a product with the
-// state, a sum across lanes, the update. A warp owns four value columns with their 128 keys (8 lanes per column, 16
-// state values each in registers), so that chain has three shuffles and no barrier; the tokens' inputs are staged
-// sixteen at a time, a block ahead. A CTA takes 16 columns: 8 CTAs per head.
-constexpr int kScanTokens = 16, kScanCols = 16;
-__device__ __forceinline__ float total4(const f32x2 (&v)[4]) {
-    float a[4], b[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) unpack2(v[i], a[i], b[i]);
-    return ((a[0] + b[0]) + (a[1] + b[1])) + ((a[2] + b[2]) + (a[3] + b[3]));
-}
-struct LongScan {
+// The gated-delta recurrence (delta.cu) over all positions, four tokens at a time. With the state S before the group, the decays'
+// products D_j = d_0 .. d_j, D_ij = d_(i+1) .. d_j and e_j = (v_j - memory read by k_j) * beta_j,
+//     e_j      = beta_j (v_j - D_j S k_j - sum_(i<j) D_ij (k_i . k_j) e_i)
+//     output_j = D_j S q_j + sum_(i<=j) D_ij (k_i . q_j) e_i
+//     S'       = D_3 S + sum_i D_i3 k_i e_i
+// so that the group's eight products with the state are independent and the chain (products, sums across lanes, update) is walked once
+// in four tokens. With u_j = v_j - D_j S k_j, e is a triangular matrix times u; k_long_coefs forms that matrix, which is the same for all
+// columns of a head, and leaves it with D_i3 (F, for the update) and with the outputs' factors (G) multiplied in.
+constexpr uint32_t kGroup = 4, kCoefs = 36;  // of a group: D[4], F[j][i], G[j][i] (zero for i > j)
+struct LongCoefs {
     const float *qkv, *decay, *beta;
+    float *coefs;  // [group][head][kCoefs]
+    uint32_t key_width, channels, heads, qk_heads, m;
+};
+// A warp per (group, key head), then a lane per factor of each of its value heads. Tokens past the last one have decay 1 and factors 0.
+__global__ void __launch_bounds__(128) k_long_coefs(const LongCoefs p) {
+    pdl_launch();
+    pdl_wait();
+    __shared__ float dots[4][kGroup][2 * kGroup];  // per warp: k_i . (k_0 .. k_3, q_0 .. q_3)
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, item = blockIdx.x * 4 + warp;
+    const uint32_t group = item / p.qk_heads, kh = item % p.qk_heads, t0 = group * kGroup;
+    if (t0 >= p.m) return;
+    float4 x[2 * kGroup];
+#pragma unroll
+    for (uint32_t j = 0; j < 2 * kGroup; ++j) {
+        const uint32_t t = t0 + j % kGroup;
+        x[j] = t < p.m ? *reinterpret_cast<const float4 *>(p.qkv + (size_t)t * p.channels + (j < kGroup ? p.key_width : 0) + kh * 128 + lane * 4)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kGroup; ++i)
+#pragma unroll
+        for (uint32_t j = i + 1; j < kGroup + kGroup; ++j) {
+            if (j >= kGroup && j - kGroup < i) continue;
+            float v = (x[i].x * x[j].x + x[i].y * x[j].y) + (x[i].z * x[j].z + x[i].w * x[j].w);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) dots[warp][i][j] = v;
+        }
+    __syncwarp();
+    const uint32_t repeat = p.heads / p.qk_heads;
+    for (uint32_t r = 0; r < repeat; ++r) {
+        const uint32_t head = kh * repeat + r;
+        float d[kGroup], beta[kGroup];
+#pragma unroll
+        for (uint32_t j = 0; j < kGroup; ++j) {
+            const bool in = t0 + j < p.m;
+            d[j] = in ? p.decay[(size_t)(t0 + j) * p.heads + head] : 1.0f;
+            beta[j] = in ? p.beta[(size_t)(t0 + j) * p.heads + head] : 0.f;
+        }
+        auto between = [&](uint32_t i, uint32_t j) {  // the decays of tokens i + 1 .. j
+            float v = 1.0f;
+#pragma unroll
+            for (uint32_t l = 0; l < kGroup; ++l)
+                if (l > i && l <= j) v *= d[l];
+            return v;
+        };
+        float kk[kGroup][kGroup], T[kGroup][kGroup];  // e = T u; every lane forms all of it
+#pragma unroll
+        for (uint32_t j = 0; j < kGroup; ++j)
+#pragma unroll
+            for (uint32_t i = 0; i < kGroup; ++i) {
+                if (i < j) kk[i][j] = between(i, j) * dots[warp][i][j];
+                T[j][i] = i == j ? 1.0f : 0.f;
+            }
+#pragma unroll
+        for (uint32_t j = 0; j < kGroup; ++j)
+#pragma unroll
+            for (uint32_t i = 0; i <= j; ++i) {
+#pragma unroll
+                for (uint32_t l = i; l < j; ++l) T[j][i] -= kk[l][j] * T[l][i];
+                T[j][i] *= beta[j];
+            }
+        float mine = 0.f, last = 0.f;  // factors `lane` and, of the first lanes, 32 + lane
+#pragma unroll
+        for (uint32_t j = 0; j < kGroup; ++j) {
+            if (lane == j) mine = d[0] * between(0, j);
+#pragma unroll
+            for (uint32_t i = 0; i <= j; ++i) {
+                if (lane == kGroup + j * kGroup + i) mine = between(j, kGroup - 1) * T[j][i];
+                float g = 0.f;
+#pragma unroll
+                for (uint32_t l = i; l <= j; ++l) g += between(l, j) * dots[warp][l][kGroup + j] * T[l][i];
+                const uint32_t at = kGroup + kGroup * kGroup + j * kGroup + i;
+                if (lane == at) mine = g;
+                if (lane + 32 == at) last = g;
+            }
+        }
+        float *out = p.coefs + ((size_t)group * p.heads + head) * kCoefs;
+        out[lane] = mine;
+        if (lane + 32 < kCoefs) out[lane + 32] = last;
+    }
+}
+
+// The scan itself. Bound by what goes through shared memory (a 16-byte read of all lanes is four cycles of its pipe, whether lanes share
+// addresses or not) and by the packed products with the state. A warp owns four value columns with their 128 keys: 16 lanes per
+// pair of columns, 2 x 8 state values each in registers, so that a key or query read serves two columns. 16 columns and 4 warps per
+// CTA, 8 CTAs per head: the fullest SM decides (48 heads: 48 columns on it, 64 with 32 columns per CTA). The tokens' inputs are
+// staged sixteen at a time, a block ahead. 999 tokens of 48 heads: 238 us and 10 for the factors; token by token with 8 lanes per column
+// 332, groups of four on that layout 309 (the shared-memory pipe 86 % busy), with two columns per 8 lanes 325 (too few warps).
+constexpr int kScanTokens = 16, kScanCols = 16, kScanThreads = kScanCols * 8, kScanCtas = 128 / kScanCols;  // CTAs per head
+struct LongScan {
+    const float *qkv, *coefs;
     float *state, *out;
     uint32_t key_width, channels, heads, qk_heads, m;
 };
-__global__ void __launch_bounds__(128) k_long_delta(const LongScan p) {
+__global__ void __launch_bounds__(kScanThreads) k_long_delta(const LongScan p) {
     pdl_launch();
     pdl_wait();
+    constexpr uint32_t kGroups = kScanTokens / kGroup;
     __shared__ __align__(16) float qs[2][kScanTokens][128], ks[2][kScanTokens][128], vs[2][kScanTokens][kScanCols];
-    __shared__ float ds[2][kScanTokens], bs[2][kScanTokens], os[kScanTokens][kScanCols];
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane & 7, c = warp * 4 + (lane >> 3);
-    const uint32_t head = blockIdx.x >> 3, col0 = (blockIdx.x & 7) * kScanCols, kh = head / (p.heads / p.qk_heads);
-    // this lane's keys are sub * 4 + 32 i .. + 3, i < 4; two of them per register pair
-    f32x2 s[8];
+    __shared__ __align__(16) float cs[2][kGroups][kCoefs];
+    __shared__ __align__(8) float os[kScanTokens][kScanCols];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane & 15, c = warp * 4 + (lane >> 4) * 2;
+    const uint32_t head = blockIdx.x / kScanCtas, col0 = blockIdx.x % kScanCtas * kScanCols, kh = head / (p.heads / p.qk_heads);
+    // this lane's keys are sub * 4 + 64 i .. + 3, i < 2, of columns c and c + 1; two keys per register pair
+    f32x2 s[2][4];
     float *state = p.state + (size_t)head * 128 * 128 + col0 + c;
+    auto state_at = [&](int i) { return reinterpret_cast<float2 *>(state + (size_t)((i >> 1) * 64 + sub * 4 + (i & 1) * 2) * 128); };
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float *at = state + (size_t)((i >> 1) * 32 + sub * 4 + (i & 1) * 2) * 128;
-        s[i] = pack2(at[0], at[128]);
+    for (int i = 0; i < 4; ++i) {
+        const float2 a = state_at(i)[0], b = state_at(i)[64];
+        s[0][i] = pack2(a.x, b.x);
+        s[1][i] = pack2(a.y, b.y);
     }
-    auto load = [&](ulonglong2(&d)[4], const float *row) {
+    auto load = [&](f32x2(&d)[4], const float *row) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) d[i] = *reinterpret_cast<const ulonglong2 *>(row + i * 32 + sub * 4);
+        for (int i = 0; i < 2; ++i) {
+            const ulonglong2 u = *reinterpret_cast<const ulonglong2 *>(row + i * 64 + sub * 4);
+            d[2 * i] = u.x;
+            d[2 * i + 1] = u.y;
+        }
     };
+    auto dot = [](const f32x2(&a)[4], const f32x2(&b)[4]) {
+        float u, v;
+        unpack2(fma2(a[3], b[3], fma2(a[2], b[2], fma2(a[1], b[1], mul2(a[0], b[0])))), u, v);
+        return u + v;
+    };
+    // After the sums over a pair's lanes, lane sub holds token sub & 3, column c + (sub >> 3), the product with its query (sub & 4) or key.
+    const bool b8 = sub & 8, b4 = sub & 4, b2 = sub & 2, b1 = sub & 1;
+    const uint32_t tok = sub & 3, of_column = (lane & 24);  // first lane of this one's column
     auto copy16 = [](void *dst, const void *src) {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                      : "memory");
     };
-    auto copy4 = [](void *dst, const void *src) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                     : "memory");
-    };
     auto fetch = [&](uint32_t t0, uint32_t b) {
-        const uint32_t n = min((uint32_t)kScanTokens, p.m - t0);
-        for (uint32_t i = tid; i < n * 32; i += 128) {
-            const float *row = p.qkv + (size_t)(t0 + (i >> 5)) * p.channels + kh * 128 + (i & 31) * 4;
-            copy16(&qs[b][i >> 5][(i & 31) * 4], row);
-            copy16(&ks[b][i >> 5][(i & 31) * 4], row + p.key_width);
+        const uint32_t n = min((uint32_t)kScanTokens, p.m - t0), groups = (n + kGroup - 1) / kGroup;
+        for (uint32_t i = tid; i < groups * kGroup * 32; i += kScanThreads) {
+            const uint32_t t = i >> 5, at = (i & 31) * 4;
+            const float *row = p.qkv + (size_t)(t0 + t) * p.channels + kh * 128 + at;
+            if (t < n) {
+                copy16(&qs[b][t][at], row);
+                copy16(&ks[b][t][at], row + p.key_width);
+            } else {  // the last group's missing tokens: their factors are 0
+                *reinterpret_cast<float4 *>(&qs[b][t][at]) = make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4 *>(&ks[b][t][at]) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
-        for (uint32_t i = tid; i < n * 4; i += 128)
-            copy16(&vs[b][i >> 2][(i & 3) * 4],
-                   p.qkv + (size_t)(t0 + (i >> 2)) * p.channels + 2 * p.key_width + head * 128 + col0 + (i & 3) * 4);
-        if (tid < n) {
-            copy4(&ds[b][tid], p.decay + (size_t)(t0 + tid) * p.heads + head);
-            copy4(&bs[b][tid], p.beta + (size_t)(t0 + tid) * p.heads + head);
+        for (uint32_t i = tid; i < groups * kGroup * (kScanCols / 4); i += kScanThreads) {
+            const uint32_t t = i / (kScanCols / 4), at = i % (kScanCols / 4) * 4;
+            if (t < n)
+                copy16(&vs[b][t][at], p.qkv + (size_t)(t0 + t) * p.channels + 2 * p.key_width + head * 128 + col0 + at);
+            else
+                *reinterpret_cast<float4 *>(&vs[b][t][at]) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        for (uint32_t i = tid; i < groups * (kCoefs / 4); i += kScanThreads)
+            copy16(&cs[b][i / (kCoefs / 4)][i % (kCoefs / 4) * 4],
+                   p.coefs + ((size_t)(t0 / kGroup + i / (kCoefs / 4)) * p.heads + head) * kCoefs + i % (kCoefs / 4) * 4);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     fetch(0, 0);
@@ -400,60 +511,72 @@ __global__ void __launch_bounds__(128) k_long_delta(const LongScan p) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        ulonglong2 k[4];
-        load(k, ks[b][0]);
-        float decay = ds[b][0], beta = bs[b][0], v = vs[b][0][c], o = 0.f;
-        for (uint32_t t = 0; t < n; ++t) {
-            ulonglong2 kn[4], q[4];
-            load(q, qs[b][t]);
-            load(kn, ks[b][t + 1 < n ? t + 1 : t]);
-            const uint32_t tn = t + 1 < n ? t + 1 : t;
-            const float decay_n = ds[b][tn], beta_n = bs[b][tn], v_n = vs[b][tn][c];
-            const f32x2 d2 = pack2(decay, decay);
-            f32x2 mem[4] = {0, 0, 0, 0}, out[4] = {0, 0, 0, 0};
+        for (uint32_t g = 0; g < (n + kGroup - 1) / kGroup; ++g) {
+            const uint32_t t = g * kGroup;
+            const float *co = cs[b][g];
+            const float D = co[tok], D3 = co[kGroup - 1], v = vs[b][t + tok][c + b8];
+            const float4 F = *reinterpret_cast<const float4 *>(co + kGroup + (b4 ? kGroup * kGroup : 0) + tok * kGroup);
+            f32x2 k[kGroup][4];
+            float x[2][2 * kGroup];
+#pragma unroll
+            for (uint32_t j = 0; j < kGroup; ++j) {
+                load(k[j], ks[b][t + j]);
+                x[0][j] = dot(s[0], k[j]);
+                x[1][j] = dot(s[1], k[j]);
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < kGroup; ++j) {
+                f32x2 q[4];
+                load(q, qs[b][t + j]);
+                x[0][kGroup + j] = dot(s[0], q);
+                x[1][kGroup + j] = dot(s[1], q);
+            }
+            float r[8], y[4], z[2];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[i] = (b8 ? x[1][i] : x[0][i]) + __shfl_xor_sync(0xffffffffu, b8 ? x[0][i] : x[1][i], 8);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[i] = (b4 ? r[4 + i] : r[i]) + __shfl_xor_sync(0xffffffffu, b4 ? r[i] : r[4 + i], 4);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) z[i] = (b2 ? y[2 + i] : y[i]) + __shfl_xor_sync(0xffffffffu, b2 ? y[i] : y[2 + i], 2);
+            const float w = (b1 ? z[1] : z[0]) + __shfl_xor_sync(0xffffffffu, b1 ? z[0] : z[1], 1);
+            const f32x2 d2 = pack2(D3, D3);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                s[2 * i] = mul2(s[2 * i], d2);
-                s[2 * i + 1] = mul2(s[2 * i + 1], d2);
-                mem[i & 1] = fma2(s[2 * i], k[i].x, mem[i & 1]);
-                mem[2 + (i & 1)] = fma2(s[2 * i + 1], k[i].y, mem[2 + (i & 1)]);
+                s[0][i] = mul2(s[0][i], d2);
+                s[1][i] = mul2(s[1][i], d2);
             }
-            float r = total4(mem);
-            // the sum over the lanes, side by side with that of the output of the token before
+            const float u = v - D * w;  // of a key's lane
+            float us[kGroup];
 #pragma unroll
-            for (int d = 1; d < 8; d <<= 1) {
-                const float r1 = __shfl_xor_sync(0xffffffffu, r, d), o1 = __shfl_xor_sync(0xffffffffu, o, d);
-                r += r1;
-                o += o1;
-            }
-            if (sub == 0 && t > 0) os[t - 1][c] = o;
-            const float delta = (v - r) * beta;
-            const f32x2 dl2 = pack2(delta, delta);
+            for (uint32_t i = 0; i < kGroup; ++i) us[i] = __shfl_sync(0xffffffffu, u, of_column + i);
+            float e = F.x * us[0];  // no term of a later token, whatever its value
+            if (b1 || b2) e += F.y * us[1];
+            if (b2) e += F.z * us[2];
+            if (b2 && b1) e += F.w * us[3];
+            if (b4) os[t + tok][c + b8] = D * w + e;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                s[2 * i] = fma2(k[i].x, dl2, s[2 * i]);
-                s[2 * i + 1] = fma2(k[i].y, dl2, s[2 * i + 1]);
-                out[i & 1] = fma2(s[2 * i], q[i].x, out[i & 1]);
-                out[2 + (i & 1)] = fma2(s[2 * i + 1], q[i].y, out[2 + (i & 1)]);
-                k[i] = kn[i];
+            for (uint32_t j = 0; j < kGroup; ++j) {
+                const float f0 = __shfl_sync(0xffffffffu, e, (lane & 16) + j), f1 = __shfl_sync(0xffffffffu, e, (lane & 16) + 8 + j);
+                const f32x2 e0 = pack2(f0, f0), e1 = pack2(f1, f1);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    s[0][i] = fma2(k[j][i], e0, s[0][i]);
+                    s[1][i] = fma2(k[j][i], e1, s[1][i]);
+                }
             }
-            o = total4(out);
-            decay = decay_n;
-            beta = beta_n;
-            v = v_n;
         }
-#pragma unroll
-        for (int d = 1; d < 8; d <<= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
-        if (sub == 0) os[n - 1][c] = o;
         __syncthreads();  // outputs complete, and buffer b free for the fetch of the next round
-        for (uint32_t i = tid; i < n * kScanCols; i += 128)
+        for (uint32_t i = tid; i < n * kScanCols; i += kScanThreads)
             p.out[((size_t)(t0 + i / kScanCols) * p.heads + head) * 128 + col0 + i % kScanCols] = os[i / kScanCols][i % kScanCols];
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        float *at = state + (size_t)((i >> 1) * 32 + sub * 4 + (i & 1) * 2) * 128;
-        unpack2(s[i], at[0], at[128]);
+    for (int i = 0; i < 4; ++i) {
+        float2 a, b;
+        unpack2(s[0][i], a.x, b.x);
+        unpack2(s[1][i], a.y, b.y);
+        state_at(i)[0] = a;
+        state_at(i)[64] = b;
     }
 }
 
@@ -685,8 +808,10 @@ ctox_status mixer(ctox_exec *e, uint32_t l, const LongOut &o, uint32_t m, uint64
                               LongGates{o, lw.a_log, lw.dt_bias, L.g, L.beta, ls.conv_state, heads, e->channels + e->value_width,
                                         e->channels, kernel, m}));
     timing_begin(ctx);
-    CTOX_CUDA(ctx, launch_pdl(k_long_delta, dim3(heads * 8), dim3(128), 0, ctx->stream,
-                              LongScan{L.qkv, L.g, L.beta, ls.delta[ls.cur], L.core, e->key_width, e->channels, heads,
+    CTOX_CUDA(ctx, launch_pdl(k_long_coefs, dim3(((m + kGroup - 1) / kGroup * c.linear_num_key_heads + 3) / 4), dim3(128), 0, ctx->stream,
+                              LongCoefs{L.qkv, L.g, L.beta, L.coefs, e->key_width, e->channels, heads, c.linear_num_key_heads, m}));
+    CTOX_CUDA(ctx, launch_pdl(k_long_delta, dim3(heads * kScanCtas), dim3(kScanThreads), 0, ctx->stream,
+                              LongScan{L.qkv, L.coefs, ls.delta[ls.cur], L.core, e->key_width, e->channels, heads,
                                        c.linear_num_key_heads, m}));
     timing_end(ctx, KC_LINEAR_ATTENTION, 2.0 * 4.0 * 128 * 128 * heads, 8.0 * 128 * 128 * heads * m);
     a.a = L.core;
@@ -751,6 +876,7 @@ ctox_status long_warmup(ctox_exec *e) {
     if (!rc) rc = get(&L->core, (size_t)cap * e->value_width);
     if (!rc) rc = get(&L->g, (size_t)cap * c.linear_num_value_heads);
     if (!rc) rc = get(&L->beta, (size_t)cap * c.linear_num_value_heads);
+    if (!rc) rc = get(&L->coefs, (size_t)(cap + kGroup - 1) / kGroup * c.linear_num_value_heads * kCoefs);
     if (!rc) rc = get(&L->aq, (size_t)cap * e->q_width);
     if (!rc) rc = get(&L->attn, (size_t)cap * c.num_attention_heads * (c.head_dim + 2));
     if (!rc) rc = get(&L->tokens, cap);

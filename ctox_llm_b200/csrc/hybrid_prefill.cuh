@@ -17,6 +17,7 @@ struct LongPass {
     float *h = nullptr, *final_hidden = nullptr;         // [cap][hidden]
     float *qkv = nullptr, *core = nullptr;               // [cap][channels], [cap][value width]
     float *g = nullptr, *beta = nullptr;                 // [cap][value heads]
+    float *coefs = nullptr;                              // [groups of four][value heads][factors of the scan]
     float *aq = nullptr, *attn = nullptr;                // [cap][query width], [cap][query heads][head_dim + 2] (all splits)
     uint32_t *tokens = nullptr;
 };
