@@ -64,7 +64,8 @@ __device__ __forceinline__ size_t attn_row(uint32_t pos, uint32_t head, uint32_t
 // Forms the next product's input row in shared memory and writes it as hi and lo parts. Bound by memory: a
 // projection's fp32 outputs are read once, four bytes per input column are written.
 enum : int { ROWS_NORM, ROWS_SWIGLU, ROWS_ATTENTION, ROWS_DELTA, ROWS_MTP };
-constexpr int kRowsThreads = 512;
+// 999 positions at a width of 5120, 512 and 256 threads: SWIGLU 53 and 59 us, NORM 36 and 30, DELTA 27 and 21, ATTENTION 31 and 23.
+__host__ __device__ constexpr int rows_threads(int mode) { return mode == ROWS_SWIGLU ? 512 : 256; }
 
 struct RowsArgs {
     LongOut o;              // NORM: addend (o.y null: none); SWIGLU: [gate | up]; ATTENTION, DELTA: where the gates are
@@ -82,115 +83,168 @@ struct RowsArgs {
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
+__global__ void __launch_bounds__(rows_threads(MODE)) k_long_rows(const RowsArgs p) {
+    constexpr uint32_t kRowsThreads = rows_threads(MODE);
     pdl_launch();
     pdl_wait();
-    extern __shared__ __align__(16) float vals[];  // [blocks_padded * 64], then the largest value of each block
+    extern __shared__ __align__(16) float vals[];  // two float4 of each unit, then the largest value of each block
     __shared__ float red[kRowsThreads / 32];
-    const uint32_t pos = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t columns = MODE == ROWS_MTP ? 2 * p.width : p.width;
+    const uint32_t pos = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const uint32_t columns = MODE == ROWS_MTP ? 2 * p.width : p.width, units = p.has_next ? p.blocks_padded * 8 : p.width / 8;
+    // A unit is what one 16-byte chunk of a part holds (inv_perm): columns c .. c + 3 and, 4 (4-bit codes) or 8 further, four more. Its
+    // thread keeps it throughout: in two places of its own in shared memory, one after the other over the lanes. Eight lanes
+    // hold a block; all lanes of a warp have a unit or none has (blocks_padded is a multiple of four).
+    const uint32_t step = p.dt ? 4 : 8;
+    auto column = [&](uint32_t unit) { return (unit >> 1) * 16 + (unit & 1) * (12 - step); };
+    float4 *first = reinterpret_cast<float4 *>(vals), *second = first + units;
+    float *block_max = vals + units * 8;
+    auto at4 = [](const float *q) { return *reinterpret_cast<const float4 *>(q); };
     float amax = 0.f;
-    auto put = [&](uint32_t c, float x) {
-        const float v = p.s_in ? x * p.s_in[c] : x;
-        vals[c] = v;
-        amax = fmaxf(amax, fabsf(v));
-    };
-    // widths are multiples of 64: NORM and SWIGLU take four columns per thread and trip
-    auto put4 = [&](uint32_t c, float4 x) {
-        if (p.s_in) {
-            const float4 w = *reinterpret_cast<const float4 *>(p.s_in + c);
-            x = make_float4(x.x * w.x, x.y * w.y, x.z * w.z, x.w * w.w);
+    auto put = [&](uint32_t unit, uint32_t c, float4 a, float4 b) {
+        if (p.s_in && c < columns) {
+            const float4 x = at4(p.s_in + c), y = at4(p.s_in + c + step);
+            a = make_float4(a.x * x.x, a.y * x.y, a.z * x.z, a.w * x.w);
+            b = make_float4(b.x * y.x, b.y * y.y, b.z * y.z, b.w * y.w);
         }
-        *reinterpret_cast<float4 *>(vals + c) = x;
-        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+        first[unit] = a;
+        second[unit] = b;
+        float mx = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
+                         fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+        if ((lane & 7) == 0) block_max[unit >> 3] = mx;
+        amax = fmaxf(amax, mx);
     };
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto sq4 = [](float4 v) { return (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); };
     if constexpr (MODE == ROWS_NORM) {
         float *h = p.h + (size_t)pos * p.width;
+        const float *base = p.a ? p.a + (size_t)pos * p.width : nullptr;
         float sq = 0.f;
-        for (uint32_t c = tid * 4; c < p.width; c += kRowsThreads * 4) {
-            float4 v = p.a ? *reinterpret_cast<const float4 *>(p.a + (size_t)pos * p.width + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (p.o.y) {
-                const float4 y = lp_out4(p.o, c, pos);
-                v = make_float4(v.x + y.x, v.y + y.y, v.z + y.z, v.w + y.w);
-            }
-            *reinterpret_cast<float4 *>(h + c) = v;
-            *reinterpret_cast<float4 *>(vals + c) = v;
-            sq += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+        for (uint32_t unit = tid; unit < units; unit += kRowsThreads) {
+            const uint32_t c = column(unit);
+            float4 v[2] = {zero, zero};
+            if (c < p.width)
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
+                    if (base) v[i] = at4(base + c + i * step);
+                    if (p.o.y) {
+                        const float4 y = lp_out4(p.o, c + i * step, pos);
+                        v[i] = make_float4(v[i].x + y.x, v[i].y + y.y, v[i].z + y.z, v[i].w + y.w);
+                    }
+                    *reinterpret_cast<float4 *>(h + c + i * step) = v[i];
+                }
+            first[unit] = v[0];
+            second[unit] = v[1];
+            sq += sq4(v[0]) + sq4(v[1]);
         }
         const float inv = 1.0f / sqrtf(lp_block<0>(sq, red) / (float)p.width + p.eps);
-        for (uint32_t c = tid * 4; c < p.width; c += kRowsThreads * 4) {  // each thread its own columns again
-            const float4 v = *reinterpret_cast<const float4 *>(vals + c), w = *reinterpret_cast<const float4 *>(p.w + c);
-            const float4 xn = make_float4(v.x * inv * (1.0f + w.x), v.y * inv * (1.0f + w.y), v.z * inv * (1.0f + w.z),
-                                          v.w * inv * (1.0f + w.w));
-            if (p.xn_out) *reinterpret_cast<float4 *>(p.xn_out + (size_t)pos * p.width + c) = xn;
-            if (p.has_next) put4(c, xn);
+        for (uint32_t unit = tid; unit < units; unit += kRowsThreads) {  // each thread its own units again
+            const uint32_t c = column(unit);
+            float4 v[2] = {first[unit], second[unit]};
+            if (c < p.width)
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
+                    const float4 w = at4(p.w + c + i * step);
+                    v[i] = make_float4(v[i].x * inv * (1.0f + w.x), v[i].y * inv * (1.0f + w.y), v[i].z * inv * (1.0f + w.z),
+                                       v[i].w * inv * (1.0f + w.w));
+                    if (p.xn_out) *reinterpret_cast<float4 *>(p.xn_out + (size_t)pos * p.width + c + i * step) = v[i];
+                }
+            if (p.has_next) put(unit, c, v[0], v[1]);
         }
         if (!p.has_next) return;
     } else if constexpr (MODE == ROWS_MTP) {
         const float *e = p.a + (size_t)pos * p.width, *h = p.b + (size_t)pos * p.width;
         float se = 0.f, sh = 0.f;
-        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
-            se += e[c] * e[c];
-            sh += h[c] * h[c];
+        for (uint32_t c = tid * 4; c < p.width; c += kRowsThreads * 4) {
+            se += sq4(at4(e + c));
+            sh += sq4(at4(h + c));
         }
         const float ie = 1.0f / sqrtf(lp_block<0>(se, red) / (float)p.width + p.eps);
         const float ih = 1.0f / sqrtf(lp_block<0>(sh, red) / (float)p.width + p.eps);
-        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
-            put(c, e[c] * ie * (1.0f + p.w[c]));
-            put(p.width + c, h[c] * ih * (1.0f + p.w2[c]));
+        for (uint32_t unit = tid; unit < units; unit += kRowsThreads) {
+            const uint32_t c = column(unit);
+            const bool hidden = c >= p.width;
+            const uint32_t cc = hidden ? c - p.width : c;
+            const float inv = hidden ? ih : ie;
+            float4 v[2] = {zero, zero};
+            if (c < columns)
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
+                    const float4 x = at4((hidden ? h : e) + cc + i * step), w = at4((hidden ? p.w2 : p.w) + cc + i * step);
+                    v[i] = make_float4(x.x * inv * (1.0f + w.x), x.y * inv * (1.0f + w.y), x.z * inv * (1.0f + w.z),
+                                       x.w * inv * (1.0f + w.w));
+                }
+            put(unit, c, v[0], v[1]);
         }
     } else if constexpr (MODE == ROWS_SWIGLU) {
-#pragma unroll 2
-        for (uint32_t c = tid * 4; c < p.width; c += kRowsThreads * 4) {
-            const float4 g = lp_out4(p.o, c, pos), u = lp_out4(p.o, p.width + c, pos);
-            put4(c, make_float4(silu_f(g.x) * u.x, silu_f(g.y) * u.y, silu_f(g.z) * u.z, silu_f(g.w) * u.w));
+        for (uint32_t unit = tid; unit < units; unit += kRowsThreads) {
+            const uint32_t c = column(unit);
+            float4 v[2] = {zero, zero};
+            if (c < p.width) {
+                const float4 g[2] = {lp_out4(p.o, c, pos), lp_out4(p.o, c + step, pos)};
+                const float4 u[2] = {lp_out4(p.o, p.width + c, pos), lp_out4(p.o, p.width + c + step, pos)};
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i)
+                    v[i] = make_float4(silu_f(g[i].x) * u[i].x, silu_f(g[i].y) * u[i].y, silu_f(g[i].z) * u[i].z, silu_f(g[i].w) * u[i].w);
+            }
+            put(unit, c, v[0], v[1]);
         }
     } else if constexpr (MODE == ROWS_ATTENTION) {
         // attention left (unnormalised output, maximum, sum) of each query; of several splits the first holds the merged one
         const uint32_t hd = p.head_dim;
-        for (uint32_t c = tid; c < p.width; c += kRowsThreads) {
-            const uint32_t hq = c / hd, d = c % hd;
-            const float *r = p.a + attn_row(pos, hq, 0, p.m, p.per_group, p.splits, p.q_heads, p.kv_heads) * (hd + 2);
-            const float gate = lp_out(p.o, hq * 2 * hd + hd + d, pos);
-            put(c, r[d] * (1.0f / r[hd + 1]) * (1.0f / (1.0f + expf(-gate))));
+        for (uint32_t unit = tid; unit < units; unit += kRowsThreads) {
+            const uint32_t c = column(unit);
+            float4 v[2] = {zero, zero};
+            if (c < p.width) {
+                const uint32_t hq = c / hd, d = c % hd;
+                const float *r = p.a + attn_row(pos, hq, 0, p.m, p.per_group, p.splits, p.q_heads, p.kv_heads) * (hd + 2);
+                const float inv = 1.0f / r[hd + 1];
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {  // rows of hd + 2 floats are aligned for two of them
+                    const float2 x = *reinterpret_cast<const float2 *>(r + d + i * step), y = *reinterpret_cast<const float2 *>(r + d + i * step + 2);
+                    const float4 g = lp_out4(p.o, hq * 2 * hd + hd + d + i * step, pos);
+                    v[i] = make_float4(x.x * inv * (1.0f / (1.0f + expf(-g.x))), x.y * inv * (1.0f / (1.0f + expf(-g.y))),
+                                       y.x * inv * (1.0f / (1.0f + expf(-g.z))), y.y * inv * (1.0f / (1.0f + expf(-g.w))));
+                }
+            }
+            put(unit, c, v[0], v[1]);
         }
     } else {
-        // rms_norm_gated per value head (reference.rs:66-93): a warp per head, four columns per lane
-        for (uint32_t head = warp; head < p.width / 128; head += kRowsThreads / 32) {
-            const uint32_t c0 = head * 128 + lane * 4;
-            const float4 v = *reinterpret_cast<const float4 *>(p.a + (size_t)pos * p.width + c0);
-            float sq = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        // rms_norm_gated per value head (reference.rs:66-93): sixteen lanes per head
+        for (uint32_t unit = tid; unit < units; unit += kRowsThreads) {
+            const uint32_t c = column(unit);
+            float4 v[2] = {zero, zero}, g[2] = {zero, zero};
+            if (c < p.width)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+                for (uint32_t i = 0; i < 2; ++i) {
+                    v[i] = at4(p.a + (size_t)pos * p.width + c + i * step);
+                    g[i] = lp_out4(p.o, p.off + c + i * step, pos);
+                }
+            float sq = sq4(v[0]) + sq4(v[1]);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
             const float inv = 1.0f / sqrtf(sq / 128.0f + p.eps);
-            const float x[4] = {v.x, v.y, v.z, v.w};
+            if (c < p.width)
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j)
-                put(c0 + j, x[j] * inv * p.w[lane * 4 + j] * silu_f(lp_out(p.o, p.off + c0 + j, pos)));
+                for (uint32_t i = 0; i < 2; ++i) {
+                    const float4 w = at4(p.w + c % 128 + i * step);
+                    v[i] = make_float4(v[i].x * inv * w.x * silu_f(g[i].x), v[i].y * inv * w.y * silu_f(g[i].y),
+                                       v[i].z * inv * w.z * silu_f(g[i].z), v[i].w * inv * w.w * silu_f(g[i].w));
+                }
+            put(unit, c, v[0], v[1]);
         }
     }
-    for (uint32_t c = columns + tid; c < p.blocks_padded * 64; c += kRowsThreads) vals[c] = 0.f;
-    amax = lp_block<1>(amax, red);  // its barriers also publish vals
-    // One unit per position: the largest value lies in [2^14, 2^15). hi + lo then keep 22 bits of every value above
+    amax = lp_block<1>(amax, red);  // its barriers also publish the blocks' largest values
+    // One unit of value per position: the largest value lies in [2^14, 2^15). hi + lo then keep 22 bits of every value above
     // 2^-28 of the largest, and an absolute 2^-50 of it below. A streaming product has a unit for each block and keeps 22
     // bits above 2^-13 (4-bit codes) or 2^-9 of the block's largest value, 2^-35 or 2^-31 of it below: the row's unit leaves
     // no block fewer unless its largest value is below 2^-15 of the row's. Then every block gets its own unit.
-    float *block_max = vals + p.blocks_padded * 64;
     auto exponent = [](float x) { return (int)((__float_as_uint(x) >> 23) & 0xff) - 127; };
     int spread = 0;
-    for (uint32_t i = tid; i < p.blocks_padded * 4; i += kRowsThreads) {  // four neighbouring lanes: a block
-        float mx = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 x = *reinterpret_cast<const float4 *>(vals + i * 16 + j * 4);
-            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
-        }
-        const uint32_t lanes = 0xfu << (lane & 28);
-        mx = fmaxf(mx, __shfl_xor_sync(lanes, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(lanes, mx, 2));
-        if ((i & 3) == 0) block_max[i >> 2] = mx;
-        if (mx > 0.f && exponent(mx) < exponent(amax) - 15) spread = 1;
-    }
+    for (uint32_t i = tid; i < p.blocks_padded; i += kRowsThreads)
+        if (block_max[i] > 0.f && exponent(block_max[i]) < exponent(amax) - 15) spread = 1;
     spread = __syncthreads_or(spread);
     auto unit_exponent = [&](float largest) {
         const int e = exponent(largest);
@@ -200,36 +254,22 @@ __global__ void __launch_bounds__(kRowsThreads) k_long_rows(const RowsArgs p) {
         p.in.unit[pos] = __uint_as_float((uint32_t)(unit_exponent(amax) - 14 + 127) << 23);
         p.in.spread[pos] = spread ? 0xff : 0;
     }
-    for (uint32_t i = tid; i < p.blocks_padded * 4; i += kRowsThreads) {  // sixteen columns: two chunks of each part
-        const uint32_t block = i >> 2, t = i & 3;
+    for (uint32_t unit = tid; unit < units; unit += kRowsThreads) {
+        const uint32_t block = unit >> 3;
         const int e = unit_exponent(spread ? block_max[block] : amax);
         const float f = __uint_as_float((uint32_t)(14 - e + 127) << 23);
-        if (t == 0) p.in.block_unit[(size_t)block * p.in.pos_pad + pos] = __uint_as_float((uint32_t)(e - 14 + 127) << 23);
-        float v[16];
+        if ((unit & 7) == 0) p.in.block_unit[(size_t)block * p.in.pos_pad + pos] = __uint_as_float((uint32_t)(e - 14 + 127) << 23);
+        const float4 a = first[unit], b = second[unit];
+        const float x[4] = {a.x * f, a.y * f, a.z * f, a.w * f}, y[4] = {b.x * f, b.y * f, b.z * f, b.w * f};
+        __align__(16) __half2 hi[4], lo[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 x = *reinterpret_cast<const float4 *>(vals + i * 16 + j * 4);
-            v[4 * j] = x.x * f;
-            v[4 * j + 1] = x.y * f;
-            v[4 * j + 2] = x.z * f;
-            v[4 * j + 3] = x.w * f;
+        for (int s = 0; s < 4; ++s) {
+            hi[s] = __floats2half2_rn(x[s], y[s]);
+            lo[s] = __floats2half2_rn((x[s] - __low2float(hi[s])) * (float)(1 << kLoShift), (y[s] - __high2float(hi[s])) * (float)(1 << kLoShift));
         }
-        __half2 hi[8], lo[8];
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {  // slots 2 s, 2 s + 1 (inv_perm)
-            const float q4a = v[(s >> 2) * 8 + (s & 3)], q4b = v[(s >> 2) * 8 + (s & 3) + 4];
-            const float x = p.dt ? q4a : v[s], y = p.dt ? q4b : v[s + 8];
-            hi[s] = __floats2half2_rn(x, y);
-            lo[s] = __floats2half2_rn((x - __low2float(hi[s])) * (float)(1 << kLoShift),
-                                      (y - __high2float(hi[s])) * (float)(1 << kLoShift));
-        }
-        uint8_t *d = p.in.x + ((size_t)block * 2 * p.in.pos_pad + pos) * 128;
-        const uint32_t c0 = ((2 * t) ^ (pos & 7)) * 16, c1 = ((2 * t + 1) ^ (pos & 7)) * 16;
-        const size_t part = (size_t)p.in.pos_pad * 128;
-        *reinterpret_cast<uint4 *>(d + c0) = *reinterpret_cast<uint4 *>(hi);
-        *reinterpret_cast<uint4 *>(d + c1) = *reinterpret_cast<uint4 *>(hi + 4);
-        *reinterpret_cast<uint4 *>(d + part + c0) = *reinterpret_cast<uint4 *>(lo);
-        *reinterpret_cast<uint4 *>(d + part + c1) = *reinterpret_cast<uint4 *>(lo + 4);
+        uint8_t *d = p.in.x + ((size_t)block * 2 * p.in.pos_pad + pos) * 128 + ((unit & 7) ^ (pos & 7)) * 16;
+        *reinterpret_cast<uint4 *>(d) = *reinterpret_cast<uint4 *>(hi);
+        *reinterpret_cast<uint4 *>(d + (size_t)p.in.pos_pad * 128) = *reinterpret_cast<uint4 *>(lo);
     }
 }
 
@@ -732,7 +772,7 @@ ctox_status rows(ctox_exec *e, RowsArgs &a, uint32_t m, ctox_matvec *next) {
         a.dt = next->parts[0].dt;
     }
     const size_t smem = (next ? (size_t)next->blocks_padded * 65 : a.width) * 4;
-    CTOX_CUDA(ctx, launch_pdl(k_long_rows<MODE>, dim3(m), dim3(kRowsThreads), smem, ctx->stream, a));
+    CTOX_CUDA(ctx, launch_pdl(k_long_rows<MODE>, dim3(m), dim3(rows_threads(MODE)), smem, ctx->stream, a));
     return CTOX_OK;
 }
 
