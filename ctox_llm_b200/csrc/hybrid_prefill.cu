@@ -61,10 +61,11 @@ __device__ __forceinline__ size_t attn_row(uint32_t pos, uint32_t head, uint32_t
 }
 
 // ------------------------------------------------------------------ rows: one CTA per position
-// Forms the next product's input row in shared memory and writes it as hi and lo parts. Bound by memory: a
-// projection's fp32 outputs are read once, four bytes per input column are written.
+// Forms the next product's input row and writes it as hi and lo parts. Bound by memory: a projection's fp32 outputs are read
+// once, four bytes per input column are written.
 enum : int { ROWS_NORM, ROWS_SWIGLU, ROWS_ATTENTION, ROWS_DELTA, ROWS_MTP };
-// 999 positions at a width of 5120, 512 and 256 threads: SWIGLU 53 and 59 us, NORM 36 and 30, DELTA 27 and 21, ATTENTION 31 and 23.
+// More threads have more of a long row's loads in flight, fewer leave room for more rows per SM. 999 positions at a width of 5120, 512
+// and 256 threads: SWIGLU 53 and 59 us, NORM 36 and 30, DELTA 27 and 21, ATTENTION 31 and 23.
 __host__ __device__ constexpr int rows_threads(int mode) { return mode == ROWS_SWIGLU ? 512 : 256; }
 
 struct RowsArgs {

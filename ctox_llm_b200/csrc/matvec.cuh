@@ -96,9 +96,9 @@ ctox_status head_accept_enqueue(ctox_ctx *ctx, uint32_t n_nodes, const int32_t *
                                 int force_accept, ctox_spec_record **record_dev);
 // Greedy token of a logit vector; token = row_ids[row] or row + row_offset. In a tensor-parallel
 // group every rank passes its shard and all ranks receive the group's token.
+ctox_status argmax_enqueue(ctox_ctx *ctx, const float *logits_dev, uint32_t n, const uint32_t *row_ids_dev,
+                           uint32_t row_offset, uint32_t *token_dev, uint32_t *status_dev);
 // The same over the outputs of a streamed pass of one position (identity activation), which go to logits_out.
 ctox_status argmax_matvec_enqueue(ctox_matvec *mv, float *logits_out, const uint32_t *row_ids_dev, uint32_t row_offset,
                                   uint32_t *token_dev, uint32_t *status_dev);
-ctox_status argmax_enqueue(ctox_ctx *ctx, const float *logits_dev, uint32_t n, const uint32_t *row_ids_dev,
-                           uint32_t row_offset, uint32_t *token_dev, uint32_t *status_dev);
 }  // namespace ctox
