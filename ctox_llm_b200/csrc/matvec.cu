@@ -1200,6 +1200,11 @@ ctox_status stream_part(ctox_matvec *mv, const MatvecPart &p, const MatvecPart::
     return CTOX_OK;
 }
 
+bool overlap(const void *a, uint64_t na, size_t size_a, const void *b, uint64_t nb, size_t size_b) {
+    const uintptr_t pa = (uintptr_t)a, pb = (uintptr_t)b;
+    return pa < pb + nb * size_b && pb < pa + na * size_a;
+}
+
 // Positions m0 .. m0 + npos of a dispatch over one or several matrices of one input.
 ctox_status dispatch_pass(ctox_ctx *ctx, const DispatchItem *it, uint64_t n, const void *x, uint32_t x_dtype, uint64_t x_stride,
                           uint32_t npos) {
@@ -1222,7 +1227,11 @@ ctox_status dispatch_pass(ctox_ctx *ctx, const DispatchItem *it, uint64_t n, con
         FinishArgs f{};
         const MatvecPart &p0 = *it[i0].part;
         const bool own = p0.kst_s * 4 * npos <= kOwnGroups;
-        const bool closed = own && plan_closed(ctx, it + i0, k, npos, &a), merged = closed || ((own || k > 1) && plan_merged(ctx, it + i0, k, npos, &a));
+        // Outputs may lie over the activations (a layer in place): a closed launch would write them while other CTAs still read.
+        bool apart = true;
+        for (uint32_t i = 0; i < k; ++i)
+            apart = apart && !overlap(x, (npos - 1) * x_stride + first->columns, esz, it[i0 + i].y, (npos - 1) * it[i0 + i].y_stride + it[i0 + i].part->rows, 4);
+        const bool closed = own && apart && plan_closed(ctx, it + i0, k, npos, &a), merged = closed || ((own || k > 1) && plan_merged(ctx, it + i0, k, npos, &a));
         auto split_of = [&](const MatvecPart &p) -> const MatvecPart::Split & {
             return p.split[npos > 4 ? 1 : !merged && p.split[kAloneSplit].warps ? kAloneSplit : 0];
         };

@@ -43,3 +43,56 @@ def test_outputs(orc, dtype, rows, columns, positions):
         m.destroy()
     assert be.allocated_bytes() == 0
     be.close()
+
+
+@pytest.mark.parametrize("rows,columns,positions,shift", [
+    ([1024], 1024, 1, 0), ([1024], 1024, 2, 0), ([256], 256, 8, 0), ([700], 512, 1, -300), ([40], 2048, 1, 2000), ([4096], 4096, 1, 0),
+    ([18945], 1024, 1, -9000), ([512, 256, 100], 512, 2, 100)])
+def test_outputs_over_the_activations(orc, rows, columns, positions, shift):
+    """The first matrix writes where the activations lie (from `shift` values behind their start): launches whose CTAs read all of them
+    and write outputs keep away from such calls, and only from those."""
+    import torch
+    be = ctox.B200Backend(0)
+    s_in = synthetic.recovery_scales_f16(columns, 5, 1)
+    ops = [ctox.FusedMatVec(Q4, synthetic.packed_weights(Q4, n, columns, i), n, columns, None, s_in=s_in,
+                            s_out=synthetic.recovery_scales_f16(n, i, 2)) for i, n in enumerate(rows)]
+    mats = [be.prepare_fused_matvec(op) for op in ops]
+    x = synthetic.activations(columns, 3, positions=positions).reshape(positions, columns)
+    stride = max(columns, rows[0])
+    memory = torch.empty(positions * stride + 2 * abs(shift), device="cuda")
+    x_at = abs(shift)
+    others = [torch.empty(positions, n, device="cuda") for n in rows[1:]]
+    apart = torch.empty(positions, stride, device="cuda")
+
+    def dispatch(y_ptr):
+        memory.zero_()
+        memory[x_at:x_at + positions * stride].view(positions, stride)[:, :columns] = torch.from_numpy(x).cuda()
+        torch.cuda.synchronize()
+        before = be.kernel_launches()
+        xp = memory.data_ptr() + 4 * x_at
+        if len(mats) == 1:
+            mats[0].dispatch_device(xp, ctox.F32, positions, stride, y_ptr, stride)
+        else:
+            be.fanout_dispatch_device(mats, xp, ctox.F32, positions, stride, [y_ptr] + [y.data_ptr() for y in others], [stride] + rows[1:])
+        be.synchronize()
+        return be.kernel_launches() - before
+
+    want = []
+    for op in ops:
+        o = to_oracle_op(orc, op)
+        want.append([])
+        for m in range(positions):
+            o.input = x[m]
+            want[-1].append(orc.fused_matvec(o))
+    closed = dispatch(apart.data_ptr()) == 1
+    assert closed == (columns <= 2048 and rows[0] < 18945)
+    over = x_at + shift
+    for _ in range(20):
+        assert dispatch(memory.data_ptr() + 4 * over) >= 2
+        got = [memory[over:over + positions * stride].view(positions, stride).cpu().numpy()] + [y.cpu().numpy() for y in others]
+        for w, n, y in zip(want, rows, got):
+            for m in range(positions):
+                assert rel_l2(y[m, :n], w[m]) <= 5e-5  # as above
+    for m in mats:
+        m.destroy()
+    be.close()
