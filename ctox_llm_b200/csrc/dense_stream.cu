@@ -169,10 +169,17 @@ __global__ void __launch_bounds__(kDsThreads, 1) k_dense_stream(const __grid_con
     const __nv_bfloat16 *src = a.w + (size_t)(r0 + first) * a.ld + (size_t)v0 * 8;
     const uint32_t my_bars = smem_addr(&bars[warp * kDsStages]), ring = smem_addr(smem) + warp * a.stages * a.stage_bytes;
     const uint32_t todo = len ? count : 0;
+    // A row is read once in a pass: its lines are the first to leave L2. With the default priority the weights push out what later
+    // kernels read again (cache rows, states, norm weights), which the loads of k_dense_matvec do not: a token's cache attention over 32-bit
+    // rows took 31 us instead of 23. A request of 134 + 31 tokens on a latent model (6 layers of width 2048, 32-bit cache) 26.4 -> 24.9 ms,
+    // 16 tokens of the eight-layer model of width 5120 16.1 -> 15.6.
+    uint64_t once;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
     auto request = [&](uint32_t row, uint32_t st) {  // one thread
         bar_expect(my_bars + 8 * st, len * 16);
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(ring + st * a.stage_bytes),
-                     "l"(src + (size_t)row * a.ld), "r"(len * 16), "r"(my_bars + 8 * st)
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+                         ring + st * a.stage_bytes),
+                     "l"(src + (size_t)row * a.ld), "r"(len * 16), "r"(my_bars + 8 * st), "l"(once)
                      : "memory");
     };
     // Half of the ring is asked for here; the rest once the input's loads are on their way, which would wait behind it.
