@@ -7,17 +7,16 @@ namespace ctox {
 
 namespace cg = cooperative_groups;
 constexpr int kMmThreads = 256, kMmWarps = kMmThreads / 32;
-// State rows a warp works on at once. A decode step is a chain of round trips: with nine rows a CTA of 65 (512 value dimensions over
-// eight CTAs, and the normaliser) takes one trip to its state instead of three.
-__host__ __device__ constexpr int mm_rows(int m) { return m == 1 ? 9 : 4; }
-
 // A cluster per head, its CTAs share the state's rows (value dimensions, the normaliser behind them). A row stays
 // in registers for all M positions: the gates' scales of every position are known before the state is touched.
 // The head's norm needs the outputs of all CTAs: they meet through distributed shared memory.
-template <int M>
+// ROWS: state rows a warp works on at once. A decode step is a chain of round trips: with nine rows a CTA of up to 72 (512 value dimensions
+// over eight CTAs and the normaliser: 65) takes one trip to its state. Up to 24 rows, three are as few trips and keep all warps at
+// work: 128 value dimensions 10.7 us a launch against 11.3 with nine and 10.7 with four (33 rows, 256 dimensions: 11.3 to 11.8 with nine,
+// 11.8 with five, 12.5 with four; 65 rows: 12.6 and, with four, 12.7).
+template <int M, int ROWS>
 __global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, const float *fan, uint32_t fan_stride,
                                                               uint32_t gate_off, uint32_t npos, uint32_t rows_per, float *__restrict__ out) {
-    constexpr int kMmRows = mm_rows(M);
     pdl_launch();
     extern __shared__ __align__(16) float sm[];
     __shared__ float keep[M], take[M], floor_s[M], part[kMmWarps][M];
@@ -81,20 +80,20 @@ __global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, co
     }
     __syncthreads();
     const float top_new = xch[0][0];
-    for (uint32_t r0 = warp * kMmRows; r0 < rows; r0 += kMmWarps * kMmRows) {
-        float acc[kMmRows][M];
-        float *sp[kMmRows];
+    for (uint32_t r0 = warp * ROWS; r0 < rows; r0 += kMmWarps * ROWS) {
+        float acc[ROWS][M];
+        float *sp[ROWS];
 #pragma unroll
-        for (int r = 0; r < kMmRows; ++r) {
+        for (int r = 0; r < ROWS; ++r) {
             sp[r] = state_row(row_beg + min(r0 + r, rows - 1));
 #pragma unroll
             for (int t = 0; t < M; ++t) acc[r][t] = 0.f;
         }
 #pragma unroll(M == 1 ? 2 : 1)
         for (uint32_t d = lane * 4; d < a.dim_pad; d += 128) {
-            float4 s[kMmRows];
+            float4 s[ROWS];
 #pragma unroll
-            for (int r = 0; r < kMmRows; ++r) s[r] = *reinterpret_cast<const float4 *>(sp[r] + d);
+            for (int r = 0; r < ROWS; ++r) s[r] = *reinterpret_cast<const float4 *>(sp[r] + d);
 #pragma unroll
             for (int t = 0; t < M; ++t) {
                 if (t >= (int)npos) break;
@@ -102,7 +101,7 @@ __global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, co
                 const float4 q = *reinterpret_cast<const float4 *>(q_s + t * a.dim_pad + d);
                 const float kp = keep[t], tk = take[t];
 #pragma unroll
-                for (int r = 0; r < kMmRows; ++r) {
+                for (int r = 0; r < ROWS; ++r) {
                     const float v = tk * v_s[t * rows_per + min(r0 + r, rows - 1)];
                     s[r].x = fmaf(kp, s[r].x, v * k.x);
                     s[r].y = fmaf(kp, s[r].y, v * k.y);
@@ -112,11 +111,11 @@ __global__ void __launch_bounds__(kMmThreads) k_matrix_memory(MatrixMemory a, co
                 }
             }
 #pragma unroll
-            for (int r = 0; r < kMmRows; ++r)
+            for (int r = 0; r < ROWS; ++r)
                 if (r0 + r < rows) *reinterpret_cast<float4 *>(sp[r] + d) = s[r];
         }
 #pragma unroll
-        for (int r = 0; r < kMmRows; ++r)
+        for (int r = 0; r < ROWS; ++r)
 #pragma unroll
             for (int t = 0; t < M; ++t) {
 #pragma unroll
@@ -182,9 +181,11 @@ ctox_status memory_launch(ctox_ctx *ctx, const MatrixMemory &a, const float *fan
     const size_t smem = (size_t)2 * M * (a.dim_pad + rows_per) * 4;
     if (smem + 2048 > (size_t)ctx->max_smem_optin)
         return fail(ctx, CTOX_MEMORY_BUDGET, "matrix memory: %u x %u per head does not fit shared memory", a.dim, a.vdim);
-    if (smem > 40 * 1024)
-        CTOX_CUDA(ctx, cudaFuncSetAttribute(k_matrix_memory<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CTOX_CUDA(ctx, launch_pdl_cluster(k_matrix_memory<M>, dim3(a.heads * ctas), dim3(kMmThreads), smem, ctx->stream, ctas, a, fan,
+    auto kernel = k_matrix_memory<M, M == 1 ? 9 : 4>;
+    if constexpr (M == 1)
+        if (rows_per <= 3 * kMmWarps) kernel = k_matrix_memory<1, 3>;
+    if (smem > 40 * 1024) CTOX_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CTOX_CUDA(ctx, launch_pdl_cluster(kernel, dim3(a.heads * ctas), dim3(kMmThreads), smem, ctx->stream, ctas, a, fan,
                                       fan_stride, gate_off, m, rows_per, out));
     return CTOX_OK;
 }
