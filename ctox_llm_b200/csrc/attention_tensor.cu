@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) k_attention_tensor(const __grid
                 const uint64_t token = (tile_beg + t) * kAtTile + tok;
                 const bool whole = (tile_beg + t + 1) * kAtTile <= slot0 + 1;  // every query sees all of the tile
 #pragma unroll
-                for (uint32_t i = 0; i < H; ++i) s[i] += lo[i];
+                for (uint32_t i = 0; i < H; ++i) s[i] = fmaxf(s[i] + lo[i], -INFINITY);  // NaN: no weight, as in k_attention_mma
                 if (!whole)
 #pragma unroll
                     for (uint32_t i = 0; i < H; ++i)

@@ -38,3 +38,28 @@ def test_short_passes_on_a_long_session(page_tokens, gain):
     finally:
         ex.unload()
         be.close()
+
+
+def test_a_key_that_is_nan_has_no_weight():
+    """Keys that overflow (norm weights of 3e38: the turn of two infinities is NaN) are passed over by short passes as by long ones; the
+    tokens ahead of the portion have other keys."""
+    be = ctox.B200Backend(0)
+    ex = ctox.B200Executor(be, ctox.qwen38_27b_config(
+        vocab_size=2048, hidden_size=1024, intermediate_size=1024, num_hidden_layers=2, full_attention_interval=2, num_attention_heads=24,
+        num_key_value_heads=4, head_dim=256, rotary_dim=64, linear_num_key_heads=4, linear_num_value_heads=8, max_context_tokens=11000,
+        max_draft_tokens=0, mtp_num_hidden_layers=0, draft_vocab=0, kv_dtype=ctox.BF16))
+    try:
+        ex.fill_synthetic(5)
+        ex.load_vector(1, N.T_K_NORM, np.full(256, 3e38, np.float32))
+        ex.warmup()
+        tokens = [int(t) for t in np.random.default_rng(1).integers(0, 2048, 20)]
+        runs = []
+        for step in (1, 4, 20):
+            ex.prefill_synthetic(9600, 3)
+            runs.append(np.concatenate([ex.extend(tokens[a:a + step], list(range(step))) for a in range(0, 20, step)]))
+        assert np.isfinite(runs[-1]).all()
+        for short in runs[:-1]:
+            assert max(rel_l2(a, b) for a, b in zip(short, runs[-1])) <= 1e-3  # as above
+    finally:
+        ex.unload()
+        be.close()
