@@ -402,9 +402,9 @@ __global__ void __launch_bounds__(512, 1) k_linear_attention(LinearAttnArgs a, i
     const uint32_t channels = 2 * a.key_width + a.value_width;
 
     // Before the dependency wait: what the pass itself does not write. The committed recurrent
-    // state and conv state were last written by the commit of the previous block, which a host
-    // copy separates from this pass; the weights never change. These loads overlap the tail of
-    // the input projection.
+    // state and conv state were last written by the commit of the previous block, and the launch that
+    // stores this pass's tokens (k_store_tokens) lets no later kernel start before that has finished;
+    // the weights never change. These loads overlap the tail of the input projection.
     const uint32_t slice = warp >> 2, rg = warp & 3, col = slice * kDeltaSlice + lane;
     float s[32];  // rows rg * 32 .. + 32 of column slice * 32 + lane
     {

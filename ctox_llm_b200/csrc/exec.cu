@@ -1082,9 +1082,11 @@ ctox_status mtp_pass(ctox_exec *e, uint32_t m, uint64_t abs_pos0, const uint32_t
 struct FewTokens {
     uint32_t v[kMaxPass + 1];
 };
+// Ahead of every short pass. No later kernel starts before all of the commit before it has finished: k_linear_attention reads the
+// committed states ahead of its own wait.
 __global__ void k_store_tokens(const __grid_constant__ FewTokens t, uint32_t n, uint32_t *dst) {
-    pdl_launch();
     pdl_wait();
+    pdl_launch();
     if (threadIdx.x < n) dst[threadIdx.x] = t.v[threadIdx.x];
 }
 

@@ -1,6 +1,10 @@
 """Attention of short passes over a long bf16 cache on tcgen05 (k_attention_tensor): 16, 24 and 32 query rows, contexts that end at
 and around the edge of a 64-token tile, scores flat and steep enough for the softmax reference to move, against long passes over the
 same session, which take k_attention_mma."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -63,3 +67,19 @@ def test_a_key_that_is_nan_has_no_weight():
     finally:
         ex.unload()
         be.close()
+
+
+@pytest.mark.parametrize("session", ["12000", "stack"])
+def test_overlap_changes_no_bit(tmp_path, session):
+    """As test_dependent_launch_overlap_changes_no_bit, where cache rows of earlier passes are copied ahead of the wait: by this kernel
+    (12000 tokens: 187 tiles in 37 parts) and by the attention of layer stacks."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    outs = []
+    for pdl in ("1", "0"):
+        env = dict(os.environ, CTOX_PDL=pdl, PYTHONPATH=os.path.dirname(here) + os.pathsep + os.environ.get("PYTHONPATH", ""))
+        path = str(tmp_path / (pdl + ".npz"))
+        r = subprocess.run([sys.executable, os.path.join(here, "pdl_worker.py"), path, session], env=env, capture_output=True, text=True, timeout=900)
+        assert r.returncode == 0, r.stderr[-2000:]
+        outs.append(np.load(path))
+    for name in outs[0]:
+        assert np.array_equal(outs[0][name], outs[1][name]), name
