@@ -242,6 +242,7 @@ SIGNATURES = {
     "ctox_exec_last_mtp_hidden": (C.c_int32, [C.c_void_p, C.c_uint32, C.c_void_p, C.POINTER(C.c_uint32)]),
     "ctox_exec_last_draft_logits": (C.c_int32, [C.c_void_p, C.c_uint32, C.c_void_p, C.POINTER(C.c_uint32),
                                                 C.POINTER(C.c_uint32)]),
+    "ctox_exec_attention_kernel": (C.c_int32, [C.c_void_p, C.c_uint64, C.c_uint32]),
     "ctox_exec_position": (C.c_int32, [C.c_void_p, C.POINTER(C.c_uint64)]),
     "ctox_exec_last_hidden": (C.c_int32, [C.c_void_p, C.c_void_p]),
     "ctox_exec_keep_logits": (C.c_int32, [C.c_void_p, C.c_int32]),

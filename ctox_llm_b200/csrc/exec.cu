@@ -549,6 +549,22 @@ ctox_status build_draft_head(ctox_exec *e) {
 
 }  // namespace
 
+namespace {
+
+AttnGeom attn_geom(const ctox_exec *e) {
+    const ctox_model_config &c = e->cfg;
+    return AttnGeom{c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.rotary_dim, c.rope_theta,
+                    c.rms_norm_epsilon, e->ctx->dev_error};
+}
+
+// Parts that the context of a short pass is cut into.
+uint32_t attn_splits(const ctox_exec *e, uint64_t slot0, uint32_t m) {
+    const uint64_t tiles = (slot0 + m + 63) / 64;
+    return (uint32_t)(tiles < e->attn_splits_max ? (tiles ? tiles : 1) : e->attn_splits_max);
+}
+
+}  // namespace
+
 extern "C" {
 
 ctox_status ctox_exec_fill_synthetic(ctox_exec *e, uint64_t seed, float mu, float sigma) {
@@ -840,6 +856,11 @@ ctox_status ctox_exec_prefill_synthetic(ctox_exec *e, uint64_t n, uint64_t seed)
     return CTOX_OK;
 }
 
+int32_t ctox_exec_attention_kernel(const ctox_exec *e, uint64_t position, uint32_t tokens) {
+    if (!e || e->stack) return -1;
+    return attention_kernel(attn_geom(e), e->cfg.kv_dtype == CTOX_BF16, position, tokens, attn_splits(e, position, tokens));
+}
+
 ctox_status ctox_exec_position(const ctox_exec *e, uint64_t *position) {
     if (!e || !position) return CTOX_INVALID_STATE;
     *position = e->position;
@@ -867,12 +888,6 @@ ctox_status ctox_exec_keep_logits(ctox_exec *e, int32_t enable) {
 
 // ------------------------------------------------------------------ passes
 namespace {
-
-AttnGeom attn_geom(const ctox_exec *e) {
-    const ctox_model_config &c = e->cfg;
-    return AttnGeom{c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.rotary_dim, c.rope_theta,
-                    c.rms_norm_epsilon, e->ctx->dev_error};
-}
 
 // Column-split projection in a tensor-parallel group: finish this rank's partial result, sum it
 // over the group and hand the sum on as a plain vector. A single GPU passes the raw sums through.
@@ -949,8 +964,7 @@ ctox_status layer_body(ctox_exec *e, uint32_t l, float *h, uint32_t m, uint64_t 
         const AttnGeom g = attn_geom(e);
         launch_attn_pre(st, fan, g, lw.q_norm, lw.k_norm, rope_pos0, slot0, m, e->aq, e->agate, ls.k_cache,
                         ls.v_cache, c.kv_dtype == CTOX_BF16, page_table, c.kv_page_tokens);
-        const uint64_t tiles = (slot0 + m + 63) / 64;
-        const uint32_t splits = (uint32_t)(tiles < e->attn_splits_max ? (tiles ? tiles : 1) : e->attn_splits_max);
+        const uint32_t splits = attn_splits(e, slot0, m);
         timing_begin(ctx);
         launch_attention(st, g, e->aq, e->agate, ls.k_cache, ls.v_cache, c.kv_dtype == CTOX_BF16, page_table,
                          c.kv_page_tokens, slot0, m, splits, e->attn_ws, out_in);

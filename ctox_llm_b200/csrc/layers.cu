@@ -1070,16 +1070,21 @@ static void launch_attention_kernel(cudaStream_t st, const AttnGeom &g, const fl
 #undef CTOX_ATTN
 }
 
+// tcgen05 from a few tiles per part of the context on: it has more to set up and to merge. Blocks of a four-layer model, all
+// attention, 24 heads over 4: with three drafts 912 (mma.sync) and 914 us at 4000 tokens, 934 / 922 at 6000, 1174 / 1075 at
+// 32000; without drafts 493 / 495 at 8000, 517 / 510 at 12000, 615 / 568 at 32000.
+AttnKernel attention_kernel(const AttnGeom &g, int kv_bf16, uint64_t cache_slot, uint32_t m, uint32_t splits) {
+    const uint32_t nq = g.q_heads / g.kv_heads * m;
+    const uint64_t tiles = (cache_slot + m + kFaTile - 1) / kFaTile;
+    if (!kv_bf16 || g.head_dim != kFaHd || nq > 32) return ATTN_CUDA_CORES;
+    return tiles >= (nq <= 16 ? 4u : 3u) * (uint64_t)splits ? ATTN_TENSOR : ATTN_MMA;
+}
+
 void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const float *gate,
                       const void *k_cache, const void *v_cache, int kv_bf16, const uint32_t *page_table,
                       uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits, float *workspace,
                       const MvIn &next) {
-    // tcgen05 from a few tiles per part of the context on: it has more to set up and to merge. Blocks of a four-layer model, all
-    // attention, 24 heads over 4: with three drafts 912 (mma.sync) and 914 us at 4000 tokens, 934 / 922 at 6000, 1174 / 1075 at
-    // 32000; without drafts 493 / 495 at 8000, 517 / 510 at 12000, 615 / 568 at 32000.
-    const uint32_t nq = g.q_heads / g.kv_heads * m;
-    const uint64_t tiles = (cache_slot + m + kFaTile - 1) / kFaTile;
-    if (kv_bf16 && g.head_dim == kFaHd && nq <= 32 && tiles >= (nq <= 16 ? 4u : 3u) * (uint64_t)splits)
+    if (attention_kernel(g, kv_bf16, cache_slot, m, splits) == ATTN_TENSOR)
         launch_attention_tensor(st, g, q, k_cache, v_cache, page_table, page_tokens, cache_slot, m, splits, workspace);
     else
         launch_attention_kernel(st, g, q, k_cache, v_cache, kv_bf16, page_table, page_tokens, cache_slot, m, m, splits, workspace);

@@ -87,6 +87,9 @@ void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const 
                       uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits, float *workspace,
                       const MvIn &next);
 
+// Which kernel a short pass takes; the numbers are those of ctox_exec_attention_kernel.
+enum AttnKernel : int { ATTN_CUDA_CORES = 0, ATTN_MMA = 1, ATTN_TENSOR = 2 };
+AttnKernel attention_kernel(const AttnGeom &g, int kv_bf16, uint64_t cache_slot, uint32_t m, uint32_t splits);
 // The part of it that runs on tcgen05 (attention_tensor.cu): head_dim 256, bf16 cache, at most 32 query rows.
 void launch_attention_tensor(cudaStream_t st, const AttnGeom &g, const float *q, const void *k_cache, const void *v_cache,
                              const uint32_t *page_table, uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits,

@@ -226,6 +226,10 @@ class B200Executor:
     def reset_session(self) -> None:
         self._b._check(self._lib.ctox_exec_reset_session(self._h))
 
+    def attention_kernel(self, position: int, tokens: int) -> int:
+        """Kernel of a short pass of `tokens` positions behind `position`: 0 CUDA cores, 1 mma.sync, 2 tcgen05; -1 for a layer stack."""
+        return int(self._lib.ctox_exec_attention_kernel(self._h, position, tokens))
+
     def position(self) -> int:
         v = C.c_uint64()
         self._b._check(self._lib.ctox_exec_position(self._h, C.byref(v)))

@@ -592,6 +592,9 @@ ctox_status ctox_exec_last_enqueue_us(const ctox_exec *exec, double *microsecond
  * (src/bin/cuda_target_mtp4_graph_bench.rs:36-64,124-136). */
 ctox_status ctox_exec_phase_timing(ctox_exec *exec, int32_t enable);
 ctox_status ctox_exec_last_phase_ms(ctox_exec *exec, float *ms4);
+/* Which attention kernel a short pass of `tokens` positions takes behind `position` tokens: 0 on CUDA cores, 1 mma.sync, 2 tcgen05; -1
+ * for a layer stack. For tests and benchmarks that mean one of them; no counterpart in the reference. */
+int32_t ctox_exec_attention_kernel(const ctox_exec *exec, uint64_t position, uint32_t tokens);
 ctox_status ctox_exec_position(const ctox_exec *exec, uint64_t *position);
 /* Final hidden state of the last committed position (device -> host), for parity tests. */
 ctox_status ctox_exec_last_hidden(ctox_exec *exec, float *out);
