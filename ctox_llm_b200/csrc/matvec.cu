@@ -855,12 +855,6 @@ ctox_status upload_f32(ctox_ctx *ctx, const float *src, uint64_t n, float **dst,
 struct StreamCfg {
     int warps, stages;
 };
-// Eight warps with four stages leave room on an SM for the kernels before and after, which then start ahead of their wait: the
-// shape of dispatches that stand alone (5120 x 17408 Q2, four positions 10.9 -> 9.7 us; 17408 x 5120 Q4, one 11.0 -> 10.7 to 11.1;
-// two stages take 9.3 and 9.8, but 35 instead of 28 us for a single Q4 dispatch from an idle GPU). In the executor's chain the body
-// gains from sixteen: two blocks of 64 layers take 12.5 ms with sixteen and 12.9 with eight, and eight for the smallest matrices alone
-// make some models of width 1024 to 2560 4 % faster and others 6 % slower.
-
 FinishItem finish_item(const ctox_matvec *mv, const MatvecPart &p, const MatvecPart::Split &sp, float *y, uint64_t y_stride) {
     const uint64_t units = (uint64_t)p.pairs * p.kst_s;
     const bool fits = (units + 1) * sp.warps_per_slice + units < (1ull << 32);  // piece_count() in 32 bits
@@ -925,6 +919,22 @@ void launch_merged(int dt, uint32_t npos, unsigned grid, size_t smem, cudaStream
         launch_pdl(k_matvec_stream<0, 16, 2, 2, FORM>, dim3(grid), dim3(512), smem, st, a);
     else
         launch_pdl(k_matvec_stream<0, 16, 2, 1, FORM>, dim3(grid), dim3(512), smem, st, a);
+}
+
+// Whether a matrix dispatched by itself takes eight warps with four stages (kAloneSplit) instead of sixteen with two. They leave room on an
+// SM for the kernels before and after, which then start ahead of their wait, but half of the warps hide less of the body's latencies. What
+// they gain is a part of the start and the end, so it falls with the work per warp (units) and with the row pairs, whose sums the
+// kernels after read: us a pass among others, matrices from HBM, sixteen / eight warps:
+//   5120 x 17408, four positions, Q2 16.8 / 14.5 and Q4 18.3 / 17.3 (pairs x units per warp = 735); 9000 x 8192, one, Q4 16.6 / 15.2 (1075);
+//   17408 x 5120, one, Q4 16.6 / 16.5 and Q2 14.1 / 13.4, but four, Q4 16.4 / 17.2 (2499); 20000 x 8192, one, Q4 22.1 / 22.9 (5279);
+//   17408 x 12288, four, Q2 23.2 / 25.6 (5999).
+// Eight warps with two stages are as good among others, but take 35 instead of 28 us for a single Q4 dispatch from an idle GPU. In the
+// executor's chain the body gains from sixteen: two blocks of 64 layers take 12.5 ms with sixteen and 12.9 with eight, and eight for
+// the smallest matrices alone make some models of width 1024 to 2560 4 % faster and others 6 % slower.
+constexpr uint64_t kAloneMost = 3000;
+bool alone(int dt, uint32_t pairs, uint64_t units, uint64_t warps, uint32_t npos) {  // units, warps: per slice, of the sixteen-warp split
+    const uint64_t limit = npos <= 2 ? kAloneMost : dt ? 1250 : 2300;
+    return pairs * units <= limit * warps;
 }
 
 // One matrix of a stand-alone dispatch and where its outputs go.
@@ -1084,9 +1094,11 @@ ctox_status prepare_part(ctox_ctx *ctx, ctox_matvec *mv, MatvecPart &part, const
         MatvecPart::Split &sp = part.split[cls];
         StreamCfg cfg = pick_stream_cfg(ctx, part.dt, part.kst_s * 4, cls == 1 ? kMaxPosPerPass : 4);
         if (cls == kAloneSplit) {
-            const StreamCfg alone{8, 4};
-            if (cfg.warps != 16 || stream_smem_bytes(part.dt, alone, part.kst_s * 4, 4) > (size_t)ctx->max_smem_optin) continue;
-            cfg = alone;
+            const StreamCfg eight{8, 4};
+            if (cfg.warps != 16 || stream_smem_bytes(part.dt, eight, part.kst_s * 4, 4) > (size_t)ctx->max_smem_optin ||
+                !alone(part.dt, part.pairs, units, part.split[0].warps_per_slice, 1))
+                continue;
+            cfg = eight;
         }
         sp.warps = cfg.warps;
         sp.stages = cfg.stages;
@@ -1233,7 +1245,10 @@ ctox_status dispatch_pass(ctox_ctx *ctx, const DispatchItem *it, uint64_t n, con
             apart = apart && !overlap(x, (npos - 1) * x_stride + first->columns, esz, it[i0 + i].y, (npos - 1) * it[i0 + i].y_stride + it[i0 + i].part->rows, 4);
         const bool closed = own && apart && plan_closed(ctx, it + i0, k, npos, &a), merged = closed || ((own || k > 1) && plan_merged(ctx, it + i0, k, npos, &a));
         auto split_of = [&](const MatvecPart &p) -> const MatvecPart::Split & {
-            return p.split[npos > 4 ? 1 : !merged && p.split[kAloneSplit].warps ? kAloneSplit : 0];
+            if (npos > 4) return p.split[1];
+            const bool eight = !merged && p.split[kAloneSplit].warps &&
+                               alone(p.dt, p.pairs, (uint64_t)p.pairs * p.kst_s, p.split[0].warps_per_slice, npos);
+            return p.split[eight ? kAloneSplit : 0];
         };
         for (uint32_t i = 0; i < k; ++i) {
             const DispatchItem &d = it[i0 + i];

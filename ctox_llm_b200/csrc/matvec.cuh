@@ -29,14 +29,14 @@ struct MatvecPart {
     size_t partial_bytes = 0;
     // The work split depends on the launch shape, which depends on the number of positions
     // (shared memory); one table per shape class: [0] 1..4 positions, [1] 5..8 positions, [kAloneSplit] 1..4 positions of
-    // one matrix dispatched by itself (warps == 0: as [0]).
+    // one matrix dispatched by itself (warps == 0: as [0]; matvec.cu says which).
     struct Split {
         int warps = 0, stages = 0;       // launch shape; warps == 0: does not fit
         uint32_t ctas_per_slice = 0, warps_per_slice = 0, max_pieces = 1;
         uint8_t *pieces = nullptr;       // [pairs][slices] partial-sum pieces
         size_t pieces_bytes = 0;
     } split[kSplits];
-    uint32_t max_pieces = 1;  // slot stride of `partial`: max over both splits
+    uint32_t max_pieces = 1;  // slot stride of `partial`: max over the splits
 };
 
 struct ctox_matvec {

@@ -96,3 +96,10 @@ def test_outputs_over_the_activations(orc, rows, columns, positions, shift):
     for m in mats:
         m.destroy()
     be.close()
+
+
+@pytest.mark.parametrize("dtype,rows,columns,positions", [
+    (Q4, 15000, 3584, 2), (Q4, 15000, 3584, 4), (Q2, 15000, 3584, 4), (Q2, 17408, 4096, 1), (Q2, 24000, 4096, 1), (Q4, 5120, 17408, 3)])
+def test_either_side_of_the_eight_warp_form(orc, dtype, rows, columns, positions):
+    """Dispatches of one matrix with eight warps per CTA and, beyond a work per warp that depends on the positions, with sixteen."""
+    test_outputs(orc, dtype, [rows], columns, positions)
