@@ -12,9 +12,10 @@ namespace ctox {
 constexpr int kDvThreads = 256, kDvWarps = kDvThreads / 32;
 constexpr uint64_t kUnitCost = 20000;                        // of a unit of rows, in columns
 constexpr uint32_t kBatch = 4;                               // vectors a thread requests at once
-// The same where attention splits are merged. One position is a chain of round trips; with more of them sixteen vectors beside the
-// positions' sums do not fit the registers (eight positions spilled: 134 prompt tokens through six latent layers 12.7 -> 13.0 ms).
-__host__ __device__ constexpr uint32_t merge_batch(int m) { return m == 1 ? 16 : 8; }
+// The same where attention splits are merged. Sixteen are padding and more code to read where a window has few splits (30 + 30 tokens through
+// four latent layers of width 512, a window of 256: 7.03 ms instead of 6.91), gain nothing with 32 (30 behind 8000: 14.4 ms either way) and
+// spill beside eight positions' sums.
+constexpr uint32_t kMergeBatch = 8;
 constexpr int kSplitLanes = (kAttnSplitsDense + 31) / 32;  // splits per lane of a merging warp
 
 __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
@@ -128,7 +129,6 @@ __global__ void __launch_bounds__(kDvThreads, 2)
                     for (int i = 0; i < kSplitLanes; ++i) mw[pm][lane + i * 32] = mv[i] / den;
             }
             __syncthreads();
-            constexpr uint32_t kMergeBatch = merge_batch(M);
             each(ldx, [&](uint32_t c) {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (c < end)
