@@ -1070,6 +1070,23 @@ static void launch_attention_kernel(cudaStream_t st, const AttnGeom &g, const fl
 #undef CTOX_ATTN
 }
 
+// Dynamic shared memory that keeps the merge's CTAs apart. They wait while k_attention_tensor's CTAs fill the SMs, and the first SMs that
+// are left would take eight each and read all parts through their few L1s: one KV head, four positions behind 38000 tokens (148 parts)
+// 46 us for both kernels, 34 with no overlap at all, 32 with a CTA per SM; four KV heads behind 32768 tokens 56 and 51.8.
+static size_t spread_smem(uint32_t ctas) {
+    constexpr size_t kMost = 190 * 1024;  // one CTA per SM; half of it two, a third three
+    static thread_local int sms[64] = {};  // per device; -1: the kernel may not ask for it
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 64) return 0;
+    if (!sms[dev] && (cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+                      cudaFuncSetAttribute(k_attn_combine_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost) != cudaSuccess)) {
+        sms[dev] = -1;
+        cudaGetLastError();
+    }
+    return sms[dev] > 0 && ctas <= 3u * sms[dev] ? kMost / ((ctas + sms[dev] - 1) / sms[dev]) : 0;
+}
+
 // tcgen05 from a few tiles per part of the context on: it has more to set up and to merge. Blocks of a four-layer model, all
 // attention, 24 heads over 4: with three drafts 912 (mma.sync) and 914 us at 4000 tokens, 934 / 922 at 6000, 1174 / 1075 at
 // 32000; without drafts 493 / 495 at 8000, 517 / 510 at 12000, 615 / 568 at 32000.
@@ -1084,11 +1101,14 @@ void launch_attention(cudaStream_t st, const AttnGeom &g, const float *q, const 
                       const void *k_cache, const void *v_cache, int kv_bf16, const uint32_t *page_table,
                       uint32_t page_tokens, uint64_t cache_slot, uint32_t m, uint32_t splits, float *workspace,
                       const MvIn &next) {
-    if (attention_kernel(g, kv_bf16, cache_slot, m, splits) == ATTN_TENSOR)
+    size_t merge_smem = 0;
+    if (attention_kernel(g, kv_bf16, cache_slot, m, splits) == ATTN_TENSOR) {
         launch_attention_tensor(st, g, q, k_cache, v_cache, page_table, page_tokens, cache_slot, m, splits, workspace);
-    else
+        merge_smem = spread_smem(m * g.q_heads);
+    } else {
         launch_attention_kernel(st, g, q, k_cache, v_cache, kv_bf16, page_table, page_tokens, cache_slot, m, m, splits, workspace);
-    launch_pdl(k_attn_combine_prep, dim3(m * g.q_heads), dim3(g.head_dim), 0, st, g, workspace, gate, (int)m, splits, next);
+    }
+    launch_pdl(k_attn_combine_prep, dim3(m * g.q_heads), dim3(g.head_dim), merge_smem, st, g, workspace, gate, (int)m, splits, next);
 }
 
 // Which kernel a long pass takes (its groups have 32 queries at most on the tensor cores).
