@@ -348,8 +348,11 @@ __device__ __forceinline__ size_t kv_slot(const uint32_t *page_table, uint32_t p
 // (1+w) RMS norm per head and the non-interleaved partial RoPE (reference.rs:115-155); k and v go
 // to the cache slot of the position. One element per thread keeps the chain of dependent loads
 // (piece count, then the partial sums) one deep.
+// 32 registers: what a CTA of the streaming product before it (4-bit codes, sixteen warps) leaves of an SM's. With 44 this kernel's CTAs did
+// not start beside it, and the first SMs to be free took several each: one token through four layers of 32 heads over 8 227 us, 202 with
+// 32 registers and a few spilled.
 template <typename T>
-__global__ void __launch_bounds__(256) k_attn_pre(MvOut fan, AttnGeom g, const float *__restrict__ q_norm,
+__global__ void __launch_bounds__(256, 8) k_attn_pre(MvOut fan, AttnGeom g, const float *__restrict__ q_norm,
                                                   const float *__restrict__ k_norm, uint64_t rope_position,
                                                   uint64_t cache_slot, int npos, float *__restrict__ q,
                                                   float *__restrict__ gate, T *__restrict__ k_cache,

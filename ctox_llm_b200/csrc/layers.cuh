@@ -229,7 +229,7 @@ __device__ __forceinline__ float out_at(const MvOut &o, const OutRef &r, uint32_
     if (!r.pieces) return out_of(o, row, pos);
     const float *first = r.first + pos * 32;
     // Pieces requested together. Twenty-four (a 5120 x 17408 product leaves 20) save a wide model nothing that can be measured in a block and
-    // cost others registers and code: 12 speculative blocks of a model of width 1024 3.97 ms instead of 3.87.
+    // cost others registers and code: eight speculative blocks of a model of width 1024 3.97 ms instead of 3.87.
     constexpr int kTrip = 8;
     float v = 0.f;
     uint32_t sl = 0, q = 0;
