@@ -82,8 +82,9 @@ ctox_status launch_dense_matvec(ctox_ctx *ctx, const DenseMat &w, uint32_t group
 
 // One position and one group through k_dense_stream (dense_stream.cu), where the matrix has at least kDenseStreamBytes and its
 // rows fit that kernel's shape; *taken says whether.
-// (Taken from 1, 4 and 12 MB on, 16 tokens of the latent model take 16.8, 16.8 and 17.1 ms, a Vasanex request 17.5, 17.2 and 17.2;
-// that was before the ring was cut to kDsRoom.)
+// Taken from 1, 4 and 12 MB on: requests of 30 + 30 tokens through four layers of width 2560, latent 8.17, 8.18 and 8.60 ms, Vasanex 7.44, 7.42
+// and 7.74; of width 1024, latent 6.91, 6.88 and 6.97, Vasanex 5.17, 5.35 and 5.35; the models of width 5120 and 2048 at kDsRoom 15.66, 15.65 and
+// 15.66, and 15.08, 15.09 and 15.32.
 constexpr size_t kDenseStreamBytes = 4 << 20;
 ctox_status launch_dense_stream(ctox_ctx *ctx, const DenseMat &w, const VecIn &in, const VecOut &out, const LatentAppend *append,
                                 bool *taken);

@@ -3,7 +3,7 @@
 //
 // What bounds it: HBM, then what a decode step's chain of launches adds to it (the prologue's round trip and block sums, about 2 us of
 // each). 17408 x 5120 and back (178 MB each) take 33 and 28 us in that chain, 5.4 and 6.4 TB/s; the chain of the latent model
-// 16.7 ms for 16 tokens against 19.3 with k_dense_matvec, whose loads go through registers, in waves of whole row units.
+// 15.6 ms for 16 tokens against 19.3 with k_dense_matvec, whose loads go through registers, in waves of whole row units.
 //
 // A CTA per SM takes an equal share of the rows; its 16 warps stand side by side on the columns (as many
 // per row as keep a warp's part of the input in registers), and every warp keeps a ring of bulk copies of its own row parts in
@@ -22,8 +22,8 @@ constexpr uint32_t kDsSteps = 5;    // vectors of eight columns per lane, at mos
 constexpr uint32_t kDsInput = 4;    // vectors of four columns of a normalised input per thread, at most
 constexpr uint32_t kDsStages = 16;  // copies in flight per warp, at most
 // Shared memory of a launch. A deeper ring holds up the prologue's loads, a shallower one leaves HBM idle meanwhile: 16 decoded tokens of
-// an eight-layer model of width 5120 / a request with 32 decoded tokens on one of width 2048 take 17.3 / 16.2 ms with 220 KB, 16.8 / 15.7
-// with 140, 16.7 / 16.1 with 108, 18.0 / 16.1 with 84.
+// an eight-layer model of width 5120 / a request with 32 decoded tokens on one of width 2048 / one of 30 + 30 tokens through four latent layers of
+// width 2560 take 16.2 / 15.3 / 8.4 ms with 220 KB, 15.65 / 15.1 / 8.2 with 140, 15.6 / 15.1 / 8.2 with 108, 15.85 / 15.3 / 8.3 with 84.
 constexpr size_t kDsRoom = 140 * 1024;
 constexpr uint32_t kDsBatch = 4;    // rows summed over the lanes together
 
