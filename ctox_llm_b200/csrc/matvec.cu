@@ -928,7 +928,8 @@ void launch_merged(int dt, uint32_t npos, unsigned grid, size_t smem, cudaStream
 //   5120 x 17408, four positions, Q2 16.8 / 14.5 and Q4 18.3 / 17.3 (pairs x units per warp = 735); 9000 x 8192, one, Q4 16.6 / 15.2 (1075);
 //   17408 x 5120, one, Q4 16.6 / 16.5 and Q2 14.1 / 13.4, but four, Q4 16.4 / 17.2 (2499); 20000 x 8192, one, Q4 22.1 / 22.9 (5279);
 //   17408 x 12288, four, Q2 23.2 / 25.6 (5999).
-// Eight warps with two stages are as good among others, but take 35 instead of 28 us for a single Q4 dispatch from an idle GPU. In the
+// Eight warps with two stages are faster still among others (17408 x 5120 Q4 9.8 us where these take 11; weights of one matrix, in L2), but take
+// 35 instead of 28 us for a single Q4 dispatch from an idle GPU. In the
 // executor's chain the body gains from sixteen: two blocks of 64 layers take 12.5 ms with sixteen and 12.9 with eight, and eight for
 // the smallest matrices alone make some models of width 1024 to 2560 4 % faster and others 6 % slower.
 constexpr uint64_t kAloneMost = 3000;
